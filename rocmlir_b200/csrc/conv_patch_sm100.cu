@@ -1,0 +1,451 @@
+// Forward convolution of an image with few channels (16-bit types, one group): the im2col tile is built by the SM itself.
+//
+// rocMLIR's implicit GEMM (ConvRewritePattern, mlir/lib/Dialect/Rock/Transforms/ConvToGemm.cpp:1133-1400) reads the image
+// through its pad -> embed -> merge coordinate map element by element, whatever the channel count. The TMA forms of this
+// library (conv_halo_sm100.cu, the im2col loads of gemm_sm100.cuh) move whole 128-byte runs of channels, so an image whose
+// pixel is not a multiple of 128 bytes - the first layer of every image network has three channels - used to be
+// expanded into an im2col matrix in memory: Y * X copies of the image written, read, padded to 16-byte rows and read
+// again. This kernel keeps that matrix on the chip:
+//
+//   * a tile is R x Qt output pixels of one image (at most 128), whose input window - a few KB - is copied once into
+//     shared memory by cp.async, zeros outside the image, one tile ahead of its use;
+//   * the 128 x K operand is gathered from the window into 128-byte-swizzled K-major blocks. A warp owns 32 pixels, a
+//     step is the same eight k values for all of them, so the offsets are warp-uniform and the reads of neighbouring
+//     pixels fall into different banks; runs of 2, 4 or 8 channels are read as one word;
+//   * the filter stays in shared memory in the same form for all tiles of the persistent CTA, tcgen05.mma accumulates
+//     into one of two TMEM buffers, and the previous tile's result is stored while the tensor core works.
+//
+// Bound: the gather (one 2-byte read per element of the operand for three channels), then HBM writes of the result. Two
+// CTAs per SM overlap one's gather with the other's stores and waits. N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2,
+// f16 channels last: 1817 us through the im2col matrix, 152 here.
+#include <cuda_runtime.h>
+#include <string.h>
+
+#include <algorithm>
+#include <string>
+
+#include "epilogue.cuh"
+#include "lib_state.h"
+#include "ptx.cuh"
+
+namespace rb {
+namespace {
+
+constexpr int kPatchThreads = 256;
+constexpr int kABlockBytes = 128 * 128;   // 128 pixels x 64 k values
+constexpr int kMaxNt = 128;               // output channels per CTA: two TMEM buffers of two CTAs fit 512 columns
+
+struct PatchParams {
+  const uint16_t* in;
+  const uint16_t* fil;
+  void* out;
+  long long i_n, i_c, i_h;          // image strides in elements; a row is (w, c) contiguous, or w contiguous (planar)
+  long long f_k;                    // filter strides in elements
+  int f_c, f_y, f_x;
+  long long o_n, o_k, o_p, o_q;     // result strides in elements
+  int N, H, W, C, P, Q, Y, X, Kout;
+  int stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
+  int planar;                       // 0: channels last, k = (y, x, c); 1: channel planes, k = (c, y, x)
+  int unit;                         // elements per image column of a row: C, or 1 when planar
+  int R, Qt, tiles_p, tiles_q;      // tile raster
+  long long num_tiles;
+  int rows, planes, pitch;          // window: planes x rows x pitch elements
+  int gran;                         // elements per window copy: 8, 4 or 2 (cp.async), 1 = plain loads
+  int kelems, ksteps, kblocks;      // k extent, MMA steps of 16, blocks of 64
+  int nbuf;                         // blocks of the operand in shared memory
+  int nt, passes;                   // output channels per CTA and CTAs groups that share a tile
+  uint32_t idesc, tmem_cols;
+  int is_bf16, out_type;
+  int wide;                         // plain result, channels contiguous: 32-byte stores
+  EpiParams epi;
+  uint32_t* status;
+  long long wait_cycles;
+};
+
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int gran, int bytes) {
+  if (gran == 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else if (gran == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+struct PatchTile {
+  int n, p0, q0;
+  __device__ PatchTile(const PatchParams& p, long long tile) {
+    const int tq = (int)(tile % p.tiles_q);
+    const long long r = tile / p.tiles_q;
+    p0 = (int)(r % p.tiles_p) * p.R;
+    n = (int)(r / p.tiles_p);
+    q0 = tq * p.Qt;
+  }
+  // position of the window's first column inside its copy granule: the copy starts on a granule of the image row
+  __device__ int skew(const PatchParams& p) const { return ((q0 * p.stride_w - p.pad_w) * p.unit) & (p.gran - 1); }
+};
+
+// Copies the input window of `tile` into `win` ([planes][rows][pitch]), zeros outside the image.
+__device__ __forceinline__ void load_window(const PatchParams& p, const PatchTile& t, uint16_t* win) {
+  const int e0 = (t.q0 * p.stride_w - p.pad_w) * p.unit;   // first element of the window inside its image row
+  const int lo0 = e0 - t.skew(p);                          // a multiple of the copy granule
+  const int h0 = t.p0 * p.stride_h - p.pad_h;
+  const int row_elems = p.W * p.unit;
+  const int gran = p.gran, per_row = p.pitch / gran;
+  const int total = p.planes * p.rows * per_row;
+  const uint16_t* img = p.in + (long long)t.n * p.i_n;
+  for (int i = threadIdx.x; i < total; i += kPatchThreads) {
+    const int v = i % per_row, pr = i / per_row;
+    const int pl = pr / p.rows, r = pr - pl * p.rows;
+    const int h = h0 + r, lo = lo0 + v * gran;
+    const bool row_ok = h >= 0 && h < p.H;
+    const int valid = (row_ok && lo >= 0) ? min(gran, max(0, row_elems - lo)) : 0;
+    const uint16_t* src = valid > 0 ? img + (long long)pl * p.i_c + (long long)h * p.i_h + lo : p.in;
+    if (gran > 1) cp_async(smem_u32(win + i * gran), src, gran, 2 * valid);
+    else win[i] = valid > 0 ? __ldg(src) : (uint16_t)0;
+  }
+}
+
+// Eight k values of one pixel from the window, in runs of VEC elements at warp-uniform offsets.
+template <int VEC>
+__device__ __forceinline__ uint4 gather8(const uint16_t* px, const int* offs, int left) {
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  if constexpr (VEC == 1) {
+    const int4 a = *reinterpret_cast<const int4*>(offs), b = *reinterpret_cast<const int4*>(offs + 4);
+    const int o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (left >= 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = (uint32_t)px[o[2 * i]] | ((uint32_t)px[o[2 * i + 1]] << 16);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < left) w[i / 2] |= (uint32_t)px[o[i]] << (16 * (i & 1));
+    }
+  } else if constexpr (VEC == 2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (2 * i < left) w[i] = *reinterpret_cast<const uint32_t*>(px + offs[2 * i]);
+  } else if constexpr (VEC == 4) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (4 * i < left) {
+        const uint2 u = *reinterpret_cast<const uint2*>(px + offs[4 * i]);
+        w[2 * i] = u.x; w[2 * i + 1] = u.y;
+      }
+  } else {
+    if (left > 0) return *reinterpret_cast<const uint4*>(px + offs[0]);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <bool EPI>
+__device__ __forceinline__ void store_tile(const PatchParams& p, const PatchTile& t, uint32_t taddr, int n0, const float* vec_scale,
+                                           const float* vec_bias) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = (warp & 3) * 32 + lane;
+  const int rr = m / p.Qt, qq = m - rr * p.Qt;
+  const bool valid = rr < p.R && t.p0 + rr < p.P && t.q0 + qq < p.Q;
+  const long long pix = (long long)t.n * p.o_n + (long long)(t.p0 + rr) * p.o_p + (long long)(t.q0 + qq) * p.o_q;
+  for (int c = (warp >> 2) * 32; c < p.nt; c += 64) {
+    const int ncols = min(32, p.Kout - n0 - c);
+    if (ncols <= 0) break;   // warp-uniform
+    uint32_t v[32];
+    tmem_ld32(taddr + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
+    tmem_ld_wait();
+    const long long o = pix + (long long)(n0 + c) * p.o_k;
+    if constexpr (!EPI) {
+      uint32_t h[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float x = __uint_as_float(v[2 * j]), y = __uint_as_float(v[2 * j + 1]);
+        if (p.is_bf16) { __nv_bfloat162 b = __floats2bfloat162_rn(x, y); h[j] = *reinterpret_cast<uint32_t*>(&b); }
+        else { __half2 b = __floats2half2_rn(x, y); h[j] = *reinterpret_cast<uint32_t*>(&b); }
+      }
+      if (valid) {
+        uint16_t* d = static_cast<uint16_t*>(p.out) + o;
+        if (p.wide && ncols == 32) {
+          st_global_v8(d, h);
+          st_global_v8(d + 16, h + 8);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (j < ncols) d[j * p.o_k] = (uint16_t)(h[j / 2] >> (16 * (j & 1)));
+        }
+      }
+    } else {
+      float x[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
+      EpiRow er;
+      if ((p.epi.flags & RB_EPI_BIAS) && (p.epi.flags & RB_EPI_BIAS_SCALAR)) er.row_bias = load_bias(p.epi.bias, p.epi.bias_type, 0);
+      er.res_stride = p.o_k;
+      er.ncols = ncols;
+      er.res = (valid && (p.epi.flags & RB_EPI_RESIDUAL))
+                   ? static_cast<const uint8_t*>(p.epi.residual) + (p.epi.res_type == RB_F32 ? 4 : 2) * o
+                   : nullptr;
+      epi_apply32(x, p.epi, vec_scale + c, vec_bias + c, er);
+      if (valid) {
+        if (p.wide && ncols == 32) {
+          uint4 w4[8];
+          const int nw = pack_row32(x, p.out_type, w4, p.epi.out_zero);
+          uint4* d = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + o * dtype_size(p.out_type));
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (i < nw) d[i] = w4[i];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (j < ncols) store_elem(p.out, o + j * p.o_k, x[j], p.out_type, p.epi.out_zero);
+        }
+      }
+    }
+  }
+}
+
+template <int VEC, bool EPI>
+__global__ void __launch_bounds__(kPatchThreads, 2)
+conv_patch_kernel(const PatchParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // [operand blocks][filter blocks][two windows][k offsets][per-channel vectors][barrier, TMEM address]
+  uint8_t* a_smem = smem;
+  uint8_t* b_smem = a_smem + p.nbuf * kABlockBytes;
+  uint16_t* win = reinterpret_cast<uint16_t*>(b_smem + (size_t)p.kblocks * p.nt * 128);
+  const int win_elems = p.planes * p.rows * p.pitch;
+  int* offs = reinterpret_cast<int*>(win + 2 * win_elems);
+  float* vec_scale = reinterpret_cast<float*>(offs + p.ksteps * 16);
+  float* vec_bias = vec_scale + p.nt;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(vec_bias + p.nt);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bar + 1);
+
+  const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
+  const int n0 = (int)(blockIdx.x % p.passes) * p.nt;
+  const long long step = gridDim.x / p.passes;
+  long long tile = blockIdx.x / p.passes;
+
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc<1>(tmem_holder, p.tmem_cols);
+    tmem_relinquish<1>();
+  }
+  if (tile < p.num_tiles) load_window(p, PatchTile(p, tile), win);
+  // offsets of every k inside a window, and (in the operand area, which is not in use yet) inside a filter row
+  int* foffs = reinterpret_cast<int*>(a_smem);
+  for (int k = threadIdx.x; k < p.ksteps * 16; k += kPatchThreads) {
+    int c, y, x;
+    if (p.planar) { x = k % p.X; const int r = k / p.X; y = r % p.Y; c = r / p.Y; }
+    else { c = k % p.C; const int r = k / p.C; x = r % p.X; y = r / p.X; }
+    const bool ok = k < p.kelems;
+    offs[k] = !ok ? 0 : p.planar ? (c * p.rows + y * p.dil_h) * p.pitch + x * p.dil_w : y * p.dil_h * p.pitch + x * p.dil_w * p.C + c;
+    foffs[k] = ok ? c * p.f_c + y * p.f_y + x * p.f_x : 0;
+  }
+  if constexpr (EPI) {
+    for (int j = threadIdx.x; j < p.nt; j += kPatchThreads) {
+      const int n = min(n0 + j, p.Kout - 1);
+      vec_scale[j] = (p.epi.flags & RB_EPI_COL_SCALE) ? __ldg(p.epi.col_scale + n) : 1.0f;
+      vec_bias[j] = epi_col_bias(p.epi.flags) ? load_bias(p.epi.bias, p.epi.bias_type, n) : 0.0f;
+    }
+  }
+  __syncthreads();
+  // the filter: row = output channel, 16-byte pieces swizzled like a TMA load would leave them, zeros past its extents
+  {
+    const int pieces = p.kblocks * 8, have = p.ksteps * 2;
+    for (int i = threadIdx.x; i < p.nt * pieces; i += kPatchThreads) {
+      const int j = i % pieces, n = i / pieces;
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+      if (j < have && n0 + n < p.Kout) {
+        const uint16_t* f = p.fil + (long long)(n0 + n) * p.f_k;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (8 * j + e < p.kelems) w[e / 2] |= (uint32_t)__ldg(f + foffs[8 * j + e]) << (16 * (e & 1));
+      }
+      *reinterpret_cast<uint4*>(b_smem + (size_t)(j >> 3) * p.nt * 128 + n * 128 + (((j & 7) ^ (n & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+
+  // this thread's pixel (operand row), the same for every tile: rows past the tile's pixels repeat pixel 0
+  const int m = (warp & 3) * 32 + lane;
+  const int rr = m / p.Qt, qq = m - rr * p.Qt;
+  const int px = rr < p.R ? rr * p.stride_h * p.pitch + qq * p.stride_w * p.unit : 0;
+  uint8_t* a_row = a_smem + m * 128;
+  const uint32_t a_lo0 = smem_desc_lo(smem_u32(a_smem), 16), b_lo0 = smem_desc_lo(smem_u32(b_smem), 16);
+  const uint32_t desc_hi = smem_desc_hi(1024);
+
+  bool ok = true;
+  uint32_t groups = 0;       // operand groups handed to the tensor core so far: phase of the barrier
+  uint32_t t = 0;
+  PatchTile prev(p, 0);
+  for (; tile < p.num_tiles; tile += step, ++t) {
+    const PatchTile cur(p, tile);
+    const uint32_t tmem_d = tmem_base + (t & 1u) * p.nt;
+    cp_async_wait_all();
+    const uint16_t* w = win + (t & 1u) * win_elems + cur.skew(p) + px;
+    for (int kb0 = 0; kb0 < p.kblocks; kb0 += p.nbuf) {
+      // the MMAs of the previous group have read the operand blocks (and, at a tile's start, finished the last tile)
+      if (groups > 0) ok = mbar_wait(bar, (groups - 1) & 1u, p.status, kStatusTimeoutMma, p.wait_cycles);
+      if (!__syncthreads_and(ok)) { ok = false; break; }
+      const int steps = min(p.nbuf * 4, p.ksteps - kb0 * 4);   // MMA steps of this group
+      for (int j = warp >> 2; j < steps * 2; j += 2) {
+        const int k = kb0 * 64 + j * 8;
+        const uint4 v = gather8<VEC>(w, offs + k, p.kelems - k);
+        *reinterpret_cast<uint4*>(a_row + (j >> 3) * kABlockBytes + (((j & 7) ^ (m & 7)) << 4)) = v;
+      }
+      fence_proxy_async();
+      tc_fence_before();   // this thread's TMEM reads of the buffer that is about to be overwritten
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        tc_fence_after();
+        for (int s = 0; s < steps; ++s) {
+          const uint32_t blk = (uint32_t)s >> 2, in = ((uint32_t)s & 3u) * 2u;
+          umma_ss<kKindF16, 1>(tmem_d, desc64(a_lo0 + blk * (kABlockBytes >> 4) + in, desc_hi),
+                               desc64(b_lo0 + (kb0 + blk) * (uint32_t)(p.nt * 8) + in, desc_hi), p.idesc, (kb0 | s) ? 1u : 0u);
+        }
+        tc_commit<1>(bar);
+      }
+      ++groups;
+    }
+    if (!ok) break;
+    if (tile + step < p.num_tiles) load_window(p, PatchTile(p, tile + step), win + ((t + 1) & 1u) * win_elems);
+    if (t > 0) {   // the previous tile's result, while the tensor core works on this one
+      tc_fence_after();
+      store_tile<EPI>(p, prev, tmem_base + ((t - 1) & 1u) * p.nt, n0, vec_scale, vec_bias);
+    }
+    prev = cur;
+  }
+  cp_async_wait_all();
+  if (ok && t > 0) {
+    ok = mbar_wait(bar, (groups - 1) & 1u, p.status, kStatusTimeoutEpilogue, p.wait_cycles);
+    if (__syncthreads_and(ok)) {
+      tc_fence_after();
+      store_tile<EPI>(p, prev, tmem_base + ((t - 1) & 1u) * p.nt, n0, vec_scale, vec_bias);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem_base, p.tmem_cols);
+  }
+}
+
+struct PatchShape {
+  int R, Qt, rows, planes, pitch, nbuf, nt, passes, ctas_per_sm, smem;
+};
+
+// Tile, operand blocks and output channels per CTA that fit. Fewest passes over the output channels first (each pass
+// gathers the operand again), then two CTAs per SM before one.
+bool choose_shape(const PatchConv& c, PatchShape* s) {
+  const int kelems = c.Y * c.X * c.C, kblocks = (kelems + 63) / 64, ksteps = (kelems + 15) / 16;
+  const int unit = c.planar ? 1 : c.C;
+  s->planes = c.planar ? c.C : 1;
+  const int cols = (c.Q + 127) / 128;
+  s->Qt = (c.Q + cols - 1) / cols;
+  for (int passes = (c.Kout + kMaxNt - 1) / kMaxNt; passes <= 4; ++passes) {
+    s->passes = passes;
+    s->nt = ((c.Kout + passes - 1) / passes + 31) / 32 * 32;
+    if ((long long)s->nt * (passes - 1) >= c.Kout) continue;   // a pass without channels
+    for (s->ctas_per_sm = 2; s->ctas_per_sm >= 1; --s->ctas_per_sm) {
+      const int limit = s->ctas_per_sm == 2 ? 115712 - 1024 : 232448;
+      for (s->R = std::min(128 / s->Qt, c.P); s->R >= 1; s->R /= 2) {
+        s->rows = (s->R - 1) * c.stride_h + (c.Y - 1) * c.dil_h + 1;
+        s->pitch = ((((s->Qt - 1) * c.stride_w + (c.X - 1) * c.dil_w + 1) * unit + 7) + 7) / 8 * 8;
+        const long long fixed = (long long)kblocks * s->nt * 128 + 4LL * s->planes * s->rows * s->pitch + ksteps * 64LL + s->nt * 8LL + 64 + 1024;
+        for (s->nbuf = std::min(kblocks, 4); s->nbuf >= std::min(kblocks, 2); --s->nbuf) {
+          // (the operand area also holds the filter offsets while the filter is loaded)
+          if (fixed + (long long)s->nbuf * kABlockBytes <= limit && ksteps * 64LL <= (long long)s->nbuf * kABlockBytes) {
+            s->smem = (int)(fixed + (long long)s->nbuf * kABlockBytes);
+            return true;
+          }
+        }
+      }
+    }
+  }
+  return false;
+}
+
+}  // namespace
+
+bool conv_patch_applicable(const PatchConv& c) {
+  // offsets inside the window, the filter and an image row are 32-bit
+  if (c.dil_h > 4096 || c.dil_w > 4096 || c.stride_h > 4096 || c.stride_w > 4096 || c.Y > 4096 || c.X > 4096) return false;
+  const long long row = ((long long)c.W + c.pad_w + c.pad_w_r) * (c.planar ? 1 : c.C);
+  const long long kelems = (long long)c.Y * c.X * c.C;
+  if (kelems > 4096 || row >= (1LL << 30) || (long long)c.H + c.pad_h + c.pad_h_r >= (1LL << 30)) return false;
+  if (c.f_c * c.C + c.f_y * c.Y + c.f_x * c.X >= (1LL << 30)) return false;
+  const long long win_cols = ((std::min(c.Q, 128) - 1LL) * c.stride_w + (c.X - 1LL) * c.dil_w + 1) * (c.planar ? 1 : c.C);
+  const long long win_rows = 127LL * c.stride_h + (c.Y - 1LL) * c.dil_h + 1;
+  if (win_cols > (1 << 20) || win_rows > (1 << 20)) return false;
+  PatchShape s;
+  return choose_shape(c, &s);
+}
+
+RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
+                        void* stream_v) {
+  const DeviceInfo* dev = device_info();
+  if (!dev) return RB_CUDA_ERROR;
+  PatchShape s;
+  if (!conv_patch_applicable(c) || !choose_shape(c, &s)) return fail(RB_UNSUPPORTED, "convolution outside the reach of the patch kernel");
+  PatchParams p;
+  memset(&p, 0, sizeof(p));
+  p.in = static_cast<const uint16_t*>(image);
+  p.fil = static_cast<const uint16_t*>(filter);
+  p.out = out;
+  p.i_n = c.i_n; p.i_c = c.planar ? c.i_c : 0; p.i_h = c.i_h;
+  p.f_k = c.f_k; p.f_c = (int)c.f_c; p.f_y = (int)c.f_y; p.f_x = (int)c.f_x;
+  p.o_n = c.o_n; p.o_k = c.o_k; p.o_p = c.o_p; p.o_q = c.o_q;
+  p.N = c.N; p.H = c.H; p.W = c.W; p.C = c.C; p.P = c.P; p.Q = c.Q; p.Y = c.Y; p.X = c.X; p.Kout = c.Kout;
+  p.stride_h = c.stride_h; p.stride_w = c.stride_w; p.dil_h = c.dil_h; p.dil_w = c.dil_w; p.pad_h = c.pad_h; p.pad_w = c.pad_w;
+  p.planar = c.planar ? 1 : 0;
+  p.unit = c.planar ? 1 : c.C;
+  p.R = s.R; p.Qt = s.Qt; p.rows = s.rows; p.planes = s.planes; p.pitch = s.pitch;
+  p.tiles_p = (c.P + s.R - 1) / s.R; p.tiles_q = (c.Q + s.Qt - 1) / s.Qt;
+  p.num_tiles = (long long)c.N * p.tiles_p * p.tiles_q;
+  // the widest copy that every image row starts on: rows, images and the base address at multiples of it
+  p.gran = 8;
+  while (p.gran > 1 && (((long long)c.W * p.unit) % p.gran || c.i_h % p.gran || c.i_n % p.gran || p.i_c % p.gran ||
+                        reinterpret_cast<uintptr_t>(image) % (2 * p.gran)))
+    p.gran /= 2;
+  p.kelems = c.Y * c.X * c.C; p.ksteps = (p.kelems + 15) / 16; p.kblocks = (p.kelems + 63) / 64;
+  p.nbuf = s.nbuf; p.nt = s.nt; p.passes = s.passes;
+  const uint32_t fmt = c.is_bf16 ? 1u : 0u;
+  p.idesc = make_idesc(1, fmt, fmt, 0, 0, 128, (uint32_t)s.nt);
+  p.tmem_cols = 32;
+  while ((int)p.tmem_cols < 2 * s.nt) p.tmem_cols *= 2;
+  p.is_bf16 = c.is_bf16;
+  p.out_type = out_type;
+  const bool with_epi = (epi && epi->flags) || out_type != (c.is_bf16 ? RB_BF16 : RB_F16);
+  const long long wide_bytes = with_epi ? 16 : 32, es_o = (long long)dtype_bytes(out_type);
+  p.wide = c.o_k == 1 && reinterpret_cast<uintptr_t>(out) % wide_bytes == 0 && (c.o_n * es_o) % wide_bytes == 0 &&
+           (c.o_p * es_o) % wide_bytes == 0 && (c.o_q * es_o) % wide_bytes == 0;
+  if (epi && epi->flags) {
+    p.epi.flags = epi->flags; p.epi.alpha = epi->alpha; p.epi.out_recip = epi->out_recip; p.epi.mid_type = epi->mid_type;
+    p.epi.bias_type = epi->bias_type; p.epi.col_scale = epi->col_scale; p.epi.bias = epi->bias;
+    p.epi.clip_lo = epi->clip_lo; p.epi.clip_hi = epi->clip_hi; p.epi.in_zero = epi->in_zero;
+    p.epi.out_zero = (epi->flags & RB_EPI_ZP_OUT) ? epi->out_zero : 0;
+    p.epi.residual = epi->residual; p.epi.res_type = epi->res_type;
+    p.epi.unary = (epi->flags & RB_EPI_UNARY) ? epi->unary : 0;
+  }
+  p.status = dev->status_word;
+  p.wait_cycles = kWaitCycles;
+  // runs of channels that can be read as one word (channels last: k walks the channels of a tap)
+  const int vec = c.planar ? 1 : c.C % 8 == 0 ? 8 : c.C % 4 == 0 ? 4 : c.C % 2 == 0 ? 2 : 1;
+  typedef void (*Kernel)(const PatchParams);
+  const Kernel kern = with_epi ? (vec == 8 ? conv_patch_kernel<8, true> : vec == 4 ? conv_patch_kernel<4, true>
+                                  : vec == 2 ? conv_patch_kernel<2, true> : conv_patch_kernel<1, true>)
+                               : (vec == 8 ? conv_patch_kernel<8, false> : vec == 4 ? conv_patch_kernel<4, false>
+                                  : vec == 2 ? conv_patch_kernel<2, false> : conv_patch_kernel<1, false>);
+  RbStatus st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), s.smem);
+  if (st != RB_SUCCESS) return st;
+  const long long per_pass = std::max<long long>(1, (long long)dev->sm_count * s.ctas_per_sm / s.passes);
+  const int grid = (int)std::min<long long>(p.num_tiles, per_pass) * s.passes;
+  kern<<<grid, kPatchThreads, s.smem, static_cast<cudaStream_t>(stream_v)>>>(p);
+  RB_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return RB_SUCCESS;
+}
+
+}  // namespace rb

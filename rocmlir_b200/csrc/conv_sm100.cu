@@ -397,6 +397,8 @@ struct ConvPlan {
   bool cls_halo = false;    //   ... and the halo kernel: up to four classes per launch, stored straight into the tensor
   bool cls_any_empty = false;
   HaloConv cls_hc[16];
+  bool patch = false;       // forward, few channels: the patch kernel gathers the operand on the SM (csrc/conv_patch_sm100.cu)
+  PatchConv pc;
 };
 
 bool is_dense_in_order(const long long* strides, const long long* sizes, const int* order, int n) {
@@ -483,6 +485,24 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
       pl->a_nchw = !in_is_mat;
       pl->a_planes = p->f32_mode == 0 ? 2 : (in_is_mat ? 0 : 1);
     }
+    // 16-bit images whose operand would have to be expanded into an im2col matrix: the patch kernel (bit 26 keeps the matrix)
+    pl->patch = false;
+    if (!pl->a_direct && !pl->a_implicit && G == 1 && (t == RB_F16 || t == RB_BF16) && !((rbGetGemmVariant() >> 26) & 1) &&
+        out_t <= RB_F8E4M3 && out_t != RB_I32) {
+      const bool last = (pl->is[2] == 1 || p->c == 1) && (pl->is[4] == p->c || p->w == 1);
+      if (last || pl->is[4] == 1 || p->w == 1) {
+        PatchConv& c = pl->pc;
+        c.N = p->n; c.H = p->h; c.W = p->w; c.C = p->c; c.P = (int)ho; c.Q = (int)wo; c.Kout = p->k; c.Y = p->y; c.X = p->x;
+        c.stride_h = p->stride_h; c.stride_w = p->stride_w; c.dil_h = p->dil_h; c.dil_w = p->dil_w;
+        c.pad_h = p->pad_h; c.pad_w = p->pad_w; c.pad_h_r = p->pad_h_r; c.pad_w_r = p->pad_w_r;
+        c.is_bf16 = t == RB_BF16;
+        c.planar = !last;
+        c.i_n = pl->is[0]; c.i_c = pl->is[2]; c.i_h = pl->is[3];
+        c.f_k = pl->fs[1]; c.f_c = pl->fs[2]; c.f_y = pl->fs[3]; c.f_x = pl->fs[4];
+        c.o_n = pl->os[0]; c.o_k = pl->os[2]; c.o_p = pl->os[3]; c.o_q = pl->os[4];
+        pl->patch = conv_patch_applicable(c);
+      }
+    }
     if (pl->a_implicit) pl->a_direct = true;   // nothing to gather
     pl->a_bytes = pl->a_implicit ? (size_t)pl->a_planes * up256((size_t)pix_i * p->c * es)
                                  : (pl->a_direct ? 0 : (size_t)G * pix_o * yxc * es);
@@ -555,6 +575,12 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
   if ((long long)gp.m != (p->direction == 0 ? pix_o : p->direction == 2 ? (long long)p->k : pix_i) ||
       pix_o > 0x7fffffffLL || pix_i > 0x7fffffffLL || yxc > 0x7fffffffLL || yxk > 0x7fffffffLL)
     return fail(RB_UNSUPPORTED, "GEMM extent exceeds 2^31");
+  if (pl->patch) {   // one kernel on the tensors as they lie
+    pl->n_classes = 0;
+    pl->gemm_ws = pl->total = 0;
+    pl->a_off = pl->b_off = pl->c_off = pl->gemm_off = 0;
+    return RB_SUCCESS;
+  }
   pl->n_classes = 0;
   if (p->direction == 1 && result_type < 0 && (p->stride_h > 1 || p->stride_w > 1) && p->dil_h == 1 && p->dil_w == 1 &&
       p->stride_h <= 4 && p->stride_w <= 4) {
@@ -753,6 +779,7 @@ extern "C" int rbConvKernelCount(const RbConvProblem* p) {
   ConvPlan pl;
   if (make_plan(p, &pl) != RB_SUCCESS) return -1;
   const bool halo_off = ((rbGetGemmVariant() >> 26) & 1) != 0;
+  if (pl.patch) return 1;
   if (pl.n_classes > 0 && pl.cls_halo && !halo_off) {
     int live = 0;
     for (int i = 0; i < pl.n_classes; ++i) live += pl.cls[i].out_off != SIZE_MAX;
@@ -819,6 +846,11 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     return fail(RB_WORKSPACE_TOO_SMALL, "workspace of " + std::to_string(pl.total) + " bytes required");
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
+  if (pl.patch) {
+    st = check_epilogue(epi, pl.gemm.c_type);
+    if (st != RB_SUCCESS) return st;
+    return conv_patch_run(pl.pc, input, filter, output, pl.gemm.c_type, epi, stream_v);
+  }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   const size_t es = dtype_bytes(p->data_type);

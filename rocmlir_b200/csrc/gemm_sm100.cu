@@ -409,6 +409,24 @@ static std::string kernel_symbol(int kind, bool a_mn, bool b_mn, int ctas, bool 
          "ELi" + std::to_string(ctas) + "ELb" + (epi ? "1" : "0") + "EEEvNS_14GemmTensorMapsENS_10GemmParamsE";
 }
 
+RbStatus rb::check_epilogue(const RbEpilogue* epi, int c_type) {
+  if (!epi) return RB_SUCCESS;
+  const uint32_t flags = epi->flags;
+  if ((flags & RB_EPI_COL_SCALE) && !epi->col_scale) return fail(RB_INVALID_PARAM, "col_scale is NULL");
+  if ((flags & RB_EPI_BIAS) && !epi->bias) return fail(RB_INVALID_PARAM, "bias is NULL");
+  if ((flags & RB_EPI_BIAS) && !(epi->bias_type == RB_F32 || epi->bias_type == RB_F16 || epi->bias_type == RB_BF16))
+    return fail(RB_INVALID_PARAM, "bias_type must be f32, f16 or bf16");
+  if ((flags & RB_EPI_BIAS_ROW) && (flags & RB_EPI_BIAS_SCALAR)) return fail(RB_INVALID_PARAM, "bias is per row or scalar, not both");
+  if ((epi->flags & RB_EPI_RESIDUAL) && !epi->residual) return fail(RB_INVALID_PARAM, "residual is NULL");
+  if ((epi->flags & RB_EPI_RESIDUAL) && !(epi->res_type == RB_F32 || epi->res_type == RB_F16 || epi->res_type == RB_BF16))
+    return fail(RB_INVALID_PARAM, "res_type must be f32, f16 or bf16");
+  if ((epi->flags & RB_EPI_UNARY) && (epi->unary <= RB_UNARY_NONE || epi->unary > RB_UNARY_TANH))
+    return fail(RB_INVALID_PARAM, "unary must name one of the RbUnary functions");
+  if ((flags & RB_EPI_CLIP) && !(epi->clip_lo <= epi->clip_hi)) return fail(RB_INVALID_PARAM, "clip needs lo <= hi");
+  if ((flags & RB_EPI_ZP_OUT) && c_type != RB_I8) return fail(RB_INVALID_PARAM, "an output zero point needs an i8 result");
+  return RB_SUCCESS;
+}
+
 RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void* a, const void* b, void* c,
                       void* workspace, size_t workspace_bytes, void* stream_v, const ConvAOperand* conva,
                       RbKernelLaunch* capture) {
@@ -441,20 +459,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
       return fail(RB_UNSUPPORTED, "store_method add exists for f32, f16 and bf16 results");
     if (epi && (epi->flags & RB_EPI_RESIDUAL)) return fail(RB_UNSUPPORTED, "store_method add cannot be combined with a residual operand");
   }
-  if (epi) {
-    if ((flags & RB_EPI_COL_SCALE) && !epi->col_scale) return fail(RB_INVALID_PARAM, "col_scale is NULL");
-    if ((flags & RB_EPI_BIAS) && !epi->bias) return fail(RB_INVALID_PARAM, "bias is NULL");
-    if ((flags & RB_EPI_BIAS) && !(epi->bias_type == RB_F32 || epi->bias_type == RB_F16 || epi->bias_type == RB_BF16))
-      return fail(RB_INVALID_PARAM, "bias_type must be f32, f16 or bf16");
-    if ((flags & RB_EPI_BIAS_ROW) && (flags & RB_EPI_BIAS_SCALAR)) return fail(RB_INVALID_PARAM, "bias is per row or scalar, not both");
-    if ((epi->flags & RB_EPI_RESIDUAL) && !epi->residual) return fail(RB_INVALID_PARAM, "residual is NULL");
-    if ((epi->flags & RB_EPI_RESIDUAL) && !(epi->res_type == RB_F32 || epi->res_type == RB_F16 || epi->res_type == RB_BF16))
-      return fail(RB_INVALID_PARAM, "res_type must be f32, f16 or bf16");
-    if ((epi->flags & RB_EPI_UNARY) && (epi->unary <= RB_UNARY_NONE || epi->unary > RB_UNARY_TANH))
-      return fail(RB_INVALID_PARAM, "unary must name one of the RbUnary functions");
-    if ((flags & RB_EPI_CLIP) && !(epi->clip_lo <= epi->clip_hi)) return fail(RB_INVALID_PARAM, "clip needs lo <= hi");
-    if ((flags & RB_EPI_ZP_OUT) && p->c_type != RB_I8) return fail(RB_INVALID_PARAM, "an output zero point needs an i8 result");
-  }
+  st = check_epilogue(epi, p->c_type);
+  if (st != RB_SUCCESS) return st;
 
   int kind;
   uint32_t fmt, fmt_b = 0xffffffffu, cfmt = 1;   // fmt_b: B's format when it differs from A's

@@ -137,6 +137,24 @@ bool gemm_gemm_on_chip_applicable(int32_t k1, int32_t n1, int32_t n2, int32_t da
 RbStatus gemm_gemm_on_chip(int32_t g, int32_t m, int32_t k1, int32_t n1, int32_t n2, int32_t data_type, const void* a,
                            const void* b1, const void* b2, void* o, void* stream);
 
+// Forward convolution of an image with few channels, 16-bit, one group (csrc/conv_patch_sm100.cu). Strides in elements:
+// image rows are (w, c) contiguous, or with `planar` w contiguous with channel planes; filter and result are arbitrary.
+struct PatchConv {
+  int N, H, W, C, P, Q, Kout, Y, X;
+  int stride_h, stride_w, dil_h, dil_w, pad_h, pad_w, pad_h_r, pad_w_r;
+  int is_bf16;
+  bool planar;
+  long long i_n, i_c, i_h;
+  long long f_k, f_c, f_y, f_x;
+  long long o_n, o_k, o_p, o_q;
+};
+bool conv_patch_applicable(const PatchConv& c);
+RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
+                        void* stream);
+
+// Whether an epilogue can be applied to a result of type c_type: RB_SUCCESS or the reason why not.
+RbStatus check_epilogue(const RbEpilogue* epi, int c_type);
+
 bool conv_wgrad_halo_applicable(const HaloConv& c);
 size_t conv_wgrad_halo_workspace(const HaloConv& c);
 RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* out_grad, void* filter_grad, void* workspace,
