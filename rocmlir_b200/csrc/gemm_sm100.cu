@@ -27,15 +27,54 @@ struct GemmChain {
 thread_local const GemmChain* t_chain = nullptr;
 
 // ---- auxiliary kernels ---------------------------------------------------------------------------
-// Copies `rows` rows of `row_bytes` bytes into rows of `pitch_bytes` bytes, zero-filling the pad.
-__global__ void pad_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, long long rows,
-                                int row_bytes, int pitch_bytes) {
-  const long long total = rows * pitch_bytes;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / pitch_bytes;
-    const int c = (int)(i - r * pitch_bytes);
-    dst[i] = c < row_bytes ? src[r * row_bytes + c] : (uint8_t)0;
+// Operands whose rows do not start on 16-byte boundaries are copied into rows that do (both of a product in one launch):
+// rows of row_bytes bytes become rows of pitch_bytes bytes, the rest of a row zero.
+struct PadJob {
+  const uint8_t* src;
+  uint8_t* dst;
+  unsigned long long rows;
+  unsigned row_bytes, pitch_bytes;
+};
+struct PadJobs {
+  PadJob job[2];
+  unsigned long long first[3];   // vectors of 16 bytes before each job
+};
+
+// Bytes [at, at + 16) of the source row that starts at `row` (any alignment), zeros from byte `n` on: the aligned 32-bit
+// words around them, shifted into place. A word is read whole only where all of it lies inside [row, row + n).
+__device__ __forceinline__ uint4 load_row16(const uint8_t* row, unsigned at, unsigned n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(row) + at;
+  const unsigned shift = (unsigned)(a & 3) * 8;
+  const unsigned lead = (unsigned)(a & 3);
+  uint32_t w[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const long long o = (long long)at - lead + 4 * i;   // offset of the word inside the row
+    w[i] = 0u;
+    if (o >= 0 && o + 4 <= (long long)n) {
+      w[i] = __ldg(reinterpret_cast<const uint32_t*>(row + o));
+    } else if (o + 4 > 0 && o < (long long)n && (i < 4 || lead)) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (o + b >= 0 && o + b < (long long)n) w[i] |= (uint32_t)__ldg(row + o + b) << (8 * b);
+    }
+  }
+  return make_uint4(__funnelshift_r(w[0], w[1], shift), __funnelshift_r(w[1], w[2], shift), __funnelshift_r(w[2], w[3], shift),
+                    __funnelshift_r(w[3], w[4], shift));
+}
+
+// One 16-byte vector of the destination per thread and step: bound by the one read and one write of the operand. (A byte
+// per thread with a 64-bit division each used to take 20 times as long as the loads and stores need.)
+__global__ void pad_rows_kernel(const PadJobs p) {
+  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < p.first[2];
+       i += (unsigned long long)gridDim.x * blockDim.x) {
+    const bool second = i >= p.first[1];
+    const PadJob j = second ? p.job[1] : p.job[0];
+    const unsigned long long v = i - (second ? p.first[1] : 0ull);
+    const unsigned per_row = j.pitch_bytes / 16;
+    const unsigned long long r = (v >> 32) ? v / per_row : (unsigned)v / per_row;
+    const unsigned at = (unsigned)(v - r * per_row) * 16;
+    *reinterpret_cast<uint4*>(j.dst + v * 16) = load_row16(j.src + r * j.row_bytes, at, j.row_bytes);
   }
 }
 
@@ -211,32 +250,71 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
 }
 
 // Sums the partial planes of a K split in a fixed order (range 0, 1, 2, ...), applies the epilogue and
-// writes C. One thread per output element; consecutive threads walk consecutive columns.
+// writes C. One thread per VEC consecutive columns of a row, the reads of up to eight planes in flight together: the pass
+// is bound by reading the planes (they are in L2), and a result of few rows has few threads to hide that latency with.
+// VEC = 4 needs rows of a multiple of four columns, C stored row-major and its rows on boundaries of four elements.
+template <int VEC>
 __global__ void splitk_reduce_kernel(const void* __restrict__ partial, int splits, long long plane, int G, int M, int N,
                                      void* __restrict__ c, int c_type, int trans_c, int acc_is_int, EpiParams epi) {
-  const long long total = (long long)G * M * N;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int n = (int)(i % N);
-    const long long gm = i / N;
-    const int m = (int)(gm % M);
-    const long long g = gm / M;
+  const long long total = (long long)G * M * N / VEC;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < total; i0 += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 * VEC;
+    const long long gm = (i >> 32) ? i / N : (long long)((unsigned)i / (unsigned)N);
+    const int n = (int)(i - gm * N);
+    const long long g = (gm >> 32) ? gm / M : (long long)((unsigned)gm / (unsigned)M);
+    const int m = (int)(gm - g * M);
     const long long o = trans_c ? (g * N + n) * (long long)M + m : i;
-    if (acc_is_int) {
-      int acc = 0;
-      for (int s = 0; s < splits; ++s) acc += reinterpret_cast<const int*>(partial)[s * plane + i];
-      if (c_type == RB_I32 && epi.flags == 0) {
-        reinterpret_cast<int*>(c)[o] = acc;
+    uint32_t acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = 0u;
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      uint32_t v[8][VEC];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        if (s0 + s < splits) {
+          const uint32_t* q = reinterpret_cast<const uint32_t*>(partial) + (s0 + s) * plane + i;
+          if constexpr (VEC == 4) {
+            const uint4 u = __ldcg(reinterpret_cast<const uint4*>(q));
+            v[s][0] = u.x; v[s][1] = u.y; v[s][2] = u.z; v[s][3] = u.w;
+          } else {
+            v[s][0] = __ldcg(q);
+          }
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s0 + s < splits) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e)
+            acc[e] = acc_is_int ? acc[e] + v[s][e] : __float_as_uint(__fadd_rn(__uint_as_float(acc[e]), __uint_as_float(v[s][e])));
+        }
+    }
+    if (acc_is_int && c_type == RB_I32 && epi.flags == 0) {
+      if constexpr (VEC == 4) *reinterpret_cast<uint4*>(static_cast<uint32_t*>(c) + o) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+      else static_cast<uint32_t*>(c)[o] = acc[0];
+      continue;
+    }
+    float x[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      x[e] = acc_is_int ? __int2float_rn((int)acc[e]) : __uint_as_float(acc[e]);
+      if (epi.flags) x[e] = epi_apply(x[e], epi, n + e, m, o + e);
+    }
+    if constexpr (VEC == 4) {
+      if (c_type == RB_F32) {
+        *reinterpret_cast<float4*>(static_cast<float*>(c) + o) = make_float4(x[0], x[1], x[2], x[3]);
+      } else if (c_type == RB_F16) {
+        __half2 h[2] = {__floats2half2_rn(x[0], x[1]), __floats2half2_rn(x[2], x[3])};
+        *reinterpret_cast<uint2*>(static_cast<__half*>(c) + o) = *reinterpret_cast<uint2*>(h);
+      } else if (c_type == RB_BF16) {
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[0], x[1]), __floats2bfloat162_rn(x[2], x[3])};
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(c) + o) = *reinterpret_cast<uint2*>(h);
       } else {
-        float x = __int2float_rn(acc);
-        if (epi.flags) x = epi_apply(x, epi, n, m, o);
-        store_elem(c, o, x, c_type, epi.out_zero);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) store_elem(c, o + e, x[e], c_type, epi.out_zero);
       }
     } else {
-      float acc = 0.0f;
-      for (int s = 0; s < splits; ++s) acc = __fadd_rn(acc, reinterpret_cast<const float*>(partial)[s * plane + i]);
-      if (epi.flags) acc = epi_apply(acc, epi, n, m, o);
-      store_elem(c, o, acc, c_type, epi.out_zero);
+      store_elem(c, o, x[0], c_type, epi.out_zero);
     }
   }
 }
@@ -560,19 +638,26 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
       b_src[0] = hi; b_src[1] = lo;
     }
   } else {
-    if (oa.needs_copy) {
-      pad_rows_kernel<<<dev->sm_count * 4, 256, 0, stream>>>(static_cast<const uint8_t*>(a), wsb + ws.a_off[0],
-                                                           (long long)p->g * oa.rows, (int)(oa.cols * es),
-                                                           (int)(oa.pitch * es));
+    PadJobs pj;
+    memset(&pj, 0, sizeof(pj));
+    int nj = 0;
+    auto add = [&](const void* src, const OperandPlan& o, size_t off) {
+      PadJob& j = pj.job[nj];
+      j.src = static_cast<const uint8_t*>(src);
+      j.dst = wsb + off;
+      j.rows = (unsigned long long)p->g * o.rows;
+      j.row_bytes = (unsigned)(o.cols * es);
+      j.pitch_bytes = (unsigned)(o.pitch * es);
+      pj.first[nj + 1] = pj.first[nj] + j.rows * (j.pitch_bytes / 16);
+      ++nj;
+    };
+    if (oa.needs_copy) { add(a, oa, ws.a_off[0]); a_src[0] = wsb + ws.a_off[0]; }
+    if (ob.needs_copy) { add(b, ob, ws.b_off[0]); b_src[0] = wsb + ws.b_off[0]; }
+    if (nj > 0) {
+      if (nj == 1) pj.first[2] = pj.first[1];
+      const int pb = (int)std::min<unsigned long long>((pj.first[2] + 255) / 256, (unsigned long long)dev->sm_count * 8);
+      pad_rows_kernel<<<pb, 256, 0, stream>>>(pj);
       count_launch();
-      a_src[0] = wsb + ws.a_off[0];
-    }
-    if (ob.needs_copy) {
-      pad_rows_kernel<<<dev->sm_count * 4, 256, 0, stream>>>(static_cast<const uint8_t*>(b), wsb + ws.b_off[0],
-                                                           (long long)p->g * ob.rows, (int)(ob.cols * es),
-                                                           (int)(ob.pitch * es));
-      count_launch();
-      b_src[0] = wsb + ws.b_off[0];
     }
   }
   RB_CUDA_TRY(cudaGetLastError());   // launch errors of the preparation kernels
@@ -807,9 +892,15 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   count_launch();
   if (splits > 1) {
     const long long total = (long long)p->g * p->m * p->n;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)dev->sm_count * 8);
-    splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(partial, splits, total, p->g, p->m, p->n, c, p->c_type,
-                                                     p->trans_c ? 1 : 0, is_int ? 1 : 0, ep);
+    const bool vec = p->n % 4 == 0 && !p->trans_c && reinterpret_cast<uintptr_t>(c) % (4 * es_c) == 0;
+    const long long threads = total / (vec ? 4 : 1);
+    const int blocks = (int)std::min<long long>((threads + 127) / 128, (long long)dev->sm_count * 16);
+    if (vec)
+      splitk_reduce_kernel<4><<<blocks, 128, 0, stream>>>(partial, splits, total, p->g, p->m, p->n, c, p->c_type,
+                                                          p->trans_c ? 1 : 0, is_int ? 1 : 0, ep);
+    else
+      splitk_reduce_kernel<1><<<blocks, 128, 0, stream>>>(partial, splits, total, p->g, p->m, p->n, c, p->c_type,
+                                                          p->trans_c ? 1 : 0, is_int ? 1 : 0, ep);
     count_launch();
   }
   return RB_SUCCESS;
