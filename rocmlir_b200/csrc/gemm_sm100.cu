@@ -91,52 +91,98 @@ __device__ __forceinline__ float tf32_round(float x) {
   if ((xb & 0x7F800000u) == 0x7F800000u) return x;  // inf / nan
   return __uint_as_float((xb + 0x1000u) & 0xFFFFE000u);
 }
-template <bool TRANSPOSE, bool SPLIT>
-__global__ void f32_prepare_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo,
-                                   int R, int C, int pitch, int tiles_x, int tiles_y, long long total_tiles) {
-  __shared__ float tile[32][33];
-  // 32 x 32 tiles dealt out over a 1-D grid: row counts of several million (im2col matrices) exceed gridDim.y
-  for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-    const long long g = t / ((long long)tiles_x * tiles_y);
-    const long long rem = t - g * (long long)tiles_x * tiles_y;
-    const int c0 = (int)(rem % tiles_x) * 32, r0 = (int)(rem / tiles_x) * 32;
-    const float* s = src + g * (long long)R * C;
+// Up to two operands per launch, dealt out in 64 x 64 tiles. Bound by one read and `planes` writes of the operand, so both
+// sides move 16 bytes per thread (the read element by element where the rows of the source do not allow it).
+struct F32Job {
+  const float* src;
+  float* hi;
+  float* lo;              // nullptr: one plane, the value itself
+  int R, C, pitch;        // src [G][R][C]; out [G][R][pitch], or with transpose [G][C][pitch]
+  int transpose;
+  int tiles_x, tiles_y;   // tiles of the output-padded extent along C and R
+};
+struct F32Jobs {
+  F32Job job[2];
+  long long first[3];     // tiles before each job
+};
+__device__ __forceinline__ void store_planes4(const F32Job& j, long long o, const float* x) {
+  if (j.lo) {
+    float h[4], l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = r0 + threadIdx.y + 8 * i, c = c0 + threadIdx.x;
-      tile[threadIdx.y + 8 * i][threadIdx.x] = (r < R && c < C) ? s[(long long)r * C + c] : 0.0f;
+    for (int e = 0; e < 4; ++e) {
+      h[e] = tf32_round(x[e]);
+      l[e] = isfinite(h[e]) ? tf32_round(x[e] - h[e]) : 0.0f;
     }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float x;
-      long long o;
-      bool ok;
-      if (TRANSPOSE) {
-        const int oc = c0 + threadIdx.y + 8 * i;  // output row = source column
-        const int orr = r0 + threadIdx.x;         // output column = source row
-        x = tile[threadIdx.x][threadIdx.y + 8 * i];
-        ok = oc < C && orr < pitch;
-        o = (g * C + oc) * (long long)pitch + orr;
-      } else {
-        const int r = r0 + threadIdx.y + 8 * i, c = c0 + threadIdx.x;
-        x = tile[threadIdx.y + 8 * i][threadIdx.x];
-        ok = r < R && c < pitch;
-        o = (g * R + r) * (long long)pitch + c;
-      }
-      if (ok) {
-        if (SPLIT) {
-          const float h = tf32_round(x);
-          const float l = isfinite(h) ? tf32_round(x - h) : 0.0f;
-          hi[o] = h;
-          lo[o] = l;
-        } else {
-          hi[o] = x;
-        }
-      }
-    }
-    __syncthreads();
+    *reinterpret_cast<float4*>(j.hi + o) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4*>(j.lo + o) = make_float4(l[0], l[1], l[2], l[3]);
+  } else {
+    *reinterpret_cast<float4*>(j.hi + o) = make_float4(x[0], x[1], x[2], x[3]);
   }
+}
+__global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p) {
+  __shared__ float tile[64][65];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
+  for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
+    const bool second = t >= p.first[1];
+    const F32Job j = second ? p.job[1] : p.job[0];
+    const long long lt = t - (second ? p.first[1] : 0), per_g = (long long)j.tiles_x * j.tiles_y;
+    const long long g = lt / per_g;
+    const int rem = (int)(lt - g * per_g);
+    const int c0 = (rem % j.tiles_x) * 64, r0 = (rem / j.tiles_x) * 64;
+    const float* s = j.src + g * (long long)j.R * j.C;
+    const bool vec = j.C % 4 == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
+    float x[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // all four reads in flight
+      const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+      const float* q = s + (long long)r * j.C + c;
+      if (vec && r < j.R && c < j.C) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
+      }
+    }
+    if (!j.transpose) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+        if (r < j.R && c < j.pitch) store_planes4(j, (g * j.R + r) * (long long)j.pitch + c, x[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tile[ty + 16 * i][tx * 4 + e] = x[i][e];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int oc = c0 + ty + 16 * i, orr = r0 + tx * 4;   // output row = source column, output column = source row
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
+        if (oc < j.C && orr < j.pitch) store_planes4(j, (g * j.C + oc) * (long long)j.pitch + orr, y);
+      }
+      __syncthreads();
+    }
+  }
+}
+// The grid covers the padded extent of whichever dimension becomes the output row (zeros past the source's extent).
+F32Job f32_job(const float* src, float* hi, float* lo, int R, int C, int pitch, bool transpose) {
+  F32Job j;
+  j.src = src; j.hi = hi; j.lo = lo; j.R = R; j.C = C; j.pitch = pitch; j.transpose = transpose ? 1 : 0;
+  j.tiles_x = ((transpose ? C : pitch) + 63) / 64;
+  j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
+  return j;
+}
+void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream) {
+  jobs.first[0] = 0;
+  for (int i = 0; i < 2; ++i)
+    jobs.first[i + 1] = jobs.first[i] + (i < count ? groups * (long long)jobs.job[i].tiles_x * jobs.job[i].tiles_y : 0);
+  const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * 32);
+  f32_prepare_kernel<<<grid, 256, 0, stream>>>(jobs);
+  count_launch();
 }
 
 // ---- dispatch ----------------------------------------------------------------------------------------
@@ -176,6 +222,9 @@ struct GemmConfig {
   int dp_tiles, sk_tiles;  // stream-K tail (see GemmParams); sk_tiles == 0: every tile is computed whole
 };
 
+// TF32 planes per operand (see kMaxPlanes)
+int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_mode == 0 ? 2 : 1; }
+
 GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false) {
   GemmConfig c;
   if (variant == 0) variant = (int)tuned_variant_gemm(p);   // the measured table, when it knows the problem
@@ -196,13 +245,15 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   }
   if (c.bn == 64 && (variant & 0xF) != 2) c.ctas = 1;        // measured: 64-column tiles run faster unpaired (345 vs 324 TFLOP/s)
   c.stages = (variant >> 4) & 0xF;
-  const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec);
+  const int planes = gemm_planes(p);
+  const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec, planes) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec, planes);
   if (c.stages <= 0 || c.stages > max_stages) c.stages = max_stages;
   // K blocks per barrier round. One round costs the issuing thread about 310 + 44 n cycles for n MMAs (measured),
   // which four 128x256x16 MMAs (512 cycles) barely hide and four narrower ones do not. Measured: two blocks per
   // round at 256 columns (4096^3 f16 1100 -> 1290 TFLOP/s with this producer loop), four at 128 and 64 columns.
   // Variant bits 28-29: 1, 2, 3 = 1, 2, 4 blocks; 0 = this rule.
-  const int kpr_code = (variant >> 28) & 3;
+  // (two TF32 planes: a K block is twelve MMAs, a round of its own)
+  const int kpr_code = planes == 2 ? 1 : (variant >> 28) & 3;
   c.kpr = kpr_code == 1 ? 1 : kpr_code == 2 ? 2 : kpr_code == 3 ? 4 : (c.bn <= 128 ? 4 : 2);
   while (c.kpr > 1 && c.stages < 2 * c.kpr) c.kpr /= 2;   // at least two rounds in flight
   c.stages = c.stages / c.kpr * c.kpr;
@@ -421,19 +472,10 @@ RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int 
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  const dim3 blk(32, 8, 1);
-  const int cx = transpose ? C : pitch, ry = transpose ? pitch : R;
-  const int tiles_x = (cx + 31) / 32, tiles_y = (ry + 31) / 32;
-  const long long total_tiles = (long long)tiles_x * tiles_y * groups;
-  const dim3 grd((unsigned)std::min<long long>(total_tiles, (long long)dev->sm_count * 64), 1, 1);
-  if (transpose) {
-    if (split) f32_prepare_kernel<true, true><<<grd, blk, 0, stream>>>(src, hi, lo, R, C, pitch, tiles_x, tiles_y, total_tiles);
-    else f32_prepare_kernel<true, false><<<grd, blk, 0, stream>>>(src, hi, lo, R, C, pitch, tiles_x, tiles_y, total_tiles);
-  } else {
-    if (split) f32_prepare_kernel<false, true><<<grd, blk, 0, stream>>>(src, hi, lo, R, C, pitch, tiles_x, tiles_y, total_tiles);
-    else f32_prepare_kernel<false, false><<<grd, blk, 0, stream>>>(src, hi, lo, R, C, pitch, tiles_x, tiles_y, total_tiles);
-  }
-  count_launch();
+  F32Jobs jobs;
+  memset(&jobs, 0, sizeof(jobs));
+  jobs.job[0] = f32_job(src, hi, split ? lo : nullptr, R, C, pitch, transpose);
+  launch_f32_jobs(jobs, 1, groups, dev->sm_count, stream);
   RB_CUDA_TRY(cudaGetLastError());
   return RB_SUCCESS;
 }
@@ -457,14 +499,14 @@ extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* ou
   out->stream_k = c.sk_tiles > 0 ? 1 : 0;
   out->grid = (uint32_t)(c.ctas * std::min<long long>(items, units));
   out->block = kGemmThreads;
-  out->dynamic_smem = (uint32_t)(c.ctas == 2 ? GemmSmemLayout<2>::total(c.stages, c.bn, false)
-                                              : GemmSmemLayout<1>::total(c.stages, c.bn, false));
+  out->dynamic_smem = (uint32_t)(c.ctas == 2 ? GemmSmemLayout<2>::total(c.stages, c.bn, false, gemm_planes(p))
+                                              : GemmSmemLayout<1>::total(c.stages, c.bn, false, gemm_planes(p)));
   // with per-column epilogue vectors (bias / column scales) the ring may be one stage shorter and the staging single
   {
     const GemmConfig ce = choose_config(p, t_variant, true);
     out->stages_epi_vec = ce.stages;
-    out->dynamic_smem_epi_vec = (uint32_t)(ce.ctas == 2 ? GemmSmemLayout<2>::total(ce.stages, ce.bn, true)
-                                                        : GemmSmemLayout<1>::total(ce.stages, ce.bn, true));
+    out->dynamic_smem_epi_vec = (uint32_t)(ce.ctas == 2 ? GemmSmemLayout<2>::total(ce.stages, ce.bn, true, gemm_planes(p))
+                                                        : GemmSmemLayout<1>::total(ce.stages, ce.bn, true, gemm_planes(p)));
   }
   out->kpr = c.kpr;
   const int bn_code = c.bn == 64 ? 1 : c.bn == 128 ? 2 : 3;
@@ -607,36 +649,20 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   uint8_t* wsb = static_cast<uint8_t*>(workspace);
   const void* a_src[2] = {a, nullptr};
   const void* b_src[2] = {b, nullptr};
-  auto prepare_f32 = [&](const void* src, const OperandPlan& o, float* hi, float* lo) {
-    const dim3 blk(32, 8, 1);
-    // the grid covers the padded extent of whichever dimension becomes the output row pitch
-    const int cx = o.src_mn_major ? o.src_cols : o.pitch, ry = o.src_mn_major ? o.pitch : o.src_rows;
-    const int tiles_x = (cx + 31) / 32, tiles_y = (ry + 31) / 32;
-    const long long total_tiles = (long long)tiles_x * tiles_y * p->g;
-    const dim3 grd((unsigned)std::min<long long>(total_tiles, (long long)dev->sm_count * 64), 1, 1);
-    const float* s = static_cast<const float*>(src);
-    if (o.src_mn_major) {
-      if (split) f32_prepare_kernel<true, true><<<grd, blk, 0, stream>>>(s, hi, lo, o.src_rows, o.src_cols, o.pitch, tiles_x, tiles_y, total_tiles);
-      else f32_prepare_kernel<true, false><<<grd, blk, 0, stream>>>(s, hi, lo, o.src_rows, o.src_cols, o.pitch, tiles_x, tiles_y, total_tiles);
-    } else {
-      if (split) f32_prepare_kernel<false, true><<<grd, blk, 0, stream>>>(s, hi, lo, o.src_rows, o.src_cols, o.pitch, tiles_x, tiles_y, total_tiles);
-      else f32_prepare_kernel<false, false><<<grd, blk, 0, stream>>>(s, hi, lo, o.src_rows, o.src_cols, o.pitch, tiles_x, tiles_y, total_tiles);
-    }
-    count_launch();
-  };
   if (is_f32) {
-    if (oa.needs_copy) {
-      float* hi = reinterpret_cast<float*>(wsb + ws.a_off[0]);
-      float* lo = split ? reinterpret_cast<float*>(wsb + ws.a_off[1]) : nullptr;
-      prepare_f32(a, oa, hi, lo);
-      a_src[0] = hi; a_src[1] = lo;
-    }
-    if (ob.needs_copy) {
-      float* hi = reinterpret_cast<float*>(wsb + ws.b_off[0]);
-      float* lo = split ? reinterpret_cast<float*>(wsb + ws.b_off[1]) : nullptr;
-      prepare_f32(b, ob, hi, lo);
-      b_src[0] = hi; b_src[1] = lo;
-    }
+    F32Jobs jobs;
+    memset(&jobs, 0, sizeof(jobs));
+    int nj = 0;
+    auto add = [&](const void* src, const OperandPlan& o, const size_t* off, const void** planes) {
+      float* hi = reinterpret_cast<float*>(wsb + off[0]);
+      float* lo = split ? reinterpret_cast<float*>(wsb + off[1]) : nullptr;
+      jobs.job[nj++] = f32_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, o.pitch, o.src_mn_major);
+      planes[0] = hi;
+      planes[1] = lo;
+    };
+    if (oa.needs_copy) add(a, oa, ws.a_off, a_src);
+    if (ob.needs_copy) add(b, ob, ws.b_off, b_src);
+    if (nj > 0) launch_f32_jobs(jobs, nj, p->g, dev->sm_count, stream);
   } else {
     PadJobs pj;
     memset(&pj, 0, sizeof(pj));
@@ -697,10 +723,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     return encode_tiled(m, dt, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
   };
   std::string err;
-  // Segment order for the split: (lo,hi), (hi,lo), (hi,hi) so that the small terms are summed first.
-  const int nseg = split ? 3 : 1;
-  const int seg_a[3] = {split ? 1 : 0, 0, 0};
-  const int seg_b[3] = {0, 1, 0};
+  const int planes = gemm_planes(p);   // [0] hi (or the operand itself), [1] lo
   if (conva) {
     const ConvAOperand& cv = *conva;
     const int che = kRowBytes / (int)es;   // elements per 128-byte run of channels
@@ -716,17 +739,16 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     const int upper[2] = {cv.pad_w_hi - (cv.X - 1) * cv.dil_w, cv.pad_h_hi - (cv.Y - 1) * cv.dil_h};
     const uint32_t trav[2] = {(uint32_t)cv.stride_w, (uint32_t)cv.stride_h};
     // A: a tile is 128 pixels (rows) x one K block of channels. B: a chunk is one K block of pixels x 64 channels.
-    for (int sg = 0; sg < (conv_a ? nseg : 1); ++sg) {
-      // f32 accurate mode: segment sg of A reads the lo or the hi plane (same order as the copied-operand path)
-      const void* plane = (conv_a && seg_a[sg] == 1) ? cv.tensor_lo : cv.tensor;
+    for (int sg = 0; sg < (conv_a ? planes : 1); ++sg) {
+      const void* plane = sg == 1 ? cv.tensor_lo : cv.tensor;
       if (!encode_im2col_nhwc(conv_a ? &maps.a[sg] : &maps.b[0], dt, plane, dims, strides, lower, upper, (uint32_t)che,
                               (uint32_t)(conv_a ? kBM : bke), trav, &err))
         return fail(RB_UNSUPPORTED, "implicit operand (im2col): " + err);
     }
   }
-  for (int s = 0; s < nseg; ++s) {
-    if (!conv_a && !encode_operand(&maps.a[s], a_src[seg_a[s]], oa, kBM, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
-    if (!conv_b && !encode_operand(&maps.b[s], b_src[seg_b[s]], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
+  for (int s = 0; s < planes; ++s) {
+    if (!conv_a && !encode_operand(&maps.a[s], a_src[s], oa, kBM, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
+    if (!conv_b && !encode_operand(&maps.b[s], b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
   }
 
   GemmParams kp;
@@ -737,7 +759,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.tiles_m = (p->m + kBM * ctas - 1) / (kBM * ctas);
   kp.tiles_n = (p->n + bn - 1) / bn;
   kp.kblocks = (p->k + bke - 1) / bke;
-  kp.nseg = nseg;
+  kp.planes = planes;
   kp.idesc = make_idesc(cfmt, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
   kp.acc_is_int = is_int ? 1 : 0;
   EpiParams ep;
@@ -846,7 +868,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   GemmKernel kern = epi_kernel ? (ctas == 2 ? pick_kernel<2, true>(kind, a_mn, b_mn) : pick_kernel<1, true>(kind, a_mn, b_mn))
                                : (ctas == 2 ? pick_kernel<2, false>(kind, a_mn, b_mn) : pick_kernel<1, false>(kind, a_mn, b_mn));
   const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
-  const int smem = ctas == 2 ? GemmSmemLayout<2>::total(stages, bn, kernel_epi_vec) : GemmSmemLayout<1>::total(stages, bn, kernel_epi_vec);
+  const int smem = ctas == 2 ? GemmSmemLayout<2>::total(stages, bn, kernel_epi_vec, planes) : GemmSmemLayout<1>::total(stages, bn, kernel_epi_vec, planes);
   {
     const RbStatus sst = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (sst != RB_SUCCESS) return sst;

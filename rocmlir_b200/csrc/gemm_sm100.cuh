@@ -51,13 +51,19 @@ struct KindTraits<kKindI8> { static constexpr int ES = 1, UMMA_K = 32; };
 template <>
 struct KindTraits<kKindF8> { static constexpr int ES = 1, UMMA_K = 32; };
 
-// A contraction may be the sum of up to kMaxSeg (A_s, B_s) products over the same K range
-// (3xTF32 split of an f32 GEMM). Segment s streams tiles from tensor maps tma[s] / tmb[s].
-constexpr int kMaxSeg = 3;
+// f32 operands in accurate mode are two TF32 planes each, hi and lo (x = hi + lo): a ring slot then holds a K block of all
+// four, [A hi][A lo][B hi][B lo], and the issuing thread runs lo.hi, hi.lo and hi.hi from it. Every other operand has the
+// one plane [0].
+// * Each tile is fetched once for its two products: 4 tiles per K block instead of the 6 that three passes over K fetched
+//   (one per product), which had the kernel waiting for the L2 -> SM fabric.
+// * The small products lo.hi + hi.lo have an accumulator of their own, added to the main one by the epilogue with
+//   round-to-nearest: the tensor core truncates what it adds to the magnitude of the accumulator, and they are 2^-11 of it.
+//   Both fit beside each other in tensor memory: two buffers of 128 + 128 columns, or one of 256 + 256.
+constexpr int kMaxPlanes = 2;
 
 struct GemmTensorMaps {
-  CUtensorMap a[kMaxSeg];
-  CUtensorMap b[kMaxSeg];
+  CUtensorMap a[kMaxPlanes];
+  CUtensorMap b[kMaxPlanes];
   CUtensorMap c;  // store map of C (box: 128 bytes of a row x 32 rows); valid when GemmParams::c_tma != 0
 };
 
@@ -80,8 +86,8 @@ struct GemmParams {
   int splits;                 // K is cut into `splits` ranges; with splits > 1 every range writes raw partial sums
   long long split_stride;     // elements between the partial planes of consecutive ranges (splits > 1)
   int tiles_m, tiles_n;       // tiles_m counts (kBM * CTAS)-row blocks
-  int kblocks;                // K blocks per segment
-  int nseg;
+  int kblocks;                // K blocks
+  int planes;                 // TF32 planes per operand: 2 for f32 in accurate mode, else 1
   uint32_t idesc;
   int acc_is_int;
   void* c;
@@ -149,7 +155,7 @@ struct GemmSmemLayout {
   static constexpr int kABytes = kBM * kRowBytes;
   static constexpr int kMaxStages = 8;
   static constexpr int kSmemBudget = 232448;  // opt-in shared memory per CTA on sm_100
-  static constexpr int stage_bytes(int bn) { return kABytes + (bn / CTAS) * kRowBytes; }
+  static constexpr int stage_bytes(int bn, int planes) { return planes * (kABytes + (bn / CTAS) * kRowBytes); }
   // Epilogue staging: per epilogue warp two 32-row x 128-byte tiles (double buffered TMA stores).
   static constexpr int kStoreTileBytes = 32 * kRowBytes;
   static constexpr int kStagingBytes = 4 * 2 * kStoreTileBytes;
@@ -160,11 +166,11 @@ struct GemmSmemLayout {
   // Per-column epilogue vectors of the current tile as f32, one private copy per epilogue warp (no cross-warp
   // barrier is needed that way): [4 warps][scale[kMaxBN], bias[kMaxBN]].
   static constexpr int kEpiVecBytes = 4 * 2 * kMaxBN * 4;
-  static constexpr int total(int stages, int bn, bool epi_vec) {
-    return stages * stage_bytes(bn) + staging_bytes(epi_vec) + (epi_vec ? kEpiVecBytes : 0) + kBarBytes + 1024;  // + alignment slack
+  static constexpr int total(int stages, int bn, bool epi_vec, int planes) {
+    return stages * stage_bytes(bn, planes) + staging_bytes(epi_vec) + (epi_vec ? kEpiVecBytes : 0) + kBarBytes + 1024;  // + alignment slack
   }
-  static constexpr int max_stages(int bn, bool epi_vec) {
-    int s = (kSmemBudget - staging_bytes(epi_vec) - (epi_vec ? kEpiVecBytes : 0) - kBarBytes - 1024) / stage_bytes(bn);
+  static constexpr int max_stages(int bn, bool epi_vec, int planes) {
+    int s = (kSmemBudget - staging_bytes(epi_vec) - (epi_vec ? kEpiVecBytes : 0) - kBarBytes - 1024) / stage_bytes(bn, planes);
     return s > kMaxStages ? kMaxStages : s;
   }
 };
@@ -381,7 +387,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   constexpr int KSTEPS = BKE / KT::UMMA_K;     // MMAs per stage (always 4)
   constexpr int CHUNK_BYTES = BKE * kRowBytes; // one MN-major chunk: BKE k-rows of 128 B
   const int bn_cta = p.bn / CTAS;              // columns of B this CTA loads
-  const int stage_bytes = L::stage_bytes(p.bn);
+  const bool two_planes = KIND == kKindTF32 && p.planes == 2;   // folds to false in every other kind
+  const int stage_bytes = L::stage_bytes(p.bn, two_planes ? 2 : 1);
+  // tensor memory: two buffers of 256 columns; with two planes a buffer is the main and the small accumulator, and a tile
+  // of 256 columns takes both buffers
+  const uint32_t buf_mask = two_planes && p.bn > kMaxBN / 2 ? 0u : 1u;
+  const uint32_t buf_shift = buf_mask;   // log2 of the number of buffers
+  const uint32_t small_cols = (uint32_t)p.bn;
   const int probe = kProbeBuild ? p.probe : 0;  // folds to 0 (and every probe branch away) in the shipped build
   const long long wait_limit = p.wait_cycles;
 
@@ -421,7 +433,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
     tmem_relinquish<CTAS>();
   }
   if (warp == 0 && lane_id() == 0) {
-    for (int s = 0; s < p.nseg; ++s) {
+    for (int s = 0; s < (two_planes ? 2 : 1); ++s) {
       prefetch_tmap(&maps.a[s]);
       prefetch_tmap(&maps.b[s]);
     }
@@ -447,7 +459,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         const int m0 = (mb * CTAS + (int)rank) * kBM;
         const int n0 = nb * p.bn + (int)rank * bn_cta;
         const int kb_begin = w.kb_begin, kb_end = w.kb_end;
-        const int ktotal = (kb_end - kb_begin) * p.nseg;
+        const int ktotal = kb_end - kb_begin;
         const int ga = g ^ (p.chain_flip & 1), gb = g ^ ((p.chain_flip >> 1) & 1);
         if (p.chain_flags != nullptr && g == 1) {   // A of this tile is the result of group 0's tiles of the same m block
           const int nw = p.tiles_n * CTAS * 4;
@@ -462,7 +474,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           base_h = op * p.conva.stride_h - p.conva.pad_h;
           base_w = (rem - op * p.conva.Q) * p.conva.stride_w - p.conva.pad_w;
         }
-        int seg = 0, kb = kb_begin;
+        int kb = kb_begin;
         // One barrier round covers up to kpr consecutive K blocks in ring slots s * kpr ... (s indexes rounds):
         // the barrier work of the issuing threads is per round, which is what bounds narrow tiles.
         for (int kk0 = 0; kk0 < ktotal; kk0 += kpr) {
@@ -481,7 +493,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           for (int j = 0; j < nblk; ++j) {
             uint8_t* sa = smem + (s * kpr + j) * stage_bytes;
-            uint8_t* sb = sa + L::kABytes;
+            uint8_t* sb = sa + (two_planes ? 2 : 1) * L::kABytes;
             const int k0 = kb * BKE;
             if ((probe & 1) || p.stall) {
               // loads switched off: the round's barrier was completed above (probe) or is left incomplete (stall)
@@ -489,33 +501,33 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
               if (!A_MN && p.conva.enabled == 1) {
                 const int tap = kb / p.conva.cchunks, cc = kb - tap * p.conva.cchunks;
                 const int fy = tap / p.conva.X, fx = tap - fy * p.conva.X;
-                tma_load_im2col_4d(sa, &maps.a[seg], &full_bar[s], cc * BKE, base_w, base_h, img,
+                tma_load_im2col_4d(sa, &maps.a[0], &full_bar[s], cc * BKE, base_w, base_h, img,
                                    (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
               } else if constexpr (!A_MN) {
-                tma_load_3d(sa, &maps.a[seg], &full_bar[s], k0, m0, ga);
+                tma_load_3d(sa, &maps.a[0], &full_bar[s], k0, m0, ga);
               } else if (p.a_fused) {
-                tma_load_4d(sa, &maps.a[seg], &full_bar[s], 0, k0, m0 / CHE, ga);
+                tma_load_4d(sa, &maps.a[0], &full_bar[s], 0, k0, m0 / CHE, ga);
               } else {
   #pragma unroll
                 for (int c = 0; c < kBM / CHE; ++c)
-                  tma_load_3d(sa + c * CHUNK_BYTES, &maps.a[seg], &full_bar[s], m0 + c * CHE, k0, ga);
+                  tma_load_3d(sa + c * CHUNK_BYTES, &maps.a[0], &full_bar[s], m0 + c * CHE, k0, ga);
               }
               if constexpr (!B_MN) {
-                tma_load_3d(sb, &maps.b[seg], &full_bar[s], k0, n0, gb);
+                tma_load_3d(sb, &maps.b[0], &full_bar[s], k0, n0, gb);
               } else if (p.conva.enabled == 2) {
                 int bi, bh, bw;
                 convb_pixel(p.conva, k0, bi, bh, bw);
                 for (int c = 0; c < bn_cta / CHE; ++c) {
                   int cc, fy, fx;
                   convb_tap(p.conva, n0 + c * CHE, p.N, CHE, cc, fy, fx);
-                  tma_load_im2col_4d(sb + c * CHUNK_BYTES, &maps.b[seg], &full_bar[s], cc * CHE, bw, bh, bi,
+                  tma_load_im2col_4d(sb + c * CHUNK_BYTES, &maps.b[0], &full_bar[s], cc * CHE, bw, bh, bi,
                                      (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
                 }
               } else if (p.b_fused) {
-                tma_load_4d(sb, &maps.b[seg], &full_bar[s], 0, k0, n0 / CHE, gb);
+                tma_load_4d(sb, &maps.b[0], &full_bar[s], 0, k0, n0 / CHE, gb);
               } else {
                 for (int c = 0; c < bn_cta / CHE; ++c)
-                  tma_load_3d(sb + c * CHUNK_BYTES, &maps.b[seg], &full_bar[s], n0 + c * CHE, k0, gb);
+                  tma_load_3d(sb + c * CHUNK_BYTES, &maps.b[0], &full_bar[s], n0 + c * CHE, k0, gb);
               }
             } else {
               // Completion of this CTA's loads is counted on the leader CTA's barrier.
@@ -523,36 +535,64 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
               if (!A_MN && p.conva.enabled == 1) {
                 const int tap = kb / p.conva.cchunks, cc = kb - tap * p.conva.cchunks;
                 const int fy = tap / p.conva.X, fx = tap - fy * p.conva.X;
-                tma_load_im2col_4d_bar(sa, &maps.a[seg], lead_full, cc * BKE, base_w, base_h, img,
+                tma_load_im2col_4d_bar(sa, &maps.a[0], lead_full, cc * BKE, base_w, base_h, img,
                                        (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
               } else if constexpr (!A_MN) {
-                tma_load_3d_bar(sa, &maps.a[seg], lead_full, k0, m0, ga);
+                tma_load_3d_bar(sa, &maps.a[0], lead_full, k0, m0, ga);
               } else if (p.a_fused) {
-                tma_load_4d_bar(sa, &maps.a[seg], lead_full, 0, k0, m0 / CHE, ga);
+                tma_load_4d_bar(sa, &maps.a[0], lead_full, 0, k0, m0 / CHE, ga);
               } else {
   #pragma unroll
                 for (int c = 0; c < kBM / CHE; ++c)
-                  tma_load_3d_bar(sa + c * CHUNK_BYTES, &maps.a[seg], lead_full, m0 + c * CHE, k0, ga);
+                  tma_load_3d_bar(sa + c * CHUNK_BYTES, &maps.a[0], lead_full, m0 + c * CHE, k0, ga);
               }
               if constexpr (!B_MN) {
-                tma_load_3d_bar(sb, &maps.b[seg], lead_full, k0, n0, gb);
+                tma_load_3d_bar(sb, &maps.b[0], lead_full, k0, n0, gb);
               } else if (p.conva.enabled == 2) {
                 int bi, bh, bw;
                 convb_pixel(p.conva, k0, bi, bh, bw);
                 for (int c = 0; c < bn_cta / CHE; ++c) {
                   int cc, fy, fx;
                   convb_tap(p.conva, n0 + c * CHE, p.N, CHE, cc, fy, fx);
-                  tma_load_im2col_4d_bar(sb + c * CHUNK_BYTES, &maps.b[seg], lead_full, cc * CHE, bw, bh, bi,
+                  tma_load_im2col_4d_bar(sb + c * CHUNK_BYTES, &maps.b[0], lead_full, cc * CHE, bw, bh, bi,
                                          (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
                 }
               } else if (p.b_fused) {
-                tma_load_4d_bar(sb, &maps.b[seg], lead_full, 0, k0, n0 / CHE, gb);
+                tma_load_4d_bar(sb, &maps.b[0], lead_full, 0, k0, n0 / CHE, gb);
               } else {
                 for (int c = 0; c < bn_cta / CHE; ++c)
-                  tma_load_3d_bar(sb + c * CHUNK_BYTES, &maps.b[seg], lead_full, n0 + c * CHE, k0, gb);
+                  tma_load_3d_bar(sb + c * CHUNK_BYTES, &maps.b[0], lead_full, n0 + c * CHE, k0, gb);
               }
             }
-            if (++kb == kb_end) { kb = kb_begin; ++seg; }
+            if constexpr (KIND == kKindTF32) {
+              if (two_planes && !((probe & 1) || p.stall)) {   // the lo planes, behind the hi planes
+                uint8_t* sa_lo = sa + L::kABytes;
+                uint8_t* sb_lo = sb + bn_cta * kRowBytes;
+                if constexpr (CTAS == 1) {
+                  if (p.conva.enabled == 1) {
+                    const int tap = kb / p.conva.cchunks, cc = kb - tap * p.conva.cchunks;
+                    const int fy = tap / p.conva.X, fx = tap - fy * p.conva.X;
+                    tma_load_im2col_4d(sa_lo, &maps.a[1], &full_bar[s], cc * BKE, base_w, base_h, img,
+                                       (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
+                  } else {
+                    tma_load_3d(sa_lo, &maps.a[1], &full_bar[s], k0, m0, ga);
+                  }
+                  tma_load_3d(sb_lo, &maps.b[1], &full_bar[s], k0, n0, gb);
+                } else {
+                  const uint32_t lead_full = mapa_u32(smem_u32(&full_bar[s]), 0);
+                  if (p.conva.enabled == 1) {
+                    const int tap = kb / p.conva.cchunks, cc = kb - tap * p.conva.cchunks;
+                    const int fy = tap / p.conva.X, fx = tap - fy * p.conva.X;
+                    tma_load_im2col_4d_bar(sa_lo, &maps.a[1], lead_full, cc * BKE, base_w, base_h, img,
+                                           (uint16_t)(fx * p.conva.dil_w), (uint16_t)(fy * p.conva.dil_h));
+                  } else {
+                    tma_load_3d_bar(sa_lo, &maps.a[1], lead_full, k0, m0, ga);
+                  }
+                  tma_load_3d_bar(sb_lo, &maps.b[1], lead_full, k0, n0, gb);
+                }
+              }
+            }
+            ++kb;
           }
           if (++s == (uint32_t)rounds) { s = 0; ph ^= 1u; }
         }
@@ -575,7 +615,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // Descriptor halves: constant high word; low word of stage 0, advanced by adds only.
       const uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), A_MN ? CHUNK_BYTES : 16);
-      const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + L::kABytes, B_MN ? CHUNK_BYTES : 16);
+      const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + (two_planes ? 2 : 1) * L::kABytes, B_MN ? CHUNK_BYTES : 16);
       const uint32_t kStageStep = (uint32_t)stage_bytes >> 4;
       constexpr uint32_t kAStep = (A_MN ? KT::UMMA_K * kRowBytes : KT::UMMA_K * ES) >> 4;
       constexpr uint32_t kBStep = (B_MN ? KT::UMMA_K * kRowBytes : KT::UMMA_K * ES) >> 4;
@@ -584,15 +624,15 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       WorkIter it(p, pair_id, num_pairs);
       WorkItem w;
       for (; ok && it.next(w); ++t) {
-        const uint32_t buf = t & 1u;
-        const uint32_t bph = (t >> 1) & 1u;
+        const uint32_t buf = t & buf_mask;
+        const uint32_t bph = (t >> buf_shift) & 1u;
         const long long tw0 = p.trace ? clock64() : 0;
         if (!mbar_wait(&tempty_bar[buf], bph ^ 1u, p.status, kStatusTimeoutMma + 0x10 + buf, wait_limit)) { ok = false; break; }
         if (p.trace) w_tempty += clock64() - tw0;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * kMaxBN;
         uint32_t accum = 0;
-        const int ktotal = (w.kb_end - w.kb_begin) * p.nseg;
+        const int ktotal = w.kb_end - w.kb_begin;
         const long long tk0 = p.trace ? clock64() : 0;
         if (kpr == 1) {
           // one K block per round: the tight loop (at 256-column tiles the four MMAs of a block execute for 512
@@ -608,11 +648,31 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
             const bool next_ready = mbar_test_wait_addr(full0 + ns * 8, nph);  // consumed after the MMAs below
             const uint32_t a_lo = a_lo0 + s * kStageStep;
             const uint32_t b_lo = b_lo0 + s * kStageStep;
+            bool done = false;
+            if constexpr (KIND == kKindTF32) {
+              if (two_planes) {   // lo.hi and hi.lo into the small accumulator, hi.hi into the main one
+                const uint32_t a_l = a_lo + (L::kABytes >> 4), b_l = b_lo + ((uint32_t)(bn_cta * kRowBytes) >> 4);
+                const uint32_t tmem_s = tmem_d + small_cols;
 #pragma unroll
-            for (int k = 0; k < KSTEPS; ++k) {
-              umma_ss<KIND, CTAS>(tmem_d, desc64(a_lo + k * kAStep, desc_hi), desc64(b_lo + k * kBStep, desc_hi), p.idesc,
-                                  accum);
-              accum = 1;
+                for (int k = 0; k < KSTEPS; ++k)
+                  umma_ss<KIND, CTAS>(tmem_s, desc64(a_l + k * kAStep, desc_hi), desc64(b_lo + k * kBStep, desc_hi), p.idesc, k ? 1u : accum);
+#pragma unroll
+                for (int k = 0; k < KSTEPS; ++k)
+                  umma_ss<KIND, CTAS>(tmem_s, desc64(a_lo + k * kAStep, desc_hi), desc64(b_l + k * kBStep, desc_hi), p.idesc, 1u);
+#pragma unroll
+                for (int k = 0; k < KSTEPS; ++k)
+                  umma_ss<KIND, CTAS>(tmem_d, desc64(a_lo + k * kAStep, desc_hi), desc64(b_lo + k * kBStep, desc_hi), p.idesc, k ? 1u : accum);
+                accum = 1;
+                done = true;
+              }
+            }
+            if (!done) {
+#pragma unroll
+              for (int k = 0; k < KSTEPS; ++k) {
+                umma_ss<KIND, CTAS>(tmem_d, desc64(a_lo + k * kAStep, desc_hi), desc64(b_lo + k * kBStep, desc_hi), p.idesc,
+                                    accum);
+                accum = 1;
+              }
             }
             if constexpr (CTAS == 1) {
               tc_commit_addr1(empty0 + s * 8);
@@ -695,8 +755,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
     for (; it.next(w); ++t) {
       int g, mb, nb;
       tile_coords(w.tile, p.tiles_m, p.tiles_n, g, mb, nb);
-      const uint32_t buf = t & 1u;
-      const uint32_t bph = (t >> 1) & 1u;
+      const uint32_t buf = t & buf_mask;
+      const uint32_t bph = (t >> buf_shift) & 1u;
       const long long tw = p.trace ? clock64() : 0;
       if (!mbar_wait_warp(&tfull_bar[buf], bph, p.status, kStatusTimeoutEpilogue + buf, wait_limit)) break;
       const long long te = p.trace ? clock64() : 0;
@@ -757,11 +817,19 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         __threadfence();
         if (!got) break;
       }
+      // f32: 32 columns of the small accumulator, added with round-to-nearest to those of the main one in v
+      auto add_small = [&](uint32_t taddr_main, uint32_t* v) {
+        uint32_t u[32];
+        tmem_ld32(taddr_main + small_cols, u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+      };
       // Fast path (whole tiles, float accumulators, no fused elementwise work, 16-bit C through TMA stores): a
       // compact loop - 64 columns = one 128-byte staging row per step. The general loop below handles every other
       // case; keeping this one small matters because the general loop's code is far larger than the instruction
       // cache and ran at about 1400 cycles per 32 columns where this one needs about 150.
-      const bool fast16 = w.kind == 0 && p.c_tma && eflags == 0 && !p.acc_is_int && !probe &&
+      const bool fast16 = !two_planes && w.kind == 0 && p.c_tma && eflags == 0 && !p.acc_is_int && !probe &&
                           (p.c_type == RB_F16 || p.c_type == RB_BF16);
       // 4-byte C (f32 results, raw i32 results, the raw planes of a K split): 32 columns = one staging row per step
       const bool fast32 = w.kind == 0 && p.c_tma && !probe &&
@@ -824,6 +892,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           if (lane == 0 && nstores >= 2) bulk_wait_read<1>();
           __syncwarp();
           tmem_ld_wait();
+          if (two_planes) add_small(taddr + c * 32, v);
           uint8_t* rowp = stg + lane * kRowBytes;
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -843,7 +912,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // code evicted the other roles' instructions (the issue loop waited twice as long for operands).
       const bool f16_mid = (eflags & RB_EPI_ROUND_MID) && (p.epi.mid_type == RB_F16 || p.epi.mid_type == RB_BF16);
       const uint32_t f16_extra = eflags & ~(uint32_t)(RB_EPI_ALPHA | RB_EPI_BIAS | RB_EPI_RELU | (f16_mid ? RB_EPI_ROUND_MID : 0));
-      const bool fast16e = eflags != 0 && w.kind == 0 && p.c_tma && f16_extra == 0 &&
+      const bool fast16e = !two_planes && eflags != 0 && w.kind == 0 && p.c_tma && f16_extra == 0 &&
                            (epi_col_bias(eflags) || !(eflags & RB_EPI_BIAS)) && !p.acc_is_int && !probe &&
                            (p.c_type == RB_F16 || p.c_type == RB_BF16);
       const bool fast8 = !fast16e && w.kind == 0 && p.c_tma && !probe && p.acc_is_int && p.c_type == RB_I8 &&
@@ -868,6 +937,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           uint32_t v[32];
           tmem_ld32(taddr + c * 32, v);
           tmem_ld_wait();
+          if (two_planes) add_small(taddr + c * 32, v);
           if (row_ok) {
             float* d = static_cast<float*>(p.c) + c_row_off + (long long)n0 * p.c_stride_n;
 #pragma unroll
@@ -894,6 +964,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
             __syncwarp();
           }
           tmem_ld_wait();
+          if (two_planes) add_small(taddr + c * 32, v);
           float x[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) x[j] = p.acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
@@ -931,6 +1002,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         const long long tl0 = p.trace ? clock64() : 0;
         tmem_ld32(tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN + c * 32, v);
         tmem_ld_wait();
+        if (two_planes) add_small(tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN + c * 32, v);
         const long long tl1 = p.trace ? clock64() : 0;
         e_ld += tl1 - tl0;
         if (w.kind == 2) {  // contributor: raw accumulators to this unit's partial tile
