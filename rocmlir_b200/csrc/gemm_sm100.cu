@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <mutex>
 
+#include "gemm_skinny.h"
 #include "lib_state.h"
 
 namespace rb {
@@ -646,6 +647,31 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   if ((reinterpret_cast<uintptr_t>(a) % 16 && !oa.needs_copy) || (reinterpret_cast<uintptr_t>(b) % 16 && !ob.needs_copy))
     return fail(RB_UNSUPPORTED, "operand base addresses must be 16-byte aligned");
 
+  EpiParams ep;
+  memset(&ep, 0, sizeof(ep));
+  if (epi) {
+    ep.flags = epi->flags; ep.alpha = epi->alpha; ep.out_recip = epi->out_recip;
+    ep.mid_type = epi->mid_type; ep.bias_type = epi->bias_type;
+    ep.col_scale = epi->col_scale; ep.bias = epi->bias;
+    ep.clip_lo = epi->clip_lo; ep.clip_hi = epi->clip_hi;
+    ep.in_zero = epi->in_zero; ep.out_zero = (epi->flags & RB_EPI_ZP_OUT) ? epi->out_zero : 0;
+    ep.residual = epi->residual; ep.res_type = epi->res_type;
+    ep.unary = (epi->flags & RB_EPI_UNARY) ? epi->unary : 0;
+  }
+  if (p->store_method == 1) {
+    // the kernel's result is rounded to C's type and added to what C holds, like an atomic add of the stored value
+    ep.flags |= RB_EPI_RESIDUAL;
+    ep.residual = c; ep.res_type = p->c_type;
+    if (!(ep.flags & RB_EPI_ROUND_MID)) { ep.flags |= RB_EPI_ROUND_MID; ep.mid_type = p->c_type; }
+  }
+
+  // few rows against weights stored N x K: the tile turned round (an explicit variant keeps this kernel)
+  if (!capture && !chain && !conva && t_variant == 0 && gemm_skinny_applicable(p) && tuned_variant_gemm(p) == 0) {
+    const int stall = t_stall_launches > 0 ? 1 : 0;
+    t_stall_launches -= stall;
+    return gemm_skinny_run(p, ep, a, b, c, kind, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, cfmt, t_wait_cycles, stall, stream_v);
+  }
+
   uint8_t* wsb = static_cast<uint8_t*>(workspace);
   const void* a_src[2] = {a, nullptr};
   const void* b_src[2] = {b, nullptr};
@@ -762,23 +788,6 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.planes = planes;
   kp.idesc = make_idesc(cfmt, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
   kp.acc_is_int = is_int ? 1 : 0;
-  EpiParams ep;
-  memset(&ep, 0, sizeof(ep));
-  if (epi) {
-    ep.flags = epi->flags; ep.alpha = epi->alpha; ep.out_recip = epi->out_recip;
-    ep.mid_type = epi->mid_type; ep.bias_type = epi->bias_type;
-    ep.col_scale = epi->col_scale; ep.bias = epi->bias;
-    ep.clip_lo = epi->clip_lo; ep.clip_hi = epi->clip_hi;
-    ep.in_zero = epi->in_zero; ep.out_zero = (epi->flags & RB_EPI_ZP_OUT) ? epi->out_zero : 0;
-    ep.residual = epi->residual; ep.res_type = epi->res_type;
-    ep.unary = (epi->flags & RB_EPI_UNARY) ? epi->unary : 0;
-  }
-  if (p->store_method == 1) {
-    // the kernel's result is rounded to C's type and added to what C holds, like an atomic add of the stored value
-    ep.flags |= RB_EPI_RESIDUAL;
-    ep.residual = c; ep.res_type = p->c_type;
-    if (!(ep.flags & RB_EPI_ROUND_MID)) { ep.flags |= RB_EPI_ROUND_MID; ep.mid_type = p->c_type; }
-  }
   const size_t es_c = dtype_bytes(p->c_type);
   void* partial = splits > 1 ? static_cast<void*>(wsb + ws.partial_off) : nullptr;
   if (splits > 1 && conva && conva->c_rows_per_img > 0)
