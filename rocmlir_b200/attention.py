@@ -11,7 +11,7 @@ from typing import Optional
 import torch
 
 from . import _lib as L
-from .gemm import rb_dtype
+from .gemm import rb_dtype, stream_address
 
 
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, trans_k: bool = False, trans_q: bool = False,
@@ -56,7 +56,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, trans_k: boo
     if mask is not None:
         assert mask.is_cuda and mask.is_contiguous() and mask.dtype == torch.int8 and tuple(mask.shape) == (g, sq, sk)
         p.mask = mask.data_ptr()
-    stream = torch.cuda.current_stream(q.device).cuda_stream
+    stream = stream_address(q.device)
     # scratch for staged operands comes from the caller's side (rbAttentionWs): the library allocates nothing
     need = int(L.lib().rbAttentionWorkspaceSize(C.byref(p)))
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):

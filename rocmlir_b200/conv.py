@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from . import _lib as L
-from .gemm import rb_dtype
+from .gemm import rb_dtype, run_with_workspace, stream_address
 
 FWD, BWD_DATA, BWD_WEIGHT = 0, 1, 2
 OPERATIONS = {"conv": FWD, "conv_bwd_data": BWD_DATA, "conv_bwd_weight": BWD_WEIGHT}
@@ -115,14 +115,10 @@ def conv(cfg: ConvConfig, direction: int, filter: torch.Tensor, input: torch.Ten
     dtype = input.dtype
     p = cfg.to_c(dtype, direction, f32_mode)
     lib = L.lib()
-    ws_bytes = int(lib.rbConvWorkspaceSize(C.byref(p)))
-    if ws_bytes and (workspace is None or workspace.numel() * workspace.element_size() < ws_bytes):
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=input.device)
-    stream = torch.cuda.current_stream(input.device).cuda_stream
-    st = lib.rbConv(C.byref(p), filter.data_ptr(), input.data_ptr(), output.data_ptr(),
-                    workspace.data_ptr() if workspace is not None else None,
-                    workspace.numel() * workspace.element_size() if workspace is not None else 0, stream)
-    L.check(st)
+    pp, stream = C.byref(p), stream_address(input.device)
+    pf, pi, po = filter.data_ptr(), input.data_ptr(), output.data_ptr()
+    L.check(run_with_workspace(lambda ws, n: lib.rbConv(pp, pf, pi, po, ws, n, stream), lambda: int(lib.rbConvWorkspaceSize(pp)),
+                               workspace, input.device, ask=lib.rbGetGemmVariant() != 0))
     return {FWD: output, BWD_DATA: input, BWD_WEIGHT: filter}[direction]
 
 
@@ -139,15 +135,12 @@ def conv_fused(cfg: ConvConfig, filter: torch.Tensor, input: torch.Tensor, outpu
     p = cfg.to_c(input.dtype, FWD, f32_mode)
     out_type = rb_dtype(output.dtype)
     lib = L.lib()
-    ws_bytes = int(lib.rbConvEpiWorkspaceSize(C.byref(p), out_type))
-    if ws_bytes and (workspace is None or workspace.numel() * workspace.element_size() < ws_bytes):
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=input.device)
-    e = epilogue.to_c() if epilogue is not None else None
-    stream = torch.cuda.current_stream(input.device).cuda_stream
-    L.check(lib.rbConvEpi(C.byref(p), C.byref(e) if e is not None else None, out_type, filter.data_ptr(),
-                          input.data_ptr(), output.data_ptr(),
-                          workspace.data_ptr() if workspace is not None else None,
-                          workspace.numel() * workspace.element_size() if workspace is not None else 0, stream))
+    e = C.byref(epilogue.to_c()) if epilogue is not None else None
+    pp, stream = C.byref(p), stream_address(input.device)
+    pf, pi, po = filter.data_ptr(), input.data_ptr(), output.data_ptr()
+    L.check(run_with_workspace(lambda ws, n: lib.rbConvEpi(pp, e, out_type, pf, pi, po, ws, n, stream),
+                               lambda: int(lib.rbConvEpiWorkspaceSize(pp, out_type)), workspace, input.device,
+                               ask=lib.rbGetGemmVariant() != 0))
     return output
 
 
@@ -252,7 +245,7 @@ def conv3d(cfg: Conv3dConfig, direction: int, filter: torch.Tensor, input: torch
     ws_bytes = int(lib.rbConv3dWorkspaceSize(C.byref(p)))
     if ws_bytes and (workspace is None or workspace.numel() * workspace.element_size() < ws_bytes):
         workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=input.device)
-    stream = torch.cuda.current_stream(input.device).cuda_stream
+    stream = stream_address(input.device)
     st = lib.rbConv3d(C.byref(p), filter.data_ptr(), input.data_ptr(), output.data_ptr(),
                       workspace.data_ptr() if workspace is not None else None,
                       workspace.numel() * workspace.element_size() if workspace is not None else 0, stream)

@@ -566,10 +566,19 @@ uint32_t tuned_variant_gemm(const RbGemmProblem* p) {
 uint32_t tuned_variant_conv(const RbConvProblem* p) {
   load_default_db();
   if (!p || g_db.size.load(std::memory_order_relaxed) == 0) return 0;
+  // the last problem asked about, per thread, by value: the key is a string of twenty numbers, and a launch asks twice
+  static thread_local RbConvProblem last_p;
+  static thread_local uint32_t last_v = 0;
+  static thread_local int last_gen = -1;
+  const int gen_now = g_db.generation.load(std::memory_order_relaxed);
+  if (last_gen == gen_now && memcmp(&last_p, p, sizeof(*p)) == 0) return last_v;
   ProblemDesc d;
   d.kind = kConv;
   d.conv = *p;
-  return db_lookup(d);
+  last_v = db_lookup(d);
+  memcpy(&last_p, p, sizeof(*p));
+  last_gen = gen_now;
+  return last_v;
 }
 
 }  // namespace rb

@@ -30,6 +30,26 @@ def torch_dtype(t: int) -> torch.dtype:
     return _RB2TORCH[t]
 
 
+def stream_address(device: torch.device) -> int:
+    """The current stream of a CUDA tensor's device (torch.cuda.current_stream makes a Stream object around it on every call)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def run_with_workspace(call, size, workspace: Optional[torch.Tensor], device: torch.device, ask: bool) -> int:
+    """Status of call(address, bytes). Small problems are bound by the host, and asking for the size plans the whole call once
+    more: a workspace that the caller brought is tried first (the library looks at its size before it launches anything), and
+    `size()` is asked only without one, when it turns out too small, or when `ask` says that the call would accept less than the
+    best."""
+    if workspace is not None and not ask:
+        st = call(workspace.data_ptr(), workspace.nbytes)
+        if st != L.WORKSPACE_TOO_SMALL:
+            return st
+    need = size()
+    if need and (workspace is None or workspace.nbytes < need):
+        workspace = torch.empty(need, dtype=torch.uint8, device=device)
+    return call(workspace.data_ptr() if workspace is not None else None, workspace.nbytes if workspace is not None else 0)
+
+
 @dataclass
 class Epilogue:
     """Fused elementwise tail of the GEMM; fields map one-to-one onto RbEpilogue."""
@@ -153,16 +173,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     try:
         if variant is not None:   # before the workspace query: a K split or a stream-K tail changes what is needed
             lib.rbSetGemmVariant(int(variant))
-        ws_bytes = workspace_size(p)
-        if ws_bytes and (workspace is None or workspace.numel() * workspace.element_size() < ws_bytes):
-            workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
-        e = epilogue.to_c() if epilogue is not None else None
-        stream = torch.cuda.current_stream(a.device).cuda_stream
-        st = lib.rbGemm(C.byref(p), C.byref(e) if e is not None else None, a.data_ptr(), b.data_ptr(), out.data_ptr(),
-                        workspace.data_ptr() if workspace is not None else None,
-                        workspace.numel() * workspace.element_size() if workspace is not None else 0, stream)
+        e = C.byref(epilogue.to_c()) if epilogue is not None else None
+        pp, pa, pb, pc, stream = C.byref(p), a.data_ptr(), b.data_ptr(), out.data_ptr(), stream_address(a.device)
+        # (a stream-K tail, bit 9 of the variant word, is left out when its partial tiles do not fit the workspace)
+        st = run_with_workspace(lambda ws, n: lib.rbGemm(pp, e, pa, pb, pc, ws, n, stream), lambda: workspace_size(p), workspace,
+                                a.device, ask=variant is not None or saved != 0)
     finally:
-        lib.rbSetGemmVariant(saved)
+        if variant is not None:
+            lib.rbSetGemmVariant(saved)
     L.check(st)
     if a.dim() == 2 and b.dim() == 2:
         out = out.view(shape[1], shape[2])
@@ -228,7 +246,7 @@ def gemm_gemm(a: torch.Tensor, b1: torch.Tensor, b2: torch.Tensor, *, out: Optio
         workspace = torch.empty(need, dtype=torch.uint8, device=a.device)
     if out is None:
         out = torch.empty((g, m, n2), dtype=a.dtype, device=a.device)
-    stream = torch.cuda.current_stream(a.device).cuda_stream
+    stream = stream_address(a.device)
     L.check(lib.rbGemmGemm(g, m, k1, n1, n2, dt, a.data_ptr(), b1.data_ptr(), b2.data_ptr(), out.data_ptr(),
                            workspace.data_ptr(), workspace.numel() * workspace.element_size(), stream))
     return out.view(m, n2) if a.dim() == 2 else out
