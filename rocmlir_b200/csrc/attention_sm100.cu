@@ -63,6 +63,9 @@ struct AttParams {
   const void* quant_bias;      // first-GEMM-quantised form: device pointers to one i8 and one f16 (else null)
   const void* quant_scale;
   unsigned long long* trace;   // optional [CTAs][16] cycle counters (two-tile kernel), see rbSetTraceBuffer
+  int splits;        // single-tile kernel: CTAs of a cluster that divide a query tile's key blocks (1, 2, 4 or 8)
+  void* o;           //   result [G][Sq][o_cols] and its row length, written directly when splits > 1
+  int o_cols;
   int linear;        // GEMM+GEMM: P = S rounded to the element type (no scale, no softmax, no division by a row sum)
 };
 
@@ -97,6 +100,18 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+constexpr int kMaxSplits = 8;   // portable cluster size
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float f16_round(float x) { return __half2float(__float2half_rn(x)); }
 
 __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __grid_constant__ AttMaps maps,
@@ -117,12 +132,20 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
 
   const int warp = threadIdx.x >> 5;
   const int lane = lane_id();
-  const int g = blockIdx.x / p.q_tiles;
+  // the CTAs of a cluster share a query tile and divide its key blocks
+  const int splits = p.splits;
+  const int part = splits > 1 ? (int)cluster_ctarank() : 0;
+  const int tile = blockIdx.x / splits;
+  const int g = tile / p.q_tiles;
   // long tiles first under a causal mask
-  const int qt = p.causal ? (p.q_tiles - 1 - blockIdx.x % p.q_tiles) : (blockIdx.x % p.q_tiles);
+  const int qt = p.causal ? (p.q_tiles - 1 - tile % p.q_tiles) : (tile % p.q_tiles);
   const int q0 = qt * kQT;
-  int nb = (p.Sk + kKT - 1) / kKT;
-  if (p.causal) nb = min(nb, (min(q0 + kQT, p.Sq) - 1) / kKT + 1);
+  int nb_all = (p.Sk + kKT - 1) / kKT;
+  if (p.causal) nb_all = min(nb_all, (min(q0 + kQT, p.Sq) - 1) / kKT + 1);
+  const int per_part = (nb_all + splits - 1) / splits;
+  const int j0 = min(part * per_part, nb_all), nb = min(per_part, nb_all - j0);   // key blocks j0 .. j0 + nb - 1 (maybe none)
+  // warps without a query row of the tile have nothing to compute: their rows of S, P and O are never looked at
+  const int live_warps = min(4, (p.Sq - q0 + 31) / 32);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -134,7 +157,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 4);
+    mbar_init(p_full, live_warps);
     mbar_init(pv_done, 1);
     fence_mbar_init();
   }
@@ -159,7 +182,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
+    if (lane == 0 && nb > 0) {
       mbar_expect_tx(q_full, q_bytes);
       for (int a = 0; a < d_atoms; ++a) tma_load_3d(smem + AttSmem::kQ + a * (kQT * 128), &maps.q, q_full, a * 64, q0, g);
       int s = 0;
@@ -169,20 +192,20 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         uint8_t* ks = smem + AttSmem::kK + s * AttSmem::kKBytes;
         mbar_expect_tx(&k_full[s], k_bytes);
         if (p.trans_k) {
-          for (int a = 0; a < d_atoms; ++a) tma_load_3d(ks + a * (kKT * 128), &maps.k, &k_full[s], a * 64, j * kKT, g);
+          for (int a = 0; a < d_atoms; ++a) tma_load_3d(ks + a * (kKT * 128), &maps.k, &k_full[s], a * 64, (j0 + j) * kKT, g);
         } else {
-          for (int c = 0; c < kKT / 64; ++c) tma_load_3d(ks + c * (p.D * 128), &maps.k, &k_full[s], j * kKT + c * 64, 0, g);
+          for (int c = 0; c < kKT / 64; ++c) tma_load_3d(ks + c * (p.D * 128), &maps.k, &k_full[s], (j0 + j) * kKT + c * 64, 0, g);
         }
         if (!mbar_wait(&v_empty[s], par ^ 1u, p.status, kStatusTimeoutProducer + 4 + s)) break;
         uint8_t* vs = smem + AttSmem::kV + s * AttSmem::kVBytes;
         mbar_expect_tx(&v_full[s], v_bytes);
-        for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, j * kKT, g);
+        for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, (j0 + j) * kKT, g);
         if (++s == NS) { s = 0; par ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (lane == 0 && nb > 0) {
       const uint32_t hi = smem_desc_hi(1024);
       const uint32_t q_addr = smem_u32(smem + AttSmem::kQ);
       int ks_stage = 0;        // ring position of the next K tile to consume
@@ -226,7 +249,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         if (++vs_stage == NS) { vs_stage = 0; vs_par ^= 1u; }
       }
     }
-  } else if (warp >= 4) {
+  } else if (warp >= 4 && warp - 4 < live_warps) {
     // ------------------------------ softmax / correction / epilogue ------------------------------
     const int wq = warp & 3;
     const int r = wq * 32 + lane;          // row within the tile == TMEM lane
@@ -237,12 +260,25 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     const float qscale = p.quant_scale ? __half2float(*static_cast<const __half*>(p.quant_scale)) : 1.0f;
     float l = 0.0f;
     bool ok = true;
+    const long long side_row = ((long long)g * p.Sq + min(row, (long long)p.Sq - 1)) * p.Sk;   // row of the [G][Sq][Sk] tensors
+    const bool mask_only = p.mask && !p.bias && !p.scale_t && !p.quant_scale && !p.causal;
+    const bool mask_vec = mask_only && p.Sk % 16 == 0 && reinterpret_cast<uintptr_t>(p.mask) % 16 == 0;
     for (int j = 0; j < nb && ok; ++j) {
       const int sb = j & 1;
+      const int key0 = (j0 + j) * kKT;
+      // this row's mask of the block, one byte a key, read while the scores are on their way
+      uint32_t mw[32];
+      if (mask_vec) {
+        const uint4* m4 = reinterpret_cast<const uint4*>(p.mask + side_row + key0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = key0 + i * 16 < p.Sk ? __ldg(m4 + i) : make_uint4(0u, 0u, 0u, 0u);   // whole words: Sk is a multiple of 16
+          mw[4 * i] = u.x; mw[4 * i + 1] = u.y; mw[4 * i + 2] = u.z; mw[4 * i + 3] = u.w;
+        }
+      }
       if (!mbar_wait(&s_full[sb], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutEpilogue + sb)) { ok = false; break; }
       tc_fence_after();
       const uint32_t tmem_s = tmem_base + lane_base + sb * 128;
-      const int key0 = j * kKT;
       const bool side_inputs = p.bias || p.mask || p.scale_t || p.quant_scale;          // per-element tensors: general path
       const bool edge = (key0 + kKT > p.Sk) || (p.causal && key0 + kKT - 1 > q0);  // key tail or diagonal block
       uint32_t v[128];
@@ -286,8 +322,21 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
           v[i] = __float_as_uint(x0); v[i + 1] = __float_as_uint(x1); v[i + 2] = __float_as_uint(x2); v[i + 3] = __float_as_uint(x3);
           mx0 = fmaxf(mx0, x0); mx1 = fmaxf(mx1, x1); mx2 = fmaxf(mx2, x2); mx3 = fmaxf(mx3, x3);
         }
+      } else if (mask_vec) {
+        // a mask tensor alone: the general branch below with its byte loads already done, sixteen at a time
+#pragma unroll
+        for (int i = 0; i < 128; i += 4) {
+          float x[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            x[t] = (mw[i / 4] & (0xffu << (8 * t))) ? __uint_as_float(v[i + t]) * p.scale_log2 : p.mask_fill * kLog2e;
+            if (key0 + i + t >= p.Sk) x[t] = -INFINITY;
+            v[i + t] = __float_as_uint(x[t]);
+          }
+          mx0 = fmaxf(mx0, x[0]); mx1 = fmaxf(mx1, x[1]); mx2 = fmaxf(mx2, x[2]); mx3 = fmaxf(mx3, x[3]);
+        }
       } else {
-        const long long side_off = ((long long)g * p.Sq + min(row, (long long)p.Sq - 1)) * p.Sk;
+        const long long side_off = side_row;
 #pragma unroll
         for (int i = 0; i < 128; ++i) {  // fully unrolled: v[] must stay in registers
           float x = __uint_as_float(v[i]);
@@ -352,8 +401,27 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
+    if (splits > 1) {
+      // this CTA's share of the row, not divided by its sum: O, reference maximum and sum go to shared memory (the key
+      // ring is idle by now) for the cluster to add up below
+      if (nb > 0 && ok && mbar_wait(pv_done, (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+        tc_fence_after();
+        const int c4mask = p.Dv / 4 - 1;   // Dv is 64 or 128
+        float4* prow = reinterpret_cast<float4*>(smem + AttSmem::kK) + r * (p.Dv / 4);
+#pragma unroll 1
+        for (int c = 0; c < p.Dv / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld32(tmem_o + lane_base + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i)   // pieces swizzled by the row: neighbouring lanes meet different banks
+            prow[((c * 8 + i) ^ r) & c4mask] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]),
+                                                          __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
+        }
+        reinterpret_cast<float2*>(smem + AttSmem::kV)[r] = make_float2(m_ref, l);
+      }
     // ---- epilogue: O / l -> element type -> staging (the Q tile is no longer needed) -> TMA store ----
-    if (ok && mbar_wait(pv_done, (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+    } else if (ok && mbar_wait(pv_done, (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
       tc_fence_after();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
       uint8_t* stg = smem + AttSmem::kQ + wq * (2 * 32 * 128);   // per warp: Dv/64 tiles of 32 rows x 128 bytes
@@ -383,6 +451,40 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     }
   }
 
+  if (splits > 1) {
+    // O = sum over the parts of 2^(m_part - m) O_part, divided by the same sum of the l_part; every CTA of the cluster
+    // does a share of the row pieces, reading the others' shared memory
+    cluster_sync();
+    const int pieces = p.Dv / 4, rows = min(kQT, p.Sq - q0);
+    const int used = (nb_all + per_part - 1) / per_part;   // parts that had a key block
+    for (int i = part * kAttThreads + (int)threadIdx.x; i < rows * pieces; i += splits * kAttThreads) {
+      const int r = i / pieces, c4 = i - r * pieces;
+      const uint32_t ml_addr = smem_u32(smem + AttSmem::kV) + r * 8;
+      const uint32_t o_addr = smem_u32(smem + AttSmem::kK) + (r * pieces + ((c4 ^ r) & (pieces - 1))) * 16;
+      float2 ml[kMaxSplits];
+      float m = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kMaxSplits; ++s)
+        if (s < used) { ml[s] = ld_cluster_f2(mapa_u32(ml_addr, s)); m = fmaxf(m, ml[s].x); }
+      const float m_use = m == -INFINITY ? 0.0f : m;
+      float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float l = 0.0f;
+#pragma unroll
+      for (int s = 0; s < kMaxSplits; ++s)
+        if (s < used) {
+          const float w = ex2(ml[s].x - m_use);
+          const float4 x = ld_cluster_f4(mapa_u32(o_addr, s));
+          l += w * ml[s].y;
+          o.x += w * x.x; o.y += w * x.y; o.z += w * x.z; o.w += w * x.w;
+        }
+      const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
+      if (c4 * 4 < p.o_cols)   // head dimensions are multiples of 8
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.o) + ((long long)g * p.Sq + q0 + r) * p.o_cols + c4 * 4) =
+            make_uint2(pack2(o.x * inv, o.y * inv, p.is_bf16), pack2(o.z * inv, o.w * inv, p.is_bf16));
+    }
+    cluster_sync();   // nobody leaves while its shared memory is being read
+  }
+
   tc_fence_before();
   __syncthreads();
   if (warp == 2) {
@@ -390,6 +492,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     tmem_dealloc<1>(tmem_base, 512);
   }
 }
+
 
 // ---------------------------------------------------------------------------------------------------------------
 // Two query tiles per CTA. One softmax group alone leaves the tensor pipe idle while it works: P_j.V_j has to wait
@@ -1117,6 +1220,20 @@ RbStatus gemm_gemm_on_chip(int32_t g, int32_t m, int32_t k1, int32_t n1, int32_t
 }
 }  // namespace rb
 
+namespace rb {
+// Key-block parts of the single-tile kernel. One CTA per query tile leaves most of the GPU idle when there are few tiles
+// (a generation step over 64 heads: 64 CTAs), and every tile then pays its whole chain of key blocks alone: 64 heads x 1
+// query x 4096 keys with a mask took 1005 us that way, 64 us with two parts per tile and the mask read as words.
+static int attention_splits(const RbAttentionProblem* p, long long ctas, int sms) {
+  if (t_attention_linear) return 1;
+  int blocks = (p->seq_k + kKT - 1) / kKT;
+  if (p->causal) blocks = std::min(blocks, (p->seq_q + kKT - 1) / kKT);   // the blocks of the longest tile
+  int splits = 1;
+  while (splits < kMaxSplits && ctas * splits * 2 <= sms && splits * 2 <= blocks) splits *= 2;
+  return splits;
+}
+}  // namespace rb
+
 static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, const void* k, const void* v, void* o,
                                   void* workspace, size_t workspace_bytes, bool own_scratch, void* stream_v) {
   if (!p) return fail(RB_INVALID_PARAM, "problem is NULL");
@@ -1256,7 +1373,25 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
     attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
   } else {
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd_kernel), AttSmem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
-    attention_fwd_kernel<<<(unsigned)ctas, kAttThreads, AttSmem::kTotal, stream>>>(maps, kp);
+    kp.splits = attention_splits(p, ctas, dev->sm_count);
+    kp.o = o;
+    kp.o_cols = p->head_v;
+    if (kp.splits == 1) {
+      attention_fwd_kernel<<<(unsigned)ctas, kAttThreads, AttSmem::kTotal, stream>>>(maps, kp);
+    } else {
+      cudaLaunchConfig_t lc;
+      memset(&lc, 0, sizeof(lc));
+      lc.gridDim = dim3((unsigned)(ctas * kp.splits), 1, 1);
+      lc.blockDim = dim3(kAttThreads, 1, 1);
+      lc.dynamicSmemBytes = AttSmem::kTotal;
+      lc.stream = stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)kp.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      lc.attrs = attr;
+      lc.numAttrs = 1;
+      RB_CUDA_TRY(cudaLaunchKernelEx(&lc, attention_fwd_kernel, maps, kp));
+    }
   }
   RB_CUDA_TRY(cudaGetLastError());
   count_launch();
