@@ -229,30 +229,32 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
           } else {
             tmem_ld_wait();
           }
-          if (!valid) continue;
-          if constexpr (F32) {
-            float* dst = static_cast<float*>(p.out) + pix + (long long)c * o_k;
-            if (o_k == 1) {   // channels last: 128 contiguous bytes per thread
+          if (valid) {
+            if constexpr (F32) {
+              float* dst = static_cast<float*>(p.out) + pix + (long long)c * o_k;
+              if (o_k == 1) {   // channels last: 128 contiguous bytes per thread
 #pragma unroll
-              for (int i = 0; i < 8; ++i)
-                reinterpret_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            } else {          // channel planes (NKHW): neighbouring lanes are neighbouring pixels of a plane
+                for (int i = 0; i < 8; ++i)
+                  reinterpret_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+              } else {          // channel planes (NKHW): neighbouring lanes are neighbouring pixels of a plane
 #pragma unroll
-              for (int j = 0; j < 32; ++j) dst[(long long)j * o_k] = __uint_as_float(v[j]);
+                for (int j = 0; j < 32; ++j) dst[(long long)j * o_k] = __uint_as_float(v[j]);
+              }
+            } else {
+              uint32_t h[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float lo = __uint_as_float(v[2 * j]), hi = __uint_as_float(v[2 * j + 1]);
+                if (is_bf16) { __nv_bfloat162 t2 = __floats2bfloat162_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
+                else { __half2 t2 = __floats2half2_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
+              }
+              uint8_t* dst = static_cast<uint8_t*>(p.out) + 2 * (pix + c);
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(dst + i * 16) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
             }
-          } else {
-            uint32_t h[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float lo = __uint_as_float(v[2 * j]), hi = __uint_as_float(v[2 * j + 1]);
-              if (is_bf16) { __nv_bfloat162 t2 = __floats2bfloat162_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
-              else { __half2 t2 = __floats2half2_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
-            }
-            uint8_t* dst = static_cast<uint8_t*>(p.out) + 2 * (pix + c);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              *reinterpret_cast<uint4*>(dst + i * 16) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
           }
+          __syncwarp();   // the warp is whole again before its next collective load from tensor memory
         }
       }
       tc_fence_before();
@@ -313,6 +315,10 @@ bool stream_shape(const HaloConv& c, int elem_bytes, long long o_k, StreamShape*
 }  // namespace
 
 bool conv_halo_stream_applicable(const HaloConv& c, int elem_bytes, long long o_k) {
+  // One tap has no halo to share, and two launches of this pipeline with a single tap per window ended in a launch failure (an
+  // f32 pointwise layer, 44 images of 128 x 52 x 52 to 128 channels; a strided form whose phase images had one tap each): the
+  // GEMM kernel takes those.
+  if (c.Y * c.X == 1) return false;
   // f32: the whole reduction of a pixel is ONE accumulation chain in TMEM, and the tensor core adds with truncation (a
   // bias that grows with the chain, csrc/gemm_sm100.cu choose_config). Chains stay at 1024 elements here, half of
   // what the GEMM kernel allows itself, since this kernel cannot cut a chain into K ranges.
