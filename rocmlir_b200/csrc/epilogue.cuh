@@ -43,6 +43,42 @@ __device__ __forceinline__ float round_to_type(float x, int t) {
   return x;
 }
 
+// N accumulators rounded to a 16-bit type and back, two per conversion, the type looked at once for all of them (a branch
+// and a one-element conversion per value took a third of a fused epilogue's time).
+template <int N>
+__device__ __forceinline__ void round_row(uint32_t* v, int t) {
+  if (t == RB_F16) {
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+      const float2 f = __half22float2(__floats2half2_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
+      v[j] = __float_as_uint(f.x); v[j + 1] = __float_as_uint(f.y);
+    }
+  } else if (t == RB_BF16) {
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+      const float2 f = __bfloat1622float2(__floats2bfloat162_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
+      v[j] = __float_as_uint(f.x); v[j + 1] = __float_as_uint(f.y);
+    }
+  }
+}
+// N accumulators as N / 2 words of a 16-bit type.
+template <int N>
+__device__ __forceinline__ void pack_row16(const uint32_t* v, uint32_t* h, bool to_bf16) {
+  if (to_bf16) {
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+      h[j] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) {
+      const __half2 b = __floats2half2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+      h[j] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+  }
+}
+
 // The MIGraphX unary elementwise ops in f32 (MIGraphX.td:134-181). sigmoid = 1 / (1 + exp(-x)) as
 // MIGraphXToTosa lowers it; recip and rsqrt are correctly rounded divisions / square roots, not the approximate forms.
 __device__ __forceinline__ float epi_unary(float x, int op) {

@@ -272,10 +272,7 @@ static __device__ __noinline__ uint32_t epi_fused16_tile(const EpiStoreCtx c, ui
     }
     __syncwarp();
     tmem_ld_wait();
-    if (f_mid) {
-#pragma unroll
-      for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(round_to_type(__uint_as_float(v[j]), mid_type));
-    }
+    if (f_mid) round_row<64>(v, mid_type);
     if (f_alpha) {
 #pragma unroll
       for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(__fmul_rn(__uint_as_float(v[j]), alpha));
@@ -290,27 +287,18 @@ static __device__ __noinline__ uint32_t epi_fused16_tile(const EpiStoreCtx c, ui
         v[j + 2] = __float_as_uint(__fadd_rn(__uint_as_float(v[j + 2]), b4.z));
         v[j + 3] = __float_as_uint(__fadd_rn(__uint_as_float(v[j + 3]), b4.w));
       }
-      if (f_mid) {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(round_to_type(__uint_as_float(v[j]), mid_type));
-      }
+      if (f_mid) round_row<64>(v, mid_type);
     }
     if (f_relu) {
 #pragma unroll
       for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
     }
     uint8_t* rowp = stg + c.lane * kRowBytes;
+    uint32_t h[32];
+    pack_row16<64>(v, h, c_type == RB_BF16);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      uint32_t h[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float lo = __uint_as_float(v[8 * i + 2 * j]), hi = __uint_as_float(v[8 * i + 2 * j + 1]);
-        if (c_type == RB_F16) { __half2 t2 = __floats2half2_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
-        else { __nv_bfloat162 t2 = __floats2bfloat162_rn(lo, hi); h[j] = *reinterpret_cast<uint32_t*>(&t2); }
-      }
-      *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
-    }
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
     fence_proxy_async();
     __syncwarp();
     if (c.lane == 0 && c.row0 < c.M) {
