@@ -88,6 +88,8 @@ gemm_skinny_kernel(const __grid_constant__ SkinnyMaps maps, const SkinnyParams p
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_launch();
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   uint32_t* part_smem = reinterpret_cast<uint32_t*>(smem);   // [nt][128] accumulators of this part, after the main loop
   bool ok = true;
@@ -128,6 +130,7 @@ gemm_skinny_kernel(const __grid_constant__ SkinnyMaps maps, const SkinnyParams p
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
       for (int m0 = 0; m0 < p.nt; m0 += 16) {
         if (m0 >= p.M) break;
+        __syncwarp();   // collective load: the lanes parted at the last stores
         uint32_t v[16];
         tmem_ld16(taddr + m0, v);
         tmem_ld_wait();
@@ -248,12 +251,15 @@ RbStatus gemm_skinny_run(const RbGemmProblem* p, const EpiParams& epi, const voi
   lc.blockDim = dim3(kSkinnyThreads, 1, 1);
   lc.dynamicSmemBytes = (size_t)smem;
   lc.stream = static_cast<cudaStream_t>(stream_v);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  lc.attrs = attr;
+  attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+  ++lc.numAttrs;
   if (kp.splits > 1) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)kp.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
+    attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[lc.numAttrs].val.clusterDim.x = (unsigned)kp.splits; attr[lc.numAttrs].val.clusterDim.y = 1; attr[lc.numAttrs].val.clusterDim.z = 1;
+    ++lc.numAttrs;
   }
   RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
   count_launch();

@@ -67,6 +67,7 @@ __device__ __forceinline__ uint4 load_row16(const uint8_t* row, unsigned at, uns
 // One 16-byte vector of the destination per thread and step: bound by the one read and one write of the operand. (A byte
 // per thread with a 64-bit division each used to take 20 times as long as the loads and stores need.)
 __global__ void pad_rows_kernel(const PadJobs p) {
+  griddep_launch();   // the product is set up meanwhile
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < p.first[2];
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const bool second = i >= p.first[1];
@@ -123,6 +124,7 @@ __device__ __forceinline__ void store_planes4(const F32Job& j, long long o, cons
 __global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p) {
   __shared__ float tile[64][65];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
+  griddep_launch();   // the product is set up meanwhile
   for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
     const bool second = t >= p.first[1];
     const F32Job j = second ? p.job[1] : p.job[0];
@@ -888,8 +890,11 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   lc.blockDim = dim3(kGemmThreads, 1, 1);
   lc.dynamicSmemBytes = (size_t)smem;
   lc.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   lc.attrs = attr;
+  attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+  ++lc.numAttrs;
   if (ctas == 2) {
     attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
     attr[lc.numAttrs].val.clusterDim.x = 2; attr[lc.numAttrs].val.clusterDim.y = 1; attr[lc.numAttrs].val.clusterDim.z = 1;

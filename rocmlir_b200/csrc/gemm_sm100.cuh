@@ -432,6 +432,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   if constexpr (CTAS == 2) cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------

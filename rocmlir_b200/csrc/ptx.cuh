@@ -42,6 +42,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch. A kernel launched with the stream-serialisation attribute may be set up (barriers, tensor
+// memory, descriptor fetches) while its predecessor in the stream still runs; griddep_wait returns when that predecessor has
+// completed and its writes are visible, and comes before the first access to global memory. griddep_launch lets the successor
+// start that early. Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
