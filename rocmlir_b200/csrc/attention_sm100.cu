@@ -127,8 +127,10 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   uint64_t* v_empty = v_full + NS;         // [NS]
   uint64_t* s_full = v_empty + NS;         // [2]
   uint64_t* p_full = s_full + 2;
+  // [2], by block parity: a softmax warp may be done with block j while the product of block j - 1 still waits for its V
+  // tile, and on one barrier the parity of j would then read as complete
   uint64_t* pv_done = p_full + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 1);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = lane_id();
@@ -158,7 +160,8 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
     mbar_init(p_full, live_warps);
-    mbar_init(pv_done, 1);
+    mbar_init(&pv_done[0], 1);
+    mbar_init(&pv_done[1], 1);
     fence_mbar_init();
   }
   if (warp == 2) {
@@ -244,7 +247,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
           const uint32_t b_lo = smem_desc_lo(v_addr + kk * 2048, kKT * 128);
           umma_ts<kKindF16>(tmem_o, tmem_p + kk * 8, desc64(b_lo, hi), p.idesc_pv, (j | kk) ? 1u : 0u);
         }
-        tc_commit<1>(pv_done);
+        tc_commit<1>(&pv_done[j & 1]);
         tc_commit<1>(&v_empty[vs_stage]);
         if (++vs_stage == NS) { vs_stage = 0; vs_par ^= 1u; }
       }
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       tmem_st32(tmem_s + 32, v + 32);
       // rescale O where a reference maximum moved (whole warp takes part: TMEM access is warp-collective)
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-        if (!mbar_wait(pv_done, (uint32_t)(j - 1) & 1u, p.status, kStatusTimeoutEpilogue + 4)) { ok = false; break; }
+        if (!mbar_wait(&pv_done[(j - 1) & 1], (uint32_t)((j - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 4)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < p.Dv / 32; ++c) {
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     if (splits > 1) {
       // this CTA's share of the row, not divided by its sum: O, reference maximum and sum go to shared memory (the key
       // ring is idle by now) for the cluster to add up below
-      if (nb > 0 && ok && mbar_wait(pv_done, (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+      if (nb > 0 && ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
         tc_fence_after();
         const int c4mask = p.Dv / 4 - 1;   // Dv is 64 or 128
         float4* prow = reinterpret_cast<float4*>(smem + AttSmem::kK) + r * (p.Dv / 4);
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         reinterpret_cast<float2*>(smem + AttSmem::kV)[r] = make_float2(m_ref, l);
       }
     // ---- epilogue: O / l -> element type -> staging (the Q tile is no longer needed) -> TMA store ----
-    } else if (ok && mbar_wait(pv_done, (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+    } else if (ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
       tc_fence_after();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
       uint8_t* stg = smem + AttSmem::kQ + wq * (2 * 32 * 128);   // per warp: Dv/64 tiles of 32 rows x 128 bytes
