@@ -106,6 +106,11 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
   asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ float ld_cluster_f1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -496,6 +501,337 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   }
 }
 
+
+// ---------------------------------------------------------------------------------------------------------------
+// At most four queries (a generation step). The single-tile kernel above gives every query a TMEM lane, so one query is one
+// lane of one warp: that warp alone computes 128 scores per key block, one after the other, and is what the block waits for
+// (8400 cycles a block with a mask; a block of keys and values needs 2800 to arrive from HBM). Here the score tile is turned
+// round: S^T = K . Q^T has the keys on its 128 lanes and the queries, padded to 16, on its columns, so each of 128 threads
+// has one key and as many exponentials as there are queries. P^T goes to shared memory as the N x K operand of
+// O^T = V^T . P^T, whose lanes are the columns of V. The row maximum needs one reduction over the four warps per block
+// (a warp maximum per query, exchanged through shared memory); the row sum is kept per thread and added up at the end.
+// Keys are divided over a cluster like above. Bound: reading K and V once. 64 heads x 1 query x 4096 keys, D = 128, masked: 57 us
+// on the single-tile kernel, 28 here. A query costs every thread some 45 instructions per block, so with more than a
+// few the single-tile kernel is the faster one again (10 queries, 429 heads x 3550 keys, D = 64: 113 us there, 183 with all
+// 16 columns computed here).
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int kNQ = 16;              // query columns of the products
+constexpr int kDecodeQ = 4;          // queries that are computed at most
+constexpr int kDecodeThreads = 192;  // producer, MMA issuer (and TMEM), four softmax warps
+
+struct DecodeSmem {
+  static constexpr int kStages = 3;
+  static constexpr int kPBytes = kNQ * 256;     // P^T of one block: two 64-key atoms of 16 rows x 128 bytes
+  // [Q][2 x P][warp maxima 2 x 4 x 16][warp sums 4 x 16][m, l][K ring][V ring][barriers]; the partial O of a part overlays Q / P
+  static constexpr int kQ = 0;
+  static constexpr int kP = kQ + kNQ * 256;
+  static constexpr int kMax = kP + 2 * kPBytes;
+  static constexpr int kSum = kMax + 2 * 4 * kNQ * 4;
+  static constexpr int kMl = kSum + 4 * kNQ * 4;
+  static constexpr int kBars = kMl + kNQ * 8;
+  static constexpr int kRing = 14336;           // 1024-byte aligned
+  static_assert(kBars + 256 <= kRing, "");
+  static constexpr int total(int Dp, int Dvp) { return kRing + kStages * kKT * 2 * (Dp + Dvp) + 1024; }
+};
+
+__device__ __forceinline__ float warp_max(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// NQT: queries computed, 1 or up to kDecodeQ
+template <int NQT>
+__global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(const __grid_constant__ AttMaps maps, const AttParams p) {
+  constexpr int NS = DecodeSmem::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + DecodeSmem::kBars);
+  uint64_t* k_full = q_full + 1;           // [NS]
+  uint64_t* k_empty = k_full + NS;         // [NS]
+  uint64_t* v_full = k_empty + NS;         // [NS]
+  uint64_t* v_empty = v_full + NS;         // [NS]
+  uint64_t* s_full = v_empty + NS;         // [2]
+  uint64_t* p_full = s_full + 2;           // [2]
+  uint64_t* pv_done = p_full + 2;          // [2]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint8_t* k_ring = smem + DecodeSmem::kRing;
+  uint8_t* v_ring = k_ring + NS * kKT * 2 * p.D;
+
+  const int warp = threadIdx.x >> 5, lane = lane_id();
+  const int splits = p.splits;
+  const int part = splits > 1 ? (int)cluster_ctarank() : 0;
+  const int g = blockIdx.x / splits;
+  int nb_all = (p.Sk + kKT - 1) / kKT;
+  if (p.causal) nb_all = min(nb_all, (p.Sq - 1) / kKT + 1);
+  const int per_part = (nb_all + splits - 1) / splits;
+  const int j0 = min(part * per_part, nb_all), nb = min(per_part, nb_all - j0);   // key blocks j0 .. j0 + nb - 1 (maybe none)
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int i = 0; i < NS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&pv_done[i], 1); }
+    fence_mbar_init();
+    prefetch_tmap(&maps.q);
+    prefetch_tmap(&maps.k);
+    prefetch_tmap(&maps.v);
+  }
+  if (warp == 1) {
+    tmem_alloc<1>(tmem_holder, 64);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  const uint32_t tmem_o = tmem_base + 32;   // scores of two blocks at columns 0 and 16, O^T at 32
+
+  const int d_atoms = p.D / 64, dv_chunks = p.Dv / 64;
+  const uint32_t k_bytes = (uint32_t)kKT * p.D * 2, v_bytes = (uint32_t)kKT * p.Dv * 2;
+
+  if (warp == 0) {
+    // ------------------------------ producer ------------------------------
+    if (lane == 0 && nb > 0) {
+      mbar_expect_tx(q_full, (uint32_t)kNQ * p.D * 2);
+      for (int a = 0; a < d_atoms; ++a) tma_load_3d(smem + DecodeSmem::kQ + a * (kNQ * 128), &maps.q, q_full, a * 64, 0, g);
+      int s = 0;
+      uint32_t par = 0;
+      for (int j = 0; j < nb; ++j) {
+        const int key0 = (j0 + j) * kKT;
+        if (!mbar_wait(&k_empty[s], par ^ 1u, p.status, kStatusTimeoutProducer + s)) break;
+        uint8_t* ks = k_ring + s * k_bytes;
+        mbar_expect_tx(&k_full[s], k_bytes);
+        if (p.trans_k) {
+          for (int a = 0; a < d_atoms; ++a) tma_load_3d(ks + a * (kKT * 128), &maps.k, &k_full[s], a * 64, key0, g);
+        } else {
+          for (int c = 0; c < kKT / 64; ++c) tma_load_3d(ks + c * (p.D * 128), &maps.k, &k_full[s], key0 + c * 64, 0, g);
+        }
+        if (!mbar_wait(&v_empty[s], par ^ 1u, p.status, kStatusTimeoutProducer + 4 + s)) break;
+        uint8_t* vs = v_ring + s * v_bytes;
+        mbar_expect_tx(&v_full[s], v_bytes);
+        for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, key0, g);
+        if (++s == NS) { s = 0; par ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer ------------------------------
+    if (lane == 0 && nb > 0) {
+      const uint32_t hi = smem_desc_hi(1024);
+      const uint32_t q_lo = smem_desc_lo(smem_u32(smem + DecodeSmem::kQ), 16);
+      const int ksteps = p.D / 16;
+      const bool trans_k = p.trans_k != 0;
+      const uint32_t idesc_s = p.idesc_s, idesc_pv = p.idesc_pv;
+      const uint32_t k_lo0 = smem_desc_lo(smem_u32(k_ring), trans_k ? 16u : (uint32_t)p.D * 128);
+      // V^T: MN-major, 64 columns of V per chunk; with 64 columns in all the second half of the 128 rows repeats the first
+      const uint32_t v_lo0 = smem_desc_lo(smem_u32(v_ring), dv_chunks == 2 ? kKT * 128 : 0);
+      const uint32_t p_lo0 = smem_desc_lo(smem_u32(smem + DecodeSmem::kP), 16);
+      int ks = 0, vs = 0;
+      uint32_t kpar = 0, vpar = 0;
+      auto issue_s = [&](int j) -> bool {
+        if (!mbar_wait(&k_full[ks], kpar, p.status, kStatusTimeoutMma + ks)) return false;
+        // (descriptors: a base per tile plus compile-time offsets; the issuing thread has some 2400 cycles per block)
+        const uint32_t a_lo = k_lo0 + ks * (k_bytes >> 4), d = tmem_base + (j & 1) * kNQ;
+        if (trans_k) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            if (kk < ksteps)
+              umma_ss<kKindF16, 1>(d, desc64(a_lo + (((kk >> 2) * (kKT * 128) + (kk & 3) * 32) >> 4), hi),
+                                   desc64(q_lo + (((kk >> 2) * (kNQ * 128) + (kk & 3) * 32) >> 4), hi), idesc_s, kk ? 1u : 0u);
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            if (kk < ksteps)
+              umma_ss<kKindF16, 1>(d, desc64(a_lo + ((kk * 2048) >> 4), hi),
+                                   desc64(q_lo + (((kk >> 2) * (kNQ * 128) + (kk & 3) * 32) >> 4), hi), idesc_s, kk ? 1u : 0u);
+        }
+        tc_commit<1>(&s_full[j & 1]);
+        tc_commit<1>(&k_empty[ks]);
+        if (++ks == NS) { ks = 0; kpar ^= 1u; }
+        return true;
+      };
+      bool ok = mbar_wait(q_full, 0, p.status, kStatusTimeoutMma + 8);
+      if (ok) ok = issue_s(0);
+      for (int j = 0; j < nb && ok; ++j) {
+        // the scores of block j - 1, in the buffer that S(j + 1) overwrites, were read before P(j - 1) was announced
+        if (j + 1 < nb) ok = issue_s(j + 1);
+        if (!ok) break;
+        if (!mbar_wait(&v_full[vs], vpar, p.status, kStatusTimeoutMma + 10 + vs)) break;
+        if (!mbar_wait(&p_full[j & 1], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutMma + 20)) break;
+        tc_fence_after();
+        const uint32_t a_lo = v_lo0 + vs * (v_bytes >> 4), b_lo = p_lo0 + (j & 1) * (DecodeSmem::kPBytes >> 4);
+#pragma unroll
+        for (int kk = 0; kk < kKT / 16; ++kk)
+          umma_ss<kKindF16, 1>(tmem_o, desc64(a_lo + ((kk * 2048) >> 4), hi), desc64(b_lo + (((kk >> 2) * (kNQ * 128) + (kk & 3) * 32) >> 4), hi),
+                               idesc_pv, (j | kk) ? 1u : 0u);
+        tc_commit<1>(&pv_done[j & 1]);
+        tc_commit<1>(&v_empty[vs]);
+        if (++vs == NS) { vs = 0; vpar ^= 1u; }
+      }
+    }
+  } else {
+    // ------------------------------ softmax / correction / epilogue ------------------------------
+    const int wq = warp & 3;
+    const int kk = wq * 32 + lane;         // key of the block, and column of V, of this thread (TMEM lane)
+    const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
+    const int Sq = p.Sq;
+    float* wmax = reinterpret_cast<float*>(smem + DecodeSmem::kMax);
+    float* wsum = reinterpret_cast<float*>(smem + DecodeSmem::kSum);
+    // this thread's column of P^T: 16-byte pieces of a row swizzled by the row
+    uint8_t* p_col = smem + DecodeSmem::kP + (kk >> 6) * (kNQ * 128) + (kk & 7) * 2;
+    const int piece = (kk & 63) >> 3;
+    const long long side_g = (long long)g * Sq * p.Sk;
+    float m_ref[NQT], l[NQT];
+#pragma unroll
+    for (int q = 0; q < NQT; ++q) { m_ref[q] = -INFINITY; l[q] = 0.0f; }
+    bool ok = true;
+    // mask byte of every query for the key of the next block, as loaded: read a block ahead and looked at then, because the
+    // latency of a load from HBM is as long as the rest of a block's work here
+    int mask_next[NQT];
+    auto load_mask = [&](int j) {
+      const int key = (j0 + j) * kKT + kk;
+      const bool in = p.mask != nullptr && j < nb && key < p.Sk;
+#pragma unroll
+      for (int q = 0; q < NQT; ++q) {
+        mask_next[q] = 1;
+        if (in && q < Sq) mask_next[q] = __ldg(p.mask + side_g + (long long)q * p.Sk + key);
+      }
+    };
+    load_mask(0);
+    // (after a wait ran out the loop goes on without waiting: the four warps meet at a barrier in every step)
+    for (int j = 0; j < nb; ++j) {
+      const int key = (j0 + j) * kKT + kk;
+      int mask_now[NQT];
+#pragma unroll
+      for (int q = 0; q < NQT; ++q) mask_now[q] = mask_next[q];
+      load_mask(j + 1);
+      // P of block j - 2 has been read
+      if (ok && j >= 2) ok = mbar_wait_warp(&pv_done[j & 1], (uint32_t)((j >> 1) - 1) & 1u, p.status, kStatusTimeoutEpilogue + 2);
+      if (ok) ok = mbar_wait_warp(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutEpilogue + (j & 1));
+      tc_fence_after();
+      uint32_t v[kNQ];
+      tmem_ld16(tmem_base + lane_base + (j & 1) * kNQ, v);
+      tmem_ld_wait();
+      float* wm = wmax + (j & 1) * (4 * kNQ);
+#pragma unroll
+      for (int q = 0; q < NQT; ++q) {
+        if (q < Sq) {   // f(S) in the log2 domain: the steps of the kernels above
+          float x = __uint_as_float(v[q]) * p.scale_log2;
+          if (key < p.Sk) {
+            const long long side = side_g + (long long)q * p.Sk + key;
+            if (p.scale_t) x *= load_elem(p.scale_t, side, p.is_bf16);
+            if (p.bias) x = fmaf(load_elem(p.bias, side, p.is_bf16), kLog2e, x);
+            if (mask_now[q] == 0) x = p.mask_fill * kLog2e;
+            if (p.causal && key > q) x = -INFINITY;
+          } else {
+            x = -INFINITY;
+          }
+          v[q] = __float_as_uint(x);
+          const float mw = warp_max(x);
+          if (lane == 0) wm[wq * kNQ + q] = mw;
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the four softmax warps (every one comes here, also after a wait ran out)
+      bool moved = false;
+      float alpha[NQT];
+      uint8_t* pc = p_col + (j & 1) * DecodeSmem::kPBytes;
+#pragma unroll
+      for (int q = 0; q < NQT; ++q) {
+        alpha[q] = 1.0f;
+        if (q < Sq) {
+          const float mx = fmaxf(fmaxf(wm[q], wm[kNQ + q]), fmaxf(wm[2 * kNQ + q], wm[3 * kNQ + q]));
+          if (mx > m_ref[q] + 8.0f || (m_ref[q] == -INFINITY && mx > -INFINITY)) {   // the same in all 128 threads
+            alpha[q] = ex2(m_ref[q] - mx);
+            m_ref[q] = mx;
+            moved = true;
+          }
+          const float e = ex2(__uint_as_float(v[q]) - (m_ref[q] == -INFINITY ? 0.0f : m_ref[q]));
+          l[q] = l[q] * alpha[q] + e;
+          *reinterpret_cast<uint16_t*>(pc + q * 128 + ((piece ^ (q & 7)) << 4)) = (uint16_t)pack2(e, 0.0f, p.is_bf16);
+        }
+      }
+      if (moved && j > 0) {   // rescale O, whose products up to block j - 1 are complete
+        if (ok) ok = mbar_wait_warp(&pv_done[(j - 1) & 1], (uint32_t)((j - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 4);
+        tc_fence_after();
+        uint32_t o[kNQ];
+        tmem_ld16(tmem_o + lane_base, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < NQT; ++q) o[q] = __float_as_uint(__uint_as_float(o[q]) * alpha[q]);
+        tmem_st16(tmem_o + lane_base, o);
+        tmem_st_wait();
+      }
+      fence_proxy_async();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
+    }
+    // row sums over the 128 keys of the lanes
+#pragma unroll
+    for (int q = 0; q < NQT; ++q) {
+      if (q < Sq) {
+        float s = l[q];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) wsum[wq * kNQ + q] = s;
+      }
+    }
+    if (ok && nb > 0) ok = mbar_wait_warp(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5);
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (nb > 0) {
+      tc_fence_after();
+      uint32_t o[kNQ];
+      tmem_ld16(tmem_o + lane_base, o);
+      tmem_ld_wait();
+      float* part_o = reinterpret_cast<float*>(smem);   // [Sq][Dv] over Q and P: every product that reads them is complete
+#pragma unroll
+      for (int q = 0; q < NQT; ++q) {
+        if (q < Sq && kk < p.Dv) {
+          const float sum = (wsum[q] + wsum[kNQ + q]) + (wsum[2 * kNQ + q] + wsum[3 * kNQ + q]);
+          if (splits > 1) {
+            part_o[q * p.Dv + kk] = __uint_as_float(o[q]);
+            if (kk == 0) reinterpret_cast<float2*>(smem + DecodeSmem::kMl)[q] = make_float2(m_ref[q], sum);
+          } else if (kk < p.o_cols) {
+            const float inv = (sum > 0.0f) ? 1.0f / sum : 0.0f;
+            static_cast<uint16_t*>(p.o)[((long long)g * Sq + q) * p.o_cols + kk] = (uint16_t)pack2(__uint_as_float(o[q]) * inv, 0.0f, p.is_bf16);
+          }
+        }
+      }
+    }
+  }
+  if (splits > 1) {
+    // the same sum over the parts as in the single-tile kernel, one element of O per thread and step
+    cluster_sync();
+    const int used = (nb_all + per_part - 1) / per_part;   // parts that had a key block
+    for (int i = part * kDecodeThreads + (int)threadIdx.x; i < p.Sq * p.o_cols; i += splits * kDecodeThreads) {
+      const int q = i / p.o_cols, c = i - q * p.o_cols;
+      const uint32_t ml_addr = smem_u32(smem + DecodeSmem::kMl) + q * 8, o_addr = smem_u32(smem) + (q * p.Dv + c) * 4;
+      float2 ml[kMaxSplits];
+      float ov[kMaxSplits];
+      float m = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kMaxSplits; ++s)
+        if (s < used) { ml[s] = ld_cluster_f2(mapa_u32(ml_addr, s)); ov[s] = ld_cluster_f1(mapa_u32(o_addr, s)); m = fmaxf(m, ml[s].x); }
+      const float m_use = m == -INFINITY ? 0.0f : m;
+      float o = 0.0f, sum = 0.0f;
+#pragma unroll
+      for (int s = 0; s < kMaxSplits; ++s)
+        if (s < used) {
+          const float w = ex2(ml[s].x - m_use);
+          sum += w * ml[s].y;
+          o += w * ov[s];
+        }
+      const float inv = (sum > 0.0f) ? 1.0f / sum : 0.0f;
+      static_cast<uint16_t*>(p.o)[((long long)g * p.Sq + q) * p.o_cols + c] = (uint16_t)pack2(o * inv, 0.0f, p.is_bf16);
+    }
+    cluster_sync();   // nobody leaves while its shared memory is being read
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem_base, 64);
+  }
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // Two query tiles per CTA. One softmax group alone leaves the tensor pipe idle while it works: P_j.V_j has to wait
@@ -1231,8 +1567,14 @@ static int attention_splits(const RbAttentionProblem* p, long long ctas, int sms
   if (t_attention_linear) return 1;
   int blocks = (p->seq_k + kKT - 1) / kKT;
   if (p->causal) blocks = std::min(blocks, (p->seq_q + kKT - 1) / kKT);   // the blocks of the longest tile
+  // rounds of CTAs x blocks of one, a CTA's start and end costing about as much as three blocks and the cluster's
+  // two meetings another two
   int splits = 1;
-  while (splits < kMaxSplits && ctas * splits * 2 <= sms && splits * 2 <= blocks) splits *= 2;
+  long long best = -1;
+  for (int s = 1; s <= kMaxSplits && s <= blocks; s *= 2) {
+    const long long cost = (ctas * s + sms - 1) / sms * ((blocks + s - 1) / s + (s > 1 ? 5 : 3));
+    if (best < 0 || cost < best) { best = cost; splits = s; }
+  }
   return splits;
 }
 }  // namespace rb
@@ -1375,25 +1717,37 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd2_kernel), Att2Smem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
     attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
   } else {
-    if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd_kernel), AttSmem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
+    // at most four queries: the score tile turned round (attention_decode_kernel)
+    const bool few = p->seq_q <= kDecodeQ && !quantized && !kp.linear;
+    if (few) {
+      kp.idesc_s = make_idesc(1, fmt, fmt, p->trans_k ? 0u : 1u, 0u, kKT, kNQ);
+      kp.idesc_pv = make_idesc(1, fmt, fmt, 1u, 0u, 128, kNQ);
+      const uint64_t dims[3] = {D, Sq, G};
+      const uint64_t str[2] = {D * 2, Sq * D * 2};
+      const uint32_t box[3] = {64, (uint32_t)kNQ, 1};
+      if (!encode_tiled(&maps.q, dt, 3, q, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, &err)) return fail(RB_UNSUPPORTED, "Q: " + err);
+    }
+    void (*const kern)(const AttMaps, const AttParams) = !few ? attention_fwd_kernel : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
+    const int threads = few ? kDecodeThreads : kAttThreads, smem = few ? DecodeSmem::total((int)Dp, (int)Dvp) : AttSmem::kTotal;
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != RB_SUCCESS) return RB_CUDA_ERROR;
     kp.splits = attention_splits(p, ctas, dev->sm_count);
     kp.o = o;
     kp.o_cols = p->head_v;
     if (kp.splits == 1) {
-      attention_fwd_kernel<<<(unsigned)ctas, kAttThreads, AttSmem::kTotal, stream>>>(maps, kp);
+      kern<<<(unsigned)ctas, threads, smem, stream>>>(maps, kp);
     } else {
       cudaLaunchConfig_t lc;
       memset(&lc, 0, sizeof(lc));
       lc.gridDim = dim3((unsigned)(ctas * kp.splits), 1, 1);
-      lc.blockDim = dim3(kAttThreads, 1, 1);
-      lc.dynamicSmemBytes = AttSmem::kTotal;
+      lc.blockDim = dim3((unsigned)threads, 1, 1);
+      lc.dynamicSmemBytes = (size_t)smem;
       lc.stream = stream;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = (unsigned)kp.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
       lc.attrs = attr;
       lc.numAttrs = 1;
-      RB_CUDA_TRY(cudaLaunchKernelEx(&lc, attention_fwd_kernel, maps, kp));
+      RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
     }
   }
   RB_CUDA_TRY(cudaGetLastError());
