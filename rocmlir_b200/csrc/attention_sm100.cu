@@ -119,6 +119,10 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 
 __device__ __forceinline__ float f16_round(float x) { return __half2float(__float2half_rn(x)); }
 
+// SPLIT: the CTAs of a cluster divide a query tile's key blocks. MASK: a mask tensor is the only side input and its rows lie on
+// 16-byte boundaries. Instantiations of their own: a tile that is neither keeps the plain loop, with all four warps at work
+// (429 heads x 10 queries x 3550 keys, D = 64, no mask: 113 us; 133 with one kernel for everything).
+template <bool SPLIT, bool MASK>
 __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __grid_constant__ AttMaps maps,
                                                                         const AttParams p) {
   constexpr int NS = AttSmem::kStages;
@@ -140,8 +144,8 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   const int warp = threadIdx.x >> 5;
   const int lane = lane_id();
   // the CTAs of a cluster share a query tile and divide its key blocks
-  const int splits = p.splits;
-  const int part = splits > 1 ? (int)cluster_ctarank() : 0;
+  const int splits = SPLIT ? p.splits : 1;
+  const int part = SPLIT ? (int)cluster_ctarank() : 0;
   const int tile = blockIdx.x / splits;
   const int g = tile / p.q_tiles;
   // long tiles first under a causal mask
@@ -149,10 +153,10 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   const int q0 = qt * kQT;
   int nb_all = (p.Sk + kKT - 1) / kKT;
   if (p.causal) nb_all = min(nb_all, (min(q0 + kQT, p.Sq) - 1) / kKT + 1);
-  const int per_part = (nb_all + splits - 1) / splits;
-  const int j0 = min(part * per_part, nb_all), nb = min(per_part, nb_all - j0);   // key blocks j0 .. j0 + nb - 1 (maybe none)
+  const int per_part = SPLIT ? (nb_all + splits - 1) / splits : nb_all;
+  const int j0 = SPLIT ? min(part * per_part, nb_all) : 0, nb = SPLIT ? min(per_part, nb_all - j0) : nb_all;   // key blocks j0 .. j0 + nb - 1 (maybe none)
   // warps without a query row of the tile have nothing to compute: their rows of S, P and O are never looked at
-  const int live_warps = min(4, (p.Sq - q0 + 31) / 32);
+  const int live_warps = SPLIT || MASK ? min(4, (p.Sq - q0 + 31) / 32) : 4;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -269,14 +273,12 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     float l = 0.0f;
     bool ok = true;
     const long long side_row = ((long long)g * p.Sq + min(row, (long long)p.Sq - 1)) * p.Sk;   // row of the [G][Sq][Sk] tensors
-    const bool mask_only = p.mask && !p.bias && !p.scale_t && !p.quant_scale && !p.causal;
-    const bool mask_vec = mask_only && p.Sk % 16 == 0 && reinterpret_cast<uintptr_t>(p.mask) % 16 == 0;
     for (int j = 0; j < nb && ok; ++j) {
       const int sb = j & 1;
       const int key0 = (j0 + j) * kKT;
       // this row's mask of the block, one byte a key, read while the scores are on their way
-      uint32_t mw[32];
-      if (mask_vec) {
+      uint32_t mw[MASK ? 32 : 1];
+      if constexpr (MASK) {
         const uint4* m4 = reinterpret_cast<const uint4*>(p.mask + side_row + key0);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -310,7 +312,20 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       }
       // f(S) in the log2 domain: scale, bias, masks
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-      if (!side_inputs && !edge) {
+      if constexpr (MASK) {
+        // the general branch below with its byte loads already done, sixteen at a time
+#pragma unroll
+        for (int i = 0; i < 128; i += 4) {
+          float x[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            x[t] = (mw[i / 4] & (0xffu << (8 * t))) ? __uint_as_float(v[i + t]) * p.scale_log2 : p.mask_fill * kLog2e;
+            if (key0 + i + t >= p.Sk) x[t] = -INFINITY;
+            v[i + t] = __float_as_uint(x[t]);
+          }
+          mx0 = fmaxf(mx0, x[0]); mx1 = fmaxf(mx1, x[1]); mx2 = fmaxf(mx2, x[2]); mx3 = fmaxf(mx3, x[3]);
+        }
+      } else if (!side_inputs && !edge) {
 #pragma unroll
         for (int i = 0; i < 128; i += 4) {
           const float x0 = __uint_as_float(v[i]) * p.scale_log2, x1 = __uint_as_float(v[i + 1]) * p.scale_log2;
@@ -329,19 +344,6 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
           const float x3 = (i + 3 < limit) ? __uint_as_float(v[i + 3]) * p.scale_log2 : -INFINITY;
           v[i] = __float_as_uint(x0); v[i + 1] = __float_as_uint(x1); v[i + 2] = __float_as_uint(x2); v[i + 3] = __float_as_uint(x3);
           mx0 = fmaxf(mx0, x0); mx1 = fmaxf(mx1, x1); mx2 = fmaxf(mx2, x2); mx3 = fmaxf(mx3, x3);
-        }
-      } else if (mask_vec) {
-        // a mask tensor alone: the general branch below with its byte loads already done, sixteen at a time
-#pragma unroll
-        for (int i = 0; i < 128; i += 4) {
-          float x[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            x[t] = (mw[i / 4] & (0xffu << (8 * t))) ? __uint_as_float(v[i + t]) * p.scale_log2 : p.mask_fill * kLog2e;
-            if (key0 + i + t >= p.Sk) x[t] = -INFINITY;
-            v[i + t] = __float_as_uint(x[t]);
-          }
-          mx0 = fmaxf(mx0, x[0]); mx1 = fmaxf(mx1, x[1]); mx2 = fmaxf(mx2, x[2]); mx3 = fmaxf(mx3, x[3]);
         }
       } else {
         const long long side_off = side_row;
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    if (splits > 1) {
+    if constexpr (SPLIT) {
       // this CTA's share of the row, not divided by its sum: O, reference maximum and sum go to shared memory (the key
       // ring is idle by now) for the cluster to add up below
       if (nb > 0 && ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
@@ -428,8 +430,9 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         }
         reinterpret_cast<float2*>(smem + AttSmem::kV)[r] = make_float2(m_ref, l);
       }
+    } else
     // ---- epilogue: O / l -> element type -> staging (the Q tile is no longer needed) -> TMA store ----
-    } else if (ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+    if (ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
       tc_fence_after();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
       uint8_t* stg = smem + AttSmem::kQ + wq * (2 * 32 * 128);   // per warp: Dv/64 tiles of 32 rows x 128 bytes
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     }
   }
 
-  if (splits > 1) {
+  if constexpr (SPLIT) {
     // O = sum over the parts of 2^(m_part - m) O_part, divided by the same sum of the l_part; every CTA of the cluster
     // does a share of the row pieces, reading the others' shared memory
     cluster_sync();
@@ -1719,6 +1722,8 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   } else {
     // at most four queries: the score tile turned round (attention_decode_kernel)
     const bool few = p->seq_q <= kDecodeQ && !quantized && !kp.linear;
+    const bool mask_words = p->mask && !p->bias && !p->scale_tensor && !quantized && !p->causal && p->seq_k % 16 == 0 &&
+                            reinterpret_cast<uintptr_t>(p->mask) % 16 == 0;
     if (few) {
       kp.idesc_s = make_idesc(1, fmt, fmt, p->trans_k ? 0u : 1u, 0u, kKT, kNQ);
       kp.idesc_pv = make_idesc(1, fmt, fmt, 1u, 0u, 128, kNQ);
@@ -1727,10 +1732,14 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
       const uint32_t box[3] = {64, (uint32_t)kNQ, 1};
       if (!encode_tiled(&maps.q, dt, 3, q, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, &err)) return fail(RB_UNSUPPORTED, "Q: " + err);
     }
-    void (*const kern)(const AttMaps, const AttParams) = !few ? attention_fwd_kernel : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
+    kp.splits = attention_splits(p, ctas, dev->sm_count);
+    const bool split = kp.splits > 1;
+    void (*const kern)(const AttMaps, const AttParams) =
+        !few ? (split ? (mask_words ? attention_fwd_kernel<true, true> : attention_fwd_kernel<true, false>)
+                      : (mask_words ? attention_fwd_kernel<false, true> : attention_fwd_kernel<false, false>))
+        : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
     const int threads = few ? kDecodeThreads : kAttThreads, smem = few ? DecodeSmem::total((int)Dp, (int)Dvp) : AttSmem::kTotal;
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != RB_SUCCESS) return RB_CUDA_ERROR;
-    kp.splits = attention_splits(p, ctas, dev->sm_count);
     kp.o = o;
     kp.o_cols = p->head_v;
     if (kp.splits == 1) {
