@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
           mw[4 * i] = u.x; mw[4 * i + 1] = u.y; mw[4 * i + 2] = u.z; mw[4 * i + 3] = u.w;
         }
       }
-      if (!mbar_wait(&s_full[sb], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutEpilogue + sb)) { ok = false; break; }
+      if (!mbar_wait_all(&s_full[sb], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutEpilogue + sb)) { ok = false; break; }
       tc_fence_after();
       const uint32_t tmem_s = tmem_base + lane_base + sb * 128;
       const bool side_inputs = p.bias || p.mask || p.scale_t || p.quant_scale;          // per-element tensors: general path
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       tmem_st32(tmem_s + 32, v + 32);
       // rescale O where a reference maximum moved (whole warp takes part: TMEM access is warp-collective)
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-        if (!mbar_wait(&pv_done[(j - 1) & 1], (uint32_t)((j - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 4)) { ok = false; break; }
+        if (!mbar_wait_all(&pv_done[(j - 1) & 1], (uint32_t)((j - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 4)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < p.Dv / 32; ++c) {
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     if constexpr (SPLIT) {
       // this CTA's share of the row, not divided by its sum: O, reference maximum and sum go to shared memory (the key
       // ring is idle by now) for the cluster to add up below
-      if (nb > 0 && ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+      if (nb > 0 && ok && mbar_wait_all(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
         tc_fence_after();
         const int c4mask = p.Dv / 4 - 1;   // Dv is 64 or 128
         float4* prow = reinterpret_cast<float4*>(smem + AttSmem::kK) + r * (p.Dv / 4);
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       }
     } else
     // ---- epilogue: O / l -> element type -> staging (the Q tile is no longer needed) -> TMA store ----
-    if (ok && mbar_wait(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
+    if (ok && mbar_wait_all(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5)) {
       tc_fence_after();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
       uint8_t* stg = smem + AttSmem::kQ + wq * (2 * 32 * 128);   // per warp: Dv/64 tiles of 32 rows x 128 bytes
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
           if (lane == 0) wm[wq * kNQ + q] = mw;
         }
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");   // the four softmax warps (every one comes here, also after a wait ran out)
+      named_barrier(1, 128);   // the four softmax warps (every one comes here, also after a wait ran out)
       bool moved = false;
       float alpha[NQT];
       uint8_t* pc = p_col + (j & 1) * DecodeSmem::kPBytes;
@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
       }
     }
     if (ok && nb > 0) ok = mbar_wait_warp(&pv_done[(nb - 1) & 1], (uint32_t)((nb - 1) >> 1) & 1u, p.status, kStatusTimeoutEpilogue + 5);
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    named_barrier(1, 128);
     if (nb > 0) {
       tc_fence_after();
       uint32_t o[kNQ];
@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
     long long sm_wait = 0, sm_busy = 0;
     for (int j = 0; j < nb && ok; ++j) {
       const long long ts0 = p.trace ? clock64() : 0;
-      if (!mbar_wait(&s_full[t], (uint32_t)j & 1u, p.status, kStatusTimeoutEpilogue + t)) { ok = false; break; }
+      if (!mbar_wait_all(&s_full[t], (uint32_t)j & 1u, p.status, kStatusTimeoutEpilogue + t)) { ok = false; break; }
       const long long ts1 = p.trace ? clock64() : 0;
       sm_wait += ts1 - ts0;
       tc_fence_after();
@@ -1220,7 +1220,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
       }
       l = l * alpha + ((l0 + l1) + (l2 + l3));
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-        if (!mbar_wait(&pv_done[t], (uint32_t)(j - 1) & 1u, p.status, kStatusTimeoutEpilogue + 4 + t)) { ok = false; break; }
+        if (!mbar_wait_all(&pv_done[t], (uint32_t)(j - 1) & 1u, p.status, kStatusTimeoutEpilogue + 4 + t)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < p.Dv / 32; ++c) {
@@ -1242,7 +1242,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
       p.trace[(size_t)blockIdx.x * 16 + 8 + 2 * t] = (unsigned long long)sm_wait;   // softmax group t: waiting for S
       p.trace[(size_t)blockIdx.x * 16 + 9 + 2 * t] = (unsigned long long)sm_busy;   //   busy (incl. rescale)
     }
-    if (ok && nb > 0 && mbar_wait(&pv_done[t], (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 6 + t)) {
+    if (ok && nb > 0 && mbar_wait_all(&pv_done[t], (uint32_t)(nb - 1) & 1u, p.status, kStatusTimeoutEpilogue + 6 + t)) {
       tc_fence_after();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
       uint8_t* stg = smem + Att2Smem::kQ + t * Att2Smem::kQBytes + wq * (2 * 32 * 128);

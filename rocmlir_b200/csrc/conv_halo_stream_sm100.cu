@@ -254,7 +254,6 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
                 *reinterpret_cast<uint4*>(dst + i * 16) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
             }
           }
-          __syncwarp();   // the warp is whole again before its next collective load from tensor memory
         }
       }
       tc_fence_before();

@@ -171,7 +171,6 @@ __device__ __forceinline__ void store_tile(const PatchParams& p, const PatchTile
   for (int c = (warp >> 2) * 32; c < p.nt; c += 64) {
     const int ncols = min(32, p.Kout - n0 - c);
     if (ncols <= 0) break;   // warp-uniform
-    __syncwarp();            // (collective loads: the lanes parted at the last stores)
     uint32_t v[32];
     tmem_ld32(taddr + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
     tmem_ld_wait();

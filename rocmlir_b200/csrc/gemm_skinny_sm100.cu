@@ -133,7 +133,6 @@ gemm_skinny_kernel(const __grid_constant__ SkinnyMaps maps, const SkinnyParams p
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
       for (int m0 = 0; m0 < p.nt; m0 += 16) {
         if (m0 >= p.M) break;
-        __syncwarp();   // collective load: the lanes parted at the last stores
         uint32_t v[16];
         tmem_ld16(taddr + m0, v);
         tmem_ld_wait();

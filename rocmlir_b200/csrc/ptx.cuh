@@ -157,6 +157,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   return ok != 0;
 }
 
+// The same wait with every lane polling (the shortest way from the barrier to the next instruction) and one answer for the
+// warp: a wait that runs out in some lanes has run out for all. All 32 lanes must call it.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code,
+                                              long long limit = kWaitCycles) {
+  const bool ok = mbar_wait(bar, parity, status, code, limit);
+  return __all_sync(0xffffffffu, ok) != 0;
+}
+
 // One 32-byte store to global memory (sm_100 and later); the address is 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t* w) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(w[0]), "r"(w[1]), "r"(w[2]),
@@ -251,9 +259,20 @@ __device__ __forceinline__ void bulk_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Barrier `id` over `threads` threads of the CTA (whole warps).
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // ---- tcgen05 / TMEM ------------------------------------------------------------------------------
+// Every instruction of this file that is `.aligned` (tensor-memory allocation, loads, stores and their waits, the cluster
+// barrier, and bar.sync) must be executed by all 32 lanes of a warp together. Lanes part at a store that only some of them
+// make, at a role or an arrival of one lane, and nothing but __syncwarp() obliges them to meet again before the next
+// instruction: so each of these functions brings the warp together itself.
 template <int CTAS>
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
+  __syncwarp();
   if constexpr (CTAS == 1)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
                  "r"(ncols)
@@ -265,6 +284,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
 }
 template <int CTAS>
 __device__ __forceinline__ void tmem_relinquish() {
+  __syncwarp();
   if constexpr (CTAS == 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   else
@@ -272,6 +292,7 @@ __device__ __forceinline__ void tmem_relinquish() {
 }
 template <int CTAS>
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t ncols) {
+  __syncwarp();
   if constexpr (CTAS == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(ncols) : "memory");
   else
@@ -355,6 +376,7 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
 
 // 32 lanes x 32-bit, 32 consecutive columns per thread.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -368,6 +390,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -378,6 +401,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -389,6 +413,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
@@ -396,8 +421,14 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_wait() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 
 // ---- descriptors -------------------------------------------------------------------------------
 // Shared-memory matrix descriptor, 128-byte swizzle, tile base 1024-byte aligned.
@@ -444,6 +475,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
