@@ -135,10 +135,12 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   uint64_t* v_full = k_empty + NS;         // [NS]
   uint64_t* v_empty = v_full + NS;         // [NS]
   uint64_t* s_full = v_empty + NS;         // [2]
+  // [2], by block parity: the scores of block j + 1 are there before P(j) is complete, so a warp may announce its P(j + 1)
+  // while a slower one still works on P(j), and one barrier would count that arrival for block j
   uint64_t* p_full = s_full + 2;
   // [2], by block parity: a softmax warp may be done with block j while the product of block j - 1 still waits for its V
   // tile, and on one barrier the parity of j would then read as complete
-  uint64_t* pv_done = p_full + 1;
+  uint64_t* pv_done = p_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 2);
 
   const int warp = threadIdx.x >> 5;
@@ -168,7 +170,8 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    mbar_init(p_full, live_warps);
+    mbar_init(&p_full[0], live_warps);
+    mbar_init(&p_full[1], live_warps);
     mbar_init(&pv_done[0], 1);
     mbar_init(&pv_done[1], 1);
     fence_mbar_init();
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         // execute in issue order.
         if (j + 1 < nb) ok = issue_s(j + 1);
         if (!ok) break;
-        if (!mbar_wait(p_full, (uint32_t)j & 1u, p.status, kStatusTimeoutMma + 9)) break;
+        if (!mbar_wait(&p_full[j & 1], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutMma + 9)) break;
         if (!mbar_wait(&v_full[vs_stage], vs_par, p.status, kStatusTimeoutMma + 10 + vs_stage)) break;
         tc_fence_after();
         const uint32_t v_addr = smem_u32(smem + AttSmem::kV + vs_stage * AttSmem::kVBytes);
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+        if (lane == 0) mbar_arrive(&p_full[j & 1]);
         l = 1.0f;
         continue;
       }
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
     }
     if constexpr (SPLIT) {
       // this CTA's share of the row, not divided by its sum: O, reference maximum and sum go to shared memory (the key

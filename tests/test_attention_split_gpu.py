@@ -36,11 +36,16 @@ def test_split_keys(cuda_device, g, sq, sk, d, dv, code):
     np.testing.assert_array_equal(np.swapaxes(swapped.reshape(g, dv, sq), 1, 2), got.reshape(g, sq, dv))
 
 
+# at most four queries: one byte per key and thread, keys divided over a cluster or not. Above: mask rows on 16-byte boundaries
+# are read as words, others byte by byte, both with the keys divided (few tiles) and not; a ragged last block of keys; one,
+# two and three live warps of a query tile
 @pytest.mark.parametrize("fill", [float("-inf"), -1000.0, float(np.finfo(np.float32).min)])
-@pytest.mark.parametrize("g,sq,sk,d,dv", [(3, 4, 1040, 128, 128), (2, 4, 1001, 64, 64), (150, 2, 272, 64, 64)])
+@pytest.mark.parametrize("g,sq,sk,d,dv", [(3, 4, 1040, 128, 128), (2, 4, 1001, 64, 64), (150, 2, 272, 64, 64),
+                                          (3, 16, 1040, 128, 128), (2, 37, 1296, 64, 64), (1, 70, 2048, 64, 128), (2, 40, 1001, 64, 64),
+                                          (2, 37, 272, 64, 64), (150, 7, 272, 64, 128), (150, 6, 277, 128, 64)])
 def test_split_keys_with_mask(cuda_device, g, sq, sk, d, dv, fill):
-    """Mask rows on 16-byte boundaries (read as words) and off them; a row without any key left, and one whose keys all lie
-    in the first block, so that the other CTAs of the cluster contribute nothing."""
+    """A row without any key left, and one whose keys all lie in the first block, so that the other CTAs of the cluster
+    contribute nothing."""
     (q, qraw), (k, kraw), (v, vraw) = make_qkv(g, sq, sk, d, dv, oracle.F16)
     scale = 1.0 / math.sqrt(d)
     mask = (np.random.Generator(np.random.PCG64(4)).random((g, sq, sk)) > 0.4).astype(np.int8)
@@ -55,6 +60,72 @@ def test_split_keys_with_mask(cuda_device, g, sq, sk, d, dv, fill):
         assert not got[0, 0].any()
         got, ref = got.reshape(g * sq, dv)[1:], np.asarray(ref).reshape(g * sq, dv)[1:]
     check(got.reshape(-1), np.asarray(ref).reshape(-1), oracle.F16)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("sk", [256, 700])
+@pytest.mark.parametrize("g,sq", [(2, 1), (160, 2), (2, 3), (2, 4), (2, 8), (160, 8)])
+def test_scale_and_bias_tensors(cuda_device, g, sq, sk, masked):
+    """Every element of the side tensors differs, so that a wrong row, key or group shows; the fill of masked keys replaces the
+    biased score."""
+    import torch
+    from rocmlir_b200.attention import attention
+    d = 64
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v = (torch.randn(s, device="cuda", generator=gen).half() for s in ((g, sq, d), (g, sk, d), (g, sk, d)))
+    st, bias = (torch.randn((g, sq, sk), device="cuda", generator=gen).half() for _ in range(2))
+    mask = (torch.rand((g, sq, sk), device="cuda", generator=gen) > 0.3).to(torch.int8) if masked else None
+    got = attention(q, k, v, trans_k=True, scale=0.1, scale_tensor=st, bias=bias, mask=mask, mask_fill=-2.0).double()
+    s = q.double() @ k.double().transpose(1, 2) * 0.1 * st.double() + bias.double()
+    if masked:
+        s = torch.where(mask != 0, s, torch.full_like(s, -2.0))
+    ref = s.softmax(-1) @ v.double()
+    check(got.cpu().numpy(), ref.cpu().numpy(), oracle.F16)
+
+
+@pytest.mark.parametrize("code", [oracle.F16, oracle.BF16])
+@pytest.mark.parametrize("g,sq,sk", [(2, 2, 100), (2, 3, 300), (160, 4, 300), (2, 4, 128), (3, 1, 300), (2, 9, 300)])
+def test_causal_few_queries(cuda_device, g, sq, sk, code):
+    """Query i sees keys 0 .. i, whatever the number of keys: one key block at most."""
+    (q, qraw), (k, kraw), (v, vraw) = make_qkv(g, sq, sk, 64, 64, code)
+    mask = np.ascontiguousarray(np.broadcast_to(np.tril(np.ones((sq, sk), np.int8)), (g, sq, sk)))
+    ref = oracle.attention(q, k, v, elem_type=oracle.F64, scale_scalar=0.125, mask=mask, mask_fill=float("-inf"),
+                           threads=oracle.max_threads())
+    got = run_attention(qraw, kraw, vraw, code, scale=0.125, causal=True)
+    check(got.reshape(-1), np.asarray(ref).reshape(-1), code)
+    check(run_attention(qraw, kraw, vraw, code, scale=0.125, mask=mask).reshape(-1), np.asarray(ref).reshape(-1), code)
+
+
+@pytest.mark.parametrize("g,sq,sk,masked", [(64, 1, 4096, True), (3, 4, 1000, False), (2, 37, 1296, True), (1, 128, 2048, False)])
+def test_divided_keys_repeat_exactly(cuda_device, g, sq, sk, masked):
+    """The parts of a divided row are added in the order of their ranks: the same bits on every call."""
+    import torch
+    from rocmlir_b200.attention import attention
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(s, device="cuda", generator=gen).half() for s in ((g, sq, 128), (g, sk, 128), (g, sk, 128)))
+    mask = (torch.rand((g, sq, sk), device="cuda", generator=gen) > 0.3).to(torch.int8) if masked else None
+    first = attention(q, k, v, trans_k=True, scale=0.1, mask=mask)
+    for _ in range(20):
+        assert torch.equal(attention(q, k, v, trans_k=True, scale=0.1, mask=mask), first)
+
+
+@pytest.mark.parametrize("g,sq,sk,masked", [(2, 3, 640, False), (2, 40, 640, False), (2, 40, 640, True), (160, 100, 256, False)])
+def test_quantised_form_with_few_queries(cuda_device, g, sq, sk, masked):
+    """First product in int8, with the keys divided over a cluster and not; the reference rounds to f16 where the form does."""
+    import torch
+    from rocmlir_b200.attention import attention
+    d = 64
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k = (torch.randint(-8, 9, s, device="cuda", generator=gen, dtype=torch.int8) for s in ((g, sq, d), (g, sk, d)))
+    v = torch.randn((g, sk, d), device="cuda", generator=gen).half()
+    mask = (torch.rand((g, sq, sk), device="cuda", generator=gen) > 0.3).to(torch.int8) if masked else None
+    qb, qs = torch.tensor([3], dtype=torch.int8, device="cuda"), torch.tensor([0.0078125], dtype=torch.float16, device="cuda")
+    got = attention(q, k, v, trans_k=True, scale=1.0, mask=mask, quant_bias=qb, quant_scale=qs).double()
+    s = (q.double() @ k.double().transpose(1, 2) - 3.0).half() * qs
+    if masked:
+        s = s.masked_fill(mask == 0, -float("inf"))
+    ref = s.double().softmax(-1) @ v.double()
+    check(got.cpu().numpy(), ref.cpu().numpy(), oracle.F16)
 
 
 def test_split_keys_with_side_tensors_and_infinities(cuda_device):
