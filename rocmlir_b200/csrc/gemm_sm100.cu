@@ -474,6 +474,9 @@ extern "C" size_t rbGemmWorkspaceSize(const RbGemmProblem* p) { return rb::gemm_
 
 RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int R, int C, int pitch, bool transpose,
                         bool split, void* stream_v) {
+  // the pass stores 16 bytes at a time (and the tensor maps over the planes ask for the same start)
+  if (reinterpret_cast<uintptr_t>(hi) % 16 || (split && reinterpret_cast<uintptr_t>(lo) % 16) || pitch % 4)
+    return fail(RB_UNSUPPORTED, "f32 planes: the workspace must be 16-byte aligned");
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
