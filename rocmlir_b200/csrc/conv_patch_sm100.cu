@@ -431,6 +431,9 @@ bool conv_patch_applicable(const PatchConv& c) {
 
 RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
                         void* stream_v) {
+  // the kernel takes its tensors element by element where they lie off wider boundaries, but not off those of an element
+  if ((reinterpret_cast<uintptr_t>(image) | reinterpret_cast<uintptr_t>(filter)) % 2 || reinterpret_cast<uintptr_t>(out) % dtype_bytes(out_type))
+    return fail(RB_UNSUPPORTED, "tensors must start on a multiple of their element size");
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
   PatchShape s;

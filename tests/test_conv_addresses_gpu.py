@@ -34,3 +34,19 @@ def test_f32_planes_in_a_workspace_off_its_boundary(cuda_device, layout, y, offs
     rc.conv(cfg, rc.FWD, fil, inp, out, workspace=space)
     torch.cuda.synchronize()
     assert L.launch_count() > launches and out.any() and L.kernel_status() == 0
+
+
+@pytest.mark.parametrize("which", ["filter", "input", "output"])
+def test_patch_kernel_tensors_off_their_elements(cuda_device, which):
+    """An address between two elements: refused, as the general kernel refuses operands it cannot load."""
+    import ctypes as C
+    import torch
+    from rocmlir_b200 import _lib as L
+    cfg, ocfg = make_cfgs(n=1, c=3, k=32, h=12, w=12, y=3, x=3, pad_h=1, pad_w=1, **LAYOUTS["nhwc"])
+    p = cfg.to_c(torch.float16, 0)
+    assert int(L.lib().rbConvWorkspaceSize(C.byref(p))) == 0
+    bufs = {n: torch.zeros(ocfg.numel(k) + 8, dtype=torch.float16, device="cuda") for n, k in (("filter", "fil"), ("input", "in"), ("output", "out"))}
+    ptr = {n: t.data_ptr() + (1 if n == which else 0) for n, t in bufs.items()}
+    launches = L.launch_count()
+    st = L.lib().rbConv(C.byref(p), ptr["filter"], ptr["input"], ptr["output"], None, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == L.UNSUPPORTED and L.launch_count() == launches
