@@ -9,9 +9,8 @@
 //     rank order, so the result is deterministic and there is no plane in memory and no second launch;
 //   * a thread of the epilogue owns an output column: its bias and scale are one load each.
 // Bound: reading the weights once from HBM, and below about 10 us the launch itself. 8 x 4096 x 4096 f16 with bias: 18.4 us a call
-// through the general kernel and its reduction, 9.8 here (32 MB of weights need 5.1 from HBM). The line to the general kernel
-// lies at 64 rows, the widest operand the two CTAs of an SM have room for: a call with 64 rows takes 12.5 us here and 19.6 through
-// the general kernel at 4096 x 4096, 25.1 and 33.2 at 11008 x 4096, so the general kernel wins nowhere below it.
+// through the general kernel and its reduction, 9.8 here (32 MB of weights need 5.1 from HBM). Where the line to the general
+// kernel lies: gemm_skinny_applicable. 64 rows are the widest operand the two CTAs of an SM have room for.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -194,9 +193,42 @@ gemm_skinny_kernel(const __grid_constant__ SkinnyMaps maps, const SkinnyParams p
 
 }  // namespace
 
-bool gemm_skinny_applicable(const RbGemmProblem* p) {
-  const size_t es = dtype_bytes(p->ab_type);
-  return p->m <= 64 && !p->trans_a && p->trans_b && !p->trans_c && p->ab_type != RB_F32 && ((size_t)p->k * es) % 16 == 0;
+namespace {
+// Parts of K: as many CTAs as fit two to an SM, at least four K blocks each (a part's fixed cost is about that of streaming
+// four blocks).
+int skinny_splits(const RbGemmProblem* p, long long tiles, int kblocks, int sms) {
+  return (int)std::max<long long>(1, std::min<long long>({(long long)kSkinnyMaxSplits, 2LL * sms / tiles, (long long)kblocks / 4}));
+}
+}  // namespace
+
+// Which of the two kernels takes a product with few rows. Here an output column is one thread's, so a row costs every CTA
+// about 0.15 us (0.05 where i32 sums are stored as they are) divided by the parts of K, while the general kernel stores a
+// tile of any height in about a microsecond, but needs a second launch when it divides K and 40 us for a tile whose rows of C
+// do not start on 16-byte boundaries. Measured, us here / there, device time of repeated calls, f16:
+//   parts of K   (16..64) x 4096 x 4096: 8.4..11.3 / 14;  64 x 1024 x 1024: 9.2 / 12.7;  33 x 11008 x 4096: 16.4 / 23.4
+//   two parts    16 x 4096 x 512: 6.8 / 9.0;  33: 9.6 / 9.0;  64: 13.7 / 9.0
+//   one part     16 x 1024 x 256: 6.7 / 7.4;  33: 9.0 / 7.4;  64: 12.8 / 7.4;  K of two blocks, 16 x 64 x 128 in 32 groups: 6.2 / 5.9
+//   long K       64 x 32000 x 4096, one part: 52.7 / 52.2;  33: 50.2 / 52.7
+//   few tiles, K cut into more ranges there than a cluster has: 16 x 128 x 8192: 8.2 / 11.5;  x 32768: 22.2 / 13.9
+//   clusters that fill the SMs to the last slot do not pack: 33 x 4096 x 4096 in 3 groups (96 clusters of 3): 29.1 / 27.1
+//   several CTAs per slot, one tile each where the general kernel is persistent: 64 x 4096 x 128 in 64 groups: 90.7 / 22.5,
+//                16: 40.8 / 20.9;  16 x 128256 x 4096: 165 / 187;  1 x 64 x 64 in 512 groups: 7.0 / 10.0
+//   C off 16 bytes: 53 x 16711 x 80: 12.4 / 43.2;  62 x 2349 x 80 in 55 groups (fp8): 47 / 164
+bool gemm_skinny_applicable(const RbGemmProblem* p, uint32_t epi_flags) {
+  const long long es = (long long)dtype_bytes(p->ab_type);
+  if (p->m > 64 || p->trans_a || !p->trans_b || p->trans_c || p->ab_type == RB_F32 || (p->k * es) % 16) return false;
+  if ((p->n * (long long)dtype_bytes(p->c_type)) % 16) return true;
+  const int sms = planning_sm_count(), kblocks = (int)((p->k * es + 127) / 128);
+  const long long slots = 2LL * sms, tiles = (long long)p->g * ((p->n + kTileN - 1) / kTileN);
+  const int rows = p->c_type == RB_I32 && epi_flags == 0 ? (p->m + 2) / 3 : p->m;
+  if (tiles > slots) return (kblocks >= 8 && 2 * rows <= kblocks) || (tiles <= 2 * slots && rows <= 6);
+  const int splits = skinny_splits(p, tiles, kblocks, sms);
+  if (splits == 1) return rows <= (kblocks >= 4 ? std::max(16, kblocks / 2) : 12);
+  if (kblocks >= 32 * splits && tiles * splits < sms) return false;
+  const bool packs = tiles * splits * 10 <= slots * 9;
+  if (rows <= (packs ? 8 : 4) * splits) return true;
+  const bool divided_there = kblocks >= 16 && 2LL * p->g * ((p->n + 255) / 256) <= sms;
+  return packs && rows <= 16 * splits && (splits >= 3 || divided_there);
 }
 
 RbStatus gemm_skinny_run(const RbGemmProblem* p, const EpiParams& epi, const void* a, const void* b, void* c, int kind, uint32_t fmt_a,
@@ -211,9 +243,7 @@ RbStatus gemm_skinny_run(const RbGemmProblem* p, const EpiParams& epi, const voi
   kp.kblocks = (p->k + bke - 1) / bke;
   kp.tiles_n = (p->n + kTileN - 1) / kTileN;
   const long long tiles = (long long)p->g * kp.tiles_n;
-  // parts of K: as many CTAs as fit two to an SM, at least four K blocks each (a part's fixed cost is about that of
-  // streaming four blocks)
-  kp.splits = (int)std::max<long long>(1, std::min<long long>({(long long)kSkinnyMaxSplits, 2LL * dev->sm_count / tiles, (long long)kp.kblocks / 4}));
+  kp.splits = skinny_splits(p, tiles, kp.kblocks, dev->sm_count);
   const int stage_bytes = kWBytes + kp.nt * 128;
   kp.stages = std::min(kSkinnyMaxStages, (115712 - 1024 - 512) / stage_bytes);   // two CTAs per SM
   kp.idesc = make_idesc(cfmt, fmt_b, fmt_a, 0, 0, (uint32_t)kTileN, (uint32_t)kp.nt);

@@ -673,7 +673,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   }
 
   // few rows against weights stored N x K: the tile turned round (an explicit variant keeps this kernel)
-  if (!capture && !chain && !conva && t_variant == 0 && gemm_skinny_applicable(p) && tuned_variant_gemm(p) == 0) {
+  if (!capture && !chain && !conva && t_variant == 0 && gemm_skinny_applicable(p, ep.flags) && tuned_variant_gemm(p) == 0) {
     const int stall = t_stall_launches > 0 ? 1 : 0;
     t_stall_launches -= stall;
     return gemm_skinny_run(p, ep, a, b, c, kind, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, cfmt, t_wait_cycles, stall, stream_v);
