@@ -25,6 +25,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <string>
 
 #include "epilogue.cuh"
@@ -413,6 +414,33 @@ bool choose_shape(const PatchConv& c, PatchShape* s) {
 }
 
 }  // namespace
+
+// Device time of both forms in microseconds, fitted to 396 convolutions (1 to 384 channels, 16 to 512 output channels, 7 x 7 to
+// 224 x 224, filters 1, 3, 5, 7, strides 1 and 2, both layouts, 5 to 2500 us): 15 % off on average for this form, 9 % for the other.
+// A tile gathers 128 x k elements however few pixels it has, once per group of 128 output channels, copies a window, and every CTA
+// brings the filter over element by element first; so taking this kernel wherever it fits made a third of those convolutions
+// slower, a pointwise layer of 512 -> 512 channels (64 channels-first images of 7 x 7) 32 -> 497 us. By this rule five of
+// the 396 are slower, at most by 13 %:
+//   64 x 224 x 224 x 3 -> 64, 7 x 7 stride 2: 102 us here, 1830 there;  32 x 28 x 28 x 24 -> 64, 3 x 3: 13.5 / 16.4
+//   16 x 14 x 14 x 96 -> 192, 3 x 3: 64 / 16;  channels first 32 x 28 x 28 x 128 -> 128, 3 x 3 stride 2: 299 / 75
+bool conv_patch_pays(const PatchConv& c, bool wide_gather, bool result_direct, int out_bytes) {
+  PatchShape s;
+  if (!choose_shape(c, &s)) return false;
+  const double sms = planning_sm_count(), pixels = 1e-6 * c.N * c.P * c.Q, k = (double)c.Y * c.X * c.C;
+  const double tiles = (double)c.N * ((c.P + s.R - 1) / s.R) * ((c.Q + s.Qt - 1) / s.Qt), rows = (double)s.planes * s.rows;
+  const double ctas = std::min(tiles, std::floor(sms * s.ctas_per_sm / s.passes));
+  const double on_one_sm = std::min<double>(s.ctas_per_sm, std::max(1.0, ctas * s.passes / sms));   // they share its issue slots
+  const double tile = 0.5 + 0.009 * s.kelems + 0.003 * s.nt + rows * (0.042 + 1e-4 * s.pitch) +
+                      (c.o_k == 1 ? 0.022 * (c.Kout % 32) : 0.0);   // (the last columns of a row one by one)
+  const double here = 4.4 + on_one_sm * (std::ceil(tiles / ctas) * tile + 0.0127 * s.nt * ((s.kelems + 63) / 64));
+  // im2col matrix (a vector or an element per thread), its rows padded to 16 bytes, product, permutation of the result
+  double there = 8.1 + pixels * (117 + 2 * k * (wide_gather ? 0.386 : 3.42)) + 0.0039 * pixels * std::max(c.Kout, 64) * k + 0.0042 * k;
+  if ((c.Y * c.X * c.C) % 8 != 0) there += 1.3 + pixels * 2 * k * 0.364;
+  if (!result_direct) there += 4.1 + pixels * 2 * c.Kout * 1.56;
+  // rows of the result off 16 bytes: the product stores element by element, 40 us a wave of tiles
+  if ((c.Kout * out_bytes) % 16) there += 35 * std::ceil(std::ceil(pixels * 1e6 / 128) * ((c.Kout + 255) / 256) / sms);
+  return here * 1.1 < there;
+}
 
 bool conv_patch_applicable(const PatchConv& c) {
   // offsets inside the window, the filter and an image row are 32-bit

@@ -149,6 +149,9 @@ struct PatchConv {
   long long o_n, o_k, o_p, o_q;
 };
 bool conv_patch_applicable(const PatchConv& c);
+// Whether it is the faster form: the other one expands an im2col matrix (wide_gather: by 16-byte vectors, else by elements) and, unless
+// result_direct, permutes the product's result.
+bool conv_patch_pays(const PatchConv& c, bool wide_gather, bool result_direct, int out_bytes);
 RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
                         void* stream);
 

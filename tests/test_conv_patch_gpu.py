@@ -1,6 +1,7 @@
 """GPU parity of the patch kernel (csrc/conv_patch_sm100.cu): 16-bit forward convolutions of one group whose channels are
 not whole 128-byte runs. Integer-valued data, so every partial sum is exact in f32 and the result must equal the oracle's
-bit for bit, and the result of the im2col form of the same library (variant bit 26)."""
+bit for bit, and the result of the im2col form of the same library (variant bit 26). Variant bit 30 takes the kernel wherever
+it fits, also where the library itself would choose the im2col form as the faster one."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,7 @@ from test_conv_gpu import LAYOUTS, make_cfgs, run_conv
 
 pytestmark = pytest.mark.gpu
 
-IM2COL = 1 << 26
+IM2COL, PATCH = 1 << 26, 1 << 30
 MIXED = dict(fil_layout="gyxck", in_layout="hngwc", out_layout="ngkwh")
 # runs of 1 / 2 / 4 / 8 channels; image rows that start on 16-, 8-, 4- and 2-byte boundaries; output rows wider than a tile,
 # several rows per tile with a ragged last one; k extents of one MMA step, of exactly one 64-element block, of more blocks than the operand area
@@ -27,6 +28,12 @@ SHAPES = [
     dict(n=1, c=96, k=64, h=6, w=6, y=3, x=3, pad_h=1, pad_w=1),
     dict(n=2, c=5, k=16, h=1, w=1, y=1, x=1),
 ]
+
+
+@pytest.fixture(autouse=True)
+def _patch_kernel(_default_gemm_variant):
+    from rocmlir_b200 import _lib as L
+    L.lib().rbSetGemmVariant(PATCH)
 
 
 def data(ocfg, code):
@@ -99,7 +106,7 @@ def test_patch_kernel_epilogue_equals_im2col_form(cuda_device, k, out_dtype, lay
     elif out_dtype == "float16" and layout == "nhwc":
         epi.residual = torch.randn(ocfg.numel("out"), device="cuda", generator=gen).half()
     res = []
-    for variant in (0, IM2COL):
+    for variant in (PATCH, IM2COL):
         out = torch.zeros(ocfg.numel("out"), dtype=dt, device="cuda")
         L.lib().rbSetGemmVariant(variant)
         try:

@@ -8,6 +8,7 @@ from test_conv_gpu import LAYOUTS, make_cfgs
 pytestmark = pytest.mark.gpu
 
 GENERAL = 1 << 27        # any explicit variant word: the general GEMM kernel with its own choice of tiles
+IM2COL, PATCH = 1 << 26, 1 << 30
 SLACK = 1.3
 
 
@@ -60,3 +61,21 @@ def test_few_rows(cuda_device, dtype, g, m, n, k):
     ws = torch.empty(max(16, workspace_size(problem(a, b, False, True, False, out))), dtype=torch.uint8, device="cuda")
     run = lambda: gemm(a, b, trans_b=True, out_dtype=out, out=c, workspace=ws)
     assert under(0, run) <= SLACK * under(GENERAL, run)
+
+
+# (layout, n, c, k, h = w, filter, stride): many channels, planes of many channels, several passes over the output channels, channel
+# counts whose pixels fall into the same banks; and the few-channel layers that the patch kernel is for
+CONVS = [("nchw", 64, 512, 512, 7, 1, 1), ("nhwc", 16, 96, 192, 14, 3, 1), ("nchw", 32, 128, 128, 28, 3, 2), ("nhwc", 18, 32, 192, 224, 3, 2),
+         ("nhwc", 125, 160, 48, 35, 3, 1), ("nchw", 42, 64, 512, 7, 3, 1), ("nhwc", 64, 3, 64, 112, 7, 2), ("nchw", 64, 3, 64, 56, 3, 1),
+         ("nhwc", 64, 16, 32, 56, 3, 1), ("nchw", 16, 48, 96, 28, 3, 1), ("nhwc", 32, 24, 33, 56, 3, 1)]
+
+
+@pytest.mark.parametrize("layout,n,c,k,hw,f,s", CONVS)
+def test_few_channels(cuda_device, layout, n, c, k, hw, f, s):
+    import torch
+    from rocmlir_b200 import conv as rc
+    cfg, ocfg = make_cfgs(n=n, c=c, k=k, h=hw, w=hw, y=f, x=f, stride_h=s, stride_w=s, pad_h=f // 2, pad_w=f // 2, **LAYOUTS[layout])
+    fil, inp, out = (torch.randn(ocfg.numel(w), device="cuda").half() for w in ("fil", "in", "out"))
+    ws = torch.empty(1 << 30, dtype=torch.uint8, device="cuda")
+    run = lambda: rc.conv(cfg, rc.FWD, fil, inp, out, workspace=ws)
+    assert under(0, run) <= SLACK * min(under(IM2COL, run), under(PATCH, run))
