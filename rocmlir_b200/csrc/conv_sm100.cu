@@ -920,7 +920,12 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
   const int fil_yxkc[5] = {0, 3, 4, 1, 2};
   const size_t es_c = dtype_bytes(pl.gemm.c_type);
 
+  // The halo kernels, the class interleaving and the weight-gradient sum store their result 16 bytes at a time at addresses that
+  // they derive from its start; the GEMM kernel looks at the address and stores by elements where it must.
+  const auto off16 = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 != 0; };
+  const bool wide_result = !off16(p->direction == 0 ? output : p->direction == 1 ? input : filter);
   if (pl.n_classes > 0) {
+    if (!wide_result) return fail(RB_UNSUPPORTED, "the input gradient of a strided convolution must be 16-byte aligned");
     ClassTable tb;
     tb.N = p->n; tb.H = p->h; tb.W = p->w; tb.G = p->g; tb.C = p->c;
     tb.s_n = pl.is[0]; tb.s_g = pl.is[1]; tb.s_c = pl.is[2]; tb.s_h = pl.is[3]; tb.s_w = pl.is[4];
@@ -1024,13 +1029,13 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
   }
 
   HaloConv uhc;
-  const bool on_halo = !capture && unit_halo(p, pl, epi != nullptr, &uhc);
+  const bool on_halo = !capture && wide_result && unit_halo(p, pl, epi != nullptr, &uhc);
   // f32 forward on the streamed-filter halo kernel (csrc/conv_halo_stream_sm100.cu): decided here because a plain KCYX
   // filter then goes to its two K-major TF32 planes in ONE transposing pass instead of a permutation and a split.
   HaloConv f32_sc;
   long long f32_o_k = 1;
   const size_t fil_plane = up256((size_t)p->k * p->y * p->x * p->c * 4);
-  const bool f32_stream = !on_halo && !capture && !epi && f32_streamed(p, pl, &f32_sc, &f32_o_k);
+  const bool f32_stream = !on_halo && !capture && !epi && wide_result && f32_streamed(p, pl, &f32_sc, &f32_o_k);
   const bool fil_kcyx = filter_is_kcyx(p, pl);
   const void* A;
   const void* B;
@@ -1059,7 +1064,7 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     if (pl.a_direct) A = output; else { permute(output, ws + pl.a_off, osz, pl.os, act_gmat, true, es); A = ws + pl.a_off; }
     if (pl.b_direct) B = input; else { gather(input, ws + pl.b_off, false, false, ho, wo, p->c); B = ws + pl.b_off; }
     C = pl.c_direct ? filter : static_cast<void*>(ws + pl.c_off);
-    if (pl.w_halo && !capture && !((rbGetGemmVariant() >> 26) & 1))
+    if (pl.w_halo && !capture && wide_result && !off16(ws) && !((rbGetGemmVariant() >> 26) & 1))
       return conv_wgrad_halo_run(pl.w_hc, input, output, filter, ws + pl.gemm_off, pl.gemm_ws, stream_v);
     if (pl.b_implicit) {
       ConvAOperand cv;
@@ -1092,7 +1097,7 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     return conv_halo_run(uhc, p->direction == 0 ? input : output, B, p->direction == 0 ? output : input, stream_v, epi, pl.gemm.c_type);
   // Filters too large to stay in shared memory, and f32 tensors (three TF32 products from two planes of window and
   // filter): the halo kernel with a streamed filter (csrc/conv_halo_stream_sm100.cu).
-  if (!capture && !epi && pl.a_implicit && !pl.a_up && p->direction <= 1 && p->stride_h == 1 && p->stride_w == 1 &&
+  if (!capture && !epi && wide_result && pl.a_implicit && !pl.a_up && p->direction <= 1 && p->stride_h == 1 && p->stride_w == 1 &&
       !((rbGetGemmVariant() >> 26) & 1)) {
     HaloConv sc;
     halo_geometry(p, &sc);

@@ -1,9 +1,10 @@
-"""Buffers of convolutions that start off the boundaries the kernels load and store on: refused before anything is launched, as
-a wide access at such an address would fault."""
+"""Buffers of convolutions that start off the boundaries the kernels load and store on: taken by a form that looks at the
+address, or refused before anything is launched, as a wide access at such an address would fault."""
+import numpy as np
 import pytest
 
 import oracle
-from helpers import to_device
+from helpers import from_device, to_device
 from test_conv_gpu import LAYOUTS, make_cfgs
 from test_conv_patch_gpu import data
 
@@ -50,3 +51,38 @@ def test_patch_kernel_tensors_off_their_elements(cuda_device, which):
     launches = L.launch_count()
     st = L.lib().rbConv(C.byref(p), ptr["filter"], ptr["input"], ptr["output"], None, 0, torch.cuda.current_stream().cuda_stream)
     assert st == L.UNSUPPORTED and L.launch_count() == launches
+
+
+# (direction, type, sizes): the halo kernel forward and backward, its streamed-filter forms, the weight-gradient kernel, and results
+# that are not stored as they come out of the product
+OFF = [("fwd", "f16", dict(c=64, k=64)), ("fwd", "f16", dict(c=256, k=64)), ("fwd", "f32", dict(c=64, k=64)),
+       ("bwd_data", "f16", dict(c=64, k=64)), ("bwd_weight", "f16", dict(c=64, k=64)),
+       ("bwd_data", "f16", dict(c=64, k=64, stride_h=2, stride_w=2))]
+
+
+@pytest.mark.parametrize("layout", ["nhwc", "nchw"])
+@pytest.mark.parametrize("direction,kind,sizes", OFF, ids=lambda v: str(v))
+def test_results_off_their_boundary(cuda_device, direction, kind, sizes, layout):
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200 import conv as rc
+    code = oracle.F16 if kind == "f16" else oracle.F32
+    cfg, ocfg = make_cfgs(n=2, h=14, w=14, y=3, x=3, pad_h=1, pad_w=1, **sizes, **LAYOUTS[layout])
+    d = {"fwd": rc.FWD, "bwd_data": rc.BWD_DATA, "bwd_weight": rc.BWD_WEIGHT}[direction]
+    which = {"fwd": 2, "bwd_data": 1, "bwd_weight": 0}[direction]
+    raws = [raw for _, raw in data(ocfg, code)]
+    results = []
+    for skip in (0, 1):
+        bufs = [to_device(raw, code).view(-1) for raw in raws]
+        space = torch.zeros(bufs[which].numel() + 16, dtype=bufs[which].dtype, device="cuda")
+        bufs[which] = space[skip:skip + bufs[which].numel()]
+        try:
+            rc.conv(cfg, d, *bufs)
+        except L.RbError as e:
+            assert e.status == L.UNSUPPORTED and skip
+            return
+        torch.cuda.synchronize()
+        results.append(from_device(bufs[which], code))
+        assert not space[:skip].any() and not space[skip + bufs[which].numel():].any() and L.kernel_status() == 0
+    assert results[0].any()
+    np.testing.assert_array_equal(results[0], results[1])
