@@ -238,6 +238,14 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   const int che = kRowBytes / es;
   const int bn_code = (variant >> 12) & 0xF;
   c.bn = bn_code == 1 ? 64 : bn_code == 2 ? 128 : bn_code == 3 ? 256 : (p->n <= 64 ? 64 : p->n <= 128 ? 128 : 256);
+  const int planes = gemm_planes(p);
+  // Two TF32 planes of 256 columns fill tensor memory with one buffer, so a tile's epilogue is exposed; with a short K that is
+  // most of the tile, and where there are more tiles than CTA pairs 128 columns with two buffers win (us, f32): 4096 x 4096 x 128
+  // 40.3 -> 36.9, x 256 56.3 -> 49.2, 2048 x 8192 x 64 30.9 -> 27.4. At K = 1024 148 against 155, and with one wave 8192 x 512 x 256
+  // 20.5 against 22.0.
+  if (bn_code == 0 && c.bn == 256 && planes == 2 && p->k <= 256 &&
+      (long long)p->g * ((p->m + 2 * kBM - 1) / (2 * kBM)) * ((p->n + 255) / 256) > planned_sms() / 2)
+    c.bn = 128;
   if (b_mn && c.bn < che) c.bn = che;                       // an MN-major B tile is loaded in whole 128-byte chunks
   c.ctas = ((variant & 0xF) == 1) ? 1 : 2;
   if (b_mn && (c.bn / 2) % che != 0) c.ctas = 1;
@@ -250,7 +258,6 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   }
   if (c.bn == 64 && (variant & 0xF) != 2) c.ctas = 1;        // measured: 64-column tiles run faster unpaired (345 vs 324 TFLOP/s)
   c.stages = (variant >> 4) & 0xF;
-  const int planes = gemm_planes(p);
   const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec, planes) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec, planes);
   if (c.stages <= 0 || c.stages > max_stages) c.stages = max_stages;
   // K blocks per barrier round. One round costs the issuing thread about 310 + 44 n cycles for n MMAs (measured),
