@@ -353,8 +353,11 @@ RB_EXPORT RbStatus rbConvEncodeLaunch(const RbConvProblem *p, const RbEpilogue *
 RB_EXPORT void rbSetGemmVariant(int variant);
 RB_EXPORT int rbGetGemmVariant(void);
 
-/* The tile configuration the library would launch for `p` under the calling thread's variant word (on a
- * 148-SM B200): the information rocMLIR attaches to a lowered kernel as block_size / grid_size attributes
+/* The tile configuration in which the GEMM kernel of the kernel image would be launched for `p` under the calling thread's
+ * variant word (on a 148-SM B200), the one rbGemmEncodeLaunch encodes. rbGemm runs some products with at most 64 rows against
+ * B stored N x K on a kernel of their own, which is not in the image and has no variants; this query, the
+ * workspace size and the tuning space keep describing the image's kernel for them, which any explicit variant word selects.
+ * The query gives the information rocMLIR attaches to a lowered kernel as block_size / grid_size attributes
  * (mlir/lib/Dialect/Rock/Transforms/AffixTuningParameters.cpp:69-87) plus what a 1-D launch cannot carry on
  * this hardware (dynamic shared memory, CTAs per cluster). Planned for the SM count of the current device (148
  * without one). `variant` is the explicit variant word that
