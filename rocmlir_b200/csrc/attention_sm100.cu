@@ -516,10 +516,11 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
 // has one key and as many exponentials as there are queries. P^T goes to shared memory as the N x K operand of
 // O^T = V^T . P^T, whose lanes are the columns of V. The row maximum needs one reduction over the four warps per block
 // (a warp maximum per query, exchanged through shared memory); the row sum is kept per thread and added up at the end.
-// Keys are divided over a cluster like above. Bound: reading K and V once. 64 heads x 1 query x 4096 keys, D = 128, masked: 57 us
-// on the single-tile kernel, 28 here. A query costs every thread some 45 instructions per block, so with more than a
-// few the single-tile kernel is the faster one again (10 queries, 429 heads x 3550 keys, D = 64: 113 us there, 183 with all
-// 16 columns computed here).
+// Keys are divided over a cluster like above. Bound: reading K and V once. 64 heads x 1 query x 4096 keys, D = 128, masked: 53 us
+// on the single-tile kernel, 28 here. A query costs every thread some 45 instructions per block, so with more than four
+// queries the single-tile kernel is the faster one again (us here / there for 1, 4, 5 and 8 queries; 5 and 8 in a build with wider
+// instantiations): 429 heads x 3550 keys, D = 64: 71, 81, 103, 128 / 119; 512 heads x 8192 keys, D = 128: 315, 332, 392, 501 / 333; 64 x 4096 x 128: 26,
+// 28, 34, 42 / 28. (With a mask the line would lie higher: 64 x 4096 x 128 5 queries 34 / 54, 9 queries 57 / 54.)
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kNQ = 16;              // query columns of the products
 constexpr int kDecodeQ = 4;          // queries that are computed at most
@@ -1583,6 +1584,22 @@ static int attention_splits(const RbAttentionProblem* p, long long ctas, int sms
   }
   return splits;
 }
+
+// Kernel of a problem: two query tiles per CTA, one, or one turned round for at most four queries.
+static bool two_query_tiles(const RbAttentionProblem* p) {   // the fast path folds the scale into the row maximum, which needs scale >= 0
+  const float scale = p->has_scale ? p->scale : 1.0f;        // an unset scale field must not pick the kernel
+  return p->seq_q > kQT && scale >= 0.0f;
+}
+static bool few_queries(const RbAttentionProblem* p) {
+  return p->seq_q <= kDecodeQ && (p->data_type == RB_F16 || p->data_type == RB_BF16) && !t_attention_linear;
+}
+void attention_launch_dims(const RbAttentionProblem* p, size_t* ctas, size_t* threads) {
+  const long long tiles = (p->seq_q + kQT - 1) / kQT;
+  const bool two = two_query_tiles(p);
+  const int splits = two ? 1 : attention_splits(p, p->g * tiles, planning_sm_count());
+  *ctas = (size_t)(p->g * (two ? (tiles + 1) / 2 : tiles) * splits);
+  *threads = two ? kAtt2Threads : few_queries(p) ? kDecodeThreads : kAttThreads;
+}
 }  // namespace rb
 
 static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, const void* k, const void* v, void* o,
@@ -1716,15 +1733,12 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   kp.trace = trace_buffer((size_t)p->g * ((kp.q_tiles + 1) / 2) * 16);
   const long long ctas = (long long)p->g * kp.q_tiles;
   if (ctas > 0x7fffffffLL) return fail(RB_UNSUPPORTED, "too many query tiles");
-  const float eff_scale = p->has_scale ? p->scale : 1.0f;   // an unset scale field must not pick the kernel
-  if (p->seq_q > kQT && eff_scale >= 0.0f) {
-    // two query tiles per CTA (the fast path folds the scale into the row maximum, which needs scale >= 0)
+  if (two_query_tiles(p)) {
     const long long ctas2 = (long long)p->g * ((kp.q_tiles + 1) / 2);
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd2_kernel), Att2Smem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
     attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
   } else {
-    // at most four queries: the score tile turned round (attention_decode_kernel)
-    const bool few = p->seq_q <= kDecodeQ && !quantized && !kp.linear;
+    const bool few = few_queries(p);
     const bool mask_words = p->mask && !p->bias && !p->scale_tensor && !quantized && !p->causal && p->seq_k % 16 == 0 &&
                             reinterpret_cast<uintptr_t>(p->mask) % 16 == 0;
     if (few) {

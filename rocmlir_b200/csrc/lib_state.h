@@ -132,6 +132,9 @@ struct TunedVariantScope {
   TunedVariantScope& operator=(const TunedVariantScope&) = delete;
 };
 
+// Grid and block of an attention problem's launch (csrc/attention_sm100.cu).
+void attention_launch_dims(const RbAttentionProblem* p, size_t* ctas, size_t* threads);
+
 // GEMM+GEMM with the intermediate kept on the SM (csrc/attention_sm100.cu): k1, n2 <= 128, 16-bit types.
 bool gemm_gemm_on_chip_applicable(int32_t k1, int32_t n1, int32_t n2, int32_t data_type);
 RbStatus gemm_gemm_on_chip(int32_t g, int32_t m, int32_t k1, int32_t n1, int32_t n2, int32_t data_type, const void* a,

@@ -195,3 +195,15 @@ def test_gemm_and_attention_extensions():
                     "-head_dim_v 64")
     with pytest.raises(ValueError):
         miir.Handle("--operation gemm --arch sm_100a -t f16 -m 0 -n 8 -k 8")
+
+
+@pytest.mark.parametrize("t,g,sq,sk,ctas,threads", [("f16", 64, 1, 4096, 128, 192), ("f16", 3, 4, 1000, 24, 192), ("f16", 3, 5, 1000, 24, 256),
+                                                    ("f16", 429, 10, 3550, 429, 256), ("bf16", 1, 128, 2048, 8, 256),
+                                                    ("f16", 150, 2, 272, 150, 192), ("f16", 2, 129, 512, 2, 384)])
+def test_attention_dims_are_those_of_the_launch(t, g, sq, sk, ctas, threads):
+    """At most four queries run on a kernel of 192 threads, and few query tiles on clusters that divide the keys."""
+    with miir.Handle(f"--operation attention --arch sm_100a -t {t} -g {g} -seq_len_q {sq} -seq_len_k {sk} "
+                     "-head_dim_qk 64 -head_dim_v 64 -transK true") as h:
+        h.lower_tuning_params()
+        n, l = h.execution_dims()
+        assert (n // l, l) == (ctas, threads)
