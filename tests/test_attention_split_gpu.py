@@ -96,6 +96,25 @@ def test_causal_few_queries(cuda_device, g, sq, sk, code):
     check(run_attention(qraw, kraw, vraw, code, scale=0.125, mask=mask).reshape(-1), np.asarray(ref).reshape(-1), code)
 
 
+@pytest.mark.parametrize("g,sq,sk,causal,masked", [(2, 300, 2048, False, False), (2, 300, 2048, True, False), (1, 700, 1000, True, False),
+                                                   (2, 300, 1040, False, True), (200, 150, 400, True, False)])
+def test_negative_scale_over_several_query_tiles(cuda_device, g, sq, sk, causal, masked):
+    """A negative scale keeps more than 128 queries on the single-tile kernel: several tiles of a group with their keys divided
+    or not, under the causal flag each tile with its own number of key blocks and parts that have none."""
+    import torch
+    from rocmlir_b200.attention import attention
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(s, device="cuda", generator=gen).half() for s in ((g, sq, 64), (g, sk, 64), (g, sk, 64)))
+    mask = (torch.rand((g, sq, sk), device="cuda", generator=gen) > 0.3).to(torch.int8) if masked else None
+    got = attention(q, k, v, trans_k=True, scale=-0.125, causal=causal, mask=mask).double()
+    s = q.double() @ k.double().transpose(1, 2) * -0.125
+    if causal:
+        s = s.masked_fill(torch.ones((sq, sk), dtype=torch.bool, device="cuda").triu(1), -float("inf"))
+    if masked:
+        s = s.masked_fill(mask == 0, -float("inf"))
+    check(got.cpu().numpy(), (s.softmax(-1) @ v.double()).cpu().numpy(), oracle.F16)
+
+
 @pytest.mark.parametrize("g,sq,sk,masked", [(64, 1, 4096, True), (3, 4, 1000, False), (2, 37, 1296, True), (1, 128, 2048, False)])
 def test_divided_keys_repeat_exactly(cuda_device, g, sq, sk, masked):
     """The parts of a divided row are added in the order of their ranks: the same bits on every call."""
