@@ -862,10 +862,6 @@ struct Att2Smem {
   static constexpr int kTotal = kBars + 256 + 1024;
 };
 
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t* r) {
-  tmem_ld32(taddr, r);
-  tmem_ld32(taddr + 32, r + 32);
-}
 
 __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const __grid_constant__ AttMaps maps,
                                                                           const AttParams p) {

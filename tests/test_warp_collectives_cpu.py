@@ -26,14 +26,34 @@ def test_collective_instructions_stand_in_the_ptx_helpers_only():
 
 
 def test_every_collective_helper_brings_the_warp_together_first():
+    """The waits for loads and stores are the exception: they follow the access, which has brought the warp together. The raw load is
+    for the helpers of this header, which do it for several of them at once."""
     text = code(os.path.join(CSRC, "ptx.cuh"))
     found = 0
     for name, body in bodies(text):
         hits = [m.start() for m in COLLECTIVE.finditer(body)]
         if hits:
-            assert 0 <= body.find("__syncwarp()") < hits[0], name
             found += len(hits)
-    assert found == len(COLLECTIVE.findall(text)) >= 10
+            if name not in ("tmem_ld_wait", "tmem_st_wait", "tmem_ld32_raw"):
+                assert 0 <= body.find("__syncwarp()") < hits[0], name
+        if "tmem_ld32_raw(" in body:
+            assert 0 <= body.find("__syncwarp()") < body.find("tmem_ld32_raw("), name
+    assert found == len(COLLECTIVE.findall(text)) >= 12
+
+
+def test_waits_follow_their_accesses():
+    """Between an access to tensor memory and its wait no lane leaves the others, or the warp meets again."""
+    for root, _, files in os.walk(CSRC):
+        for name in files:
+            if not name.endswith((".cu", ".cuh")) or name == "ptx.cuh":
+                continue
+            text = code(os.path.join(root, name))
+            for m in re.finditer(r"\btmem_(ld|st)_wait\(\);", text):
+                before = text[:m.start()]
+                access = max(before.rfind(f"tmem_{m.group(1)}{n}(") for n in (16, 32, 64))
+                between = before[access:]
+                parted = re.search(r"\blane(?:_id\(\))? == 0|\bvalid\b|\brow_ok\b|\bleader\b", between)
+                assert access >= 0 and (not parted or between.rfind("__syncwarp()") > parted.start()), (name, between[-200:])
 
 
 def test_waits_of_the_softmax_warps_end_alike_in_all_lanes():
