@@ -1,6 +1,7 @@
 """Calls on both sides of the lines between two kernels that compute the same: the library's own choice is not slower than the form
-an explicit variant word selects. Device times, the lower of several; 1.3 leaves room for clocks and for what the lines
-leave on the table (at most 14 % where they were fitted); the choices that this guards against were 1.7 to 16 times slower."""
+an explicit variant word selects. Device times of graph replays, the lowest of several; 1.5 leaves room for clocks and for what
+the lines leave on the table (at most 13 % where they were fitted); most choices that this guards against were 1.7 to 16
+times slower."""
 import pytest
 
 from test_conv_gpu import LAYOUTS, make_cfgs
@@ -9,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 GENERAL = 1 << 27        # any explicit variant word: the general GEMM kernel with its own choice of tiles
 IM2COL, PATCH = 1 << 26, 1 << 30
-SLACK = 1.3
+SLACK = 1.5
 
 
 def device_us(run):
