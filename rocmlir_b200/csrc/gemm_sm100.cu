@@ -814,7 +814,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     kp.c_stride_g = (long long)p->m * p->n;
     kp.split_stride = (long long)p->g * p->m * p->n;
     kp.vec_ok = (p->n % 4 == 0) ? 1 : 0;
-    kp.c_tma = (kp.vec_ok && !cfg.plain_stores) ? 1 : 0;   // planes are stored like a C of splits * g groups
+    kp.c_tma = cfg.plain_stores ? 0 : kp.vec_ok ? 1 : 2;   // planes are stored like a C of splits * g groups
   } else {
     kp.c = c;
     kp.c_type = p->c_type;
@@ -823,7 +823,10 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     if (chain)   // signed distance from group 0's result to group 1's, in elements
       kp.c_stride_g = (reinterpret_cast<intptr_t>(chain->c2) - reinterpret_cast<intptr_t>(c)) / (intptr_t)es_c;
     kp.vec_ok = (!p->trans_c && ((size_t)p->n * es_c) % 16 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0) ? 1 : 0;
-    kp.c_tma = (kp.vec_ok && !cfg.plain_stores) ? 1 : 0;
+    // rows off 16-byte boundaries: staged like the others, copied out by the warps (us, element stores from the registers before): 3 x 640 x
+    // 2279, K = 768, bf16 with bias and ReLU 182 -> 51; 2000 x 3001 x 640 97 -> 33; 4096 x 4095 x 4096 f16 228 -> 127; f32 768 x 1043 x 3648
+    // 102 -> 70
+    kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok ? 1 : 2;
     if (conva && conva->c_rows_per_img > 0) {   // NKHW result: strided element stores, coalesced along the pixels
       kp.c_rows_per_img = conva->c_rows_per_img;
       kp.c_img_stride = conva->c_img_stride;
@@ -834,7 +837,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     }
     kp.epi = ep;
   }
-  if (kp.c_tma) {
+  if (kp.c_tma == 1) {
     const int st_type = kp.c_type;                      // what the kernel stores: C's type, or raw planes
     const size_t es_st = dtype_bytes(st_type);
     const CUtensorMapDataType cdt = st_type == RB_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16

@@ -65,7 +65,7 @@ constexpr int kMaxPlanes = 2;
 struct GemmTensorMaps {
   CUtensorMap a[kMaxPlanes];
   CUtensorMap b[kMaxPlanes];
-  CUtensorMap c;  // store map of C (box: 128 bytes of a row x 32 rows); valid when GemmParams::c_tma != 0
+  CUtensorMap c;  // store map of C (box: 128 bytes of a row x 32 rows); valid when GemmParams::c_tma == 1
 };
 
 // A operand fetched straight from an NHWC activation tensor (implicit GEMM): row m of A is output pixel m
@@ -95,7 +95,8 @@ struct GemmParams {
   long long c_stride_g, c_stride_m, c_stride_n;  // in elements
   int c_type;
   int vec_ok;                 // rows of C start 16-byte aligned and c_stride_n == 1
-  int c_tma;                  // C is written by TMA stores from a shared-memory staging tile
+  int c_tma;                  // rows of C go through a shared-memory staging tile: 1 = and from there by TMA stores, 2 = and are
+                              // copied out by the warp (rows off 16-byte boundaries, see copy_staged_rows); 0 = plain stores
   EpiParams epi;
   uint32_t* status;
   unsigned long long* trace;  // optional [gridDim.x][16] cycle counters per CTA (see rbSetTraceBuffer), or NULL
@@ -244,7 +245,10 @@ struct WorkIter {
 // never executed by such a problem - the C = 256 -> K = 64 pointwise layers lost 12 % (forward) and 6 % (backward data).
 // They are therefore separate functions, called by the tiles that need them.
 struct EpiStoreCtx {
-  const CUtensorMap* cmap;   // store map of C
+  const CUtensorMap* cmap;   // store map of C, or nullptr: the staged rows are copied out from here
+  uint8_t* dst;              // without a map: C at (row0, column 0 of the matrix), its pitch in elements, bytes per element
+  long long pitch;
+  int es;
   uint8_t* staging;          // this warp's staging buffers
   uint32_t stg_bufs;         // 1 or 2
   uint32_t taddr;            // this warp's quarter of the accumulator buffer
@@ -252,6 +256,61 @@ struct EpiStoreCtx {
   int bn, N, M;
   int row0, gz, lane;
 };
+
+// Copies the staged rows of a warp (32 rows of 128 bytes, 16-byte pieces XOR-swizzled by the row) to rows of C that start
+// anywhere: row r goes to dst + r * pitch, of which `cols` elements and the first `rows` rows exist, with a store per 32
+// neighbouring elements. Stored straight from the registers, as the general loop does, every store instruction touches 32 rows.
+// (Aligned words with the two ends of a row by themselves were tried first: 300 cycles a row, most of them instructions.)
+template <typename T>
+__device__ __forceinline__ void copy_rows(const uint8_t* stg, T* dst, long long pitch, int rows, int cols, int lane) {
+  constexpr int kPer = kRowBytes / 32 / (int)sizeof(T);   // elements of a row per lane: columns lane, lane + 32, ...
+  bool in[kPer];
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) in[e] = lane + 32 * e < cols;
+  T* d = dst + lane;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += 8) {   // the words of eight rows in flight, then their stores
+    T w[8][kPer];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) {
+        const int at = (lane + 32 * e) * (int)sizeof(T);
+        w[i][e] = *reinterpret_cast<const T*>(stg + (r0 + i) * kRowBytes + ((at & ~15) ^ (i << 4)) + (at & 15));
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (r0 + i < rows) {
+#pragma unroll
+        for (int e = 0; e < kPer; ++e)
+          if (in[e]) d[32 * e] = w[i][e];
+      }
+      d += pitch;
+    }
+  }
+}
+static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t* dst, long long pitch, int es, int rows, int cols,
+                                                     int lane) {
+  __syncwarp();
+  if (es == 2) copy_rows(stg, reinterpret_cast<uint16_t*>(dst), pitch, rows, cols, lane);
+  else if (es == 4) copy_rows(stg, reinterpret_cast<uint32_t*>(dst), pitch, rows, cols, lane);
+  else copy_rows(stg, dst, pitch, rows, cols, lane);
+  __syncwarp();
+}
+
+// The staged rows of this warp, whose first column is n0, on their way to C.
+__device__ __forceinline__ void emit_staged(const EpiStoreCtx& c, const uint8_t* stg, int n0) {
+  if (c.cmap) {
+    fence_proxy_async();
+    __syncwarp();
+    if (c.lane == 0 && c.row0 < c.M) {
+      tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
+      bulk_commit();
+    }
+  } else {
+    copy_staged_rows(stg, c.dst + (long long)n0 * c.es, c.pitch, c.es, min(32, c.M - c.row0), c.N - n0, c.lane);
+  }
+}
 
 // 16-bit C from float accumulators with the common float tails: [round to mid] -> [x alpha] -> [+ bias[n], round to mid]
 // -> [ReLU] -> convert; the operations and their order are those of epi_apply32. Returns the updated store count.
@@ -300,12 +359,7 @@ static __device__ __noinline__ uint32_t epi_fused16_tile(const EpiStoreCtx c, ui
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
-    fence_proxy_async();
-    __syncwarp();
-    if (c.lane == 0 && c.row0 < c.M) {
-      tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
-      bulk_commit();
-    }
+    emit_staged(c, stg, n0);
     ++nstores;
   }
   return nstores;
@@ -347,12 +401,7 @@ static __device__ __noinline__ uint32_t epi_requant8_tile(const EpiStoreCtx c, c
     *reinterpret_cast<uint4*>(stg + c.lane * kRowBytes + (((sub * 2 + 1) ^ (c.lane & 7)) << 4)) = make_uint4(wd[4], wd[5], wd[6], wd[7]);
     const bool last_group = (sub == 3) || (n0 + 32 >= c.N) || (g == ngroups - 1);
     if (last_group) {
-      fence_proxy_async();
-      __syncwarp();
-      if (c.lane == 0 && c.row0 < c.M) {
-        tma_store_3d(c.cmap, stg, n0 - sub * 32, c.row0, c.gz);
-        bulk_commit();
-      }
+      emit_staged(c, stg, n0 - sub * 32);
       ++nstores;
     }
   }
@@ -426,7 +475,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       prefetch_tmap(&maps.a[s]);
       prefetch_tmap(&maps.b[s]);
     }
-    if (p.c_tma) prefetch_tmap(&maps.c);
+    if (p.c_tma == 1) prefetch_tmap(&maps.c);
   }
   tc_fence_before();
   __syncthreads();
@@ -824,6 +873,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // 4-byte C (f32 results, raw i32 results, the raw planes of a K split): 32 columns = one staging row per step
       const bool fast32 = w.kind == 0 && p.c_tma && !probe &&
                           ((eflags == 0 && !p.acc_is_int && p.c_type == RB_F32) || raw_i32);
+      EpiStoreCtx ec;
+      ec.cmap = p.c_tma == 1 ? &maps.c : nullptr;
+      ec.dst = static_cast<uint8_t*>(p.c) + ((long long)w.split * p.split_stride + (long long)g * p.c_stride_g + row0 * p.c_stride_m) * es_c;
+      ec.pitch = p.c_stride_m; ec.es = es_c;
+      ec.staging = my_staging; ec.stg_bufs = stg_bufs;
+      ec.taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
+      ec.col0 = nb * p.bn; ec.bn = p.bn; ec.N = p.N; ec.M = p.M; ec.row0 = (int)row0; ec.gz = gz; ec.lane = lane;
       if (fast16) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
         const int nsteps = p.bn / 64;
@@ -862,12 +918,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
               *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
             }
           }
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0 && row0 < p.M) {
-            tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
-            bulk_commit();
-          }
+          emit_staged(ec, stg, n0);
           ++nstores;
         }
       } else if (fast32) {
@@ -887,12 +938,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
 #pragma unroll
           for (int i = 0; i < 8; ++i)
             *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0 && row0 < p.M) {
-            tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
-            bulk_commit();
-          }
+          emit_staged(ec, stg, n0);
           ++nstores;
         }
       }
@@ -908,10 +954,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       const bool fast8 = !fast16e && w.kind == 0 && p.c_tma && !probe && p.acc_is_int && p.c_type == RB_I8 &&
                          (eflags & ~(uint32_t)RB_EPI_ZP_OUT) == (uint32_t)(RB_EPI_COL_SCALE | RB_EPI_REQUANT);
       if (fast16e || fast8) {
-        EpiStoreCtx ec;
-        ec.cmap = &maps.c; ec.staging = my_staging; ec.stg_bufs = stg_bufs;
-        ec.taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
-        ec.col0 = nb * p.bn; ec.bn = p.bn; ec.N = p.N; ec.M = p.M; ec.row0 = (int)row0; ec.gz = gz; ec.lane = lane;
         if (fast16e) nstores = epi_fused16_tile(ec, eflags, p.epi.mid_type, p.epi.alpha, vec_bias, p.c_type, nstores);
         else nstores = epi_requant8_tile(ec, vec_scale, p.epi.out_recip, p.epi.out_zero, nstores);
       }
@@ -973,12 +1015,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0 && row0 < p.M) {
-              tma_store_3d(&maps.c, stg, n0 - sub * 32, (int)row0, gz);
-              bulk_commit();
-            }
+            emit_staged(ec, stg, n0 - sub * 32);
             ++nstores;
           }
         }
@@ -1064,12 +1101,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0 && row0 < p.M && !(probe & 4)) {
-              tma_store_3d(&maps.c, stg, n0 - sub * 32, (int)row0, gz);
-              bulk_commit();
-            }
+            if (!(probe & 4)) emit_staged(ec, stg, n0 - sub * 32);
             ++nstores;
           }
         } else if (nw > 0 && row_ok && !(probe & 4)) {
@@ -1100,7 +1132,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       if (p.chain_flags != nullptr && g == 0) {
         // this warp's rows of the intermediate are complete in global memory before its flag says so
-        if (p.c_tma && lane == 0) { bulk_wait<0>(); fence_proxy_async_all(); }
+        if (p.c_tma == 1 && lane == 0) { bulk_wait<0>(); fence_proxy_async_all(); }
         __threadfence();
         __syncwarp();
         if (lane == 0)
@@ -1108,7 +1140,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       if (p.trace) e_work += clock64() - te;
     }
-    if (p.c_tma && lane == 0) bulk_wait<0>();  // every store of this thread has completed before the CTA exits
+    if (p.c_tma == 1 && lane == 0) bulk_wait<0>();  // every store of this thread has completed before the CTA exits
     if (p.trace && warp == 4 && lane == 0) {
       p.trace[blockIdx.x * 16 + 6] = (unsigned long long)w_tfull;
       p.trace[blockIdx.x * 16 + 7] = (unsigned long long)e_work;
