@@ -58,6 +58,7 @@ struct AttParams {
   const void* scale_t;  // optional multiplicative [G][Sq][Sk], element type (applied before the bias)
   const int8_t* mask;  // optional [G][Sq][Sk]: score kept where mask != 0, else mask_fill
   float mask_fill;
+  long long mask_bytes;   // size of the mask
   uint32_t idesc_s, idesc_pv;
   uint32_t* status;
   const void* quant_bias;      // first-GEMM-quantised form: device pointers to one i8 and one f16 (else null)
@@ -119,10 +120,24 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 
 __device__ __forceinline__ float f16_round(float x) { return __half2float(__float2half_rn(x)); }
 
-// SPLIT: the CTAs of a cluster divide a query tile's key blocks. MASK: a mask tensor is the only side input and its rows lie on
-// 16-byte boundaries. Instantiations of their own: a tile that is neither keeps the plain loop, with all four warps at work
-// (429 heads x 10 queries x 3550 keys, D = 64, no mask: 113 us; 133 with one kernel for everything).
-template <bool SPLIT, bool MASK>
+// Four bytes of a tensor of n bytes from offset o on; the address is a multiple of four. A word that reaches beyond either end of the
+// tensor is put together from the bytes that exist, zeros for the others.
+__device__ __forceinline__ uint32_t load_word_within(const int8_t* t, long long n, long long o) {
+  if (o >= 0 && o + 4 <= n) return __ldg(reinterpret_cast<const uint32_t*>(t + o));
+  uint32_t w = 0u;
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if (o + b >= 0 && o + b < n) w |= (uint32_t)(uint8_t)__ldg(t + o + b) << (8 * b);
+  return w;
+}
+
+// SPLIT: the CTAs of a cluster divide a query tile's key blocks. MASK: a mask tensor is the only side input; its rows lie on 16-byte
+// boundaries (1) or anywhere (2: the aligned words around a row's 128 bytes, shifted into place). Instantiations of their own: a tile
+// that is neither keeps the plain loop, with all four warps at work (429 heads x 10 queries x 3550 keys, D = 64, no mask: 113 us; 133 with
+// one kernel for everything). Rows anywhere used to take the general branch, 128 dependent byte loads a block in a loop of a few
+// thousand instructions: 55 heads x 6 queries x 300 keys, D = 64,
+// bf16 102 -> 22 us; 300 x 9 x 1003 840 -> 140; 100 x 16 x 4097, D = 128 1234 -> 207.
+template <bool SPLIT, int MASK>
 __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __grid_constant__ AttMaps maps,
                                                                         const AttParams p) {
   constexpr int NS = AttSmem::kStages;
@@ -158,7 +173,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   const int per_part = SPLIT ? (nb_all + splits - 1) / splits : nb_all;
   const int j0 = SPLIT ? min(part * per_part, nb_all) : 0, nb = SPLIT ? min(per_part, nb_all - j0) : nb_all;   // key blocks j0 .. j0 + nb - 1 (maybe none)
   // warps without a query row of the tile have nothing to compute: their rows of S, P and O are never looked at
-  const int live_warps = SPLIT || MASK ? min(4, (p.Sq - q0 + 31) / 32) : 4;
+  const int live_warps = SPLIT || MASK != 0 ? min(4, (p.Sq - q0 + 31) / 32) : 4;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -281,7 +296,17 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       const int key0 = (j0 + j) * kKT;
       // this row's mask of the block, one byte a key, read while the scores are on their way
       uint32_t mw[MASK ? 32 : 1];
-      if constexpr (MASK) {
+      if constexpr (MASK == 2) {
+        const long long first = side_row + key0;
+        const uint32_t lead = (uint32_t)reinterpret_cast<uintptr_t>(p.mask + first) & 3u;
+        const int n = min(kKT, p.Sk - key0);
+        uint32_t w[33];
+#pragma unroll
+        for (int i = 0; i < 33; ++i) w[i] = 4 * i - (int)lead < n ? load_word_within(p.mask, p.mask_bytes, first - lead + 4 * i) : 0u;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) mw[i] = __funnelshift_r(w[i], w[i + 1], 8 * lead);
+      }
+      if constexpr (MASK == 1) {
         const uint4* m4 = reinterpret_cast<const uint4*>(p.mask + side_row + key0);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -315,7 +340,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       }
       // f(S) in the log2 domain: scale, bias, masks
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-      if constexpr (MASK) {
+      if constexpr (MASK != 0) {
         // the general branch below with its byte loads already done, sixteen at a time
 #pragma unroll
         for (int i = 0; i < 128; i += 4) {
@@ -1721,6 +1746,7 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   kp.quant_scale = quantized ? p->quant_scale : nullptr;
   kp.mask = p->mask;
   kp.mask_fill = p->mask_fill;
+  kp.mask_bytes = (long long)p->g * p->seq_q * p->seq_k;
   kp.linear = t_attention_linear ? 1 : 0;
   const uint32_t fmt = kp.is_bf16 ? 1u : 0u;
   kp.idesc_s = make_idesc(1, fmt, fmt, 0, p->trans_k ? 0u : 1u, kQT, kKT);
@@ -1735,8 +1761,8 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
     attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
   } else {
     const bool few = few_queries(p);
-    const bool mask_words = p->mask && !p->bias && !p->scale_tensor && !quantized && !p->causal && p->seq_k % 16 == 0 &&
-                            reinterpret_cast<uintptr_t>(p->mask) % 16 == 0;
+    const bool mask_only = p->mask && !p->bias && !p->scale_tensor && !quantized && !p->causal;
+    const int mask = !mask_only ? 0 : p->seq_k % 16 == 0 && reinterpret_cast<uintptr_t>(p->mask) % 16 == 0 ? 1 : 2;
     if (few) {
       kp.idesc_s = make_idesc(1, fmt, fmt, p->trans_k ? 0u : 1u, 0u, kKT, kNQ);
       kp.idesc_pv = make_idesc(1, fmt, fmt, 1u, 0u, 128, kNQ);
@@ -1748,8 +1774,8 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
     kp.splits = attention_splits(p, ctas, dev->sm_count);
     const bool split = kp.splits > 1;
     void (*const kern)(const AttMaps, const AttParams) =
-        !few ? (split ? (mask_words ? attention_fwd_kernel<true, true> : attention_fwd_kernel<true, false>)
-                      : (mask_words ? attention_fwd_kernel<false, true> : attention_fwd_kernel<false, false>))
+        !few ? (split ? (mask == 1 ? attention_fwd_kernel<true, 1> : mask == 2 ? attention_fwd_kernel<true, 2> : attention_fwd_kernel<true, 0>)
+                      : (mask == 1 ? attention_fwd_kernel<false, 1> : mask == 2 ? attention_fwd_kernel<false, 2> : attention_fwd_kernel<false, 0>))
         : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
     const int threads = few ? kDecodeThreads : kAttThreads, smem = few ? DecodeSmem::total((int)Dp, (int)Dvp) : AttSmem::kTotal;
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != RB_SUCCESS) return RB_CUDA_ERROR;

@@ -164,3 +164,23 @@ def test_split_keys_with_side_tensors_and_infinities(cuda_device):
     assert torch.isinf(got[1, :, 3]).all() and (got[1, :, 3] > 0).all()
     got[1, :, 3] = 0
     assert torch.isfinite(got).all()
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 16])
+@pytest.mark.parametrize("g,sq,sk", [(2, 5, 128), (2, 16, 129), (3, 7, 300), (150, 9, 255), (1, 6, 1), (1, 100, 1023)])
+def test_mask_rows_anywhere(cuda_device, g, sq, sk, offset):
+    """Masks whose rows start on any byte, in a tensor that begins and ends on any byte: equal, bit for bit, to the same mask as a
+    bias-free general call (a bias tensor of zeros takes the element-wise path)."""
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200.attention import attention
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(s, device="cuda", generator=gen).half() for s in ((g, sq, 64), (g, sk, 64), (g, sk, 64)))
+    buf = torch.full((g * sq * sk + 64,), 1, dtype=torch.int8, device="cuda")
+    mask = buf[offset:offset + g * sq * sk].view(g, sq, sk)
+    mask.copy_((torch.rand((g, sq, sk), device="cuda", generator=gen) > 0.4).to(torch.int8))
+    got = attention(q, k, v, trans_k=True, scale=0.125, mask=mask)
+    zeros = torch.zeros((g, sq, sk), dtype=torch.float16, device="cuda")
+    ref = attention(q, k, v, trans_k=True, scale=0.125, mask=mask.clone(), bias=zeros)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref) and L.kernel_status() == 0
