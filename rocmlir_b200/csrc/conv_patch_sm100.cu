@@ -28,9 +28,8 @@
 #include <cmath>
 #include <string>
 
-#include "epilogue.cuh"
+#include "conv_patch.cuh"
 #include "lib_state.h"
-#include "ptx.cuh"
 
 namespace rb {
 namespace {
@@ -67,13 +66,6 @@ struct PatchParams {
   long long wait_cycles;
 };
 
-__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int gran, int bytes) {
-  if (gran == 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-  else if (gran == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 struct PatchTile {
   int n, p0, q0;
   __device__ PatchTile(const PatchParams& p, unsigned tile) {   // 32-bit: a 64-bit division is two hundred instructions
@@ -108,14 +100,6 @@ __device__ __forceinline__ void load_window(const PatchParams& p, const PatchTil
       else dst[v] = valid > 0 ? __ldg(src) : (uint16_t)0;
     }
   }
-}
-
-// Shared memory by byte offset from the start of the dynamic allocation: plain loads and stores that the compiler knows to be
-// in shared memory (through an aligned-up pointer they are generic ones) and may schedule freely between barriers.
-extern __shared__ __align__(16) uint8_t smem_raw[];
-template <typename T>
-__device__ __forceinline__ T lds(uint32_t off) {
-  return *reinterpret_cast<const T*>(smem_raw + off);
 }
 
 // Eight k values of one pixel from the window (`px`: where the pixel lies in shared memory; `offs`: where the step's eight
@@ -172,51 +156,7 @@ __device__ __forceinline__ void store_tile(const PatchParams& p, const PatchTile
   for (int c = (warp >> 2) * 32; c < p.nt; c += 64) {
     const int ncols = min(32, p.Kout - n0 - c);
     if (ncols <= 0) break;   // warp-uniform
-    uint32_t v[32];
-    tmem_ld32(taddr + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
-    tmem_ld_wait();
-    const long long o = pix + (long long)(n0 + c) * p.o_k;
-    if constexpr (!EPI) {
-      uint32_t h[16];
-      pack_row16<32>(v, h, p.is_bf16 != 0);
-      if (valid) {
-        uint16_t* d = static_cast<uint16_t*>(p.out) + o;
-        if (p.wide && ncols == 32) {
-          st_global_v8(d, h);
-          st_global_v8(d + 16, h + 8);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < ncols) d[j * p.o_k] = (uint16_t)(h[j / 2] >> (16 * (j & 1)));
-        }
-      }
-    } else {
-      float x[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
-      EpiRow er;
-      if ((p.epi.flags & RB_EPI_BIAS) && (p.epi.flags & RB_EPI_BIAS_SCALAR)) er.row_bias = load_bias(p.epi.bias, p.epi.bias_type, 0);
-      er.res_stride = p.o_k;
-      er.ncols = ncols;
-      er.res = (valid && (p.epi.flags & RB_EPI_RESIDUAL))
-                   ? static_cast<const uint8_t*>(p.epi.residual) + (p.epi.res_type == RB_F32 ? 4 : 2) * o
-                   : nullptr;
-      epi_apply32(x, p.epi, vec_scale + c, vec_bias + c, er);
-      if (valid) {
-        if (p.wide && ncols == 32) {
-          uint4 w4[8];
-          const int nw = pack_row32(x, p.out_type, w4, p.epi.out_zero);
-          uint4* d = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + o * dtype_size(p.out_type));
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (i < nw) d[i] = w4[i];
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < ncols) store_elem(p.out, o + j * p.o_k, x[j], p.out_type, p.epi.out_zero);
-        }
-      }
-    }
+    store_pixel<EPI>(p, valid, pix, taddr + ((uint32_t)((warp & 3) * 32) << 16) + c, n0 + c, ncols, vec_scale + c, vec_bias + c);
   }
 }
 
@@ -423,7 +363,8 @@ bool choose_shape(const PatchConv& c, PatchShape* s) {
 // the 396 are slower, at most by 13 %:
 //   64 x 224 x 224 x 3 -> 64, 7 x 7 stride 2: 102 us here, 1830 there;  32 x 28 x 28 x 24 -> 64, 3 x 3: 13.5 / 16.4
 //   16 x 14 x 14 x 96 -> 192, 3 x 3: 64 / 16;  channels first 32 x 28 x 28 x 128 -> 128, 3 x 3 stride 2: 299 / 75
-bool conv_patch_pays(const PatchConv& c, bool wide_gather, bool result_direct, int out_bytes) {
+bool conv_patch_pays(PatchConv* conv, bool wide_gather, bool result_direct, int out_bytes) {
+  const PatchConv& c = *conv;
   PatchShape s;
   if (!choose_shape(c, &s)) return false;
   const double sms = planning_sm_count(), pixels = 1e-6 * c.N * c.P * c.Q, k = (double)c.Y * c.X * c.C;
@@ -439,7 +380,10 @@ bool conv_patch_pays(const PatchConv& c, bool wide_gather, bool result_direct, i
   if (!result_direct) there += 4.1 + pixels * 2 * c.Kout * 1.56;
   // rows of the result off 16 bytes: the product stores element by element, 40 us a wave of tiles
   if ((c.Kout * out_bytes) % 16) there += 35 * std::ceil(std::ceil(pixels * 1e6 / 128) * ((c.Kout + 255) / 256) / sms);
-  return here * 1.1 < there;
+  const int variant = rbGetGemmVariant();
+  const double window = ((variant >> 10) & 1) ? -1.0 : conv_window_plan(conv);
+  if (window < 0 || (((variant >> 30) & 1) == 0 && window > here)) conv->win_q = 0;
+  return (conv->win_q ? std::min(here, window) : here) * 1.1 < there;
 }
 
 bool conv_patch_applicable(const PatchConv& c) {
@@ -462,6 +406,7 @@ RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filte
   // the kernel takes its tensors element by element where they lie off wider boundaries, but not off those of an element
   if ((reinterpret_cast<uintptr_t>(image) | reinterpret_cast<uintptr_t>(filter)) % 2 || reinterpret_cast<uintptr_t>(out) % dtype_bytes(out_type))
     return fail(RB_UNSUPPORTED, "tensors must start on a multiple of their element size");
+  if (conv_window_fits(c, image)) return conv_window_run(c, image, filter, out, out_type, epi, stream_v);
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
   PatchShape s;

@@ -486,7 +486,7 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
       pl->a_planes = p->f32_mode == 0 ? 2 : (in_is_mat ? 0 : 1);
     }
     // 16-bit images whose operand would have to be expanded into an im2col matrix: the patch kernel where it is the faster form (bit
-    // 26 keeps the matrix, bit 30 takes the kernel wherever it fits)
+    // 26 keeps the matrix, bit 30 takes the patch kernels wherever they fit, bit 10 the gathering one of them)
     pl->patch = false;
     if (!pl->a_direct && !pl->a_implicit && G == 1 && (t == RB_F16 || t == RB_BF16) && !((rbGetGemmVariant() >> 26) & 1) &&
         out_t <= RB_F8E4M3 && out_t != RB_I32) {
@@ -501,9 +501,9 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
         c.i_n = pl->is[0]; c.i_c = pl->is[2]; c.i_h = pl->is[3];
         c.f_k = pl->fs[1]; c.f_c = pl->fs[2]; c.f_y = pl->fs[3]; c.f_x = pl->fs[4];
         c.o_n = pl->os[0]; c.o_k = pl->os[2]; c.o_p = pl->os[3]; c.o_q = pl->os[4];
+        c.win_q = c.win_r = 0;
         pl->patch = conv_patch_applicable(c) &&
-                    (((rbGetGemmVariant() >> 30) & 1) ||
-                     conv_patch_pays(c, pl->is[2] == 1 && p->c % 8 == 0, pl->c_direct, (int)es_o));
+                    (conv_patch_pays(&c, pl->is[2] == 1 && p->c % 8 == 0, pl->c_direct, (int)es_o) || ((rbGetGemmVariant() >> 30) & 1));
       }
     }
     if (pl->a_implicit) pl->a_direct = true;   // nothing to gather

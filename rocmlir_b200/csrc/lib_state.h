@@ -150,13 +150,21 @@ struct PatchConv {
   long long i_n, i_c, i_h;
   long long f_k, f_c, f_y, f_x;
   long long o_n, o_k, o_p, o_q;
+  int win_q, win_r;   // tile of the window kernel (csrc/conv_window_sm100.cu), 0: the patch kernel's gather
 };
 bool conv_patch_applicable(const PatchConv& c);
 // Whether it is the faster form: the other one expands an im2col matrix (wide_gather: by 16-byte vectors, else by elements) and, unless
 // result_direct, permutes the product's result.
-bool conv_patch_pays(const PatchConv& c, bool wide_gather, bool result_direct, int out_bytes);
+bool conv_patch_pays(PatchConv* c, bool wide_gather, bool result_direct, int out_bytes);
 RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
                         void* stream);
+
+// The window kernel: its tile for this convolution and an estimate of its time in microseconds (negative: it does not take it);
+// whether it takes this image with that tile (not off 16 bytes).
+double conv_window_plan(PatchConv* c);
+bool conv_window_fits(const PatchConv& c, const void* image);
+RbStatus conv_window_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
+                         void* stream);
 
 // Whether an epilogue can be applied to a result of type c_type: RB_SUCCESS or the reason why not.
 RbStatus check_epilogue(const RbEpilogue* epi, int c_type);

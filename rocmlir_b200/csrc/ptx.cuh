@@ -461,6 +461,9 @@ __device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr, uint32_t lbo_by
 __device__ __forceinline__ uint32_t smem_desc_hi(uint32_t sbo_bytes) {
   return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
 }
+// No swizzle: core matrices of eight rows x 16 contiguous bytes, `sbo` bytes from one group of eight rows to the next; the
+// leading byte offset of a K-major tile is the distance of its second 16 bytes of K from the first.
+__device__ __forceinline__ uint32_t smem_desc_hi_plain(uint32_t sbo_bytes) { return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14); }
 __device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
