@@ -136,7 +136,8 @@ __device__ __forceinline__ uint32_t load_word_within(const int8_t* t, long long 
 // that is neither keeps the plain loop, with all four warps at work (429 heads x 10 queries x 3550 keys, D = 64, no mask: 113 us; 133 with
 // one kernel for everything). Rows anywhere used to take the general branch, 128 dependent byte loads a block in a loop of a few
 // thousand instructions: 55 heads x 6 queries x 300 keys, D = 64,
-// bf16 102 -> 22 us; 300 x 9 x 1003 840 -> 140; 100 x 16 x 4097, D = 128 1234 -> 207.
+// bf16 102 -> 13 us; 300 x 9 x 1003 862 -> 57; 100 x 16 x 4097, D = 128 1243 -> 71; rows on 16 bytes, 64 x 8 x 4096, D = 128
+// 54 -> 34 (read a block ahead).
 template <bool SPLIT, int MASK>
 __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __grid_constant__ AttMaps maps,
                                                                         const AttParams p) {
@@ -291,20 +292,21 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
     float l = 0.0f;
     bool ok = true;
     const long long side_row = ((long long)g * p.Sq + min(row, (long long)p.Sq - 1)) * p.Sk;   // row of the [G][Sq][Sk] tensors
-    for (int j = 0; j < nb && ok; ++j) {
-      const int sb = j & 1;
+    // this row's mask of a block, one byte a key, read a block ahead: its latency is as long as a block's work. Rows that start anywhere:
+    // the aligned words that hold the 128 bytes.
+    uint32_t mw[MASK == 2 ? 33 : MASK == 1 ? 32 : 1];
+    const uint32_t lead = MASK == 2 ? (uint32_t)reinterpret_cast<uintptr_t>(p.mask + side_row) & 3u : 0u;
+    auto load_mask = [&](int j) {
       const int key0 = (j0 + j) * kKT;
-      // this row's mask of the block, one byte a key, read while the scores are on their way
-      uint32_t mw[MASK ? 32 : 1];
       if constexpr (MASK == 2) {
-        const long long first = side_row + key0;
-        const uint32_t lead = (uint32_t)reinterpret_cast<uintptr_t>(p.mask + first) & 3u;
-        const int n = min(kKT, p.Sk - key0);
-        uint32_t w[33];
+        const long long first = side_row + key0 - lead;
+        if (__all_sync(0xffffffffu, first >= 0 && first + 132 <= p.mask_bytes)) {
 #pragma unroll
-        for (int i = 0; i < 33; ++i) w[i] = 4 * i - (int)lead < n ? load_word_within(p.mask, p.mask_bytes, first - lead + 4 * i) : 0u;
+          for (int i = 0; i < 33; ++i) mw[i] = __ldg(reinterpret_cast<const uint32_t*>(p.mask + first + 4 * i));
+        } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) mw[i] = __funnelshift_r(w[i], w[i + 1], 8 * lead);
+          for (int i = 0; i < 33; ++i) mw[i] = load_word_within(p.mask, p.mask_bytes, first + 4 * i);
+        }
       }
       if constexpr (MASK == 1) {
         const uint4* m4 = reinterpret_cast<const uint4*>(p.mask + side_row + key0);
@@ -314,6 +316,11 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
           mw[4 * i] = u.x; mw[4 * i + 1] = u.y; mw[4 * i + 2] = u.z; mw[4 * i + 3] = u.w;
         }
       }
+    };
+    if (MASK != 0 && nb > 0) load_mask(0);
+    for (int j = 0; j < nb && ok; ++j) {
+      const int sb = j & 1;
+      const int key0 = (j0 + j) * kKT;
       if (!mbar_wait_all(&s_full[sb], (uint32_t)(j >> 1) & 1u, p.status, kStatusTimeoutEpilogue + sb)) { ok = false; break; }
       tc_fence_after();
       const uint32_t tmem_s = tmem_base + lane_base + sb * 128;
@@ -341,17 +348,24 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
       // f(S) in the log2 domain: scale, bias, masks
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
       if constexpr (MASK != 0) {
-        // the general branch below with its byte loads already done, sixteen at a time
+        // the general branch below with its byte loads already done
+        const float fill = p.mask_fill * kLog2e;
 #pragma unroll
         for (int i = 0; i < 128; i += 4) {
-          float x[4];
+          const uint32_t m = MASK == 2 ? __funnelshift_r(mw[i / 4], mw[MASK == 2 ? i / 4 + 1 : 0], 8 * lead) : mw[i / 4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            x[t] = (mw[i / 4] & (0xffu << (8 * t))) ? __uint_as_float(v[i + t]) * p.scale_log2 : p.mask_fill * kLog2e;
-            if (key0 + i + t >= p.Sk) x[t] = -INFINITY;
-            v[i + t] = __float_as_uint(x[t]);
-          }
-          mx0 = fmaxf(mx0, x[0]); mx1 = fmaxf(mx1, x[1]); mx2 = fmaxf(mx2, x[2]); mx3 = fmaxf(mx3, x[3]);
+          for (int t = 0; t < 4; ++t) v[i + t] = (m & (0xffu << (8 * t))) ? __float_as_uint(__uint_as_float(v[i + t]) * p.scale_log2) : __float_as_uint(fill);
+        }
+        if (j + 1 < nb) load_mask(j + 1);
+        if (key0 + kKT > p.Sk) {
+#pragma unroll
+          for (int i = 0; i < 128; ++i)
+            if (key0 + i >= p.Sk) v[i] = 0xff800000u;
+        }
+#pragma unroll
+        for (int i = 0; i < 128; i += 4) {
+          mx0 = fmaxf(mx0, __uint_as_float(v[i])); mx1 = fmaxf(mx1, __uint_as_float(v[i + 1]));
+          mx2 = fmaxf(mx2, __uint_as_float(v[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(v[i + 3]));
         }
       } else if (!side_inputs && !edge) {
 #pragma unroll
