@@ -103,22 +103,32 @@ def workspace_size(cfg: ConvConfig, dtype: torch.dtype, direction: int, f32_mode
     return int(L.lib().rbConvWorkspaceSize(C.byref(p)))
 
 
+def check_tensors(cfg: ConvConfig, filter: torch.Tensor, input: torch.Tensor, output: torch.Tensor) -> None:
+    if not (filter.is_cuda and input.is_cuda and output.is_cuda and filter.is_contiguous() and input.is_contiguous() and
+            output.is_contiguous()):
+        raise L.RbError(L.INVALID_PARAM, "tensors must be contiguous CUDA buffers (the library has no CPU path)")
+    for t_, name in ((filter, "fil"), (input, "in"), (output, "out")):
+        if t_.numel() != cfg.numel(name):
+            raise L.RbError(L.INVALID_PARAM, f"{name} has {t_.numel()} elements, expected {cfg.numel(name)}")
+
+
 def conv(cfg: ConvConfig, direction: int, filter: torch.Tensor, input: torch.Tensor, output: torch.Tensor, *,
          workspace: Optional[torch.Tensor] = None, f32_mode: int = 0) -> torch.Tensor:
     """Runs the convolution; writes and returns the tensor the direction produces. All three tensors are flat
     (or any-shape contiguous) CUDA buffers in their layout order; the output of an i8 convolution is int32."""
-    for t_, name in ((filter, "fil"), (input, "in"), (output, "out")):
-        if not t_.is_cuda or not t_.is_contiguous():
-            raise L.RbError(L.INVALID_PARAM, "tensors must be contiguous CUDA buffers (the library has no CPU path)")
-        if t_.numel() != cfg.numel(name):
-            raise L.RbError(L.INVALID_PARAM, f"{name} has {t_.numel()} elements, expected {cfg.numel(name)}")
-    dtype = input.dtype
-    p = cfg.to_c(dtype, direction, f32_mode)
+    check_tensors(cfg, filter, input, output)
+    p = cfg.to_c(input.dtype, direction, f32_mode)
     lib = L.lib()
     pp, stream = C.byref(p), stream_address(input.device)
     pf, pi, po = filter.data_ptr(), input.data_ptr(), output.data_ptr()
-    L.check(run_with_workspace(lambda ws, n: lib.rbConv(pp, pf, pi, po, ws, n, stream), lambda: int(lib.rbConvWorkspaceSize(pp)),
-                               workspace, input.device, ask=lib.rbGetGemmVariant() != 0))
+    st, ask = L.WORKSPACE_TOO_SMALL, lib.rbGetGemmVariant() != 0
+    if workspace is not None and not ask:   # as run_with_workspace does, which small calls are too short for
+        st, ask = lib.rbConv(pp, pf, pi, po, workspace.data_ptr(), workspace.nbytes, stream), True
+    if st == L.WORKSPACE_TOO_SMALL:
+        st = run_with_workspace(lambda ws, n: lib.rbConv(pp, pf, pi, po, ws, n, stream), lambda: int(lib.rbConvWorkspaceSize(pp)),
+                                workspace, input.device, ask=ask)
+    if st != L.SUCCESS:
+        L.check(st)
     return {FWD: output, BWD_DATA: input, BWD_WEIGHT: filter}[direction]
 
 
@@ -127,11 +137,7 @@ def conv_fused(cfg: ConvConfig, filter: torch.Tensor, input: torch.Tensor, outpu
     """Forward convolution with a fused elementwise tail (rbConvEpi): `epilogue` is a rocmlir_b200.gemm.Epilogue whose
     vectors are indexed by the output channel; the element type of `output` is the result type after the epilogue
     (e.g. int8 for a requantised i8 convolution)."""
-    for t_, name in ((filter, "fil"), (input, "in"), (output, "out")):
-        if not t_.is_cuda or not t_.is_contiguous():
-            raise L.RbError(L.INVALID_PARAM, "tensors must be contiguous CUDA buffers (the library has no CPU path)")
-        if t_.numel() != cfg.numel(name):
-            raise L.RbError(L.INVALID_PARAM, f"{name} has {t_.numel()} elements, expected {cfg.numel(name)}")
+    check_tensors(cfg, filter, input, output)
     p = cfg.to_c(input.dtype, FWD, f32_mode)
     out_type = rb_dtype(output.dtype)
     lib = L.lib()

@@ -50,6 +50,12 @@ def run_with_workspace(call, size, workspace: Optional[torch.Tensor], device: to
     return call(workspace.data_ptr() if workspace is not None else None, workspace.nbytes if workspace is not None else 0)
 
 
+def f32_reciprocal(x: float) -> float:
+    """fl32(1 / fl32(x)): the quotient in 64 bits, rounded once more, is the correctly rounded one in 32."""
+    x = C.c_float(x).value
+    return 1.0 / x if x else float(np.float32(1.0) / np.float32(x))
+
+
 @dataclass
 class Epilogue:
     """Fused elementwise tail of the GEMM; fields map one-to-one onto RbEpilogue."""
@@ -71,7 +77,7 @@ class Epilogue:
         flags = 0
         if self.alpha is not None:
             flags |= L.EPI_ALPHA
-            e.alpha = float(np.float32(self.alpha))
+            e.alpha = self.alpha   # (rounded to f32 by the field)
         if self.col_scale is not None:
             assert self.col_scale.dtype == torch.float32 and self.col_scale.is_cuda and self.col_scale.is_contiguous()
             flags |= L.EPI_COL_SCALE
@@ -103,7 +109,7 @@ class Epilogue:
             flags |= L.EPI_RELU
         if self.requant_scale is not None:
             flags |= L.EPI_REQUANT
-            e.out_recip = float(np.float32(1.0) / np.float32(self.requant_scale))
+            e.out_recip = f32_reciprocal(self.requant_scale)
         if self.mid_type is not None:
             flags |= L.EPI_ROUND_MID
             e.mid_type = int(self.mid_type)
@@ -117,14 +123,18 @@ def _as3d(t: torch.Tensor) -> torch.Tensor:
 
 def problem(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: bool, trans_c: bool, out_dtype: torch.dtype,
             f32_mode: int = 0, accumulate: bool = False) -> L.RbGemmProblem:
-    a3, b3 = _as3d(a), _as3d(b)
-    g = a3.shape[0]
-    m, k = (a3.shape[2], a3.shape[1]) if trans_a else (a3.shape[1], a3.shape[2])
-    kb, n = (b3.shape[2], b3.shape[1]) if trans_b else (b3.shape[1], b3.shape[2])
-    if kb != k or b3.shape[0] != g:
+    sa, sb = a.shape, b.shape
+    g, m, k = (1, sa[0], sa[1]) if len(sa) == 2 else (sa[0], sa[1], sa[2])
+    gb, kb, n = (1, sb[0], sb[1]) if len(sb) == 2 else (sb[0], sb[1], sb[2])
+    if trans_a:
+        m, k = k, m
+    if trans_b:
+        kb, n = n, kb
+    if kb != k or gb != g:
         raise L.RbError(L.INVALID_PARAM, f"shape mismatch: A {tuple(a.shape)} B {tuple(b.shape)}")
-    if a.dtype == b.dtype:
-        ab = rb_dtype(a.dtype)
+    ta = a.dtype
+    if ta == b.dtype:
+        ab = rb_dtype(ta)
     elif (a.dtype, b.dtype) == (torch.float8_e4m3fn, torch.float8_e5m2):
         ab = L.F8E4M3_E5M2      # rocmlir-gen's -t fp8_bf8
     elif (a.dtype, b.dtype) == (torch.float8_e5m2, torch.float8_e4m3fn):
@@ -161,29 +171,33 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         raise L.RbError(L.INVALID_PARAM, "operands must be contiguous")
     out_dtype = out_dtype or default_out_dtype(a.dtype)
     p = problem(a, b, trans_a, trans_b, trans_c, out_dtype, f32_mode, accumulate)
-    shape = (p.g, p.n, p.m) if trans_c else (p.g, p.m, p.n)
     if out is None:
-        out = torch.empty(shape, dtype=out_dtype, device=a.device)
+        out = torch.empty((p.g, p.n, p.m) if trans_c else (p.g, p.m, p.n), dtype=out_dtype, device=a.device)
     else:
         assert out.is_contiguous() and out.dtype == out_dtype and out.numel() == p.g * p.m * p.n
     lib = L.lib()
     # The variant word is state of the calling thread inside the library: set it for this call only and put the
     # caller's value back, so that a tuned call does not change what later calls (of any operator) run.
     saved = lib.rbGetGemmVariant()
-    try:
-        if variant is not None:   # before the workspace query: a K split or a stream-K tail changes what is needed
-            lib.rbSetGemmVariant(int(variant))
-        e = C.byref(epilogue.to_c()) if epilogue is not None else None
-        pp, pa, pb, pc, stream = C.byref(p), a.data_ptr(), b.data_ptr(), out.data_ptr(), stream_address(a.device)
-        # (a stream-K tail, bit 9 of the variant word, is left out when its partial tiles do not fit the workspace)
-        st = run_with_workspace(lambda ws, n: lib.rbGemm(pp, e, pa, pb, pc, ws, n, stream), lambda: workspace_size(p), workspace,
-                                a.device, ask=variant is not None or saved != 0)
-    finally:
-        if variant is not None:
-            lib.rbSetGemmVariant(saved)
-    L.check(st)
+    e = C.byref(epilogue.to_c()) if epilogue is not None else None
+    pp, pa, pb, pc, stream = C.byref(p), a.data_ptr(), b.data_ptr(), out.data_ptr(), stream_address(a.device)
+    st = L.WORKSPACE_TOO_SMALL
+    if workspace is not None and variant is None and saved == 0:   # as run_with_workspace does, which small calls are too short for
+        st = lib.rbGemm(pp, e, pa, pb, pc, workspace.data_ptr(), workspace.nbytes, stream)
+    if st == L.WORKSPACE_TOO_SMALL:
+        try:
+            if variant is not None:   # before the workspace query: a K split or a stream-K tail changes what is needed
+                lib.rbSetGemmVariant(int(variant))
+            # (a stream-K tail, bit 9 of the variant word, is left out when its partial tiles do not fit the workspace)
+            st = run_with_workspace(lambda ws, n: lib.rbGemm(pp, e, pa, pb, pc, ws, n, stream), lambda: workspace_size(p), workspace,
+                                    a.device, ask=True)
+        finally:
+            if variant is not None:
+                lib.rbSetGemmVariant(saved)
+    if st != L.SUCCESS:
+        L.check(st)
     if a.dim() == 2 and b.dim() == 2:
-        out = out.view(shape[1], shape[2])
+        out = out.view(p.n, p.m) if trans_c else out.view(p.m, p.n)
     return out
 
 
