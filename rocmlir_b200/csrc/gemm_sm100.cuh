@@ -96,7 +96,8 @@ struct GemmParams {
   int c_type;
   int vec_ok;                 // rows of C start 16-byte aligned and c_stride_n == 1
   int c_tma;                  // rows of C go through a shared-memory staging tile: 1 = and from there by TMA stores, 2 = and are
-                              // copied out by the warp (rows off 16-byte boundaries, see copy_staged_rows); 0 = plain stores
+                              // copied out by the warp (rows off 16-byte boundaries or tiles narrower than a staged row, see copy_staged_rows); 0 = plain stores
+  int c_add;                  // f32, two K ranges: both are added to a C of zeros by TMA reductions (the order of two addends does not matter)
   EpiParams epi;
   uint32_t* status;
   unsigned long long* trace;  // optional [gridDim.x][16] cycle counters per CTA (see rbSetTraceBuffer), or NULL
@@ -805,7 +806,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       const long long row = row0 + lane;
       const bool row_ok = row < p.M;
       const int ngroups = p.bn / 32;
-      const int gz = w.split * p.G + (g ^ ((p.chain_flip >> 2) & 1));   // group coordinate of the store map (K-split planes are stacked groups)
+      const int gz = (KIND == kKindTF32 && p.c_add ? 0 : w.split * p.G) + (g ^ ((p.chain_flip >> 2) & 1));   // group coordinate of the store map (K-split planes are stacked groups)
       // Per-column scales / biases of this tile, converted to f32, in this warp's private copy.
       float* vec_scale = epi_vecs + q * (2 * kMaxBN);
       float* vec_bias = vec_scale + kMaxBN;
@@ -873,13 +874,28 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // 4-byte C (f32 results, raw i32 results, the raw planes of a K split): 32 columns = one staging row per step
       const bool fast32 = w.kind == 0 && p.c_tma && !probe &&
                           ((eflags == 0 && !p.acc_is_int && p.c_type == RB_F32) || raw_i32);
-      EpiStoreCtx ec;
-      ec.cmap = p.c_tma == 1 ? &maps.c : nullptr;
-      ec.dst = static_cast<uint8_t*>(p.c) + ((long long)w.split * p.split_stride + (long long)g * p.c_stride_g + row0 * p.c_stride_m) * es_c;
-      ec.pitch = p.c_stride_m; ec.es = es_c;
-      ec.staging = my_staging; ec.stg_bufs = stg_bufs;
-      ec.taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
-      ec.col0 = nb * p.bn; ec.bn = p.bn; ec.N = p.N; ec.M = p.M; ec.row0 = (int)row0; ec.gz = gz; ec.lane = lane;
+      // rows that are copied out: where they start in C (such launches run the EPI instantiation, see there)
+      auto copy_base = [&]() {
+        return static_cast<uint8_t*>(p.c) + ((long long)w.split * p.split_stride + (long long)g * p.c_stride_g + row0 * p.c_stride_m) * es_c;
+      };
+      auto copy_staged = [&](const uint8_t* stg, int n0) {
+        copy_staged_rows(stg, copy_base() + (long long)n0 * es_c, p.c_stride_m, es_c, min(32, p.M - (int)row0),
+                         min(min(p.N, (nb + 1) * p.bn) - n0, kRowBytes / es_c), lane);
+      };
+      auto store_map = [&](const uint8_t* stg, int n0) {
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0 && row0 < p.M) {
+          if (KIND == kKindTF32 && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
+          else tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
+          bulk_commit();
+        }
+      };
+      const bool copied = EPI && p.c_tma == 2 && (fast16 || fast32);
+      if (copied) {
+        epi_copy_tile(my_staging, tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN, copy_base(), p.c_stride_m, es_c, nb * p.bn,
+                      min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u);
+      } else
       if (fast16) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
         const int nsteps = p.bn / 64;
