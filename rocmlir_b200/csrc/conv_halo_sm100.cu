@@ -104,6 +104,7 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
   // EPI: the bias of every output channel as f32, behind the barriers (at most 256 channels: 1 KB of the region's 2 KB)
   float* vec_bias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);
   static_assert((2 * kHaloMaxStages + 6) * 8 <= 256, "barriers and the bias vector share one region");
+  const bool packed_bias = EPI && epi_packed_bias(p.epi, p.out_type) && epi_col_bias(p.epi.flags);   // biases kept as they are
   const int warp = warp_id_uniform();
   const long long wait_limit = p.wait_cycles;
 
@@ -120,7 +121,10 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
   if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.in); prefetch_tmap(&maps.fil); }
   if constexpr (EPI) {
     if (epi_col_bias(p.epi.flags))
-      for (int j = threadIdx.x; j < p.Kout; j += kHaloThreads) vec_bias[j] = load_bias(p.epi.bias, p.epi.bias_type, j);
+      for (int j = threadIdx.x; j < p.Kout; j += kHaloThreads) {
+        if (packed_bias) reinterpret_cast<uint16_t*>(vec_bias)[j] = __ldg(static_cast<const uint16_t*>(p.epi.bias) + j);
+        else vec_bias[j] = load_bias(p.epi.bias, p.epi.bias_type, j);
+      }
   }
   tc_fence_before();
   __syncthreads();
@@ -294,7 +298,7 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
           uint32_t v[32];
           tmem_ld32(taddr + c, v);
           tmem_ld_wait();
-          if constexpr (EPI) {
+          if (EPI && !packed_bias) {
             if (f_mid) round_row<32>(v, mid_type);
             if (f_alpha) {
 #pragma unroll
@@ -318,6 +322,7 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
           }
           uint32_t h[16];
           pack_row16<32>(v, h, to_bf16);
+          if (EPI && packed_bias) bias_row16<32>(h, reinterpret_cast<const uint32_t*>(vec_bias) + c / 2, to_bf16, f_relu);
           if (valid) {
             if (wide) {   // 32 bytes per store: half as many trips through the load/store unit
               st_global_v8(dst + c * 2, h);

@@ -79,6 +79,38 @@ __device__ __forceinline__ void pack_row16(const uint32_t* v, uint32_t* h, bool 
   }
 }
 
+// The commonest tail, [round to a 16-bit type] -> [+ bias of that type, round] -> [ReLU] with a result of that type, on packed pairs: the sum
+// of two f16 (bf16) values rounded to f32 and then to f16 is the one rounded at once (24 >= 2 x 11 + 2 bits), so this is bit for
+// bit what the steps in f32 give, in 3 instructions a pair instead of 11.
+__host__ __device__ __forceinline__ bool epi_packed_bias(const EpiParams& e, int c_type) {
+  return (e.flags & ~(uint32_t)RB_EPI_RELU) == (uint32_t)(RB_EPI_BIAS | RB_EPI_ROUND_MID) && (c_type == RB_F16 || c_type == RB_BF16) &&
+         e.mid_type == c_type && e.bias_type == c_type;
+}
+// h: N / 2 words of rounded values; bias2: as many of biases (shared memory, 16-byte aligned).
+template <int N>
+__device__ __forceinline__ void bias_row16(uint32_t* h, const uint32_t* bias2, bool is_bf16, bool relu) {
+#pragma unroll
+  for (int j = 0; j < N / 2; j += 4) {
+    const uint4 b4 = *reinterpret_cast<const uint4*>(bias2 + j);
+    const uint32_t b[4] = {b4.x, b4.y, b4.z, b4.w};
+    if (is_bf16) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        __nv_bfloat162 x = __hadd2_rn(*reinterpret_cast<__nv_bfloat162*>(&h[j + i]), *reinterpret_cast<const __nv_bfloat162*>(&b[i]));
+        if (relu) x = __hmax2(x, __nv_bfloat162(__float2bfloat16(0.0f), __float2bfloat16(0.0f)));
+        h[j + i] = *reinterpret_cast<uint32_t*>(&x);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        __half2 x = __hadd2_rn(*reinterpret_cast<__half2*>(&h[j + i]), *reinterpret_cast<const __half2*>(&b[i]));
+        if (relu) x = __hmax2(x, __half2(__float2half(0.0f), __float2half(0.0f)));
+        h[j + i] = *reinterpret_cast<uint32_t*>(&x);
+      }
+    }
+  }
+}
+
 // The MIGraphX unary elementwise ops in f32 (MIGraphX.td:134-181). sigmoid = 1 / (1 + exp(-x)) as
 // MIGraphXToTosa lowers it; recip and rsqrt are correctly rounded divisions / square roots, not the approximate forms.
 __device__ __forceinline__ float epi_unary(float x, int op) {

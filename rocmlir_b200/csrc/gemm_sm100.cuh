@@ -414,6 +414,35 @@ static __device__ __noinline__ uint32_t epi_requant8_tile(const EpiStoreCtx c, c
 // one run the EPI = false instantiation, in which every such branch folds away: the per-tile path of problems with a
 // short K loop follows the size of the code around it (measured: the pointwise C = 256 -> K = 64 layers lost 12 % and
 // 6 % when two never-executed fused loops were added to the one kernel, inlined or not).
+// The same for the commonest of those tails (epi_packed_bias), on packed pairs.
+template <typename Ctx>
+static __device__ __noinline__ uint32_t epi_bias16_tile(const Ctx c, bool relu, const uint32_t* bias2, int c_type, uint32_t nstores) {
+  const int nsteps = c.bn / 64;
+#pragma unroll 1
+  for (int cp = 0; cp < nsteps; ++cp) {
+    const int n0 = c.col0 + cp * 64;
+    if (n0 >= c.N) break;  // warp-uniform
+    uint32_t v[64];
+    tmem_ld64(c.taddr + cp * 64, v);
+    uint8_t* stg = c.staging + (c.stg_bufs == 2 ? (nstores & 1u) : 0u) * (32 * kRowBytes);
+    if (c.lane == 0 && nstores >= c.stg_bufs) {   // the store that last used this buffer has read it
+      if (c.stg_bufs == 2) bulk_wait_read<1>(); else bulk_wait_read<0>();
+    }
+    __syncwarp();
+    tmem_ld_wait();
+    uint32_t h[32];
+    pack_row16<64>(v, h, c_type == RB_BF16);
+    bias_row16<64>(h, bias2 + cp * 32, c_type == RB_BF16, relu);
+    uint8_t* rowp = stg + c.lane * kRowBytes;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+    emit_staged(c, stg, n0);
+    ++nstores;
+  }
+  return nstores;
+}
+
 template <int KIND, bool A_MN, bool B_MN, int CTAS, bool EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParams p) {
@@ -815,7 +844,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         for (int j = lane; j < p.bn; j += 32) {
           const int n = min(nb * p.bn + j, p.N - 1);
           if (eflags & RB_EPI_COL_SCALE) vec_scale[j] = __ldg(p.epi.col_scale + n);
-          if (epi_col_bias(eflags)) vec_bias[j] = load_bias(p.epi.bias, p.epi.bias_type, n);
+          if (packed_bias) reinterpret_cast<uint16_t*>(vec_bias)[j] = __ldg(static_cast<const uint16_t*>(p.epi.bias) + n);
+          else if (epi_col_bias(eflags)) vec_bias[j] = load_bias(p.epi.bias, p.epi.bias_type, n);
         }
         __syncwarp();
       }
@@ -838,6 +868,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
                        : nullptr;
       };
       // stream-K: 16-byte word i of column group c of this thread's row in the partial tile of unit u
+    // the tail on packed pairs, whose biases are kept as they are (every tile is a whole one then)
+    const bool packed_bias = EPI && epi_packed_bias(p.epi, p.c_type) && !p.acc_is_int && !two_planes && p.c_tma && p.sk_tiles == 0 && !probe;
       const int tile_row = (int)rank * kBM + q * 32 + lane;
       auto sk_word = [&](int u, int c, int i) -> uint4* {
         return reinterpret_cast<uint4*>(p.sk_partial) +
@@ -970,8 +1002,25 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       const bool fast8 = !fast16e && w.kind == 0 && p.c_tma && !probe && p.acc_is_int && p.c_type == RB_I8 &&
                          (eflags & ~(uint32_t)RB_EPI_ZP_OUT) == (uint32_t)(RB_EPI_COL_SCALE | RB_EPI_REQUANT);
       if (fast16e || fast8) {
-        if (fast16e) nstores = epi_fused16_tile(ec, eflags, p.epi.mid_type, p.epi.alpha, vec_bias, p.c_type, nstores);
-        else nstores = epi_requant8_tile(ec, vec_scale, p.epi.out_recip, p.epi.out_zero, nstores);
+        auto set_context = [&](EpiStoreCtx& ec) {
+          ec.cmap = &maps.c; ec.staging = my_staging; ec.stg_bufs = stg_bufs;
+          ec.taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
+          ec.col0 = nb * p.bn; ec.bn = p.bn; ec.N = p.N; ec.M = p.M; ec.row0 = (int)row0; ec.gz = gz; ec.lane = lane;
+        };
+        if (p.c_tma == 1) {
+          EpiStoreCtx ec;
+          set_context(ec);
+          if (packed_bias) nstores = epi_bias16_tile<EpiStoreCtx>(ec, (eflags & RB_EPI_RELU) != 0, reinterpret_cast<const uint32_t*>(vec_bias), p.c_type, nstores);
+          else if (fast16e) nstores = epi_fused16_tile<EpiStoreCtx>(ec, eflags, p.epi.mid_type, p.epi.alpha, vec_bias, p.c_type, nstores);
+          else nstores = epi_requant8_tile<EpiStoreCtx>(ec, vec_scale, p.epi.out_recip, p.epi.out_zero, nstores);
+        } else {
+          EpiCopyCtx ec;
+          set_context(ec);
+          ec.dst = copy_base(); ec.pitch = p.c_stride_m; ec.es = es_c;
+          if (packed_bias) nstores = epi_bias16_tile<EpiCopyCtx>(ec, (eflags & RB_EPI_RELU) != 0, reinterpret_cast<const uint32_t*>(vec_bias), p.c_type, nstores);
+          else if (fast16e) nstores = epi_fused16_tile<EpiCopyCtx>(ec, eflags, p.epi.mid_type, p.epi.alpha, vec_bias, p.c_type, nstores);
+          else nstores = epi_requant8_tile<EpiCopyCtx>(ec, vec_scale, p.epi.out_recip, p.epi.out_zero, nstores);
+        }
       }
       // Channel-major f32 result of a convolution (NKHW): one store per column, the warp's 32 lanes are 32 consecutive
       // pixels of the column's image plane
