@@ -230,7 +230,63 @@ struct GemmConfig {
 // TF32 planes per operand (see kMaxPlanes)
 int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_mode == 0 ? 2 : 1; }
 
-GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false) {
+// Tile and K split of a plain product by an estimate of its time, where nobody has asked for one. A launch costs `fixed`; a CTA (or
+// pair) then walks its tiles, K block by K block: at least `block` (operand fetch and issue of its MMAs), and no faster than all
+// CTAs together draw operands through the L2 -> SM fabric; a tile shorter than the store of the tile before it waits for that; the
+// last store is exposed. A K split adds the planes and the pass that sums them. Constants in microseconds, fitted to 24 products in up to
+// eleven configurations each (f16 / bf16 / fp8 / i8, 256^3 to 2048 x 2048 x 4096, replayed graphs; 8 % off on average; what a launch
+// costs by the width of its tiles has gone into `column`). The rule before - 256 columns in pairs whatever the size, a K split as soon as
+// half of the pairs idle - lost most where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.3 / 9.1
+// (64 columns, no split), 1536^3 bf16 28.8 / 16.9, 2048 x 1024 x 2048 f16 21.8 / 14.3, 364 x 1344 x 1792 i8 15.9 / 9.8. From three waves on the
+// rule stays: such products are bound by memory or by power.
+struct TileCost {
+  int ctas, bn;
+  double fixed, block, kb_per_block;   // kb_per_block: KB a CTA fetches per K block
+};
+constexpr TileCost kTileCosts[] = {{1, 64, 3.7, 0.252, 24}, {1, 128, 2.1, 0.326, 32}, {2, 128, 3.6, 0.246, 24}, {1, 256, 0.0, 0.404, 48}, {2, 256, 0.8, 0.335, 32}};
+
+// *ctas and *bn come in as the rule gives them and stay unless another tile, or no K split, is estimated at 15 % less.
+// f32 with two planes (the operand passes included); only where the rule does not cut K, so that no accumulation chain gets longer
+constexpr TileCost kTileCostsF32[] = {{1, 64, 6.9, 0.57, 48}, {1, 128, 5.3, 0.67, 64}, {2, 128, 6.4, 0.56, 48}, {1, 256, 5.5, 0.95, 96}, {2, 256, 4.4, 0.87, 64}};
+
+void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, int* ctas, int* bn, int* splits) {
+  // store of a column of a tile: an 8-bit result is requantised, rows off 16 bytes are copied out by the warps
+  const double column = 0.025 * (p->c_type == RB_I8 ? 1.56 : 1.0) * ((long long)p->n * (long long)dtype_bytes(p->c_type) % 16 ? 2.0 : 1.0);
+  auto estimate = [&](const TileCost& t, bool split, long long* s, long long* waves) {
+    const long long tiles = (long long)p->g * ((p->m + kBM * t.ctas - 1) / (kBM * t.ctas)) * ((p->n + t.bn - 1) / t.bn);
+    const long long units = sms / t.ctas;
+    *s = split && tiles * 2 <= units && kblocks >= 16 ? std::max<long long>(1, std::min<long long>(std::min(units / tiles, kblocks / 8), 128)) : 1;
+    const long long items = tiles * *s, kb = (kblocks + *s - 1) / *s;
+    *waves = (items + units - 1) / units;
+    const double busy = (double)std::min(items, units) * t.ctas;
+    const double block = std::max(t.block, busy * t.kb_per_block / 12500.0), store = t.bn * (*s > 1 ? 0.025 : column);
+    double us = t.fixed + std::max(kb * block, store) * (double)(*waves - 1) + kb * block + store;
+    if (*s > 1) us += 3.7 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.283;
+    return us;
+  };
+  const int rule_ctas = *ctas, rule_bn = *bn;
+  const bool f32 = p->ab_type == RB_F32;
+  const TileCost* const costs = f32 ? kTileCostsF32 : kTileCosts;
+  double best = 0;
+  long long s = 1, waves = 1;
+  for (int i = 0; i < 5; ++i) {
+    const TileCost& t = costs[i];
+    if (t.ctas == rule_ctas && t.bn == rule_bn) best = 0.85 * estimate(t, true, &s, &waves);
+  }
+  if (best == 0 || waves > 3 || (f32 && (s > 1 || p->k > 2048))) return;   // (s and waves are those of the rule's tile)
+  for (int i = 0; i < 5; ++i) {
+    const TileCost& t = costs[i];
+    if (f32 && t.ctas == 1 && t.bn == 256) continue;
+    if (b_mn && (t.bn / t.ctas) % che != 0) continue;
+    if (t.ctas == 2 && (p->m <= kBM || kblocks <= 2)) continue;   // (see choose_config)
+    for (int split = 0; split < (f32 ? 1 : 2); ++split) {
+      const double us = estimate(t, split != 0, &s, &waves);
+      if (us < best) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
+    }
+  }
+}
+
+GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false) {
   GemmConfig c;
   if (variant == 0) variant = (int)tuned_variant_gemm(p);   // the measured table, when it knows the problem
   const int es = (int)dtype_bytes(p->ab_type);
@@ -257,6 +313,9 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
     if (kb <= 2 && (variant & 0xF) != 2) c.ctas = 1;
   }
   if (c.bn == 64 && (variant & 0xF) != 2) c.ctas = 1;        // measured: 64-column tiles run faster unpaired (345 vs 324 TFLOP/s)
+  int est_splits = 0;
+  if (variant == 0 && !implicit && (p->ab_type != RB_F32 || planes == 2))
+    estimate_tile(p, b_mn, che, (p->k + kRowBytes / es - 1) / (kRowBytes / es), planned_sms(), &c.ctas, &c.bn, &est_splits);
   c.stages = (variant >> 4) & 0xF;
   const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec, planes) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec, planes);
   if (c.stages <= 0 || c.stages > max_stages) c.stages = max_stages;
@@ -274,7 +333,7 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   const long long kblocks = (p->k + bke - 1) / bke;
   const long long tiles = (long long)p->g * ((p->m + kBM * c.ctas - 1) / (kBM * c.ctas)) * ((p->n + c.bn - 1) / c.bn);
   const long long units = planned_sms() / c.ctas;
-  c.splits = (variant >> 16) & 0xFF;
+  c.splits = est_splits ? est_splits : (variant >> 16) & 0xFF;
   if (c.splits == 0) {
     c.splits = 1;
     if (tiles * 2 <= units && kblocks >= 16) {
@@ -474,7 +533,7 @@ size_t rb::gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand) {
   OperandPlan ob = plan_operand(p->trans_b == 0, p->n, p->k, es, f32, split);
   if (implicit_operand == 0) oa.needs_copy = false;
   if (implicit_operand == 1) ob.needs_copy = false;
-  return plan_workspace(p, oa, ob, choose_config(p, t_variant)).total;
+  return plan_workspace(p, oa, ob, choose_config(p, t_variant, false, implicit_operand >= 0)).total;
 }
 
 extern "C" size_t rbGemmWorkspaceSize(const RbGemmProblem* p) { return rb::gemm_workspace_bytes(p, -1); }
@@ -624,7 +683,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   }
   const bool a_mn = oa.mn_major, b_mn = ob.mn_major;
   const bool epi_vec = epi_needs_col_vectors(flags);
-  GemmConfig cfg = choose_config(p, t_variant, epi_vec);
+  GemmConfig cfg = choose_config(p, t_variant, epi_vec, conva != nullptr);
   Workspace ws = plan_workspace(p, oa, ob, cfg);
   if (cfg.sk_tiles > 0 && (!workspace || workspace_bytes < ws.total)) {
     // the stream-K tail is an optimisation: without room for its partial tiles every tile is computed whole
@@ -686,6 +745,13 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     return gemm_skinny_run(p, ep, a, b, c, kind, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, cfmt, t_wait_cycles, stall, stream_v);
   }
 
+  // Two K ranges of an f32 product (chains of at most 2048 elements, see choose_config): both are added to a C of zeros by TMA reductions
+  // instead of going through planes and a pass that sums them. 0 + x + y and 0 + y + x are the same number, so the result does not
+  // depend on which comes first; of three ranges it would. 4096^3: 668 us -> 632 in all.
+  const bool add_ranges = cfg.splits == 2 && is_f32 && p->c_type == RB_F32 && ep.flags == 0 && !p->trans_c && !cfg.plain_stores && !chain &&
+                          p->n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0;
+  if (add_ranges) RB_CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)p->g * p->m * p->n * sizeof(float), stream));
+
   uint8_t* wsb = static_cast<uint8_t*>(workspace);
   const void* a_src[2] = {a, nullptr};
   const void* b_src[2] = {b, nullptr};
@@ -745,13 +811,6 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   const bool a_fused = oa.mn_major && oa.cols % bke == 0 && oa.pitch == oa.cols;
   const bool b_fused = ob.mn_major && ob.cols % bke == 0 && ob.pitch == ob.cols;
   auto encode_operand = [&](CUtensorMap* m, const void* base, const OperandPlan& o, int box_rows_kmajor,
-  // Two K ranges of an f32 product (chains of at most 2048 elements, see choose_config): both are added to a C of zeros by TMA reductions
-  // instead of going through planes and a pass that sums them. 0 + x + y and 0 + y + x are the same number, so the result does not
-  // depend on which comes first; of three ranges it would. 4096^3: 668 us -> 632 in all.
-  const bool add_ranges = cfg.splits == 2 && is_f32 && p->c_type == RB_F32 && ep.flags == 0 && !p->trans_c && !cfg.plain_stores && !chain &&
-                          p->n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0;
-  if (add_ranges) RB_CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)p->g * p->m * p->n * sizeof(float), stream));
-
                             std::string* err) {
     const bool fused = (&o == &oa) ? a_fused : b_fused;
     const int ci = (&o == &oa) ? 0 : 1;
@@ -833,7 +892,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     // rows off 16-byte boundaries: staged like the others, copied out by the warps (us, element stores from the registers before): 3 x 640 x
     // 2279, K = 768, bf16 with bias and ReLU 182 -> 51; 2000 x 3001 x 640 97 -> 33; 4096 x 4095 x 4096 f16 228 -> 127; f32 768 x 1043 x 3648
     // 102 -> 70
-    kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok ? 1 : 2;
+    // (and so is an 8-bit result in tiles of 64 columns: the box of the store map is a staged row, 128 of them)
+    kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok && bn * es_c >= (size_t)kRowBytes ? 1 : 2;
     if (conva && conva->c_rows_per_img > 0) {   // NKHW result: strided element stores, coalesced along the pixels
       kp.c_rows_per_img = conva->c_rows_per_img;
       kp.c_img_stride = conva->c_img_stride;
@@ -859,6 +919,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     if (!encode_tiled(&maps.c, cdt, 3, cbase, cdims, cstrides, cbox, CU_TENSOR_MAP_SWIZZLE_128B, &err))
       return fail(RB_UNSUPPORTED, "C: " + err);
   }
+  kp.c_add = add_ranges ? 1 : 0;
   kp.status = dev->status_word;
   kp.stages = stages;
   kp.kpr = cfg.kpr;
@@ -896,8 +957,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     kp.sk_token = next_token.fetch_add(1, std::memory_order_relaxed);
   }
 
-  // the instantiation with the fused elementwise code only when this launch has such work (see gemm_tcgen05_kernel)
-  const bool epi_kernel = kp.epi.flags != 0;
+  // the instantiation with the fused elementwise code and the copied rows only when this launch has such work (see gemm_tcgen05_kernel)
+  const bool epi_kernel = kp.epi.flags != 0 || kp.c_tma == 2;
   GemmKernel kern = epi_kernel ? (ctas == 2 ? pick_kernel<2, true>(kind, a_mn, b_mn) : pick_kernel<1, true>(kind, a_mn, b_mn))
                                : (ctas == 2 ? pick_kernel<2, false>(kind, a_mn, b_mn) : pick_kernel<1, false>(kind, a_mn, b_mn));
   const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
@@ -919,7 +980,6 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   ++lc.numAttrs;
   if (ctas == 2) {
     attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
-  kp.c_add = add_ranges ? 1 : 0;
     attr[lc.numAttrs].val.clusterDim.x = 2; attr[lc.numAttrs].val.clusterDim.y = 1; attr[lc.numAttrs].val.clusterDim.z = 1;
     ++lc.numAttrs;
     const int pairs = dev->sm_count / 2;

@@ -246,16 +246,20 @@ struct WorkIter {
 // never executed by such a problem - the C = 256 -> K = 64 pointwise layers lost 12 % (forward) and 6 % (backward data).
 // They are therefore separate functions, called by the tiles that need them.
 struct EpiStoreCtx {
-  const CUtensorMap* cmap;   // store map of C, or nullptr: the staged rows are copied out from here
-  uint8_t* dst;              // without a map: C at (row0, column 0 of the matrix), its pitch in elements, bytes per element
-  long long pitch;
-  int es;
+  const CUtensorMap* cmap;   // store map of C
   uint8_t* staging;          // this warp's staging buffers
   uint32_t stg_bufs;         // 1 or 2
   uint32_t taddr;            // this warp's quarter of the accumulator buffer
   int col0;                  // first column of the tile
   int bn, N, M;
   int row0, gz, lane;
+};
+// The same for rows that are copied out of the staging buffers. Instantiations of their own of the loops below: with both ends in one
+// loop aligned results were 3 to 7 % slower.
+struct EpiCopyCtx : EpiStoreCtx {
+  uint8_t* dst;              // C at (row0, column 0 of the matrix), its pitch in elements, bytes per element
+  long long pitch;
+  int es;
 };
 
 // Copies the staged rows of a warp (32 rows of 128 bytes, 16-byte pieces XOR-swizzled by the row) to rows of C that start
@@ -293,7 +297,15 @@ __device__ __forceinline__ void copy_rows(const uint8_t* stg, T* dst, long long 
 static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t* dst, long long pitch, int es, int rows, int cols,
                                                      int lane) {
   __syncwarp();
-  if (es == 2) copy_rows(stg, reinterpret_cast<uint16_t*>(dst), pitch, rows, cols, lane);
+  const int bytes = cols * es;
+  if (((reinterpret_cast<uintptr_t>(dst) | (uintptr_t)(pitch * es) | (uintptr_t)bytes) & 15) == 0) {
+    // aligned after all, but not whole 128-byte rows (an 8-bit tile of 64 columns): 16 bytes at a time
+    const int pieces = bytes >> 4;
+    for (int i = lane; i < rows * pieces; i += 32) {
+      const int r = i / pieces, j = i - r * pieces;
+      *reinterpret_cast<uint4*>(dst + r * pitch * es + j * 16) = *reinterpret_cast<const uint4*>(stg + r * kRowBytes + ((j ^ (r & 7)) << 4));
+    }
+  } else if (es == 2) copy_rows(stg, reinterpret_cast<uint16_t*>(dst), pitch, rows, cols, lane);
   else if (es == 4) copy_rows(stg, reinterpret_cast<uint32_t*>(dst), pitch, rows, cols, lane);
   else copy_rows(stg, dst, pitch, rows, cols, lane);
   __syncwarp();
@@ -301,21 +313,57 @@ static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t
 
 // The staged rows of this warp, whose first column is n0, on their way to C.
 __device__ __forceinline__ void emit_staged(const EpiStoreCtx& c, const uint8_t* stg, int n0) {
-  if (c.cmap) {
-    fence_proxy_async();
-    __syncwarp();
-    if (c.lane == 0 && c.row0 < c.M) {
-      tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
-      bulk_commit();
+  fence_proxy_async();
+  __syncwarp();
+  if (c.lane == 0 && c.row0 < c.M) {
+    tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
+    bulk_commit();
+  }
+}
+__device__ __forceinline__ void emit_staged(const EpiCopyCtx& c, const uint8_t* stg, int n0) {
+  copy_staged_rows(stg, c.dst + (long long)n0 * c.es, c.pitch, c.es, min(32, c.M - c.row0), min(min(c.N, c.col0 + c.bn) - n0, kRowBytes / c.es),
+                   c.lane);
+}
+
+// Rows without fused work that are copied out: 16-bit C, or 32-bit words as they are (f32 with `small_cols` columns further on its small
+// accumulator, added with round-to-nearest; raw i32; the planes of a K split). Out of line, so that the loops of aligned rows stay short.
+static __device__ __noinline__ void epi_copy_tile(uint8_t* staging, uint32_t taddr, uint8_t* dst, long long pitch, int es, int col0, int col_end,
+                                                  int rows, int lane, int c_type, bool bits32, uint32_t small_cols) {
+  const int width = bits32 ? 32 : 64;   // columns of a staged row
+  uint8_t* rowp = staging + lane * kRowBytes;
+#pragma unroll 1
+  for (int n0 = col0; n0 < col_end; n0 += width, taddr += width) {
+    if (bits32) {
+      uint32_t v[32];
+      tmem_ld32(taddr, v);
+      tmem_ld_wait();
+      if (small_cols) {
+        uint32_t u[32];
+        tmem_ld32(taddr + small_cols, u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else {
+      uint32_t v[64], h[32];
+      tmem_ld64(taddr, v);
+      tmem_ld_wait();
+      pack_row16<64>(v, h, c_type == RB_BF16);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
     }
-  } else {
-    copy_staged_rows(stg, c.dst + (long long)n0 * c.es, c.pitch, c.es, min(32, c.M - c.row0), c.N - n0, c.lane);
+    copy_staged_rows(staging, dst + (long long)n0 * es, pitch, es, rows, min(col_end - n0, width), lane);
   }
 }
 
 // 16-bit C from float accumulators with the common float tails: [round to mid] -> [x alpha] -> [+ bias[n], round to mid]
 // -> [ReLU] -> convert; the operations and their order are those of epi_apply32. Returns the updated store count.
-static __device__ __noinline__ uint32_t epi_fused16_tile(const EpiStoreCtx c, uint32_t flags, int mid_type, float alpha,
+template <typename Ctx>
+static __device__ __noinline__ uint32_t epi_fused16_tile(const Ctx c, uint32_t flags, int mid_type, float alpha,
                                                          const float* vec_bias, int c_type, uint32_t nstores) {
   const bool f_mid = (flags & RB_EPI_ROUND_MID) != 0, f_alpha = (flags & RB_EPI_ALPHA) != 0;
   const bool f_bias = (flags & RB_EPI_BIAS) != 0, f_relu = (flags & RB_EPI_RELU) != 0;
@@ -366,9 +414,39 @@ static __device__ __noinline__ uint32_t epi_fused16_tile(const EpiStoreCtx c, ui
   return nstores;
 }
 
+// The same for the commonest of those tails (epi_packed_bias), on packed pairs.
+template <typename Ctx>
+static __device__ __noinline__ uint32_t epi_bias16_tile(const Ctx c, bool relu, const uint32_t* bias2, int c_type, uint32_t nstores) {
+  const int nsteps = c.bn / 64;
+#pragma unroll 1
+  for (int cp = 0; cp < nsteps; ++cp) {
+    const int n0 = c.col0 + cp * 64;
+    if (n0 >= c.N) break;  // warp-uniform
+    uint32_t v[64];
+    tmem_ld64(c.taddr + cp * 64, v);
+    uint8_t* stg = c.staging + (c.stg_bufs == 2 ? (nstores & 1u) : 0u) * (32 * kRowBytes);
+    if (c.lane == 0 && nstores >= c.stg_bufs) {   // the store that last used this buffer has read it
+      if (c.stg_bufs == 2) bulk_wait_read<1>(); else bulk_wait_read<0>();
+    }
+    __syncwarp();
+    tmem_ld_wait();
+    uint32_t h[32];
+    pack_row16<64>(v, h, c_type == RB_BF16);
+    bias_row16<64>(h, bias2 + cp * 32, c_type == RB_BF16, relu);
+    uint8_t* rowp = stg + c.lane * kRowBytes;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+    emit_staged(c, stg, n0);
+    ++nstores;
+  }
+  return nstores;
+}
+
 // Quantised linear layer: i32 accumulator x scale[n] x 1 / output scale -> i8 (round half even, saturate, plus the
 // output zero point). 32 columns are 32 bytes of a staging row; four groups make one 128-byte-wide store.
-static __device__ __noinline__ uint32_t epi_requant8_tile(const EpiStoreCtx c, const float* vec_scale, float recip, int zp,
+template <typename Ctx>
+static __device__ __noinline__ uint32_t epi_requant8_tile(const Ctx c, const float* vec_scale, float recip, int zp,
                                                           uint32_t nstores) {
   const int ngroups = c.bn / 32;
 #pragma unroll 1
@@ -410,39 +488,11 @@ static __device__ __noinline__ uint32_t epi_requant8_tile(const EpiStoreCtx c, c
 }
 
 
-// EPI: the instantiation that carries the fused elementwise epilogues (RbEpilogue flags, C += A.B). Launches without
-// one run the EPI = false instantiation, in which every such branch folds away: the per-tile path of problems with a
+// EPI: the instantiation that carries the fused elementwise epilogues (RbEpilogue flags, C += A.B) and the rows that are copied out
+// (GemmParams::c_tma == 2; in the other instantiation, never taken, they cost those layers 5 to 8 %). Launches without
+// either run the EPI = false instantiation, in which every such branch folds away: the per-tile path of problems with a
 // short K loop follows the size of the code around it (measured: the pointwise C = 256 -> K = 64 layers lost 12 % and
 // 6 % when two never-executed fused loops were added to the one kernel, inlined or not).
-// The same for the commonest of those tails (epi_packed_bias), on packed pairs.
-template <typename Ctx>
-static __device__ __noinline__ uint32_t epi_bias16_tile(const Ctx c, bool relu, const uint32_t* bias2, int c_type, uint32_t nstores) {
-  const int nsteps = c.bn / 64;
-#pragma unroll 1
-  for (int cp = 0; cp < nsteps; ++cp) {
-    const int n0 = c.col0 + cp * 64;
-    if (n0 >= c.N) break;  // warp-uniform
-    uint32_t v[64];
-    tmem_ld64(c.taddr + cp * 64, v);
-    uint8_t* stg = c.staging + (c.stg_bufs == 2 ? (nstores & 1u) : 0u) * (32 * kRowBytes);
-    if (c.lane == 0 && nstores >= c.stg_bufs) {   // the store that last used this buffer has read it
-      if (c.stg_bufs == 2) bulk_wait_read<1>(); else bulk_wait_read<0>();
-    }
-    __syncwarp();
-    tmem_ld_wait();
-    uint32_t h[32];
-    pack_row16<64>(v, h, c_type == RB_BF16);
-    bias_row16<64>(h, bias2 + cp * 32, c_type == RB_BF16, relu);
-    uint8_t* rowp = stg + c.lane * kRowBytes;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      *reinterpret_cast<uint4*>(rowp + ((i ^ (c.lane & 7)) << 4)) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
-    emit_staged(c, stg, n0);
-    ++nstores;
-  }
-  return nstores;
-}
-
 template <int KIND, bool A_MN, bool B_MN, int CTAS, bool EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParams p) {
@@ -817,6 +867,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
     const bool raw_i32 = p.acc_is_int && p.c_type == RB_I32 && eflags == 0;
     const uint32_t stg_bufs = epi_vec ? 1u : 2u;   // staging buffers per warp
     uint8_t* my_staging = staging + q * stg_bufs * L::kStoreTileBytes;
+    // the tail on packed pairs, whose biases are kept as they are (every tile is a whole one then)
+    const bool packed_bias = EPI && epi_packed_bias(p.epi, p.c_type) && !p.acc_is_int && !two_planes && p.c_tma && p.sk_tiles == 0 && !probe;
     uint32_t t = 0, nstores = 0;
     long long w_tfull = 0, e_work = 0, e_ld = 0, e_cv = 0;
     WorkIter it(p, pair_id, num_pairs);
@@ -868,8 +920,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
                        : nullptr;
       };
       // stream-K: 16-byte word i of column group c of this thread's row in the partial tile of unit u
-    // the tail on packed pairs, whose biases are kept as they are (every tile is a whole one then)
-    const bool packed_bias = EPI && epi_packed_bias(p.epi, p.c_type) && !p.acc_is_int && !two_planes && p.c_tma && p.sk_tiles == 0 && !probe;
       const int tile_row = (int)rank * kBM + q * 32 + lane;
       auto sk_word = [&](int u, int c, int i) -> uint4* {
         return reinterpret_cast<uint4*>(p.sk_partial) +
@@ -966,7 +1016,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
               *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
             }
           }
-          emit_staged(ec, stg, n0);
+          store_map(stg, n0);
           ++nstores;
         }
       } else if (fast32) {
@@ -986,7 +1036,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
 #pragma unroll
           for (int i = 0; i < 8; ++i)
             *reinterpret_cast<uint4*>(rowp + ((i ^ (lane & 7)) << 4)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          emit_staged(ec, stg, n0);
+          store_map(stg, n0);
           ++nstores;
         }
       }
@@ -1080,7 +1130,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            emit_staged(ec, stg, n0 - sub * 32);
+            if (EPI && p.c_tma == 2) copy_staged(stg, n0 - sub * 32);
+            else store_map(stg, n0 - sub * 32);
             ++nstores;
           }
         }
@@ -1166,7 +1217,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            if (!(probe & 4)) emit_staged(ec, stg, n0 - sub * 32);
+            if (EPI && p.c_tma == 2) copy_staged(stg, n0 - sub * 32);
+            else if (!(probe & 4)) store_map(stg, n0 - sub * 32);
             ++nstores;
           }
         } else if (nw > 0 && row_ok && !(probe & 4)) {

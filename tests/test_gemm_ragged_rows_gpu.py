@@ -58,3 +58,17 @@ def test_fused_tails_equal_element_stores(cuda_device, g, m, n, k, off):
         got = [run(a, b, out, off, epilogue=Epilogue(**kw), variant=v) for v in (1, 1 | PLAIN)]
         assert torch.equal(got[0], got[1]), (dt, out, kw.keys())
     assert L.kernel_status() == 0
+
+
+@pytest.mark.parametrize("m,n", [(64, 128), (33, 192), (200, 80), (130, 1344), (128, 65)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_eight_bit_results_in_narrow_tiles(cuda_device, m, n, off):
+    """Tiles of 64 columns are half of a staged row of bytes: they do not touch the columns of their neighbours."""
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200.gemm import Epilogue
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    a, b = (torch.randint(-9, 10, (1, r, 256), device="cuda", generator=gen).to(torch.int8) for r in (m, n))
+    epi = Epilogue(col_scale=torch.rand(n, device="cuda", generator=gen), requant_scale=3.0)
+    got = [run(a, b, torch.int8, off, epilogue=epi, variant=v) for v in (0x1001, 0x2001 | PLAIN)]   # 64 columns, 128
+    assert torch.equal(got[0], got[1]) and L.kernel_status() == 0
