@@ -673,7 +673,7 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
   if (p->direction == 0 && !pl->c_direct && pl->a_implicit && G == 1 && pl->os[4] == 1 && pl->os[3] == wo &&
       pl->os[2] == ho * wo && pl->os[0] == (long long)p->k * ho * wo) {
     RbGemmConfigInfo info;
-    if (rbGemmGetConfig(&gp, &info) == RB_SUCCESS && info.splits == 1) {
+    if (gemm_config(&gp, 0, &info) == RB_SUCCESS && info.splits == 1) {
       pl->c_remap = true;
       pl->c_bytes = 0;
     }
@@ -775,6 +775,12 @@ extern "C" RbStatus rbConvGetGemmProblem(const RbConvProblem* p, RbGemmProblem* 
   if (!out) return fail(RB_INVALID_PARAM, "out is NULL");
   *out = pl.gemm;
   return RB_SUCCESS;
+}
+
+RbStatus rb::conv_gemm_config(const RbConvProblem* p, RbGemmConfigInfo* out) {
+  ConvPlan pl;
+  const RbStatus st = make_plan(p, &pl);
+  return st == RB_SUCCESS ? gemm_config(&pl.gemm, pl.a_implicit ? 0 : pl.b_implicit ? 1 : -1, out) : st;
 }
 
 extern "C" int rbConvKernelCount(const RbConvProblem* p) {

@@ -554,11 +554,13 @@ RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int 
   return RB_SUCCESS;
 }
 
-extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* out) {
+extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* out) { return rb::gemm_config(p, -1, out); }
+
+RbStatus rb::gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmConfigInfo* out) {
   RbStatus st = check_problem(p);
   if (st != RB_SUCCESS) return st;
   if (!out) return fail(RB_INVALID_PARAM, "out is NULL");
-  const GemmConfig c = choose_config(p, t_variant);
+  const GemmConfig c = choose_config(p, t_variant, false, implicit_operand >= 0);
   const int es = (int)dtype_bytes(p->ab_type);
   const long long tiles = (long long)p->g * ((p->m + kBM * c.ctas - 1) / (kBM * c.ctas)) * ((p->n + c.bn - 1) / c.bn);
   const long long items = tiles * c.splits;
@@ -577,7 +579,7 @@ extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* ou
                                               : GemmSmemLayout<1>::total(c.stages, c.bn, false, gemm_planes(p)));
   // with per-column epilogue vectors (bias / column scales) the ring may be one stage shorter and the staging single
   {
-    const GemmConfig ce = choose_config(p, t_variant, true);
+    const GemmConfig ce = choose_config(p, t_variant, true, implicit_operand >= 0);
     out->stages_epi_vec = ce.stages;
     out->dynamic_smem_epi_vec = (uint32_t)(ce.ctas == 2 ? GemmSmemLayout<2>::total(ce.stages, ce.bn, true, gemm_planes(p))
                                                         : GemmSmemLayout<1>::total(ce.stages, ce.bn, true, gemm_planes(p)));

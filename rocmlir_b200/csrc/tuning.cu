@@ -106,7 +106,7 @@ void build_space(const ProblemDesc& d, RbTuningParamSetKind kind, Space* sp) {
   const int saved = rbGetGemmVariant();
   rbSetGemmVariant(0);
   RbGemmConfigInfo own;
-  const bool have_own = rbGemmGetConfig(&gp, &own) == RB_SUCCESS;
+  const bool have_own = (d.kind == kConv ? rb::conv_gemm_config(&d.conv, &own) : rbGemmGetConfig(&gp, &own)) == RB_SUCCESS;
   rbSetGemmVariant(saved);
   std::set<uint32_t> seen_q, seen;
   if (have_own) {
