@@ -17,6 +17,8 @@
 //   * the filter stays in shared memory in the same form for all tiles of the persistent CTA, tcgen05.mma accumulates
 //     into one of two TMEM buffers, and the previous tile's result is stored while the tensor core works.
 //
+// (Images of up to 24 channels take conv_window_sm100.cu where its estimate is the lower one.)
+//
 // Bound: the gather (one 2-byte read per element of the operand for three channels), then HBM writes of the result. Two
 // CTAs per SM overlap one's gather with the other's stores and waits. N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2,
 // f16 channels last: 1826 us through the im2col matrix, 102 here. (152 with 64-bit tile arithmetic and element reads: the kernel
