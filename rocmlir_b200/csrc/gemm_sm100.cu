@@ -747,12 +747,14 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     return gemm_skinny_run(p, ep, a, b, c, kind, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, cfmt, t_wait_cycles, stall, stream_v);
   }
 
-  // Two K ranges of an f32 product (chains of at most 2048 elements, see choose_config): both are added to a C of zeros by TMA reductions
-  // instead of going through planes and a pass that sums them. 0 + x + y and 0 + y + x are the same number, so the result does not
-  // depend on which comes first; of three ranges it would. 4096^3: 668 us -> 632 in all.
-  const bool add_ranges = cfg.splits == 2 && is_f32 && p->c_type == RB_F32 && ep.flags == 0 && !p->trans_c && !cfg.plain_stores && !chain &&
+  // Two K ranges of an f32 product in full accuracy: both are added to a C of zeros by TMA reductions instead of going through planes and a
+  // pass that sums them. 0 + x + y and 0 + y + x are the same number, so the result does not depend on which comes first; of three
+  // ranges it would. Subnormal partial sums and results are kept (tests/test_gemm_f32_ranges_gpu.py). 4096^3: 668 us -> 632 in all.
+  // C is cleared right before the launch: by then both operands have been read into their planes (hence full accuracy only; a single TF32
+  // pass may read them in place), so C may lie over one of them as with any other number of ranges. The workspace query knows neither C's
+  // address nor the epilogue and counts the planes all the same.
+  const bool add_ranges = cfg.splits == 2 && split && p->c_type == RB_F32 && ep.flags == 0 && !p->trans_c && !cfg.plain_stores && !chain &&
                           p->n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0;
-  if (add_ranges) RB_CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)p->g * p->m * p->n * sizeof(float), stream));
 
   uint8_t* wsb = static_cast<uint8_t*>(workspace);
   const void* a_src[2] = {a, nullptr};
@@ -1009,6 +1011,10 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     return RB_SUCCESS;
   }
   kp.trace = trace_buffer((size_t)lc.gridDim.x * 16);
+  if (add_ranges) {
+    attr[0].val.programmaticStreamSerializationAllowed = 0;   // (nothing to set up early: what runs before is the clearing)
+    RB_CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)p->g * p->m * p->n * sizeof(float), stream));
+  }
   RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
   count_launch();
   if (splits > 1 && !add_ranges) {
