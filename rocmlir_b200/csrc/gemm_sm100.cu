@@ -1,7 +1,7 @@
 // Host side of rbGemm: validates a rock.gemm problem, prepares operands that TMA cannot address
 // directly (row pitch not a multiple of 16 bytes -> padded copy in the caller's workspace; f32 ->
 // TF32 hi/lo split), encodes the tensor maps and launches the persistent tcgen05 kernel.
-#include "gemm_sm100.cuh"
+#include "gemm_pick.cuh"
 
 #include <atomic>
 #include <cstdio>
@@ -188,26 +188,6 @@ void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaSt
   const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * 32);
   f32_prepare_kernel<<<grid, 256, 0, stream>>>(jobs);
   count_launch();
-}
-
-// ---- dispatch ----------------------------------------------------------------------------------------
-typedef void (*GemmKernel)(const GemmTensorMaps, const GemmParams);
-
-template <int KIND, int CTAS, bool EPI>
-GemmKernel pick_major(bool a_mn, bool b_mn) {
-  if (!a_mn && !b_mn) return gemm_tcgen05_kernel<KIND, false, false, CTAS, EPI>;
-  if (!a_mn && b_mn) return gemm_tcgen05_kernel<KIND, false, true, CTAS, EPI>;
-  if (a_mn && !b_mn) return gemm_tcgen05_kernel<KIND, true, false, CTAS, EPI>;
-  return gemm_tcgen05_kernel<KIND, true, true, CTAS, EPI>;
-}
-template <int CTAS, bool EPI>
-GemmKernel pick_kernel(int kind, bool a_mn, bool b_mn) {
-  switch (kind) {
-    case kKindF16: return pick_major<kKindF16, CTAS, EPI>(a_mn, b_mn);
-    case kKindTF32: return gemm_tcgen05_kernel<kKindTF32, false, false, CTAS, EPI>;  // f32 operands are made K-major first
-    case kKindI8: return pick_major<kKindI8, CTAS, EPI>(a_mn, b_mn);
-    default: return pick_major<kKindF8, CTAS, EPI>(a_mn, b_mn);
-  }
 }
 
 // ---- tile configuration -----------------------------------------------------------------------
@@ -599,10 +579,10 @@ extern "C" RbStatus rbGemm(const RbGemmProblem* p, const RbEpilogue* epi, const 
 }
 
 // Name of an instantiation of gemm_tcgen05_kernel inside the cubin image (Itanium mangling of
-// rb::gemm_tcgen05_kernel<KIND, A_MN, B_MN, CTAS, EPI>(GemmTensorMaps, GemmParams)).
-static std::string kernel_symbol(int kind, bool a_mn, bool b_mn, int ctas, bool epi) {
+// rb::gemm_tcgen05_kernel<KIND, A_MN, B_MN, CTAS, TAIL>(GemmTensorMaps, GemmParams)).
+static std::string kernel_symbol(int kind, bool a_mn, bool b_mn, int ctas, int tail) {
   return "_ZN2rb19gemm_tcgen05_kernelILi" + std::to_string(kind) + "ELb" + (a_mn ? "1" : "0") + "ELb" + (b_mn ? "1" : "0") +
-         "ELi" + std::to_string(ctas) + "ELb" + (epi ? "1" : "0") + "EEEvNS_14GemmTensorMapsENS_10GemmParamsE";
+         "ELi" + std::to_string(ctas) + "ELi" + std::to_string(tail) + "EEEvNS_14GemmTensorMapsENS_10GemmParamsE";
 }
 
 RbStatus rb::check_epilogue(const RbEpilogue* epi, int c_type) {
@@ -961,10 +941,11 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     kp.sk_token = next_token.fetch_add(1, std::memory_order_relaxed);
   }
 
-  // the instantiation with the fused elementwise code and the copied rows only when this launch has such work (see gemm_tcgen05_kernel)
-  const bool epi_kernel = kp.epi.flags != 0 || kp.c_tma == 2;
-  GemmKernel kern = epi_kernel ? (ctas == 2 ? pick_kernel<2, true>(kind, a_mn, b_mn) : pick_kernel<1, true>(kind, a_mn, b_mn))
-                               : (ctas == 2 ? pick_kernel<2, false>(kind, a_mn, b_mn) : pick_kernel<1, false>(kind, a_mn, b_mn));
+  // fused elementwise code and copied rows only in launches that have such work (see GemmTail)
+  const int tail = kp.c_tma == 2 ? kTailCopied : kp.epi.flags != 0 ? kTailFused : kTailNone;
+  const GemmKernel kern = tail == kTailCopied  ? gemm_kernel_copied(kind, a_mn, b_mn, ctas)
+                          : tail == kTailFused ? gemm_kernel_fused(kind, a_mn, b_mn, ctas)
+                                               : gemm_kernel_plain(kind, a_mn, b_mn, ctas);
   const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
   const int smem = ctas == 2 ? GemmSmemLayout<2>::total(stages, bn, kernel_epi_vec, planes) : GemmSmemLayout<1>::total(stages, bn, kernel_epi_vec, planes);
   {
@@ -994,7 +975,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   if (capture) {
     static_assert(sizeof(GemmTensorMaps) + sizeof(GemmParams) + 64 <= sizeof(capture->params), "parameter block too small");
     memset(capture, 0, sizeof(*capture));
-    const std::string sym = kernel_symbol(kind, kind == kKindTF32 ? false : a_mn, kind == kKindTF32 ? false : b_mn, ctas, epi_kernel);
+    const std::string sym = kernel_symbol(kind, kind == kKindTF32 ? false : a_mn, kind == kKindTF32 ? false : b_mn, ctas, tail);
     snprintf(capture->symbol, sizeof(capture->symbol), "%s", sym.c_str());
     capture->grid = lc.gridDim.x;
     capture->block = kGemmThreads;

@@ -488,15 +488,20 @@ static __device__ __noinline__ uint32_t epi_requant8_tile(const Ctx c, const flo
 }
 
 
-// EPI: the instantiation that carries the fused elementwise epilogues (RbEpilogue flags, C += A.B) and the rows that are copied out
-// (GemmParams::c_tma == 2; in the other instantiation, never taken, they cost those layers 5 to 8 %). Launches without
-// either run the EPI = false instantiation, in which every such branch folds away: the per-tile path of problems with a
-// short K loop follows the size of the code around it (measured: the pointwise C = 256 -> K = 64 layers lost 12 % and
-// 6 % when two never-executed fused loops were added to the one kernel, inlined or not).
-template <int KIND, bool A_MN, bool B_MN, int CTAS, bool EPI>
+// TAIL: what a launch does between accumulator and C. kTailNone: nothing but a conversion; every branch for fused work folds away, since the
+// per-tile path of problems with a short K loop follows the size of the code around it (measured: the pointwise C = 256 -> K = 64
+// layers lost 12 % and 6 % when two never-executed fused loops were added to the one kernel, inlined or not). kTailFused: the elementwise
+// epilogues (RbEpilogue flags, C += A.B). kTailCopied: rows that are copied out (GemmParams::c_tma == 2), with or without those. In the plain
+// instantiation, never taken, the copying code cost pointwise layers 5 to 8 %; in the fused one it cost every launch 70 to 90 bytes of
+// spilled registers (2048 x 11008 x 4096 i8, requantised: 82.8 -> 83.7 us).
+enum GemmTail { kTailNone = 0, kTailFused = 1, kTailCopied = 2 };
+template <int KIND, bool A_MN, bool B_MN, int CTAS, int TAIL>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParams p) {
+  constexpr bool EPI = TAIL != kTailNone, COPY = TAIL == kTailCopied;
   const uint32_t eflags = EPI ? p.epi.flags : 0u;   // compile-time zero without EPI
+  const int c_tma = COPY ? 2 : p.c_tma;             // 0 or 1 otherwise
+  const bool acc_is_int = EPI ? KIND == kKindI8 : p.acc_is_int != 0;   // (the plain instantiation keeps the code it was measured with)
   using KT = KindTraits<KIND>;
   using L = GemmSmemLayout<CTAS>;
   constexpr int ES = KT::ES;
@@ -555,7 +560,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       prefetch_tmap(&maps.a[s]);
       prefetch_tmap(&maps.b[s]);
     }
-    if (p.c_tma == 1) prefetch_tmap(&maps.c);
+    if (c_tma == 1) prefetch_tmap(&maps.c);
   }
   tc_fence_before();
   __syncthreads();
@@ -864,11 +869,11 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
     const int es_c = dtype_size(p.c_type);
     const int cols_per_store = kRowBytes / es_c;          // columns covered by one 128-byte staging row
     const int groups_per_store = cols_per_store / 32;     // 32-column TMEM loads per staging row: 1, 2 or 4
-    const bool raw_i32 = p.acc_is_int && p.c_type == RB_I32 && eflags == 0;
+    const bool raw_i32 = acc_is_int && p.c_type == RB_I32 && eflags == 0;
     const uint32_t stg_bufs = epi_vec ? 1u : 2u;   // staging buffers per warp
     uint8_t* my_staging = staging + q * stg_bufs * L::kStoreTileBytes;
     // the tail on packed pairs, whose biases are kept as they are (every tile is a whole one then)
-    const bool packed_bias = EPI && epi_packed_bias(p.epi, p.c_type) && !p.acc_is_int && !two_planes && p.c_tma && p.sk_tiles == 0 && !probe;
+    const bool packed_bias = EPI && (KIND == kKindF16 || KIND == kKindF8) && epi_packed_bias(p.epi, p.c_type) && c_tma && p.sk_tiles == 0 && !probe;
     uint32_t t = 0, nstores = 0;
     long long w_tfull = 0, e_work = 0, e_ld = 0, e_cv = 0;
     WorkIter it(p, pair_id, num_pairs);
@@ -951,12 +956,12 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // compact loop - 64 columns = one 128-byte staging row per step. The general loop below handles every other
       // case; keeping this one small matters because the general loop's code is far larger than the instruction
       // cache and ran at about 1400 cycles per 32 columns where this one needs about 150.
-      const bool fast16 = !two_planes && w.kind == 0 && p.c_tma && eflags == 0 && !p.acc_is_int && !probe &&
+      const bool fast16 = !two_planes && w.kind == 0 && c_tma && eflags == 0 && !acc_is_int && !probe &&
                           (p.c_type == RB_F16 || p.c_type == RB_BF16);
       // 4-byte C (f32 results, raw i32 results, the raw planes of a K split): 32 columns = one staging row per step
-      const bool fast32 = w.kind == 0 && p.c_tma && !probe &&
-                          ((eflags == 0 && !p.acc_is_int && p.c_type == RB_F32) || raw_i32);
-      // rows that are copied out: where they start in C (such launches run the EPI instantiation, see there)
+      const bool fast32 = w.kind == 0 && c_tma && !probe &&
+                          ((eflags == 0 && !acc_is_int && p.c_type == RB_F32) || raw_i32);
+      // rows that are copied out: where they start in C
       auto copy_base = [&]() {
         return static_cast<uint8_t*>(p.c) + ((long long)w.split * p.split_stride + (long long)g * p.c_stride_g + row0 * p.c_stride_m) * es_c;
       };
@@ -973,12 +978,11 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           bulk_commit();
         }
       };
-      const bool copied = EPI && p.c_tma == 2 && (fast16 || fast32);
-      if (copied) {
-        epi_copy_tile(my_staging, tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN, copy_base(), p.c_stride_m, es_c, nb * p.bn,
-                      min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u);
-      } else
-      if (fast16) {
+      if constexpr (COPY) {
+        if (fast16 || fast32)
+          epi_copy_tile(my_staging, tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN, copy_base(), p.c_stride_m, es_c, nb * p.bn,
+                        min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u);
+      } else if (fast16) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
         const int nsteps = p.bn / 64;
 #pragma unroll 1
@@ -1046,10 +1050,10 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       // code evicted the other roles' instructions (the issue loop waited twice as long for operands).
       const bool f16_mid = (eflags & RB_EPI_ROUND_MID) && (p.epi.mid_type == RB_F16 || p.epi.mid_type == RB_BF16);
       const uint32_t f16_extra = eflags & ~(uint32_t)(RB_EPI_ALPHA | RB_EPI_BIAS | RB_EPI_RELU | (f16_mid ? RB_EPI_ROUND_MID : 0));
-      const bool fast16e = !two_planes && eflags != 0 && w.kind == 0 && p.c_tma && f16_extra == 0 &&
-                           (epi_col_bias(eflags) || !(eflags & RB_EPI_BIAS)) && !p.acc_is_int && !probe &&
+      const bool fast16e = !two_planes && eflags != 0 && w.kind == 0 && c_tma && f16_extra == 0 &&
+                           (epi_col_bias(eflags) || !(eflags & RB_EPI_BIAS)) && !acc_is_int && !probe &&
                            (p.c_type == RB_F16 || p.c_type == RB_BF16);
-      const bool fast8 = !fast16e && w.kind == 0 && p.c_tma && !probe && p.acc_is_int && p.c_type == RB_I8 &&
+      const bool fast8 = !fast16e && w.kind == 0 && c_tma && !probe && acc_is_int && p.c_type == RB_I8 &&
                          (eflags & ~(uint32_t)RB_EPI_ZP_OUT) == (uint32_t)(RB_EPI_COL_SCALE | RB_EPI_REQUANT);
       if (fast16e || fast8) {
         auto set_context = [&](EpiStoreCtx& ec) {
@@ -1057,7 +1061,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           ec.taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
           ec.col0 = nb * p.bn; ec.bn = p.bn; ec.N = p.N; ec.M = p.M; ec.row0 = (int)row0; ec.gz = gz; ec.lane = lane;
         };
-        if (p.c_tma == 1) {
+        if constexpr (!COPY) {
           EpiStoreCtx ec;
           set_context(ec);
           if (packed_bias) nstores = epi_bias16_tile<EpiStoreCtx>(ec, (eflags & RB_EPI_RELU) != 0, reinterpret_cast<const uint32_t*>(vec_bias), p.c_type, nstores);
@@ -1074,7 +1078,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       // Channel-major f32 result of a convolution (NKHW): one store per column, the warp's 32 lanes are 32 consecutive
       // pixels of the column's image plane
-      const bool fast_remap = w.kind == 0 && p.c_rows_per_img && eflags == 0 && !p.acc_is_int && !probe && p.c_type == RB_F32;
+      const bool fast_remap = w.kind == 0 && p.c_rows_per_img && eflags == 0 && !acc_is_int && !probe && p.c_type == RB_F32;
       if (fast_remap) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
 #pragma unroll 1
@@ -1095,7 +1099,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       // Fused elementwise work (or 1-byte / converted outputs) on whole tiles through TMA stores: the general loop's
       // body without its stream-K and plain-store branches.
-      const bool fast_epi = !fast8 && !fast16 && !fast16e && !fast32 && !fast_remap && w.kind == 0 && p.c_tma && !probe && !raw_i32;
+      const bool fast_epi = !fast8 && !fast16 && !fast16e && !fast32 && !fast_remap && w.kind == 0 && c_tma && !probe && !raw_i32;
       if (fast_epi) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
 #pragma unroll 1
@@ -1114,7 +1118,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           if (two_planes) add_small(taddr + c * 32, v);
           float x[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = p.acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
+          for (int j = 0; j < 32; ++j) x[j] = acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
           if (eflags) {
             set_res(n0);
             epi_apply32(x, p.epi, vec_scale + c * 32, vec_bias + c * 32, erow);
@@ -1130,7 +1134,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            if (EPI && p.c_tma == 2) copy_staged(stg, n0 - sub * 32);
+            if constexpr (COPY) copy_staged(stg, n0 - sub * 32);
             else store_map(stg, n0 - sub * 32);
             ++nstores;
           }
@@ -1158,7 +1162,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const uint4 x4 = __ldcg(sk_word(u, c, i));
-              if (p.acc_is_int) {
+              if (acc_is_int) {
                 v[4 * i] += x4.x; v[4 * i + 1] += x4.y; v[4 * i + 2] += x4.z; v[4 * i + 3] += x4.w;
               } else {
                 v[4 * i] = __float_as_uint(__fadd_rn(__uint_as_float(v[4 * i]), __uint_as_float(x4.x)));
@@ -1179,14 +1183,14 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           float x[32];
           if (eflags == 0) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = p.acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
+            for (int j = 0; j < 32; ++j) x[j] = acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = p.acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
+            for (int j = 0; j < 32; ++j) x[j] = acc_is_int ? __int2float_rn((int)v[j]) : __uint_as_float(v[j]);
             set_res(n0);
             epi_apply32(x, p.epi, vec_scale + c * 32, vec_bias + c * 32, erow);
           }
-          if (p.c_tma || (p.vec_ok && n0 + 32 <= p.N)) {
+          if (c_tma || (p.vec_ok && n0 + 32 <= p.N)) {
             nw = pack_row32(x, p.c_type, w4, p.epi.out_zero);
           } else {
             nw = 0;
@@ -1198,7 +1202,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
         }
         if (p.trace) e_cv += clock64() - tl1;
-        if (p.c_tma) {
+        if (c_tma) {
           // Stage 32 rows x 128 bytes per store: row `lane` at lane * 128, its 16-byte pieces XOR-swizzled with
           // (lane & 7) exactly as the 128-byte-swizzled store map expects (also free of bank conflicts).
           const int sub = c % groups_per_store;
@@ -1217,7 +1221,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           }
           const bool last_group = (sub == groups_per_store - 1) || (n0 + 32 >= p.N) || (c == ngroups - 1);
           if (last_group) {
-            if (EPI && p.c_tma == 2) copy_staged(stg, n0 - sub * 32);
+            if constexpr (COPY) copy_staged(stg, n0 - sub * 32);
             else if (!(probe & 4)) store_map(stg, n0 - sub * 32);
             ++nstores;
           }
@@ -1249,7 +1253,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       if (p.chain_flags != nullptr && g == 0) {
         // this warp's rows of the intermediate are complete in global memory before its flag says so
-        if (p.c_tma == 1 && lane == 0) { bulk_wait<0>(); fence_proxy_async_all(); }
+        if (c_tma == 1 && lane == 0) { bulk_wait<0>(); fence_proxy_async_all(); }
         __threadfence();
         __syncwarp();
         if (lane == 0)
@@ -1257,7 +1261,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       }
       if (p.trace) e_work += clock64() - te;
     }
-    if (p.c_tma == 1 && lane == 0) bulk_wait<0>();  // every store of this thread has completed before the CTA exits
+    if (c_tma == 1 && lane == 0) bulk_wait<0>();  // every store of this thread has completed before the CTA exits
     if (p.trace && warp == 4 && lane == 0) {
       p.trace[blockIdx.x * 16 + 6] = (unsigned long long)w_tfull;
       p.trace[blockIdx.x * 16 + 7] = (unsigned long long)e_work;
