@@ -217,18 +217,26 @@ int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_
 // eleven configurations each (f16 / bf16 / fp8 / i8, 256^3 to 2048 x 2048 x 4096, replayed graphs; 8 % off on average; what a launch
 // costs by the width of its tiles has gone into `column`). The rule before - 256 columns in pairs whatever the size, a K split as soon as
 // half of the pairs idle - lost most where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.3 / 9.1
-// (64 columns, no split), 1536^3 bf16 28.8 / 16.9, 2048 x 1024 x 2048 f16 21.8 / 14.3, 364 x 1344 x 1792 i8 15.9 / 9.8. From three waves on the
-// rule stays: such products are bound by memory or by power.
+// (64 columns, no split), 1536^3 bf16 28.8 / 16.9, 2048 x 1024 x 2048 f16 21.8 / 14.3, 364 x 1344 x 1792 i8 15.9 / 9.8. Beyond three
+// waves of the rule's tiles the rule stays, such products being bound by memory or by power, and beyond three of the estimate's own too: their
+// stores take longer than estimated (3 x 180 x 7720 x 213 bf16 in tiles of 64 columns 20.9 us, by the rule 18.0; of 19 such products ten were
+// slower). Of 600 further products whose tile or split it changes (200 of them of two or three waves), one is more than 2 % slower than by the rule,
+// 3 x 321 x 1360 x 3833 fp8 24.5 -> 27.0; the mean is 0.79 of the rule's time. The chained pair of rbGemmGemm goes by the same estimate: 13 sizes from
+// 128 x 256 x 256 to 4096 x 1024 x 1024 took 0.72 to 1.01 of the rule's time.
 struct TileCost {
   int ctas, bn;
   double fixed, block, kb_per_block;   // kb_per_block: KB a CTA fetches per K block
 };
 constexpr TileCost kTileCosts[] = {{1, 64, 3.7, 0.252, 24}, {1, 128, 2.1, 0.326, 32}, {2, 128, 3.6, 0.246, 24}, {1, 256, 0.0, 0.404, 48}, {2, 256, 0.8, 0.335, 32}};
 
-// *ctas and *bn come in as the rule gives them and stay unless another tile, or no K split, is estimated at 15 % less.
 // f32 with two planes (the operand passes included); only where the rule does not cut K, so that no accumulation chain gets longer
 constexpr TileCost kTileCostsF32[] = {{1, 64, 6.9, 0.57, 48}, {1, 128, 5.3, 0.67, 64}, {2, 128, 6.4, 0.56, 48}, {1, 256, 5.5, 0.95, 96}, {2, 256, 4.4, 0.87, 64}};
 
+// *ctas and *bn come in as the rule gives them and stay unless another tile, or fewer K ranges, is estimated at 15 % less. K is not cut where
+// the rule does not cut it: such a product needs no planes in its workspace and can be handed out as one kernel. An f32 result keeps
+// accumulation chains no longer than the rule's: the tensor core truncates what it adds, and of two chains in place of one the error of f16 and
+// fp8 products against 64 bits is half (1.2e-6 -> 0.6e-6 at K = 1024; values of one sign 6.1e-6 -> 2.8e-6). In a 16-bit result its rounding hides that
+// (2.067e-4 both ways).
 void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, int* ctas, int* bn, int* splits) {
   // store of a column of a tile: an 8-bit result is requantised, rows off 16 bytes are copied out by the warps
   const double column = 0.025 * (p->c_type == RB_I8 ? 1.56 : 1.0) * ((long long)p->n * (long long)dtype_bytes(p->c_type) % 16 ? 2.0 : 1.0);
@@ -239,7 +247,9 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     const long long items = tiles * *s, kb = (kblocks + *s - 1) / *s;
     *waves = (items + units - 1) / units;
     const double busy = (double)std::min(items, units) * t.ctas;
-    const double block = std::max(t.block, busy * t.kb_per_block / 12500.0), store = t.bn * (*s > 1 ? 0.025 : column);
+    // (a byte per element in 64 columns: half of a staged row, copied out by the warps; 3.2 us a requantised tile)
+    const double narrow = t.bn == 64 && dtype_bytes(p->c_type) == 1 ? 1.3 : 1.0;
+    const double block = std::max(t.block, busy * t.kb_per_block / 12500.0), store = t.bn * (*s > 1 ? 0.025 : column * narrow);
     double us = t.fixed + std::max(kb * block, store) * (double)(*waves - 1) + kb * block + store;
     if (*s > 1) us += 3.7 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.283;
     return us;
@@ -254,14 +264,15 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     if (t.ctas == rule_ctas && t.bn == rule_bn) best = 0.85 * estimate(t, true, &s, &waves);
   }
   if (best == 0 || waves > 3 || (f32 && (s > 1 || p->k > 2048))) return;   // (s and waves are those of the rule's tile)
+  const long long rule_splits = s, chain = p->c_type == RB_F32 && p->ab_type != RB_I8 ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
     if (f32 && t.ctas == 1 && t.bn == 256) continue;
     if (b_mn && (t.bn / t.ctas) % che != 0) continue;
     if (t.ctas == 2 && (p->m <= kBM || kblocks <= 2)) continue;   // (see choose_config)
-    for (int split = 0; split < (f32 ? 1 : 2); ++split) {
+    for (int split = 0; split < (rule_splits > 1 ? 2 : 1); ++split) {
       const double us = estimate(t, split != 0, &s, &waves);
-      if (us < best) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
+      if (us < best && (kblocks + s - 1) / s <= chain && waves <= 3) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
     }
   }
 }
