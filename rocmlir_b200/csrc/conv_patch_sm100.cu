@@ -17,7 +17,7 @@
 //   * the filter stays in shared memory in the same form for all tiles of the persistent CTA, tcgen05.mma accumulates
 //     into one of two TMEM buffers, and the previous tile's result is stored while the tensor core works.
 //
-// (Images of up to 24 channels take conv_window_sm100.cu where its estimate is the lower one.)
+// (Images of up to 24 channels that start on 16 bytes take conv_window_sm100.cu where its estimate is the lower one.)
 //
 // Bound: the gather (one 2-byte read per element of the operand for three channels), then HBM writes of the result. Two
 // CTAs per SM overlap one's gather with the other's stores and waits. N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2,
@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <numeric>
 #include <string>
 
 #include "conv_patch.cuh"
@@ -355,37 +356,52 @@ bool choose_shape(const PatchConv& c, PatchShape* s) {
   return false;
 }
 
+// Runs of channels that can be read as one word (channels last: k walks the channels of a tap); 0: padded runs, by single elements.
+int gather_run(const PatchConv& c, const PatchShape& s) {
+  return s.run_pad != s.run ? 0 : c.planar ? 1 : c.C % 8 == 0 ? 8 : c.C % 4 == 0 ? 4 : c.C % 2 == 0 ? 2 : 1;
+}
+
 }  // namespace
 
-// Device time of both forms in microseconds, fitted to 396 convolutions (1 to 384 channels, 16 to 512 output channels, 7 x 7 to
-// 224 x 224, filters 1, 3, 5, 7, strides 1 and 2, both layouts, 5 to 2500 us): 15 % off on average for this form, 9 % for the other.
-// A tile gathers 128 x k elements however few pixels it has, once per group of 128 output channels, copies a window, and every CTA
-// brings the filter over element by element first; so taking this kernel wherever it fits made a third of those convolutions
-// slower, a pointwise layer of 512 -> 512 channels (64 channels-first images of 7 x 7) 32 -> 497 us. By this rule five of
-// the 396 are slower, at most by 13 %:
+// Device times of the forms in microseconds, replayed graphs. The product of an im2col matrix: fitted to 396 convolutions (1 to 384 channels, 16 to
+// 512 output channels, 7 x 7 to 224 x 224, filters 1, 3, 5, 7, strides 1 and 2, both layouts, 5 to 2500 us), 9 % off on average. This kernel and
+// the window kernel: fitted to 1900 of 1 to 96 channels and 1 to 256 output channels, strides to 4, images of 5 x 5 to 224 x 300, 11 and 8 % off.
+// A tile gathers 128 x k elements however few pixels it has, once per group of 128 output channels, copies a window, by single elements where
+// image rows start on any even byte, and every CTA brings the filter over element by element first; so taking this kernel
+// wherever it fits made a third of the convolutions slower, a pointwise layer of 512 -> 512 channels (64 channels-first images of 7 x 7) 32 -> 497 us:
 //   64 x 224 x 224 x 3 -> 64, 7 x 7 stride 2: 102 us here, 1830 there;  32 x 28 x 28 x 24 -> 64, 3 x 3: 13.5 / 16.4
 //   16 x 14 x 14 x 96 -> 192, 3 x 3: 64 / 16;  channels first 32 x 28 x 28 x 128 -> 128, 3 x 3 stride 2: 299 / 75
-bool conv_patch_pays(PatchConv* conv, bool wide_gather, bool result_direct, int out_bytes) {
+// An image off 16 bytes can not take the window kernel and goes by the other two estimates (*off16: whether to this kernel).
+bool conv_patch_pays(PatchConv* conv, bool wide_gather, bool result_direct, int out_bytes, bool* off16) {
   const PatchConv& c = *conv;
+  *off16 = false;
   PatchShape s;
   if (!choose_shape(c, &s)) return false;
   const double sms = planning_sm_count(), pixels = 1e-6 * c.N * c.P * c.Q, k = (double)c.Y * c.X * c.C;
   const double tiles = (double)c.N * ((c.P + s.R - 1) / s.R) * ((c.Q + s.Qt - 1) / s.Qt), rows = (double)s.planes * s.rows;
   const double ctas = std::min(tiles, std::floor(sms * s.ctas_per_sm / s.passes));
   const double on_one_sm = std::min<double>(s.ctas_per_sm, std::max(1.0, ctas * s.passes / sms));   // they share its issue slots
-  const double tile = 0.5 + 0.009 * s.kelems + 0.003 * s.nt + rows * (0.042 + 1e-4 * s.pitch) +
-                      (c.o_k == 1 ? 0.022 * (c.Kout % 32) : 0.0);   // (the last columns of a row one by one)
-  const double here = 4.4 + on_one_sm * (std::ceil(tiles / ctas) * tile + 0.0127 * s.nt * ((s.kelems + 63) / 64));
-  // im2col matrix (a vector or an element per thread), its rows padded to 16 bytes, product, permutation of the result
+  // result: whole groups of 32 columns (in the last group of a row, all columns where rows are off 32 bytes, or in channel planes one by one)
+  const double columns = std::min(c.Kout, s.nt), fill = std::min(1.0, s.R * s.Qt / 128.0);
+  const double one_by_one = c.o_k != 1 ? 0.004 * columns : fill * ((c.Kout * out_bytes) % 32 ? 0.124 * columns : 0.093 * (c.Kout % 32));
+  const long long starts = (long long)c.W * (c.planar ? 1 : c.C) | c.i_h | c.i_n | (c.planar ? c.i_c : 0);
+  const double row = starts % 4 == 0 ? 0.033 + 8e-5 * s.pitch : starts % 2 == 0 ? 0.030 + 2.1e-4 * s.pitch : 0.025 + 8.6e-4 * s.pitch;
+  // pixels of a warp that fall into the same banks: `ways` of the lanes that shared memory serves at a time
+  const int word = 2 * gather_run(c, s) < 4 ? 4 : 2 * gather_run(c, s), step = c.stride_w * (c.planar ? 1 : c.C) * 2;
+  const double ways = (128.0 / word) / std::min(128.0 / word, std::max(1.0, 128.0 / std::gcd(step, 128)));
+  const double tile = 0.225 + 0.0047 * s.kelems * (1 + 0.07 * (ways - 1)) + 0.0077 * std::max(0, s.kelems - 400) + 0.0047 * s.nt + rows * row + one_by_one;
+  const double here = 4.4 + on_one_sm * (std::ceil(tiles / ctas) * tile + 0.0140 * s.nt * ((s.kelems + 63) / 64));
+  // im2col matrix (a vector or an element per thread), its rows padded to 16 bytes, product (rows of it off 16 bytes are copied out),
+  // permutation of the result
   double there = 8.1 + pixels * (117 + 2 * k * (wide_gather ? 0.386 : 3.42)) + 0.0039 * pixels * std::max(c.Kout, 64) * k + 0.0042 * k;
   if ((c.Y * c.X * c.C) % 8 != 0) there += 1.3 + pixels * 2 * k * 0.364;
   if (!result_direct) there += 4.1 + pixels * 2 * c.Kout * 1.56;
-  // rows of the result off 16 bytes: the product stores element by element, 40 us a wave of tiles
-  if ((c.Kout * out_bytes) % 16) there += 35 * std::ceil(std::ceil(pixels * 1e6 / 128) * ((c.Kout + 255) / 256) / sms);
+  if ((c.Kout * out_bytes) % 16) there += 2.6 + pixels * (54 + 2.0 * c.Kout);
   const int variant = rbGetGemmVariant();
   const double window = ((variant >> 10) & 1) ? -1.0 : conv_window_plan(conv);
-  if (window < 0 || (((variant >> 30) & 1) == 0 && window > here)) conv->win_q = 0;
-  return (conv->win_q ? std::min(here, window) : here) * 1.1 < there;
+  if (window < 0 || (((variant >> 30) & 1) == 0 && window > 0.95 * here)) conv->win_q = 0;
+  *off16 = here * 1.05 < there;
+  return (conv->win_q ? std::min(here, window) : here) * 1.05 < there;
 }
 
 bool conv_patch_applicable(const PatchConv& c) {
@@ -408,7 +424,7 @@ RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filte
   // the kernel takes its tensors element by element where they lie off wider boundaries, but not off those of an element
   if ((reinterpret_cast<uintptr_t>(image) | reinterpret_cast<uintptr_t>(filter)) % 2 || reinterpret_cast<uintptr_t>(out) % dtype_bytes(out_type))
     return fail(RB_UNSUPPORTED, "tensors must start on a multiple of their element size");
-  if (conv_window_fits(c, image)) return conv_window_run(c, image, filter, out, out_type, epi, stream_v);
+  if (c.win_q > 0 && reinterpret_cast<uintptr_t>(image) % 16 == 0) return conv_window_run(c, image, filter, out, out_type, epi, stream_v);
   const DeviceInfo* dev = device_info();
   if (!dev) return RB_CUDA_ERROR;
   PatchShape s;
@@ -456,8 +472,7 @@ RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filte
   }
   p.status = dev->status_word;
   p.wait_cycles = kWaitCycles;
-  // runs of channels that can be read as one word (channels last: k walks the channels of a tap)
-  const int vec = s.run_pad != s.run ? 0 : c.planar ? 1 : c.C % 8 == 0 ? 8 : c.C % 4 == 0 ? 4 : c.C % 2 == 0 ? 2 : 1;
+  const int vec = gather_run(c, s);
   typedef void (*Kernel)(const PatchParams);
   const Kernel kern = with_epi ? (vec == 8 ? conv_patch_kernel<8, true> : vec == 4 ? conv_patch_kernel<4, true>
                                   : vec == 2 ? conv_patch_kernel<2, true> : vec == 1 ? conv_patch_kernel<1, true> : conv_patch_kernel<0, true>)

@@ -398,6 +398,7 @@ struct ConvPlan {
   bool cls_any_empty = false;
   HaloConv cls_hc[16];
   bool patch = false;       // forward, few channels: the patch kernel gathers the operand on the SM (csrc/conv_patch_sm100.cu)
+  bool patch_off16 = false; // also for an image that starts off 16 bytes
   PatchConv pc;
 };
 
@@ -411,7 +412,7 @@ bool is_dense_in_order(const long long* strides, const long long* sizes, const i
   return true;
 }
 
-RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
+RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, bool image_on_16 = true) {
   if (!p) return fail(RB_INVALID_PARAM, "problem is NULL");
   if (p->n <= 0 || p->g <= 0 || p->c <= 0 || p->k <= 0 || p->h <= 0 || p->w <= 0 || p->y <= 0 || p->x <= 0 ||
       p->stride_h <= 0 || p->stride_w <= 0 || p->dil_h <= 0 || p->dil_w <= 0 || p->pad_h < 0 || p->pad_w < 0 ||
@@ -502,8 +503,11 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1) {
         c.f_k = pl->fs[1]; c.f_c = pl->fs[2]; c.f_y = pl->fs[3]; c.f_x = pl->fs[4];
         c.o_n = pl->os[0]; c.o_k = pl->os[2]; c.o_p = pl->os[3]; c.o_q = pl->os[4];
         c.win_q = c.win_r = 0;
+        const bool wherever = ((rbGetGemmVariant() >> 30) & 1) != 0;
         pl->patch = conv_patch_applicable(c) &&
-                    (conv_patch_pays(&c, pl->is[2] == 1 && p->c % 8 == 0, pl->c_direct, (int)es_o) || ((rbGetGemmVariant() >> 30) & 1));
+                    (conv_patch_pays(&c, pl->is[2] == 1 && p->c % 8 == 0, pl->c_direct, (int)es_o, &pl->patch_off16) || wherever);
+        pl->patch_off16 = pl->patch && (pl->patch_off16 || wherever);
+        if (!image_on_16) pl->patch = pl->patch_off16;
       }
     }
     if (pl->a_implicit) pl->a_direct = true;   // nothing to gather
@@ -763,7 +767,9 @@ size_t rb::conv_workspace_bytes(const RbConvProblem* p, int result_type) {
   TunedVariantScope tuned(tuned_variant_conv(p));
   ConvPlan pl;
   if (make_plan(p, &pl, result_type) != RB_SUCCESS) return 0;
-  return pl.total;
+  size_t total = pl.total;
+  if (pl.patch && !pl.patch_off16 && make_plan(p, &pl, result_type, false) == RB_SUCCESS) total = std::max(total, pl.total);
+  return total;
 }
 
 extern "C" size_t rbConvWorkspaceSize(const RbConvProblem* p) { return rb::conv_workspace_bytes(p, -1); }
@@ -842,6 +848,11 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
   ConvPlan pl;
   RbStatus st = make_plan(p, &pl, result_type);
   if (st != RB_SUCCESS) return st;
+  if (pl.patch && !pl.patch_off16 && reinterpret_cast<uintptr_t>(input) % 16 && workspace) {
+    // the form for an image off 16 bytes, where its matrix fits the workspace
+    ConvPlan off;
+    if (make_plan(p, &off, result_type, false) == RB_SUCCESS && off.total <= workspace_bytes) pl = off;
+  }
   if (capture && (pl.n_classes > 0 || !pl.a_direct || !pl.b_direct || !pl.c_direct || pl.a_up || pl.a_planes > 0 ||
                   (p->direction == 1 && pl.a_implicit)))
     return fail(RB_UNSUPPORTED, "this convolution runs as several kernels (layout, filter or reduction passes): it has no "

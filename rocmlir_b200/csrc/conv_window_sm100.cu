@@ -19,8 +19,9 @@
 //   * Bound: what the sixteen warps do for an item (2800 cycles of preparation, 2900 of stores, 1400 of copies for four tiles of 64 channels),
 //     against 3000 cycles of products. us, the gathering form before: N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2 100 -> 71; 30 x 7 -> 32
 //     channels, 184 x 184, 7 x 7 stride 2 81 -> 26; 20 x 16 -> 32, 223 x 223, 3 x 3 116 -> 39; 109 x 8 -> 64, 62 x 62, 5 x 5 53 -> 31;
-//     36 x 3 -> 32, 195 x 195, 3 x 3 stride 2 83 -> 19 (rows that start on any even byte). Of 69 convolutions of 3 to 16 channels the
-//     rule in conv_patch_pays took the slower form by more than 6 % in nine, all below 22 us.
+//     36 x 3 -> 32, 195 x 195, 3 x 3 stride 2 83 -> 19 (rows that start on any even byte). Of 1000 convolutions
+//     that the estimates in conv_patch_pays were not fitted to, they take a form more than 6 % slower than the fastest in 80, and 15 are
+//     more than 5 % slower than without this kernel (the worst 14.2 -> 18.3 us).
 //   * sixteen warps prepare item i + 1 and store item i - 1 while the seventeenth issues item i: two windows, two sets of
 //     accumulators in tensor memory, the raw rows of the next item on their way by cp.async meanwhile.
 #include <cuda_runtime.h>
@@ -421,13 +422,14 @@ struct WindowShape {
   int R, Qt, Wp, mtiles;
   int segs, tasks;
   int raw_pitch, win_bytes, smem;
+  int max_ctas;
+  double store_cycles, tensor_cycles;   // of a tile of 128 raster positions
   double us;   // estimated time
 };
 
 // What does not depend on the tile (rows_ph and raw_rows without the tile's rows).
-bool window_operand(const PatchConv& c, const void* image, WindowShape* s) {
+bool window_operand(const PatchConv& c, WindowShape* s) {
   if (c.stride_h > kMaxPhases || c.stride_w > kMaxPhases || c.Y > 32 || c.X > 32 || c.C > kWindowMaxC) return false;
-  if (reinterpret_cast<uintptr_t>(image) % 16) return false;   // raw rows are copied by the image's 16-byte granules
   const int unit = c.planar ? 1 : c.C;
   // runs waste the last entry of a filter row, pixels the last entry of a pixel
   s->pixels = c.C > 4;
@@ -457,6 +459,9 @@ bool window_operand(const PatchConv& c, const void* image, WindowShape* s) {
   s->nt = ((c.Kout + s->passes - 1) / s->passes + 31) / 32 * 32;
   if (s->passes > 8 || (long long)s->nt * (s->passes - 1) >= c.Kout) return false;   // (no pass without channels)
   s->mmas = (s->chunks + 1) / 2;
+  s->max_ctas = std::max(1, planning_sm_count() / s->passes);
+  s->store_cycles = 4.0 * (s->nt / 32) * 130 * (c.o_k == 1 && c.Kout % 32 == 0 ? 1 : 1.6);
+  s->tensor_cycles = (double)s->mmas * (4096 + 32 * s->nt) / 90.0;
   s->phases = 0;
   int last_row = 0;
   for (int f = 0; f < c.stride_h; ++f) {
@@ -474,14 +479,21 @@ bool window_operand(const PatchConv& c, const void* image, WindowShape* s) {
 }
 
 // The kernel on tiles of R x Qt output pixels: whether it fits, and an estimate of its time: the longer of an item's two sides, the
-// products and what the sixteen warps do meanwhile, times the items of a CTA.
-bool window_tile(const PatchConv& c, const WindowShape& operand, int Qt, int R, WindowShape* out) {
+// products and what the sixteen warps do meanwhile, times the items of a CTA. (A tile that cannot be faster than `limit` microseconds by the
+// products and stores alone is not looked at further: most of a search ends there, and its 1 us is a tenth of a small call.)
+bool window_tile(const PatchConv& c, const WindowShape& operand, int Qt, int R, double limit, WindowShape* out) {
+  const unsigned mtiles = (unsigned)(R * (Qt + operand.halo) + 127) / 128;
+  const unsigned items = (unsigned)c.N * ((unsigned)(c.P + R - 1) / (unsigned)R) * ((unsigned)(c.Q + Qt - 1) / (unsigned)Qt);   // (at most N x P x Q < 2^30)
+  const unsigned ctas = std::min(items, (unsigned)operand.max_ctas);
+  const double per_cta = (double)((items + ctas - 1) / ctas);
+  const double store = mtiles * operand.store_cycles, tensor = mtiles * operand.tensor_cycles + 250;
+  if (4.5 + per_cta * std::max(tensor, store / 1.2 + 1200) / 1900 >= limit) return false;
   WindowShape s = operand;
   const int unit = c.planar ? 1 : c.C, raw_planes = c.planar ? c.C : 1;
   s.Qt = Qt;
   s.R = R;
   s.Wp = Qt + s.halo;
-  s.mtiles = (R * s.Wp + 127) / 128;
+  s.mtiles = (int)mtiles;
   s.rows_ph += R;
   s.raw_rows += s.rows_ph * c.stride_h;
   const long long entries = (long long)s.planes * s.phases * s.rows_ph * s.Wp;
@@ -499,33 +511,48 @@ bool window_tile(const PatchConv& c, const WindowShape& operand, int Qt, int R, 
   const double lanes = (double)s.planes * s.phases * s.rows_ph * s.segs;   // warp steps of the preparation
   const double prep = lanes * (s.fetch == kDirect ? 14 : s.fetch == kElements ? 44 : s.fetch == kShifted ? 26 : 18) +
                       (s.fetch == kDirect ? 0.0 : (double)raw_planes * s.raw_rows * (30 + s.raw_pitch / 256.0 * 16));
-  const double store = s.mtiles * 4.0 * (s.nt / 32) * 130 * (c.o_k == 1 && c.Kout % 32 == 0 ? 1 : 1.6);
-  const double tensor = (double)s.mtiles * s.mmas * (4096 + 32 * s.nt) / 90.0 + 250;
   const double item = std::max(tensor, (prep + store) / 1.2 + 1200);
-  const double items = (double)c.N * ((c.P + R - 1) / R) * ((c.Q + Qt - 1) / Qt);
-  const double ctas = std::min(items, (double)std::max(1, planning_sm_count() / s.passes));
-  s.us = 4.5 + (s.fetch == kElements ? 1.0 : 0.0) + (std::ceil(items / ctas) * item + tensor + 6.0 * s.mmas * s.nt) / 1900;   // + the filter
+  s.us = 4.5 + (s.fetch == kElements ? 1.0 : 0.0) + (per_cta * item + tensor + 6.0 * s.mmas * s.nt) / 1900;   // + the filter
   *out = s;
   return true;
 }
 
 // The fastest tile by that estimate among a few: columns cut evenly, as many rows as one to all of the accumulators hold.
-bool window_shape(const PatchConv& c, const void* image, WindowShape* best) {
+bool window_shape(const PatchConv& c, WindowShape* best) {
   WindowShape s, t;
   memset(&s, 0, sizeof(s));
-  if (!window_operand(c, image, &s)) return false;
+  if (!window_operand(c, &s)) return false;
   bool found = false;
   const int max_tiles = 256 / s.nt;
   for (int cols = (c.Q + 255) / 256, tries = 0; cols <= c.Q && tries < 6; ++cols, ++tries) {
     const int Qt = (c.Q + cols - 1) / cols;
     if (tries && Qt < 8) break;
-    for (int tiles = max_tiles; tiles >= 1; --tiles) {
+    for (int tiles = max_tiles, last = 0; tiles >= 1; --tiles) {
       const int R = std::min(c.P, tiles * 128 / (Qt + s.halo));
       if (R < 1) break;
-      if (window_tile(c, s, Qt, R, &t) && (!found || t.us < best->us)) { *best = t; found = true; }
+      if (R == last) continue;   // (a low image: the same tile again)
+      last = R;
+      if (window_tile(c, s, Qt, R, found ? best->us : 1e30, &t) && (!found || t.us < best->us)) { *best = t; found = true; }
     }
   }
   return found;
+}
+
+// The kernel's time with that tile, for the choice between kernels. (The estimate above ranks the tiles of one convolution; between
+// convolutions it was up to five times too low: it knew nothing of what results off 32 bytes, element by element, and filters by channel planes
+// cost, and rows of single channels by element.) Cycles fitted to 1500 convolutions.
+double window_time(const PatchConv& c, const WindowShape& s) {
+  static const double kEntries[] = {23, 14, 14, 65, 46};   // of 32 entries, by Fetch
+  const double columns = std::min(c.Kout, s.nt), units = 4.0 * s.mtiles, fill = s.R * s.Qt / (128.0 * s.mtiles);
+  const double prep = (double)s.planes * s.phases * s.rows_ph * s.segs * kEntries[s.fetch] +
+                      (s.fetch == kDirect ? 0.0 : 58.0 * (c.planar ? c.C : 1) * s.raw_rows);
+  const double store = units * (c.o_k != 1 ? 5.2 * columns : c.Kout % 16 ? 62 * fill * columns : 99 * std::floor(columns / 32) + 62 * fill * (c.Kout % 32));
+  const double tensor = (double)s.mtiles * s.mmas * (4096 + 32 * s.nt) / 75.0 + 250, entries = (double)s.mmas * s.nt;
+  // a filter whose channels are not neighbours comes element by element, from L2 once it no longer fits what is left of the L1
+  const double filter = c.f_c == 1 ? 5.8 * entries : 7.0 * entries + 26 * std::max(0.0, entries - 3000);
+  const double items = (double)c.N * ((c.P + s.R - 1) / s.R) * ((c.Q + s.Qt - 1) / s.Qt);
+  const double ctas = std::min(items, (double)s.max_ctas);
+  return 4.0 + (std::ceil(items / ctas) * std::max(tensor, prep + store + 1820) + tensor + filter) / 1900;
 }
 
 }  // namespace
@@ -533,16 +560,10 @@ bool window_shape(const PatchConv& c, const void* image, WindowShape* best) {
 double conv_window_plan(PatchConv* c) {
   WindowShape s;
   c->win_q = c->win_r = 0;
-  if (!window_shape(*c, nullptr, &s)) return -1.0;
+  if (!window_shape(*c, &s)) return -1.0;
   c->win_q = s.Qt;
   c->win_r = s.R;
-  return s.us;
-}
-
-bool conv_window_fits(const PatchConv& c, const void* image) {
-  WindowShape s;
-  memset(&s, 0, sizeof(s));
-  return c.win_q > 0 && window_operand(c, image, &s) && window_tile(c, s, c.win_q, c.win_r, &s);
+  return window_time(*c, s);
 }
 
 RbStatus conv_window_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
@@ -552,7 +573,8 @@ RbStatus conv_window_run(const PatchConv& c, const void* image, const void* filt
   const bool with_epi = (epi && epi->flags) || out_type != (c.is_bf16 ? RB_BF16 : RB_F16);
   WindowShape s;
   memset(&s, 0, sizeof(s));
-  if (c.win_q <= 0 || !window_operand(c, image, &s) || !window_tile(c, s, c.win_q, c.win_r, &s))
+  // (raw rows are copied by the image's 16-byte granules)
+  if (c.win_q <= 0 || reinterpret_cast<uintptr_t>(image) % 16 || !window_operand(c, &s) || !window_tile(c, s, c.win_q, c.win_r, 1e30, &s))
     return fail(RB_UNSUPPORTED, "convolution outside the reach of the window kernel");
   WindowParams p;
   memset(&p, 0, sizeof(p));

@@ -157,15 +157,14 @@ struct PatchConv {
 };
 bool conv_patch_applicable(const PatchConv& c);
 // Whether it is the faster form: the other one expands an im2col matrix (wide_gather: by 16-byte vectors, else by elements) and, unless
-// result_direct, permutes the product's result.
-bool conv_patch_pays(PatchConv* c, bool wide_gather, bool result_direct, int out_bytes);
+// result_direct, permutes the product's result. *off16: the same for an image that starts off 16 bytes.
+bool conv_patch_pays(PatchConv* c, bool wide_gather, bool result_direct, int out_bytes, bool* off16);
 RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
                         void* stream);
 
-// The window kernel: its tile for this convolution and an estimate of its time in microseconds (negative: it does not take it);
-// whether it takes this image with that tile (not off 16 bytes).
+// The window kernel: its tile for this convolution and an estimate of its time in microseconds (negative: it does not take it). It takes
+// images that start on 16 bytes.
 double conv_window_plan(PatchConv* c);
-bool conv_window_fits(const PatchConv& c, const void* image);
 RbStatus conv_window_run(const PatchConv& c, const void* image, const void* filter, void* out, int out_type, const RbEpilogue* epi,
                          void* stream);
 
