@@ -203,24 +203,27 @@ int skinny_splits(const RbGemmProblem* p, long long tiles, int kblocks, int sms)
 
 // Which of the two kernels takes a product with few rows. Here an output column is one thread's, so a row costs every CTA
 // about 0.15 us (0.05 where i32 sums are stored as they are) divided by the parts of K, while the general kernel stores a
-// tile of any height in about a microsecond, but needs a second launch when it divides K and 40 us for a tile whose rows of C
-// do not start on 16-byte boundaries. Measured, us here / there, device time of repeated calls, f16:
-//   parts of K   (16..64) x 4096 x 4096: 8.4..11.3 / 14;  64 x 1024 x 1024: 9.2 / 12.7;  33 x 11008 x 4096: 16.4 / 23.4
-//   two parts    16 x 4096 x 512: 6.8 / 9.0;  33: 9.6 / 9.0;  64: 13.7 / 9.0
-//   one part     16 x 1024 x 256: 6.7 / 7.4;  33: 9.0 / 7.4;  64: 12.8 / 7.4;  K of two blocks, 16 x 64 x 128 in 32 groups: 6.2 / 5.9
-//   long K       64 x 32000 x 4096, one part: 52.7 / 52.2;  33: 50.2 / 52.7
-//   few tiles, K cut into more ranges there than a cluster has: 16 x 128 x 8192: 8.2 / 11.5;  x 32768: 22.2 / 13.9
-//   clusters that fill the SMs to the last slot do not pack: 33 x 4096 x 4096 in 3 groups (96 clusters of 3): 29.1 / 27.1
-//   several CTAs per slot, one tile each where the general kernel is persistent: 64 x 4096 x 128 in 64 groups: 90.7 / 22.5,
-//                16: 40.8 / 20.9;  16 x 128256 x 4096: 165 / 187;  1 x 64 x 64 in 512 groups: 7.0 / 10.0
-//   C off 16 bytes: 53 x 16711 x 80: 12.4 / 43.2;  62 x 2349 x 80 in 55 groups (fp8): 47 / 164
+// tile of any height in about a microsecond (twice that where rows of C do not start on 16-byte boundaries), but needs a second launch
+// when it divides K. Measured, us here / there, device time of repeated calls, f16:
+//   parts of K   (16..64) x 4096 x 4096: 9.6..12.1 / 14.7..16.2;  64 x 1024 x 1024: 8.9 / 8.4;  33 x 11008 x 4096: 21.5 / 26.4
+//   two parts    16 x 4096 x 512: 6.6 / 7.1;  33: 9.6 / 7.1;  64: 13.7 / 7.0
+//   one part     16 x 1024 x 256: 6.4 / 5.9;  33: 9.0 / 6.0;  64: 12.8 / 6.0;  K of two blocks, 16 x 64 x 128 in 32 groups: 6.2 / 5.5
+//   long K       64 x 32000 x 4096, one part: 52.7 / 50.7;  33: 50.2 / 50.4
+//   few tiles, K cut into more ranges there than a cluster has: 16 x 128 x 8192: 8.1 / 11.1;  x 32768: 22.2 / 13.7
+//   clusters that fill the SMs to the last slot do not pack: 33 x 4096 x 4096 in 3 groups (96 clusters of 3): 29.1 / 28.2
+//   several CTAs per slot, one tile each where the general kernel is persistent: 64 x 4096 x 128 in 64 groups: 90.7 / 22.9,
+//                16: 40.8 / 22.0;  16 x 128256 x 4096: 165 / 183;  1 x 64 x 64 in 512 groups: 8.0 / 11.5
+//   C off 16 bytes, one part, short K: 35 x 10245 x 64: 8.6 / 10.0;  64 x 1023 x 256: 12.2 / 8.5;  64 x 4095 x 128 in 64 groups: 90.5 / 83
+// Of 600 products of up to 64 rows on 16 bytes, four are more than 5 % slower by these lines than on the general kernel (64 x 1024 x 1024 by 5 %:
+// drawn before that one chose its tiles by an estimate). Of 300 off 16 bytes two are; taking this kernel for all of them, 42 of 700 were
+// more than 6 % slower.
 bool gemm_skinny_applicable(const RbGemmProblem* p, uint32_t epi_flags) {
   const long long es = (long long)dtype_bytes(p->ab_type);
   if (p->m > 64 || p->trans_a || !p->trans_b || p->trans_c || p->ab_type == RB_F32 || (p->k * es) % 16) return false;
-  if ((p->n * (long long)dtype_bytes(p->c_type)) % 16) return true;
   const int sms = planning_sm_count(), kblocks = (int)((p->k * es + 127) / 128);
   const long long slots = 2LL * sms, tiles = (long long)p->g * ((p->n + kTileN - 1) / kTileN);
   const int rows = p->c_type == RB_I32 && epi_flags == 0 ? (p->m + 2) / 3 : p->m;
+  if ((p->n * (long long)dtype_bytes(p->c_type)) % 16) return rows <= 36 || kblocks > 8 || skinny_splits(p, tiles, kblocks, sms) > 1;
   if (tiles > slots) return (kblocks >= 8 && 2 * rows <= kblocks) || (tiles <= 2 * slots && rows <= 6);
   const int splits = skinny_splits(p, tiles, kblocks, sms);
   if (splits == 1) return rows <= (kblocks >= 4 ? std::max(16, kblocks / 2) : 12);

@@ -221,8 +221,8 @@ int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_
 // waves of the rule's tiles the rule stays, such products being bound by memory or by power, and beyond three of the estimate's own too: their
 // stores take longer than estimated (3 x 180 x 7720 x 213 bf16 in tiles of 64 columns 20.9 us, by the rule 18.0; of 19 such products ten were
 // slower). Of 600 further products whose tile or split it changes (200 of them of two or three waves), one is more than 2 % slower than by the rule,
-// 3 x 321 x 1360 x 3833 fp8 24.5 -> 27.0; the mean is 0.79 of the rule's time. The chained pair of rbGemmGemm goes by the same estimate: 13 sizes from
-// 128 x 256 x 256 to 4096 x 1024 x 1024 took 0.72 to 1.01 of the rule's time.
+// 3 x 321 x 1360 x 3833 fp8 24.5 -> 27.0; the mean is 0.79 of the rule's time. The chained pair of rbGemmGemm goes by the same estimate: 12 sizes from
+// 128 x 256 x 256 to 2048 x 2048 x 2048, f16 and bf16, took 0.71 to 1.00 of the rule's time.
 struct TileCost {
   int ctas, bn;
   double fixed, block, kb_per_block;   // kb_per_block: KB a CTA fetches per K block

@@ -72,3 +72,21 @@ def test_eight_bit_results_in_narrow_tiles(cuda_device, m, n, off):
     epi = Epilogue(col_scale=torch.rand(n, device="cuda", generator=gen), requant_scale=3.0)
     got = [run(a, b, torch.int8, off, epilogue=epi, variant=v) for v in (0x1001, 0x2001 | PLAIN)]   # 64 columns, 128
     assert torch.equal(got[0], got[1]) and L.kernel_status() == 0
+
+
+@pytest.mark.parametrize("dt,g,m,n,k", [("float16", 1, 64, 1023, 256), ("bfloat16", 1, 63, 567, 64), ("float16", 1, 36, 1030, 256), ("float16", 1, 37, 1030, 256),
+                                        ("float16", 1, 35, 10245, 64), ("float16", 1, 64, 1023, 4096), ("bfloat16", 3, 64, 515, 2048)])
+def test_few_rows_take_the_faster_kernel(cuda_device, dt, g, m, n, k):
+    """At most 64 rows against weights stored N x K: the library's choice against the general kernel in its own configuration."""
+    import ctypes as C
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200.gemm import gemm, problem, workspace_size
+    from test_dispatch_lines_gpu import under
+    t = getattr(torch, dt)
+    a, b, c = (torch.randn(s, device="cuda").to(t) for s in ((g, m, k), (g, n, k), (g, m, n)))
+    p, general = problem(a, b, False, True, False, t), L.RbGemmConfigInfo()
+    ws = torch.empty(max(16, workspace_size(p)), dtype=torch.uint8, device="cuda")
+    L.check(L.lib().rbGemmGetConfig(C.byref(p), C.byref(general)))
+    run = lambda: gemm(a, b, trans_b=True, out=c, workspace=ws)
+    assert under(0, run) <= 1.25 * under(general.variant, run)
