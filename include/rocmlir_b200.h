@@ -204,6 +204,11 @@ RB_EXPORT size_t rbConvWorkspaceSize(const RbConvProblem *p);
  * miirGetKernelCount, Miir.h:54-58); -1 for an invalid problem. */
 RB_EXPORT int rbConvKernelCount(const RbConvProblem *p);
 
+/* Which kernel reads a few-channel image of a forward convolution as it lies, for an image that starts on 16 bytes: 0 = none (the
+ * convolution takes another form), 1 = the one that gathers its operand, 2 = the one whose operand is the input window; -1 for an invalid
+ * problem. */
+RB_EXPORT int rbConvPatchKernel(const RbConvProblem *p);
+
 /* The GEMM a convolution is computed as (the reference's GemmSize::fromConvolution and the backward variants,
  * mlir/lib/Dialect/Rock/IR/RockDialect.cpp:509-533,671-749): forward M = N*Ho*Wo, N = K, K = Y*X*C; backward
  * data M = N*H*W, N = C, K = Y*X*K; backward weight M = K, N = Y*X*C, K = N*Ho*Wo (per group). */

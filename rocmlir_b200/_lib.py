@@ -116,6 +116,8 @@ def lib() -> C.CDLL:
         l.rbConvWorkspaceSize.argtypes = [C.POINTER(RbConvProblem)]
         l.rbConvKernelCount.restype = C.c_int
         l.rbConvKernelCount.argtypes = [C.POINTER(RbConvProblem)]
+        l.rbConvPatchKernel.restype = C.c_int
+        l.rbConvPatchKernel.argtypes = [C.POINTER(RbConvProblem)]
         l.rbConv.restype = C.c_int
         l.rbConv.argtypes = [C.POINTER(RbConvProblem), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t,
                              C.c_void_p]

@@ -820,6 +820,13 @@ extern "C" int rbConvKernelCount(const RbConvProblem* p) {
   return 1 + (pl.a_direct ? 0 : 1) + (pl.b_direct ? 0 : 1) + ((pl.c_direct || pl.c_remap) ? 0 : 1);
 }
 
+extern "C" int rbConvPatchKernel(const RbConvProblem* p) {
+  TunedVariantScope tuned(tuned_variant_conv(p));
+  ConvPlan pl;
+  if (make_plan(p, &pl) != RB_SUCCESS) return -1;
+  return !pl.patch ? 0 : pl.pc.win_q > 0 ? 2 : 1;
+}
+
 extern "C" RbStatus rbConv(const RbConvProblem* p, void* filter, void* input, void* output, void* workspace,
                            size_t workspace_bytes, void* stream_v) {
   return rb::conv_run(p, -1, filter, input, output, workspace, workspace_bytes, stream_v);
