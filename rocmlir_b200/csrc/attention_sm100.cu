@@ -136,7 +136,7 @@ __device__ __forceinline__ uint32_t load_word_within(const int8_t* t, long long 
 // that is neither keeps the plain loop, with all four warps at work (429 heads x 10 queries x 3550 keys, D = 64, no mask: 113 us; 133 with
 // one kernel for everything). Rows anywhere used to take the general branch, 128 dependent byte loads a block in a loop of a few
 // thousand instructions: 55 heads x 6 queries x 300 keys, D = 64,
-// bf16 102 -> 13 us; 300 x 9 x 1003 862 -> 57; 100 x 16 x 4097, D = 128 1243 -> 71; rows on 16 bytes, 64 x 8 x 4096, D = 128
+// bf16 102 -> 13 us; 300 x 9 x 1003 836 -> 57; 100 x 16 x 4097, D = 128 1238 -> 71; rows on 16 bytes, 64 x 8 x 4096, D = 128
 // 54 -> 34 (read a block ahead).
 template <bool SPLIT, int MASK>
 __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __grid_constant__ AttMaps maps,

@@ -16,10 +16,11 @@
 //     neighbours again. Images channels last with whole groups of eight channels need no preparation: cp.async puts them there.
 //   * input rows are kept by phase of the vertical stride too, so a tile's raster (R output rows of Wp positions) is contiguous for
 //     every filter row. Rows of an instruction past the raster read whatever follows; their results are not stored.
-//   * Bound: what the sixteen warps do for an item (2800 cycles of preparation, 2900 of stores, 1400 of copies for four tiles of 64 channels),
-//     against 3000 cycles of products. us, the gathering form before: N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2 100 -> 71; 30 x 7 -> 32
-//     channels, 184 x 184, 7 x 7 stride 2 81 -> 26; 20 x 16 -> 32, 223 x 223, 3 x 3 116 -> 39; 109 x 8 -> 64, 62 x 62, 5 x 5 53 -> 31;
-//     36 x 3 -> 32, 195 x 195, 3 x 3 stride 2 83 -> 19 (rows that start on any even byte). Of 1000 convolutions
+//   * Bound: what the sixteen warps do for an item, one after the other: of 9360 cycles (with clocks read in between) for four tiles of 64 channels
+//     3340 go into preparation, 3260 into stores, 1560 into copies and 990 into waits, beside 2980 of products. us, the gathering form before:
+//     N = 64, 3 -> 64 channels, 224 x 224, 7 x 7 stride 2 100 -> 71; 30 x 7 -> 32 channels, 184 x 184, 7 x 7 stride 2 82 -> 25; 20 x 16 -> 32,
+//     223 x 223, 3 x 3 116 -> 39; 109 x 8 -> 64, 62 x 62, 5 x 5 54 -> 31; 36 x 3 -> 32, 195 x 195, 3 x 3 stride 2 107 -> 19 (rows that start on any
+//     even byte). Of 1000 convolutions
 //     that the estimates in conv_patch_pays were not fitted to, they take a form more than 6 % slower than the fastest in 80, and 15 are
 //     more than 5 % slower than without this kernel (the worst 14.2 -> 18.3 us).
 //   * sixteen warps prepare item i + 1 and store item i - 1 while the seventeenth issues item i: two windows, two sets of

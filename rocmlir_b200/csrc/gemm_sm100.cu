@@ -225,8 +225,8 @@ int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_
 // last store is exposed. A K split adds the planes and the pass that sums them. Constants in microseconds, fitted to 24 products in up to
 // eleven configurations each (f16 / bf16 / fp8 / i8, 256^3 to 2048 x 2048 x 4096, replayed graphs; 8 % off on average; what a launch
 // costs by the width of its tiles has gone into `column`). The rule before - 256 columns in pairs whatever the size, a K split as soon as
-// half of the pairs idle - lost most where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.3 / 9.1
-// (64 columns, no split), 1536^3 bf16 28.8 / 16.9, 2048 x 1024 x 2048 f16 21.8 / 14.3, 364 x 1344 x 1792 i8 15.9 / 9.8. Beyond three
+// half of the pairs idle - lost most where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.0 / 8.9
+// (64 columns, no split), 1536^3 bf16 22.5 / 12.7, 2048 x 1024 x 2048 f16 21.7 / 14.5, 364 x 1344 x 1792 i8 15.2 / 9.7. Beyond three
 // waves of the rule's tiles the rule stays, such products being bound by memory or by power, and beyond three of the estimate's own too: their
 // stores take longer than estimated (3 x 180 x 7720 x 213 bf16 in tiles of 64 columns 20.9 us, by the rule 18.0; of 19 such products ten were
 // slower). Of 600 further products whose tile or split it changes (200 of them of two or three waves), one is more than 2 % slower than by the rule,
@@ -894,8 +894,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
       kp.c_stride_g = (reinterpret_cast<intptr_t>(chain->c2) - reinterpret_cast<intptr_t>(c)) / (intptr_t)es_c;
     kp.vec_ok = (!p->trans_c && ((size_t)p->n * es_c) % 16 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0) ? 1 : 0;
     // rows off 16-byte boundaries: staged like the others, copied out by the warps (us, element stores from the registers before): 3 x 640 x
-    // 2279, K = 768, bf16 with bias and ReLU 182 -> 51; 2000 x 3001 x 640 97 -> 33; 4096 x 4095 x 4096 f16 228 -> 127; f32 768 x 1043 x 3648
-    // 102 -> 70
+    // 2279, K = 768, bf16 with bias and ReLU 179 -> 30; 2000 x 3001 x 640 95 -> 29; 4096 x 4095 x 4096 f16 243 -> 149; f32 768 x 1043 x 3648
+    // 98 -> 64
     // (and so is an 8-bit result in tiles of 64 columns: the box of the store map is a staged row, 128 of them)
     kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok && bn * es_c >= (size_t)kRowBytes ? 1 : 2;
     if (conva && conva->c_rows_per_img > 0) {   // NKHW result: strided element stores, coalesced along the pixels

@@ -248,7 +248,8 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* s
                "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-// The same, added to what C holds (f32, each element rounded to nearest).
+// The same, added to what C holds (f32, each element rounded to nearest; subnormal numbers are kept, which
+// tests/test_gemm_f32_ranges_gpu.py holds).
 __device__ __forceinline__ void tma_add_3d(const CUtensorMap* m, const void* src, int c0, int c1, int c2) {
   asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(m)),
