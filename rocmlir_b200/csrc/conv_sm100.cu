@@ -783,10 +783,10 @@ extern "C" RbStatus rbConvGetGemmProblem(const RbConvProblem* p, RbGemmProblem* 
   return RB_SUCCESS;
 }
 
-RbStatus rb::conv_gemm_config(const RbConvProblem* p, RbGemmConfigInfo* out) {
+RbStatus rb::conv_gemm_config(const RbConvProblem* p, RbGemmConfigInfo* out, bool one_kernel) {
   ConvPlan pl;
   const RbStatus st = make_plan(p, &pl);
-  return st == RB_SUCCESS ? gemm_config(&pl.gemm, pl.a_implicit ? 0 : pl.b_implicit ? 1 : -1, out) : st;
+  return st == RB_SUCCESS ? gemm_config(&pl.gemm, pl.a_implicit ? 0 : pl.b_implicit ? 1 : -1, out, one_kernel) : st;
 }
 
 extern "C" int rbConvKernelCount(const RbConvProblem* p) {

@@ -245,8 +245,8 @@ constexpr TileCost kTileCostsF32[] = {{1, 64, 6.9, 0.57, 48}, {1, 128, 5.3, 0.67
 // the rule does not cut it: such a product needs no planes in its workspace and can be handed out as one kernel. An f32 result keeps
 // accumulation chains no longer than the rule's: the tensor core truncates what it adds, and of two chains in place of one the error of f16 and
 // fp8 products against 64 bits is half (1.2e-6 -> 0.6e-6 at K = 1024; values of one sign 6.1e-6 -> 2.8e-6). In a 16-bit result its rounding hides that
-// (2.067e-4 both ways).
-void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, int* ctas, int* bn, int* splits) {
+// (2.067e-4 both ways). any_chain: without that (see choose_one_kernel).
+void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, bool any_chain, int* ctas, int* bn, int* splits) {
   // store of a column of a tile: an 8-bit result is requantised, rows off 16 bytes are copied out by the warps
   const double column = 0.025 * (p->c_type == RB_I8 ? 1.56 : 1.0) * ((long long)p->n * (long long)dtype_bytes(p->c_type) % 16 ? 2.0 : 1.0);
   auto estimate = [&](const TileCost& t, bool split, long long* s, long long* waves) {
@@ -256,8 +256,8 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     const long long items = tiles * *s, kb = (kblocks + *s - 1) / *s;
     *waves = (items + units - 1) / units;
     const double busy = (double)std::min(items, units) * t.ctas;
-    // (a byte per element in 64 columns: half of a staged row, copied out by the warps; 3.2 us a requantised tile)
-    const double narrow = t.bn == 64 && dtype_bytes(p->c_type) == 1 ? 1.3 : 1.0;
+    // (a byte per element in 64 columns: half of a staged row, copied out by the warps; 3.2 us a requantised tile where tiles follow one another)
+    const double narrow = t.bn == 64 && dtype_bytes(p->c_type) == 1 && *waves > 1 ? 1.3 : 1.0;
     const double block = std::max(t.block, busy * t.kb_per_block / 12500.0), store = t.bn * (*s > 1 ? 0.025 : column * narrow);
     double us = t.fixed + std::max(kb * block, store) * (double)(*waves - 1) + kb * block + store;
     if (*s > 1) us += 3.7 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.283;
@@ -273,7 +273,7 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     if (t.ctas == rule_ctas && t.bn == rule_bn) best = 0.85 * estimate(t, true, &s, &waves);
   }
   if (best == 0 || waves > 3 || (f32 && (s > 1 || p->k > 2048))) return;   // (s and waves are those of the rule's tile)
-  const long long rule_splits = s, chain = p->c_type == RB_F32 && p->ab_type != RB_I8 ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
+  const long long rule_splits = s, chain = p->c_type == RB_F32 && p->ab_type != RB_I8 && !any_chain ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
     if (f32 && t.ctas == 1 && t.bn == 256) continue;
@@ -286,7 +286,7 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
   }
 }
 
-GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false) {
+GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false, bool any_chain = false) {
   GemmConfig c;
   if (variant == 0) variant = (int)tuned_variant_gemm(p);   // the measured table, when it knows the problem
   const int es = (int)dtype_bytes(p->ab_type);
@@ -315,7 +315,7 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   if (c.bn == 64 && (variant & 0xF) != 2) c.ctas = 1;        // measured: 64-column tiles run faster unpaired (345 vs 324 TFLOP/s)
   int est_splits = 0;
   if (variant == 0 && !implicit && (p->ab_type != RB_F32 || planes == 2))
-    estimate_tile(p, b_mn, che, (p->k + kRowBytes / es - 1) / (kRowBytes / es), planned_sms(), &c.ctas, &c.bn, &est_splits);
+    estimate_tile(p, b_mn, che, (p->k + kRowBytes / es - 1) / (kRowBytes / es), planned_sms(), any_chain, &c.ctas, &c.bn, &est_splits);
   c.stages = (variant >> 4) & 0xF;
   const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec, planes) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec, planes);
   if (c.stages <= 0 || c.stages > max_stages) c.stages = max_stages;
@@ -369,6 +369,15 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
     }
   }
   return c;
+}
+
+// The configuration of a launch that is to be one kernel, or has no room for the planes of K ranges: ranges that only keep the sums of an
+// f32 result short are left out, others stay.
+GemmConfig choose_one_kernel(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false) {
+  const GemmConfig c = choose_config(p, variant, epi_vec, implicit);
+  if (c.splits == 1) return c;
+  const GemmConfig whole = choose_config(p, variant, epi_vec, implicit, true);
+  return whole.splits == 1 ? whole : c;
 }
 
 // Sums the partial planes of a K split in a fixed order (range 0, 1, 2, ...), applies the epilogue and
@@ -525,7 +534,7 @@ extern "C" void rbSetWaitLimit(uint64_t sm_cycles) {
 }
 extern "C" void rbInjectStall(int launches) { t_stall_launches = launches > 0 ? launches : 0; }
 
-size_t rb::gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand) {
+size_t rb::gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand, bool least) {
   if (check_problem(p) != RB_SUCCESS) return 0;
   const size_t es = dtype_bytes(p->ab_type);
   const bool f32 = p->ab_type == RB_F32, split = f32 && p->f32_mode == 0;
@@ -533,7 +542,8 @@ size_t rb::gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand) {
   OperandPlan ob = plan_operand(p->trans_b == 0, p->n, p->k, es, f32, split);
   if (implicit_operand == 0) oa.needs_copy = false;
   if (implicit_operand == 1) ob.needs_copy = false;
-  return plan_workspace(p, oa, ob, choose_config(p, t_variant, false, implicit_operand >= 0)).total;
+  return plan_workspace(p, oa, ob, (least ? choose_one_kernel(p, t_variant, false, implicit_operand >= 0)
+                                          : choose_config(p, t_variant, false, implicit_operand >= 0))).total;
 }
 
 extern "C" size_t rbGemmWorkspaceSize(const RbGemmProblem* p) { return rb::gemm_workspace_bytes(p, -1); }
@@ -556,11 +566,14 @@ RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int 
 
 extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* out) { return rb::gemm_config(p, -1, out); }
 
-RbStatus rb::gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmConfigInfo* out) {
+RbStatus rb::gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmConfigInfo* out, bool one_kernel) {
   RbStatus st = check_problem(p);
   if (st != RB_SUCCESS) return st;
   if (!out) return fail(RB_INVALID_PARAM, "out is NULL");
-  const GemmConfig c = choose_config(p, t_variant, false, implicit_operand >= 0);
+  const auto choose = [&](bool epi_vec) {
+    return one_kernel ? choose_one_kernel(p, t_variant, epi_vec, implicit_operand >= 0) : choose_config(p, t_variant, epi_vec, implicit_operand >= 0);
+  };
+  const GemmConfig c = choose(false);
   const int es = (int)dtype_bytes(p->ab_type);
   const long long tiles = (long long)p->g * ((p->m + kBM * c.ctas - 1) / (kBM * c.ctas)) * ((p->n + c.bn - 1) / c.bn);
   const long long items = tiles * c.splits;
@@ -579,7 +592,7 @@ RbStatus rb::gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmCon
                                               : GemmSmemLayout<1>::total(c.stages, c.bn, false, gemm_planes(p)));
   // with per-column epilogue vectors (bias / column scales) the ring may be one stage shorter and the staging single
   {
-    const GemmConfig ce = choose_config(p, t_variant, true, implicit_operand >= 0);
+    const GemmConfig ce = choose(true);
     out->stages_epi_vec = ce.stages;
     out->dynamic_smem_epi_vec = (uint32_t)(ce.ctas == 2 ? GemmSmemLayout<2>::total(ce.stages, ce.bn, true, gemm_planes(p))
                                                         : GemmSmemLayout<1>::total(ce.stages, ce.bn, true, gemm_planes(p)));
@@ -687,6 +700,10 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   const bool epi_vec = epi_needs_col_vectors(flags);
   GemmConfig cfg = choose_config(p, t_variant, epi_vec, conva != nullptr);
   Workspace ws = plan_workspace(p, oa, ob, cfg);
+  if (cfg.splits > 1 && (capture || !workspace || workspace_bytes < ws.total)) {
+    cfg = choose_one_kernel(p, t_variant, epi_vec, conva != nullptr);
+    ws = plan_workspace(p, oa, ob, cfg);
+  }
   if (cfg.sk_tiles > 0 && (!workspace || workspace_bytes < ws.total)) {
     // the stream-K tail is an optimisation: without room for its partial tiles every tile is computed whole
     cfg.sk_tiles = 0;
@@ -1077,7 +1094,8 @@ extern "C" RbStatus rbGemmNoAlloc(const RbGemmProblem* p, const RbEpilogue* epi,
                                   void* stream) {
   RbStatus st = rb::check_problem(p);
   if (st != RB_SUCCESS) return st;
-  const size_t need = rbGemmWorkspaceSize(p);
+  size_t need = rbGemmWorkspaceSize(p);
+  if (need > kNoAllocScratchBytes) need = rb::gemm_workspace_bytes(p, -1, true);
   if (need > kNoAllocScratchBytes)
     return rb::fail(RB_WORKSPACE_TOO_SMALL,
                     "rbGemmNoAlloc: this problem needs " + std::to_string(need) + " bytes of scratch, the built-in "

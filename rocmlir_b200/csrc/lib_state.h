@@ -68,10 +68,11 @@ RbStatus gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void* a, 
 
 // rbGemmWorkspaceSize when operand `implicit_operand` (0 = A, 1 = B, -1 = none) is fetched in place by im2col loads
 // and therefore needs neither a pitched copy nor TF32 planes inside the GEMM's own workspace.
-size_t gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand);
-// rbGemmGetConfig for such a GEMM, and for the GEMM that a convolution runs as.
-RbStatus gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmConfigInfo* out);
-RbStatus conv_gemm_config(const RbConvProblem* p, RbGemmConfigInfo* out);
+size_t gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand, bool least = false);
+// rbGemmGetConfig for such a GEMM, and for the GEMM that a convolution runs as. one_kernel: of the launch that rbGemmEncodeLaunch describes, where
+// there is one. (least: the workspace of that.)
+RbStatus gemm_config(const RbGemmProblem* p, int implicit_operand, RbGemmConfigInfo* out, bool one_kernel = false);
+RbStatus conv_gemm_config(const RbConvProblem* p, RbGemmConfigInfo* out, bool one_kernel = false);
 // TF32 planes of an f32 matrix stack [groups][R][C]: hi (and lo when `split`) with row pitch `pitch` elements;
 // with `transpose` the output is [groups][C][pitch >= R]. x = hi + lo, both exactly representable in TF32.
 RbStatus f32_planes(const float* src, float* hi, float* lo, int groups, int R, int C, int pitch, bool transpose,

@@ -54,7 +54,7 @@ MiirStatus lower(Handle* h, bool binary) {
     const int saved_variant = rbGetGemmVariant();
     rbSetGemmVariant((int)h->d.variant);
     RbGemmConfigInfo info;
-    const RbStatus st = h->d.kind == kConv ? rb::conv_gemm_config(&h->d.conv, &info) : rbGemmGetConfig(&gp, &info);
+    const RbStatus st = h->d.kind == kConv ? rb::conv_gemm_config(&h->d.conv, &info, true) : rb::gemm_config(&gp, -1, &info, true);
     rbSetGemmVariant(saved_variant);
     if (st != RB_SUCCESS) return MIIR_BUILD_FAILURE;
     h->grid = info.grid;

@@ -1255,7 +1255,7 @@ bool run_applicability(Operation* mod) {
   const int saved = rbGetGemmVariant();
   rbSetGemmVariant((int)L.variant);
   RbGemmConfigInfo info;
-  const bool ok = gemm_of(L, &gp) && (L.kind == kGemmKind ? rbGemmGetConfig(&gp, &info) : rb::conv_gemm_config(&L.conv, &info)) == RB_SUCCESS;
+  const bool ok = gemm_of(L, &gp) && (L.kind == kGemmKind ? rb::gemm_config(&gp, -1, &info, true) : rb::conv_gemm_config(&L.conv, &info, true)) == RB_SUCCESS;
   rbSetGemmVariant(saved);
   if (!ok) { mod->diagnostic = std::string("no kernel for the problem: ") + rbGetLastError(); return false; }
   if (L.variant) {   // an explicit configuration must be one the problem can really take

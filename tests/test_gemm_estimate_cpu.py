@@ -48,3 +48,17 @@ def test_eight_bit_results_of_several_waves_keep_wide_tiles():
     """896 x 6016 x 1024, requantised: tiles of 64 columns take 22 us, of 128 17, the rule's 20."""
     p = L.RbGemmProblem(1, 896, 6016, 1024, 0, 1, 0, L.I8, L.I8, 0, 0)
     assert query(p, 0)[0].tile_n >= 128
+
+
+def test_dimensions_of_a_handle_are_those_of_the_one_kernel():
+    """K is cut for the sake of the f32 sums: the handle names the grid of the kernel that a client launches itself, which sums all of K. Cut for
+    speed there is no such kernel, and the grid is the library's."""
+    from rocmlir_b200 import miir
+    for m, n, k, cut, one in ((1024, 1024, 1024, True, True), (64, 576, 8192, True, False), (4096, 4096, 1024, False, False)):
+        p = L.RbGemmProblem(1, m, n, k, 0, 0, 0, L.F16, L.F32, 0, 0)
+        info, ws = query(p, 0)
+        assert (info.splits > 1) == cut and (ws > 0) == cut
+        with miir.Handle(f"--operation gemm --arch sm_100a -t f16 -out_datatype f32 -transA false -transB false -g 1 -m {m} -n {n} -k {k}") as h:
+            h.lower_bin()
+            glob, loc = h.execution_dims()
+            assert (glob // loc != info.grid) == one
