@@ -222,33 +222,42 @@ int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_
 // Tile and K split of a plain product by an estimate of its time, where nobody has asked for one. A launch costs `fixed`; a CTA (or
 // pair) then walks its tiles, K block by K block: at least `block` (operand fetch and issue of its MMAs), and no faster than all
 // CTAs together draw operands through the L2 -> SM fabric; a tile shorter than the store of the tile before it waits for that; the
-// last store is exposed. A K split adds the planes and the pass that sums them. Constants in microseconds, fitted to 24 products in up to
-// eleven configurations each (f16 / bf16 / fp8 / i8, 256^3 to 2048 x 2048 x 4096, replayed graphs; 8 % off on average; what a launch
-// costs by the width of its tiles has gone into `column`). The rule before - 256 columns in pairs whatever the size, a K split as soon as
-// half of the pairs idle - lost most where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.0 / 8.9
-// (64 columns, no split), 1536^3 bf16 22.5 / 12.7, 2048 x 1024 x 2048 f16 21.7 / 14.5, 364 x 1344 x 1792 i8 15.2 / 9.7. Beyond three
-// waves of the rule's tiles the rule stays, such products being bound by memory or by power, and beyond three of the estimate's own too: their
-// stores take longer than estimated (3 x 180 x 7720 x 213 bf16 in tiles of 64 columns 20.9 us, by the rule 18.0; of 19 such products ten were
-// slower). Of 600 further products whose tile or split it changes (200 of them of two or three waves), one is more than 2 % slower than by the rule,
-// 3 x 321 x 1360 x 3833 fp8 24.5 -> 27.0; the mean is 0.79 of the rule's time. The chained pair of rbGemmGemm goes by the same estimate: 12 sizes from
-// 128 x 256 x 256 to 2048 x 2048 x 2048, f16 and bf16, took 0.71 to 1.00 of the rule's time.
+// last store is exposed. A K split adds the planes and the pass that sums them. Constants in microseconds, fitted to every tile of 1600 products (f16,
+// bf16, fp8, i8; up to three waves of the rule's tiles, with and without K ranges; replayed graphs; 7 % off on average, on others too), for f32 to six
+// products, operand passes included. The rule before - 256 columns in pairs whatever the size, a K split as soon as half of the pairs idle - lost most
+// where a product is a wave of tiles or less, us before and by the estimate: 1024^3 f16 15.0 / 8.9 (64 columns, no split), 1536^3 bf16 22.5 / 12.7,
+// 2048 x 1024 x 2048 f16 21.7 / 14.5, 364 x 1344 x 1792 i8 15.2 / 9.7. Beyond three waves of its tiles the rule stays, such products being bound by memory
+// or by power. Of 2831 products, 700 of them new to the fit, 15 are more than 2 % slower than by the rule (1536 x 448 x 4736 f16 18.1 -> 19.2 the most),
+// of 600 more two, and the mean is 0.86 of its time, 1.005 of the fastest tile's. An estimate that took the store of every tile for the exposed one had to be beaten by
+// 15 % and made 34 slower, narrow tiles in many waves above all (3 x 180 x 7720 x 213 bf16 18.0 -> 20.9, 896 x 6016 x 1024 i8 20.4 -> 22.1).
+// The chained pair of rbGemmGemm goes by the same estimate: 12 sizes from 128 x 256 x 256 to 2048 x 2048 x 2048, f16 and bf16, take 0.71 to 1.02 of the
+// rule's time.
 struct TileCost {
   int ctas, bn;
   double fixed, block, kb_per_block;   // kb_per_block: KB a CTA fetches per K block
 };
-constexpr TileCost kTileCosts[] = {{1, 64, 3.7, 0.252, 24}, {1, 128, 2.1, 0.326, 32}, {2, 128, 3.6, 0.246, 24}, {1, 256, 0.0, 0.404, 48}, {2, 256, 0.8, 0.335, 32}};
-
-// f32 with two planes (the operand passes included); only where the rule does not cut K, so that no accumulation chain gets longer
+struct StoreCost {
+  double last, tile, column, ragged, margin;   // a column of the exposed store; a tile and a column of the others; rows off 16 bytes; what an estimate must beat
+};
+constexpr TileCost kTileCosts[] = {{1, 64, 4.75, 0.239, 24}, {1, 128, 4.35, 0.311, 32}, {2, 128, 5.68, 0.233, 24}, {1, 256, 3.50, 0.446, 48}, {2, 256, 4.91, 0.324, 32}};
+constexpr StoreCost kStoreCost = {0.0087, 0.84, 0.0084, 2.58, 0.97};
+// f32 with two planes; only where the rule does not cut K, so that no accumulation chain gets longer
 constexpr TileCost kTileCostsF32[] = {{1, 64, 6.9, 0.57, 48}, {1, 128, 5.3, 0.67, 64}, {2, 128, 6.4, 0.56, 48}, {1, 256, 5.5, 0.95, 96}, {2, 256, 4.4, 0.87, 64}};
+constexpr StoreCost kStoreCostF32 = {0.025, 0.0, 0.025, 2.0, 0.85};
 
-// *ctas and *bn come in as the rule gives them and stay unless another tile, or fewer K ranges, is estimated at 15 % less. K is not cut where
+// *ctas and *bn come in as the rule gives them and stay unless another tile, or fewer K ranges, is estimated faster by the margin. K is not cut where
 // the rule does not cut it: such a product needs no planes in its workspace and can be handed out as one kernel. An f32 result keeps
 // accumulation chains no longer than the rule's: the tensor core truncates what it adds, and of two chains in place of one the error of f16 and
 // fp8 products against 64 bits is half (1.2e-6 -> 0.6e-6 at K = 1024; values of one sign 6.1e-6 -> 2.8e-6). In a 16-bit result its rounding hides that
-// (2.067e-4 both ways). any_chain: without that (see choose_one_kernel).
-void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, bool any_chain, int* ctas, int* bn, int* splits) {
-  // store of a column of a tile: an 8-bit result is requantised, rows off 16 bytes are copied out by the warps
-  const double column = 0.025 * (p->c_type == RB_I8 ? 1.56 : 1.0) * ((long long)p->n * (long long)dtype_bytes(p->c_type) % 16 ? 2.0 : 1.0);
+// (2.067e-4 both ways). whole: only all of K at once, whatever the result, where that is no slower than the rule (see choose_one_kernel).
+void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, bool whole, int* ctas, int* bn, int* splits) {
+  const bool f32 = p->ab_type == RB_F32;
+  const TileCost* const costs = f32 ? kTileCostsF32 : kTileCosts;
+  const StoreCost& sc = f32 ? kStoreCostF32 : kStoreCost;
+  const int es_c = (int)dtype_bytes(p->c_type);
+  // an 8-bit result is requantised, 4-byte ones (and planes) are two staged rows for one; rows off 16 bytes are copied out by the warps
+  const double words = f32 ? 1.0 : 1.45;
+  const double width = (p->c_type == RB_I8 ? 2.76 : es_c == 4 ? words : 1.0) * ((long long)p->n * es_c % 16 ? sc.ragged : 1.0);
   auto estimate = [&](const TileCost& t, bool split, long long* s, long long* waves) {
     const long long tiles = (long long)p->g * ((p->m + kBM * t.ctas - 1) / (kBM * t.ctas)) * ((p->n + t.bn - 1) / t.bn);
     const long long units = sms / t.ctas;
@@ -256,37 +265,37 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     const long long items = tiles * *s, kb = (kblocks + *s - 1) / *s;
     *waves = (items + units - 1) / units;
     const double busy = (double)std::min(items, units) * t.ctas;
-    // (a byte per element in 64 columns: half of a staged row, copied out by the warps; 3.2 us a requantised tile where tiles follow one another)
-    const double narrow = t.bn == 64 && dtype_bytes(p->c_type) == 1 && *waves > 1 ? 1.3 : 1.0;
-    const double block = std::max(t.block, busy * t.kb_per_block / 12500.0), store = t.bn * (*s > 1 ? 0.025 : column * narrow);
-    double us = t.fixed + std::max(kb * block, store) * (double)(*waves - 1) + kb * block + store;
-    if (*s > 1) us += 3.7 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.283;
+    const double block = std::max(t.block, busy * t.kb_per_block / 12500.0);
+    // (a byte per element in 64 columns: half of a staged row, copied out by the warps)
+    const double columns = t.bn * (*s > 1 ? words : t.bn == 64 && es_c == 1 ? 1.52 * width : width);
+    double us = t.fixed + std::max(kb * block, sc.tile + sc.column * columns) * (double)(*waves - 1) + kb * block + sc.last * columns;
+    if (*s > 1) us += 2.13 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.265;
     return us;
   };
   const int rule_ctas = *ctas, rule_bn = *bn;
-  const bool f32 = p->ab_type == RB_F32;
-  const TileCost* const costs = f32 ? kTileCostsF32 : kTileCosts;
   double best = 0;
   long long s = 1, waves = 1;
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
-    if (t.ctas == rule_ctas && t.bn == rule_bn) best = 0.85 * estimate(t, true, &s, &waves);
+    if (t.ctas == rule_ctas && t.bn == rule_bn) best = (whole ? 1.0 : sc.margin) * estimate(t, true, &s, &waves);
   }
   if (best == 0 || waves > 3 || (f32 && (s > 1 || p->k > 2048))) return;   // (s and waves are those of the rule's tile)
-  const long long rule_splits = s, chain = p->c_type == RB_F32 && p->ab_type != RB_I8 && !any_chain ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
+  const long long rule_splits = whole ? 1 : s;
+  const long long chain = p->c_type == RB_F32 && p->ab_type != RB_I8 && !whole ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
     if (f32 && t.ctas == 1 && t.bn == 256) continue;
     if (b_mn && (t.bn / t.ctas) % che != 0) continue;
     if (t.ctas == 2 && (p->m <= kBM || kblocks <= 2)) continue;   // (see choose_config)
     for (int split = 0; split < (rule_splits > 1 ? 2 : 1); ++split) {
-      const double us = estimate(t, split != 0, &s, &waves);
-      if (us < best && (kblocks + s - 1) / s <= chain && waves <= 3) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
+      double us = estimate(t, split != 0, &s, &waves);
+      if (s > 1) us *= 1.08;   // (K ranges other than the rule's are the less certain ones)
+      if (us < best && (kblocks + s - 1) / s <= chain) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
     }
   }
 }
 
-GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false, bool any_chain = false) {
+GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false, bool whole = false) {
   GemmConfig c;
   if (variant == 0) variant = (int)tuned_variant_gemm(p);   // the measured table, when it knows the problem
   const int es = (int)dtype_bytes(p->ab_type);
@@ -315,7 +324,7 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   if (c.bn == 64 && (variant & 0xF) != 2) c.ctas = 1;        // measured: 64-column tiles run faster unpaired (345 vs 324 TFLOP/s)
   int est_splits = 0;
   if (variant == 0 && !implicit && (p->ab_type != RB_F32 || planes == 2))
-    estimate_tile(p, b_mn, che, (p->k + kRowBytes / es - 1) / (kRowBytes / es), planned_sms(), any_chain, &c.ctas, &c.bn, &est_splits);
+    estimate_tile(p, b_mn, che, (p->k + kRowBytes / es - 1) / (kRowBytes / es), planned_sms(), whole, &c.ctas, &c.bn, &est_splits);
   c.stages = (variant >> 4) & 0xF;
   const int max_stages = c.ctas == 2 ? GemmSmemLayout<2>::max_stages(c.bn, epi_vec, planes) : GemmSmemLayout<1>::max_stages(c.bn, epi_vec, planes);
   if (c.stages <= 0 || c.stages > max_stages) c.stages = max_stages;
@@ -372,7 +381,7 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
 }
 
 // The configuration of a launch that is to be one kernel, or has no room for the planes of K ranges: ranges that only keep the sums of an
-// f32 result short are left out, others stay.
+// f32 result short, or gain little, are left out; others stay.
 GemmConfig choose_one_kernel(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false) {
   const GemmConfig c = choose_config(p, variant, epi_vec, implicit);
   if (c.splits == 1) return c;
