@@ -214,9 +214,9 @@ int skinny_splits(const RbGemmProblem* p, long long tiles, int kblocks, int sms)
 //   several CTAs per slot, one tile each where the general kernel is persistent: 64 x 4096 x 128 in 64 groups: 90.7 / 22.9,
 //                16: 40.8 / 22.0;  16 x 128256 x 4096: 165 / 183;  1 x 64 x 64 in 512 groups: 8.0 / 11.5
 //   C off 16 bytes, one part, short K: 35 x 10245 x 64: 8.6 / 10.0;  64 x 1023 x 256: 12.2 / 8.5;  64 x 4095 x 128 in 64 groups: 90.5 / 83
-// Of 600 products of up to 64 rows on 16 bytes, four are more than 5 % slower by these lines than on the general kernel (64 x 1024 x 1024 by 5 %:
-// drawn before that one chose its tiles by an estimate). Of 300 off 16 bytes two are; taking this kernel for all of them, 42 of 700 were
-// more than 6 % slower.
+// Of 600 products of up to 64 rows on 16 bytes, one is more than 5 % slower by these lines than on the general kernel (48 x 224 x 992 i8, 9.1 / 6.8).
+// Of 400 off 16 bytes five are (59 x 2246 x 2288 fp8 in 57 groups 90 / 75); taking this kernel for all of them, 42 of 700 were more than 6 %
+// slower.
 bool gemm_skinny_applicable(const RbGemmProblem* p, uint32_t epi_flags) {
   const long long es = (long long)dtype_bytes(p->ab_type);
   if (p->m > 64 || p->trans_a || !p->trans_b || p->trans_c || p->ab_type == RB_F32 || (p->k * es) % 16) return false;
