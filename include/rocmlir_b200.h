@@ -135,7 +135,9 @@ typedef struct RbGemmProblem {
                            rounded to C's type and added in it; f32 / f16 / bf16 results. Deterministic: no atomics. */
 } RbGemmProblem;
 
-/* Bytes of caller-provided device workspace rbGemm needs for this problem (0 for most). */
+/* Bytes of caller-provided device workspace rbGemm needs for this problem (0 for most). With less, a product whose K would be cut into
+ * ranges runs uncut where that is estimated to be about as fast (sums of an f32 result are then longer); everything else is refused with
+ * RB_WORKSPACE_TOO_SMALL. */
 RB_EXPORT size_t rbGemmWorkspaceSize(const RbGemmProblem *p);
 
 /* Runs the GEMM on `stream`. Returns RB_UNSUPPORTED for problems outside the kernel's reach. */
@@ -153,7 +155,7 @@ RB_EXPORT RbStatus rbGemm(const RbGemmProblem *p, const RbEpilogue *epi /* may b
  * fixed RB_NO_ALLOC_SCRATCH_BYTES array inside the library image instead. It calls no cudaMalloc, cudaFree or
  * allocating library routine. The inputs and the output are still the caller's.
  *
- *  - Problems whose scratch need (rbGemmWorkspaceSize) exceeds RB_NO_ALLOC_SCRATCH_BYTES are rejected with
+ *  - Problems whose scratch need (rbGemmWorkspaceSize; uncut, where rbGemm would run them so) exceeds RB_NO_ALLOC_SCRATCH_BYTES are rejected with
  *    RB_WORKSPACE_TOO_SMALL and a message naming both sizes; nothing is launched.
  *  - The first call on each device looks up the scratch array's device address (cudaGetSymbolAddress, with that
  *    device current). Make that first call before any stream capture begins.
@@ -197,7 +199,8 @@ typedef struct RbConvProblem {
 } RbConvProblem;
 
 /* Bytes of device workspace rbConv needs (gathered operand matrices, split-K planes); the counterpart of
- * miirGetWorkspaceSize (mlir/tools/rocmlir-lib/Miir.h:60-66). 0 also for an invalid problem. */
+ * miirGetWorkspaceSize (mlir/tools/rocmlir-lib/Miir.h:60-66). 0 also for an invalid problem. For some few-channel images it is what an image
+ * off 16 bytes is better computed with; those run with less, too. */
 RB_EXPORT size_t rbConvWorkspaceSize(const RbConvProblem *p);
 
 /* Number of kernels one rbConv call launches besides those inside its GEMM (counterpart of
@@ -359,7 +362,7 @@ RB_EXPORT void rbSetGemmVariant(int variant);
 RB_EXPORT int rbGetGemmVariant(void);
 
 /* The tile configuration in which the GEMM kernel of the kernel image would be launched for `p` under the calling thread's
- * variant word (on a 148-SM B200), the one rbGemmEncodeLaunch encodes. rbGemm runs some products with at most 64 rows against
+ * variant word (on a 148-SM B200) with its workspace; rbGemmEncodeLaunch encodes the same, or the uncut form of a product whose K is cut. rbGemm runs some products with at most 64 rows against
  * B stored N x K on a kernel of their own, which is not in the image and has no variants; this query, the
  * workspace size and the tuning space keep describing the image's kernel for them, which any explicit variant word selects.
  * The query gives the information rocMLIR attaches to a lowered kernel as block_size / grid_size attributes
