@@ -25,50 +25,15 @@
 //            cancels the stale reference); final O / l and TMA store.
 // S_{j+1} is issued before P_j is awaited, so the score MMA of the next block overlaps the softmax of this one.
 // MMAs of one issuing thread execute in order, which is what makes P_j safe in the buffer S_{j+2} will overwrite.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include <algorithm>
 #include <string>
 
-#include "epilogue.cuh"
-#include "lib_state.h"
-#include "ptx.cuh"
+#include "attention.cuh"
 
 namespace rb {
 namespace {
 
-constexpr int kQT = 128;    // query rows per CTA
-constexpr int kKT = 128;    // keys per block
 constexpr int kAttThreads = 256;
-constexpr float kLog2e = 1.4426950408889634f;
-
-struct AttMaps {
-  CUtensorMap q, k, v, o;
-};
-
-struct AttParams {
-  int G, Sq, Sk, D, Dv;
-  int trans_k;       // K stored [G][Sk][D] (K-major) instead of [G][D][Sk]
-  int is_bf16;
-  int causal;
-  int q_tiles;
-  float scale_log2;  // scale * log2(e)
-  const void* bias;  // optional additive [G][Sq][Sk], element type
-  const void* scale_t;  // optional multiplicative [G][Sq][Sk], element type (applied before the bias)
-  const int8_t* mask;  // optional [G][Sq][Sk]: score kept where mask != 0, else mask_fill
-  float mask_fill;
-  long long mask_bytes;   // size of the mask
-  uint32_t idesc_s, idesc_pv;
-  uint32_t* status;
-  const void* quant_bias;      // first-GEMM-quantised form: device pointers to one i8 and one f16 (else null)
-  const void* quant_scale;
-  unsigned long long* trace;   // optional [CTAs][16] cycle counters (two-tile kernel), see rbSetTraceBuffer
-  int splits;        // single-tile kernel: CTAs of a cluster that divide a query tile's key blocks (1, 2, 4 or 8)
-  void* o;           //   result [G][Sq][o_cols] and its row length, written directly when splits > 1
-  int o_cols;
-  int linear;        // GEMM+GEMM: P = S rounded to the element type (no scale, no softmax, no division by a row sum)
-};
 
 struct AttSmem {
   static constexpr int kQBytes = kQT * 256;        // up to D = 128 f16
@@ -81,25 +46,6 @@ struct AttSmem {
   static constexpr int kBars = kV + kStages * kVBytes;
   static constexpr int kTotal = kBars + 256 + 1024;
 };
-
-__device__ __forceinline__ float load_elem(const void* p, long long i, int is_bf16) {
-  return is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i])
-                 : __half2float(reinterpret_cast<const __half*>(p)[i]);
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b, int is_bf16) {
-  if (is_bf16) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&h);
-  }
-  __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 constexpr int kMaxSplits = 8;   // portable cluster size
 __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
@@ -880,7 +826,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Two query tiles per CTA. One softmax group alone leaves the tensor pipe idle while it works: P_j.V_j has to wait
+// Two query tiles per CTA, scores with side tensors (scale, bias, mask, quantised) or without a softmax; without side tensors
+// attention_prefill_sm100.cu. One softmax group alone leaves the tensor pipe idle while it works: P_j.V_j has to wait
 // for softmax(j). With two 128-row query tiles (A, B) that share every K/V tile, the products of one tile run while
 // the other tile's softmax group computes:   ... PV_A(j)  S_A(j+1)  PV_B(j)  S_B(j+1) ...
 // 384 threads: warp 0 producer, warp 1 MMA issuer, warp 2 TMEM allocator, warps 4-7 softmax of tile A, warps 8-11
@@ -1114,8 +1061,6 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
       sm_wait += ts1 - ts0;
       tc_fence_after();
       const int key0 = j * kKT;
-      const bool side_inputs = p.bias || p.mask || p.scale_t || p.quant_scale;
-      const bool edge = (key0 + kKT > p.Sk) || (p.causal && key0 + kKT - 1 > tq0);
       const int limit = min(p.Sk - key0, p.causal ? (int)min(row - key0 + 1, (long long)kKT) : kKT);
       const long long side_off = ((long long)g * p.Sq + min(row, (long long)p.Sq - 1)) * p.Sk + key0;
       // x(i): score of key key0 + i in the log2 domain after scale, bias and masks
@@ -1134,7 +1079,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
           return x * p.scale_log2;
         }
         x *= p.scale_log2;
-        if (side_inputs && i < p.Sk - key0) {
+        if (i < p.Sk - key0) {
           if (p.scale_t) x *= load_elem(p.scale_t, side_off + i, p.is_bf16);
           if (p.bias) x = fmaf(load_elem(p.bias, side_off + i, p.is_bf16), kLog2e, x);
           if (p.mask && p.mask[side_off + i] == 0) x = p.mask_fill * kLog2e;
@@ -1166,10 +1111,10 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
         continue;
       }
       // pass 1: row maximum over both halves
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+      float mx = -INFINITY;
       float m_use = 0.0f;
-      // exponent argument x(i) - m; without a bias it is the same single fused multiply-add as on the fast path, so
-      // that a mask tensor and the analytic causal mask give bit-identical results
+      // exponent argument x(i) - m; without a bias it is the same single fused multiply-add as in the kernel without side
+      // tensors, so that a mask tensor and the analytic causal mask give bit-identical results
       auto fe = [&](uint32_t raw, int i) -> float {
         float a = (p.bias || p.scale_t || p.quant_scale) ? fx(raw, i) - m_use : fmaf(__uint_as_float(raw), p.scale_log2, -m_use);
         if (p.mask && i < p.Sk - key0 && p.mask[side_off + i] == 0) a = p.mask_fill * kLog2e - m_use;
@@ -1180,32 +1125,12 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
         uint32_t v[64];
         tmem_ld64(tmem_s + h * 64, v);
         tmem_ld_wait();
-        if (!side_inputs && !edge) {
 #pragma unroll
-          for (int i = 0; i < 64; i += 4) {
-            mx0 = fmaxf(mx0, __uint_as_float(v[i])); mx1 = fmaxf(mx1, __uint_as_float(v[i + 1]));
-            mx2 = fmaxf(mx2, __uint_as_float(v[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(v[i + 3]));
-          }
-        } else if (!side_inputs) {
-          // key tail / diagonal block: keys at or past `limit` are dropped with a select
-#pragma unroll
-          for (int i = 0; i < 64; i += 4) {
-            const int c0 = h * 64 + i;
-            mx0 = fmaxf(mx0, (c0 < limit) ? __uint_as_float(v[i]) : -INFINITY);
-            mx1 = fmaxf(mx1, (c0 + 1 < limit) ? __uint_as_float(v[i + 1]) : -INFINITY);
-            mx2 = fmaxf(mx2, (c0 + 2 < limit) ? __uint_as_float(v[i + 2]) : -INFINITY);
-            mx3 = fmaxf(mx3, (c0 + 3 < limit) ? __uint_as_float(v[i + 3]) : -INFINITY);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const float x = (h * 64 + i < limit) ? fx(v[i], h * 64 + i) : -INFINITY;
-            mx0 = fmaxf(mx0, x);
-          }
+        for (int i = 0; i < 64; ++i) {
+          const float x = (h * 64 + i < limit) ? fx(v[i], h * 64 + i) : -INFINITY;
+          mx = fmaxf(mx, x);
         }
       }
-      float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-      if (!side_inputs) mx *= p.scale_log2;   // the scale is positive: max commutes with it (-inf stays -inf)
       float alpha = 1.0f;
       if (mx > m_ref + 8.0f || (m_ref == -INFINITY && mx > -INFINITY)) {
         alpha = ex2(m_ref - mx);
@@ -1220,38 +1145,13 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
         tmem_ld64(tmem_s + h * 64, v);
         tmem_ld_wait();
         uint32_t w[32];
-        if (!side_inputs && !edge) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float p0 = ex2(fmaf(__uint_as_float(v[2 * i]), p.scale_log2, -m_use));
-            const float p1 = ex2(fmaf(__uint_as_float(v[2 * i + 1]), p.scale_log2, -m_use));
-            const float p2 = ex2(fmaf(__uint_as_float(v[2 * i + 2]), p.scale_log2, -m_use));
-            const float p3 = ex2(fmaf(__uint_as_float(v[2 * i + 3]), p.scale_log2, -m_use));
-            l0 += p0; l1 += p1; l2 += p2; l3 += p3;
-            w[i] = pack2(p0, p1, p.is_bf16);
-            w[i + 1] = pack2(p2, p3, p.is_bf16);
-          }
-        } else if (!side_inputs) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const int c0 = h * 64 + 2 * i;
-            const float p0 = (c0 < limit) ? ex2(fmaf(__uint_as_float(v[2 * i]), p.scale_log2, -m_use)) : 0.0f;
-            const float p1 = (c0 + 1 < limit) ? ex2(fmaf(__uint_as_float(v[2 * i + 1]), p.scale_log2, -m_use)) : 0.0f;
-            const float p2 = (c0 + 2 < limit) ? ex2(fmaf(__uint_as_float(v[2 * i + 2]), p.scale_log2, -m_use)) : 0.0f;
-            const float p3 = (c0 + 3 < limit) ? ex2(fmaf(__uint_as_float(v[2 * i + 3]), p.scale_log2, -m_use)) : 0.0f;
-            l0 += p0; l1 += p1; l2 += p2; l3 += p3;
-            w[i] = pack2(p0, p1, p.is_bf16);
-            w[i + 1] = pack2(p2, p3, p.is_bf16);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int c0 = h * 64 + 2 * i;
-            const float p0 = (c0 < limit) ? ex2(fe(v[2 * i], c0)) : 0.0f;
-            const float p1 = (c0 + 1 < limit) ? ex2(fe(v[2 * i + 1], c0 + 1)) : 0.0f;
-            if (i & 1) { l2 += p0; l3 += p1; } else { l0 += p0; l1 += p1; }   // same summation order as the fast path
-            w[i] = pack2(p0, p1, p.is_bf16);
-          }
+        for (int i = 0; i < 32; ++i) {
+          const int c0 = h * 64 + 2 * i;
+          const float p0 = (c0 < limit) ? ex2(fe(v[2 * i], c0)) : 0.0f;
+          const float p1 = (c0 + 1 < limit) ? ex2(fe(v[2 * i + 1], c0 + 1)) : 0.0f;
+          if (i & 1) { l2 += p0; l3 += p1; } else { l0 += p0; l1 += p1; }   // the order of the kernel without side tensors
+          w[i] = pack2(p0, p1, p.is_bf16);
         }
         // half h of P -> columns 32h .. 32h+31 (both halves of S are in registers or consumed by now only for
         // h = 1; for h = 0 the columns 0..31 written here belong to the half already read)
@@ -1769,7 +1669,12 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   kp.trace = trace_buffer((size_t)p->g * ((kp.q_tiles + 1) / 2) * 16);
   const long long ctas = (long long)p->g * kp.q_tiles;
   if (ctas > 0x7fffffffLL) return fail(RB_UNSUPPORTED, "too many query tiles");
-  if (two_query_tiles(p)) {
+  kp.o = o;
+  kp.o_cols = p->head_v;
+  if (two_query_tiles(p) && !p->bias && !p->scale_tensor && !p->mask && !quantized && !kp.linear) {
+    const RbStatus st = attention_prefill_launch(maps, kp, stream);
+    if (st != RB_SUCCESS) return st;
+  } else if (two_query_tiles(p)) {
     const long long ctas2 = (long long)p->g * ((kp.q_tiles + 1) / 2);
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd2_kernel), Att2Smem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
     attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
@@ -1793,8 +1698,6 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
         : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
     const int threads = few ? kDecodeThreads : kAttThreads, smem = few ? DecodeSmem::total((int)Dp, (int)Dvp) : AttSmem::kTotal;
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != RB_SUCCESS) return RB_CUDA_ERROR;
-    kp.o = o;
-    kp.o_cols = p->head_v;
     if (kp.splits == 1) {
       kern<<<(unsigned)ctas, threads, smem, stream>>>(maps, kp);
     } else {

@@ -487,6 +487,66 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t c_fmt, uint32_t a_fmt
          ((m >> 4) << 24);
 }
 
+// ---- registers of a warpgroup -------------------------------------------------------------------
+// All warps of the warpgroup (four, aligned) execute it. What one group gives up another may take: the shares of a block's
+// groups add up to what it was launched with.
+template <int REGS>
+__device__ __forceinline__ void regs_inc() {
+  __syncwarp();
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+template <int REGS>
+__device__ __forceinline__ void regs_dec() {
+  __syncwarp();
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+
+// ---- work of CTAs that have not started ------------------------------------------------------------
+// Asks for the next CTA of the grid that has not started: it is cancelled and the caller does its work. The 16-byte answer
+// arrives on `bar` (the caller expects the bytes). After an answer without a CTA no other request may follow.
+__device__ __forceinline__ void cta_request(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// The blockIdx.x of the answer, or -1.
+__device__ __forceinline__ int cta_answer(const void* answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 A;\n\t.reg .b64 L, H;\n\t.reg .pred P;\n\t"
+      "ld.shared.v2.b64 {L, H}, [%1];\n\t"
+      "mov.b128 A, {L, H};\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 P, A;\n\t"
+      "@P clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, A;\n\t}"
+      : "=r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return x;
+}
+
+// ---- two f32 values in one instruction (each rounded as the scalar form rounds it) ------------------
+__device__ __forceinline__ uint64_t pair_f32(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpair_f32(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // ---- cluster helpers ------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
