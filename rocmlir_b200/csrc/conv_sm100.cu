@@ -530,8 +530,9 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, b
     if (pl->b_implicit) pl->b_direct = true;
     // unit stride, dense NHWK output gradient and KYXC filter gradient: the halo form (input window loaded once per tile)
     pl->w_halo = false;
-    if (pl->b_implicit && pl->a_direct && pl->c_direct && p->stride_h == 1 && p->stride_w == 1) {
+    if (pl->b_implicit && pl->a_direct && pl->c_direct && p->stride_h <= 2 && p->stride_w <= 2) {
       HaloConv& h = pl->w_hc;
+      h.stride_h = p->stride_h; h.stride_w = p->stride_w;
       h.is_bf16 = t == RB_BF16;
       h.N = p->n; h.H = p->h; h.W = p->w; h.C = p->c; h.P = (int)ho; h.Q = (int)wo; h.Kout = p->k;
       h.Y = p->y; h.X = p->x; h.dil_h = p->dil_h; h.dil_w = p->dil_w;

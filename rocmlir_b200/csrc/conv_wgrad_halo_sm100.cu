@@ -1,4 +1,4 @@
-// Backward weight of a unit-stride NHWC convolution without an im2col matrix and without re-reading the input once
+// Backward weight of an NHWC convolution without an im2col matrix and without re-reading the input once
 // per filter tap.
 //
 // rocMLIR lowers rock.conv_bwd_weight to a GEMM whose reduction runs over the output pixels
@@ -40,20 +40,26 @@ namespace {
 constexpr int kWgThreads = 256;
 constexpr int kWgMaxStages = 6;
 constexpr int kWgMaxPairs = 32;
+constexpr int kWgMaxGroups = 16;
+constexpr int kWgMaxLoads = 96;       // windows of all groups
+constexpr int kWgMaxPhases = 4;
 constexpr int kWgSlack = 160 * 128;   // rows that shifted descriptors may touch past the last stage
 
 struct WgradMaps {
-  CUtensorMap x;    // {C, W, H, N} of the NHWC input, box {64, Wp, rows_box, 1}
+  CUtensorMap x[kWgMaxPhases];   // {C, W, H, N} of the NHWC input (stride: of every stride-th pixel of it), box {64, Wp, rows_box, 1}
   CUtensorMap dy;   // {Kout, Q, P, N} of the NHWK output gradient, box {64, Wp, R, 1}
 };
 
 struct WgradParams {
   int Kout, cchunks, kchunks, yxc;
-  int pad_h, pad_w;
   int Wp, R, ksteps;                 // padded raster width, output rows per tile, 16-pixel reduction steps per tile
   int tiles_per_img, num_tiles;
-  int x_plane_bytes, dy_plane_bytes, x_box_bytes, dy_box_bytes, stage_bytes, stages;
+  int x_plane_bytes, dy_plane_bytes, x_box_bytes, dy_box_bytes, stage_bytes, stages, dy_off;
   int npairs, pairs_per_cta, groups;
+  // windows that a group's taps read: loads [load_begin[g], load_begin[g + 1]), one behind the other in a stage
+  int load_begin[kWgMaxGroups + 1];
+  uint8_t load_phase[kWgMaxLoads], load_cc[kWgMaxLoads];
+  int phase_h[kWgMaxPhases], phase_w[kWgMaxPhases];   // the window's first pixel relative to (first output row, 0)
   uint32_t idesc;
   int is_bf16;
   float* slabs;                      // [ctas of a group][Kout][Y * X * C] partial sums (each CTA writes its share of the columns)
@@ -104,7 +110,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
   }
-  if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.x); prefetch_tmap(&maps.dy); }
+  if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.x[0]); prefetch_tmap(&maps.dy); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -114,16 +120,19 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
     // ------------------------------ producer ------------------------------
     if (lane_id() == 0) {
       uint32_t s = 0, ph = 0;
-      const uint32_t tx_bytes = (uint32_t)(p.cchunks * p.x_box_bytes + p.kchunks * p.dy_box_bytes);
+      const int l0 = p.load_begin[group], l1 = p.load_begin[group + 1];
+      const uint32_t tx_bytes = (uint32_t)((l1 - l0) * p.x_box_bytes + p.kchunks * p.dy_box_bytes);
       for (int tile = cta; tile < p.num_tiles; tile += ctas) {
         const int n = tile / p.tiles_per_img;
         const int p0 = (tile - n * p.tiles_per_img) * p.R;
         if (!mbar_wait(&empty_bar[s], ph ^ 1u, p.status, kStatusTimeoutProducer + s, wait_limit)) break;
         mbar_expect_tx(&full_bar[s], tx_bytes);
         uint8_t* st = smem + (size_t)s * p.stage_bytes;
-        for (int cc = 0; cc < p.cchunks; ++cc)
-          tma_load_4d(st + (size_t)cc * p.x_plane_bytes, &maps.x, &full_bar[s], cc * 64, -p.pad_w, p0 - p.pad_h, n);
-        uint8_t* dy = st + (size_t)p.cchunks * p.x_plane_bytes;
+        for (int l = l0; l < l1; ++l) {
+          const int ph_i = p.load_phase[l];
+          tma_load_4d(st + (size_t)(l - l0) * p.x_plane_bytes, &maps.x[ph_i], &full_bar[s], p.load_cc[l] * 64, p.phase_w[ph_i], p0 + p.phase_h[ph_i], n);
+        }
+        uint8_t* dy = st + p.dy_off;
         for (int kc = 0; kc < p.kchunks; ++kc)
           tma_load_4d(dy + (size_t)kc * p.dy_plane_bytes, &maps.dy, &full_bar[s], kc * 64, 0, p0, n);
         if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
@@ -139,7 +148,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
     const bool tracing = p.trace != nullptr;
     const uint32_t desc_hi = smem_desc_hi(1024);
     const uint32_t x_lo0 = smem_desc_lo(smem_u32(smem), 0);
-    const uint32_t dy_lo0 = smem_desc_lo(smem_u32(smem) + (uint32_t)(p.cchunks * p.x_plane_bytes), (uint32_t)p.dy_plane_bytes);
+    const uint32_t dy_lo0 = smem_desc_lo(smem_u32(smem) + (uint32_t)p.dy_off, (uint32_t)p.dy_plane_bytes);
     const uint32_t stage_step = (uint32_t)p.stage_bytes >> 4;
     constexpr uint32_t kStep = (16 * 128) >> 4;   // sixteen pixels = sixteen 128-byte rows on
     uint32_t s = 0, ph = 0;
@@ -262,22 +271,50 @@ conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, vo
   }
 }
 
-struct WgradShape {
-  int Wp, R, rows_box, ksteps, cchunks, kchunks, units, npairs, pairs_per_cta, groups;
-  int x_plane_bytes, dy_plane_bytes, stage_bytes, stages;
+// A tap (y, x) reads input row p * stride + t with t = y * dil - pad: row p + o of the pixels a, a + stride, ... where t = o * stride + a.
+struct WgradPhase {
+  int a_h, a_w;              // first pixel of the phase
+  int lo_h, hi_h, lo_w, hi_w;  // smallest and largest o of its taps
+  int taps;
 };
 
-// Units in (tap, channel block) order; consecutive units share an MMA: the half at the lower address comes first and
-// the leading-dimension offset is the (positive) distance to the other. False when a distance does not fit the
-// descriptor's 14-bit field.
+struct WgradShape {
+  int Wp, R, rows_box, ksteps, cchunks, kchunks, units, npairs, pairs_per_cta, groups, planes;
+  int x_plane_bytes, dy_plane_bytes, stage_bytes, stages;
+  int nphases;
+  WgradPhase phase[kWgMaxPhases];
+  // units (tap, channel block), by phase, channel block and tap: a group of consecutive ones reads few windows
+  uint8_t tap[2 * kWgMaxPairs], cc[2 * kWgMaxPairs], ph[2 * kWgMaxPairs];
+};
+
+int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+int tap_offset(int tap, int dil, int pad, int stride) { return floor_div(tap * dil - pad, stride); }
+int tap_phase(int tap, int dil, int pad, int stride) { return tap * dil - pad - tap_offset(tap, dil, pad, stride) * stride; }
+
+// The windows that a group reads, in the order of its units: (phase, channel block) of each into `win`; returns their number.
+int wgrad_windows(const WgradShape& s, int group, int (*win)[2]) {
+  int n = 0;
+  const int u1 = std::min(s.units, (group + 1) * s.pairs_per_cta * 2);
+  for (int u = group * s.pairs_per_cta * 2; u < u1; ++u)
+    if (n == 0 || win[n - 1][0] != s.ph[u] || win[n - 1][1] != s.cc[u]) { win[n][0] = s.ph[u]; win[n][1] = s.cc[u]; ++n; }
+  return n;
+}
+
+// Consecutive units share an MMA: the half at the lower address comes first and the leading-dimension offset is the (positive)
+// distance to the other. False when a distance does not fit the descriptor's 14-bit field.
 bool wgrad_pairs(const HaloConv& c, const WgradShape& s, uint32_t* off, uint32_t* lbo, int* col0, int* col1) {
   for (int u = 0; u < s.units; u += 2) {
+    int win[2 * kWgMaxPairs][2];
+    const int nwin = wgrad_windows(s, u / 2 / s.pairs_per_cta, win);
     long long o[2] = {0, 0};
     int col[2] = {-1, -1};
     for (int h = 0; h < 2 && u + h < s.units; ++h) {
-      const int tap = (u + h) / s.cchunks, cc = (u + h) % s.cchunks;
-      const int y = tap / c.X, x = tap % c.X;
-      o[h] = (long long)cc * s.x_plane_bytes + ((long long)y * c.dil_h * s.Wp + (long long)x * c.dil_w) * 128;
+      const int tap = s.tap[u + h], cc = s.cc[u + h], y = tap / c.X, x = tap % c.X;
+      const WgradPhase& f = s.phase[s.ph[u + h]];
+      int w = 0;
+      while (w + 1 < nwin && (win[w][0] != s.ph[u + h] || win[w][1] != cc)) ++w;
+      const int dh = tap_offset(y, c.dil_h, c.pad_h, c.stride_h) - f.lo_h, dw = tap_offset(x, c.dil_w, c.pad_w, c.stride_w) - f.lo_w;
+      o[h] = (long long)w * s.x_plane_bytes + ((long long)dh * s.Wp + dw) * 128;
       col[h] = tap * c.C + cc * 64;
     }
     const bool lone = u + 1 >= s.units;
@@ -297,20 +334,68 @@ bool wgrad_pairs(const HaloConv& c, const WgradShape& s, uint32_t* off, uint32_t
 bool wgrad_shape(const HaloConv& c, WgradShape* s) {
   if (c.C % 64 || c.Kout % 64 || c.Kout > 256 || c.Kout < 64) return false;
   if (c.dil_h < 1 || c.dil_w < 1 || c.pad_h < 0 || c.pad_w < 0 || c.Y * c.X > 49) return false;
-  s->Wp = c.Q + (c.X - 1) * c.dil_w;
-  if (s->Wp > 128 || s->Wp != c.W + c.pad_w + c.pad_w_r) return false;
-  if (c.P + (c.Y - 1) * c.dil_h != c.H + c.pad_h + c.pad_h_r) return false;
   s->cchunks = c.C / 64;
   s->kchunks = c.Kout / 64;
+  s->units = c.Y * c.X * s->cchunks;
+  s->npairs = (s->units + 1) / 2;
+  if (s->npairs > kWgMaxPairs) return false;
+  s->nphases = 0;
+  for (int tap = 0; tap < c.Y * c.X; ++tap) {
+    const int y = tap / c.X, x = tap % c.X;
+    const int ah = tap_phase(y, c.dil_h, c.pad_h, c.stride_h), aw = tap_phase(x, c.dil_w, c.pad_w, c.stride_w);
+    const int oh = tap_offset(y, c.dil_h, c.pad_h, c.stride_h), ow = tap_offset(x, c.dil_w, c.pad_w, c.stride_w);
+    if (ah >= c.H || aw >= c.W) return false;   // a phase without pixels
+    int f = 0;
+    while (f < s->nphases && (s->phase[f].a_h != ah || s->phase[f].a_w != aw)) ++f;
+    if (f == s->nphases) {
+      if (f == kWgMaxPhases) return false;
+      s->phase[s->nphases++] = {ah, aw, oh, oh, ow, ow, 0};
+    }
+    WgradPhase& q = s->phase[f];
+    q.lo_h = std::min(q.lo_h, oh); q.hi_h = std::max(q.hi_h, oh);
+    q.lo_w = std::min(q.lo_w, ow); q.hi_w = std::max(q.hi_w, ow);
+    ++q.taps;
+  }
+  int n = 0, more_w = 0, more_h = 0;
+  for (int f = 0; f < s->nphases; ++f) {
+    const WgradPhase& q = s->phase[f];
+    more_w = std::max(more_w, q.hi_w - q.lo_w);
+    more_h = std::max(more_h, q.hi_h - q.lo_h);
+    for (int cc = 0; cc < s->cchunks; ++cc)
+      for (int tap = 0; tap < c.Y * c.X; ++tap)
+        if (tap_phase(tap / c.X, c.dil_h, c.pad_h, c.stride_h) == q.a_h && tap_phase(tap % c.X, c.dil_w, c.pad_w, c.stride_w) == q.a_w) {
+          s->tap[n] = (uint8_t)tap;
+          s->cc[n] = (uint8_t)cc;
+          s->ph[n++] = (uint8_t)f;
+        }
+  }
+  s->Wp = c.Q + more_w;
+  if (s->Wp > 128) return false;
+  if (c.stride_h == 1 && c.P + (c.Y - 1) * c.dil_h != c.H + c.pad_h + c.pad_h_r) return false;
+  if (c.stride_w == 1 && s->Wp != c.W + c.pad_w + c.pad_w_r) return false;
+  // pairs of taps by groups of CTAs, as evenly as they go: a group's time is its pairs
+  s->groups = (s->npairs + 512 / c.Kout - 1) / (512 / c.Kout);
+  if (s->groups > kWgMaxGroups) return false;
+  s->pairs_per_cta = (s->npairs + s->groups - 1) / s->groups;
+  s->groups = (s->npairs + s->pairs_per_cta - 1) / s->pairs_per_cta;
+  s->planes = 0;
+  int loads = 0;
+  for (int g = 0; g < s->groups; ++g) {
+    int win[2 * kWgMaxPairs][2];
+    const int w = wgrad_windows(*s, g, win);
+    s->planes = std::max(s->planes, w);
+    loads += w;
+  }
+  if (loads > kWgMaxLoads) return false;
   // Output rows per tile: the reduction runs along the raster, so a tile may be any number of rows long. More rows
   // share the window's halo rows and waste less of the last 16-pixel step; the ring must still hold three stages.
   // Among the sizes that fit, the one with the fewest reduction steps per image wins.
   int best_r = 0;
   long long best_steps = 0;
   for (int r = 1; r <= std::min(c.P, 16); ++r) {
-    const int rows_box = r + (c.Y - 1) * c.dil_h;
+    const int rows_box = r + more_h;
     const int ksteps = (r * s->Wp + 15) / 16;
-    const long long stage = (long long)s->cchunks * ((s->Wp * rows_box + 7) / 8 * 8 * 128) + (long long)s->kchunks * ksteps * 16 * 128;
+    const long long stage = (long long)s->planes * ((s->Wp * rows_box + 7) / 8 * 8 * 128) + (long long)s->kchunks * ksteps * 16 * 128;
     if (rows_box > 256 || (232448 - 1024 - kWgSlack - 1024) / stage < 3) continue;
     const long long steps = (long long)((c.P + r - 1) / r) * (ksteps + 2);   // + the barrier work of a tile, about two steps' worth
     if (best_r == 0 || steps <= best_steps) { best_r = r; best_steps = steps; }
@@ -319,17 +404,12 @@ bool wgrad_shape(const HaloConv& c, WgradShape* s) {
     best_r = std::min(128 / s->Wp, c.P);
   }
   s->R = best_r;
-  s->rows_box = s->R + (c.Y - 1) * c.dil_h;
+  s->rows_box = s->R + more_h;
   if (s->R < 1 || s->rows_box > 256) return false;
   s->ksteps = (s->R * s->Wp + 15) / 16;
-  s->units = c.Y * c.X * s->cchunks;
-  s->npairs = (s->units + 1) / 2;
-  if (s->npairs > kWgMaxPairs) return false;
-  s->pairs_per_cta = std::min(s->npairs, 512 / c.Kout);
-  s->groups = (s->npairs + s->pairs_per_cta - 1) / s->pairs_per_cta;
   s->x_plane_bytes = (s->Wp * s->rows_box + 7) / 8 * 8 * 128;
   s->dy_plane_bytes = s->ksteps * 16 * 128;
-  s->stage_bytes = s->cchunks * s->x_plane_bytes + s->kchunks * s->dy_plane_bytes;
+  s->stage_bytes = s->planes * s->x_plane_bytes + s->kchunks * s->dy_plane_bytes;
   s->stages = std::min(kWgMaxStages, (232448 - 1024 - kWgSlack - 1024) / s->stage_bytes);
   return s->stages >= 2 && wgrad_pairs(c, *s, nullptr, nullptr, nullptr, nullptr);
 }
@@ -371,14 +451,20 @@ RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* o
   WgradParams p;
   memset(&p, 0, sizeof(p));
   p.Kout = c.Kout; p.cchunks = s.cchunks; p.kchunks = s.kchunks; p.yxc = c.Y * c.X * c.C;
-  p.pad_h = c.pad_h; p.pad_w = c.pad_w;
   p.Wp = s.Wp; p.R = s.R; p.ksteps = s.ksteps;
   p.tiles_per_img = (c.P + s.R - 1) / s.R;
   p.num_tiles = c.N * p.tiles_per_img;
   p.x_plane_bytes = s.x_plane_bytes; p.dy_plane_bytes = s.dy_plane_bytes;
   p.x_box_bytes = s.Wp * s.rows_box * 128; p.dy_box_bytes = s.Wp * s.R * 128;
   p.stage_bytes = s.stage_bytes; p.stages = s.stages;
+  p.dy_off = s.planes * s.x_plane_bytes;
   p.npairs = s.npairs; p.pairs_per_cta = s.pairs_per_cta; p.groups = s.groups;
+  for (int g = 0; g < s.groups; ++g) {
+    int win[2 * kWgMaxPairs][2];
+    const int n = wgrad_windows(s, g, win);
+    for (int i = 0; i < n; ++i) { p.load_phase[p.load_begin[g] + i] = (uint8_t)win[i][0]; p.load_cc[p.load_begin[g] + i] = (uint8_t)win[i][1]; }
+    p.load_begin[g + 1] = p.load_begin[g] + n;
+  }
   const uint32_t fmt = c.is_bf16 ? 1u : 0u;
   p.idesc = make_idesc(1, fmt, fmt, 1, 1, 128, (uint32_t)c.Kout);
   p.is_bf16 = c.is_bf16;
@@ -392,11 +478,15 @@ RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* o
   memset(&maps, 0, sizeof(maps));
   std::string err;
   const CUtensorMapDataType dt = c.is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  {
-    const uint64_t dims[4] = {(uint64_t)c.C, (uint64_t)c.W, (uint64_t)c.H, (uint64_t)c.N};
-    const uint64_t strides[3] = {(uint64_t)c.C * 2, (uint64_t)c.W * c.C * 2, (uint64_t)c.H * c.W * c.C * 2};
+  for (int f = 0; f < s.nphases; ++f) {
+    const WgradPhase& q = s.phase[f];
+    p.phase_h[f] = q.lo_h;
+    p.phase_w[f] = q.lo_w;
+    const uint64_t dims[4] = {(uint64_t)c.C, (uint64_t)((c.W - q.a_w + c.stride_w - 1) / c.stride_w), (uint64_t)((c.H - q.a_h + c.stride_h - 1) / c.stride_h), (uint64_t)c.N};
+    const uint64_t strides[3] = {(uint64_t)c.stride_w * c.C * 2, (uint64_t)c.stride_h * c.W * c.C * 2, (uint64_t)c.H * c.W * c.C * 2};
     const uint32_t box[4] = {64u, (uint32_t)s.Wp, (uint32_t)s.rows_box, 1u};
-    if (!encode_tiled(&maps.x, dt, 4, image, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, &err))
+    const uint8_t* base = static_cast<const uint8_t*>(image) + ((size_t)q.a_h * c.W + q.a_w) * c.C * 2;
+    if (!encode_tiled(&maps.x[f], dt, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, &err))
       return fail(RB_UNSUPPORTED, "halo weight-gradient kernel, input: " + err);
   }
   {

@@ -263,9 +263,64 @@ struct EpiCopyCtx : EpiStoreCtx {
 };
 
 // Copies the staged rows of a warp (32 rows of 128 bytes, 16-byte pieces XOR-swizzled by the row) to rows of C that start
-// anywhere: row r goes to dst + r * pitch, of which `cols` elements and the first `rows` rows exist, with a store per 32
-// neighbouring elements. Stored straight from the registers, as the general loop does, every store instruction touches 32 rows.
-// (Aligned words with the two ends of a row by themselves were tried first: 300 cycles a row, most of them instructions.)
+// anywhere: row r goes to dst + r * pitch, of which `cols` elements and the first `rows` rows exist. Stored straight from the
+// registers, as the general loop does, every store instruction touches 32 rows.
+//
+// 2- and 4-byte elements: eight lanes to a row, each an aligned 16 bytes of C put together from the two staged pieces it lies across;
+// what is left of a 128-byte run at its ends, 16 bytes in all, element by element. Bound by the load/store unit's instructions: 16 stores
+// for 32 rows of 64 columns where one per 32 neighbouring elements makes 64. 1344x997x144 f16 13.2 -> FIG1 us, 1675x918x1960 bf16
+// 24.1 -> FIG2 (17.98 with 920 columns).
+template <int ES>
+__device__ __forceinline__ void copy_rows_wide(const uint8_t* stg, uint8_t* dst, long long pitch_bytes, int rows, int bytes, int lane) {
+  const int j = lane & 7, row0 = lane >> 3;
+  uint8_t* g = dst + row0 * pitch_bytes;
+  const long long step = 4 * pitch_bytes;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {   // four rows of each lane in flight
+    uint4 cur[4], prv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = row0 + 16 * half + 4 * i, x = (row & 7) << 4;
+      cur[i] = *reinterpret_cast<const uint4*>(stg + row * kRowBytes + ((j << 4) ^ x));
+      prv[i] = *reinterpret_cast<const uint4*>(stg + row * kRowBytes + ((((j - 1) & 7) << 4) ^ x));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i, g += step) {
+      const int a = (int)(reinterpret_cast<uintptr_t>(g) & 15);   // C's aligned pieces begin a bytes before the staged ones
+      // bytes 16 - a .. 31 - a of prv, cur: by eight bytes, by four, by single ones
+      const uint32_t w[8] = {prv[i].x, prv[i].y, prv[i].z, prv[i].w, cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+      uint32_t u[6], v[5], o[4];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) u[k] = (a & 8) ? w[k] : w[k + 2];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) v[k] = (a & 4) ? u[k] : u[k + 1];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] = ES == 4 ? v[k + 1] : __funnelshift_rc(v[k], v[k + 1], (4 - (a & 3)) * 8);
+      const int at = 16 * j - a;
+      if (row0 + 16 * half + 4 * i < rows && at >= 0 && at + 16 <= bytes) *reinterpret_cast<uint4*>(g + at) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  // the ends: of a whole run 16 bytes in all, an element to a lane; fewer columns may leave up to twice that
+  constexpr int kEnds = 16 / ES;                // elements, a power of two
+  const int sub = lane & (kEnds - 1);
+#pragma unroll 1
+  for (int first = 0; first < 2 * kEnds - 1; first += kEnds) {
+    if (first && bytes == kRowBytes) break;
+#pragma unroll 4
+    for (int r = lane / kEnds; r < 32; r += 32 / kEnds) {
+      uint8_t* gr = dst + r * pitch_bytes;
+      const int a = (int)(reinterpret_cast<uintptr_t>(gr) & 15);
+      const int head = a ? min(16 - a, bytes) : 0, tail = head + ((bytes - head) & ~15);
+      const int e = (first + sub) * ES, off = e < head ? e : tail + e - head;
+      if (r < rows && off < bytes) {
+        const uint8_t* from = stg + r * kRowBytes + ((off & ~15) ^ ((r & 7) << 4)) + (off & 15);
+        if (ES == 4) *reinterpret_cast<uint32_t*>(gr + off) = *reinterpret_cast<const uint32_t*>(from);
+        else *reinterpret_cast<uint16_t*>(gr + off) = *reinterpret_cast<const uint16_t*>(from);
+      }
+    }
+  }
+}
+// Single bytes: a store per 32 neighbouring elements.
 template <typename T>
 __device__ __forceinline__ void copy_rows(const uint8_t* stg, T* dst, long long pitch, int rows, int cols, int lane) {
   constexpr int kPer = kRowBytes / 32 / (int)sizeof(T);   // elements of a row per lane: columns lane, lane + 32, ...
@@ -305,8 +360,8 @@ static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t
       const int r = i / pieces, j = i - r * pieces;
       *reinterpret_cast<uint4*>(dst + r * pitch * es + j * 16) = *reinterpret_cast<const uint4*>(stg + r * kRowBytes + ((j ^ (r & 7)) << 4));
     }
-  } else if (es == 2) copy_rows(stg, reinterpret_cast<uint16_t*>(dst), pitch, rows, cols, lane);
-  else if (es == 4) copy_rows(stg, reinterpret_cast<uint32_t*>(dst), pitch, rows, cols, lane);
+  } else if (es == 2) copy_rows_wide<2>(stg, dst, pitch * 2, rows, bytes, lane);
+  else if (es == 4) copy_rows_wide<4>(stg, dst, pitch * 4, rows, bytes, lane);
   else copy_rows(stg, dst, pitch, rows, cols, lane);
   __syncwarp();
 }

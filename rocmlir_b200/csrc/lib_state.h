@@ -95,6 +95,7 @@ struct HaloConv {
   int pad_h, pad_w, pad_h_r, pad_w_r;
   int is_bf16;
   long long o_n, o_p, o_q;
+  int stride_h = 1, stride_w = 1;   // the weight-gradient kernel only; 1 elsewhere
   // Backward data reading the KYXC filter tensor as it lies (no rearranged copy): `filter_matrix` is then the filter
   // itself, [C = conv output channels][FY][FX][Kout = conv input channels, contiguous] with element strides f_sk, f_sy,
   // f_sx, and tap (y', x') of the raster is filter tap (fy0 + fsy * (Y-1-y'), fx0 + fsx * (X-1-x')).
