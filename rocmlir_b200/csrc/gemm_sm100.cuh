@@ -268,55 +268,39 @@ struct EpiCopyCtx : EpiStoreCtx {
 //
 // 2- and 4-byte elements: eight lanes to a row, each an aligned 16 bytes of C put together from the two staged pieces it lies across;
 // what is left of a 128-byte run at its ends, 16 bytes in all, element by element. Bound by the load/store unit's instructions: 16 stores
-// for 32 rows of 64 columns where one per 32 neighbouring elements makes 64. 1344x997x144 f16 13.2 -> FIG1 us, 1675x918x1960 bf16
-// 24.1 -> FIG2 (17.98 with 920 columns).
+// for 32 rows of 64 columns where one per 32 neighbouring elements makes 64. 1344x997x144 f16 13.2 -> 12.5 us, 1675x918x1960 bf16
+// 24.1 -> 22.8 (18.0 with 920 columns). All rows' loads ahead of the stores: 13.2 and 23.2 (twice the code, and a tile runs it once).
 template <int ES>
 __device__ __forceinline__ void copy_rows_wide(const uint8_t* stg, uint8_t* dst, long long pitch_bytes, int rows, int bytes, int lane) {
-  const int j = lane & 7, row0 = lane >> 3;
-  uint8_t* g = dst + row0 * pitch_bytes;
-  const long long step = 4 * pitch_bytes;
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {   // four rows of each lane in flight
-    uint4 cur[4], prv[4];
+  const int j = lane & 7;
+#pragma unroll 2
+  for (int r0 = 0; r0 < 32; r0 += 4) {
+    const int row = r0 + (lane >> 3);
+    uint8_t* g = dst + row * pitch_bytes;
+    const int a = (int)(reinterpret_cast<uintptr_t>(g) & 15);   // C's aligned pieces begin a bytes before the staged ones
+    const uint8_t* srow = stg + row * kRowBytes;
+    const int x = (row & 7) << 4;
+    const uint4 cur = *reinterpret_cast<const uint4*>(srow + ((j << 4) ^ x));
+    const uint4 prv = *reinterpret_cast<const uint4*>(srow + ((((j - 1) & 7) << 4) ^ x));
+    // bytes 16 - a .. 31 - a of prv, cur: by eight bytes, by four, by single ones
+    const uint32_t w[8] = {prv.x, prv.y, prv.z, prv.w, cur.x, cur.y, cur.z, cur.w};
+    uint32_t u[6], v[5], o[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = row0 + 16 * half + 4 * i, x = (row & 7) << 4;
-      cur[i] = *reinterpret_cast<const uint4*>(stg + row * kRowBytes + ((j << 4) ^ x));
-      prv[i] = *reinterpret_cast<const uint4*>(stg + row * kRowBytes + ((((j - 1) & 7) << 4) ^ x));
-    }
+    for (int i = 0; i < 6; ++i) u[i] = (a & 8) ? w[i] : w[i + 2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i, g += step) {
-      const int a = (int)(reinterpret_cast<uintptr_t>(g) & 15);   // C's aligned pieces begin a bytes before the staged ones
-      // bytes 16 - a .. 31 - a of prv, cur: by eight bytes, by four, by single ones
-      const uint32_t w[8] = {prv[i].x, prv[i].y, prv[i].z, prv[i].w, cur[i].x, cur[i].y, cur[i].z, cur[i].w};
-      uint32_t u[6], v[5], o[4];
+    for (int i = 0; i < 5; ++i) v[i] = (a & 4) ? u[i] : u[i + 1];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) u[k] = (a & 8) ? w[k] : w[k + 2];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) v[k] = (a & 4) ? u[k] : u[k + 1];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o[k] = ES == 4 ? v[k + 1] : __funnelshift_rc(v[k], v[k + 1], (4 - (a & 3)) * 8);
-      const int at = 16 * j - a;
-      if (row0 + 16 * half + 4 * i < rows && at >= 0 && at + 16 <= bytes) *reinterpret_cast<uint4*>(g + at) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  }
-  // the ends: of a whole run 16 bytes in all, an element to a lane; fewer columns may leave up to twice that
-  constexpr int kEnds = 16 / ES;                // elements, a power of two
-  const int sub = lane & (kEnds - 1);
-#pragma unroll 1
-  for (int first = 0; first < 2 * kEnds - 1; first += kEnds) {
-    if (first && bytes == kRowBytes) break;
-#pragma unroll 4
-    for (int r = lane / kEnds; r < 32; r += 32 / kEnds) {
-      uint8_t* gr = dst + r * pitch_bytes;
-      const int a = (int)(reinterpret_cast<uintptr_t>(gr) & 15);
-      const int head = a ? min(16 - a, bytes) : 0, tail = head + ((bytes - head) & ~15);
-      const int e = (first + sub) * ES, off = e < head ? e : tail + e - head;
-      if (r < rows && off < bytes) {
-        const uint8_t* from = stg + r * kRowBytes + ((off & ~15) ^ ((r & 7) << 4)) + (off & 15);
-        if (ES == 4) *reinterpret_cast<uint32_t*>(gr + off) = *reinterpret_cast<const uint32_t*>(from);
-        else *reinterpret_cast<uint16_t*>(gr + off) = *reinterpret_cast<const uint16_t*>(from);
-      }
+    for (int i = 0; i < 4; ++i) o[i] = ES == 4 ? v[i + 1] : __funnelshift_rc(v[i], v[i + 1], (4 - (a & 3)) * 8);
+    const int at = 16 * j - a;
+    const bool there = row < rows;
+    if (there && at >= 0 && at + 16 <= bytes) *reinterpret_cast<uint4*>(g + at) = make_uint4(o[0], o[1], o[2], o[3]);
+    const int head = a ? min(16 - a, bytes) : 0, tail = head + ((bytes - head) & ~15);
+    const int rest = there ? head + bytes - tail : 0;
+    for (int e = j * ES; e < rest; e += 8 * ES) {
+      const int off = e < head ? e : tail + e - head;
+      const uint8_t* from = srow + ((off & ~15) ^ x) + (off & 15);
+      if (ES == 4) *reinterpret_cast<uint32_t*>(g + off) = *reinterpret_cast<const uint32_t*>(from);
+      else *reinterpret_cast<uint16_t*>(g + off) = *reinterpret_cast<const uint16_t*>(from);
     }
   }
 }
