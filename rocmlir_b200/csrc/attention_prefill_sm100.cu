@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "attention.cuh"
+#include "launch.cuh"
 
 namespace rb {
 namespace {
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) attention_prefill_kernel(c
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) attention_prefill_kernel(c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;   // S_A 0, S_B 128, O_A 256, O_B 384
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   // Item n of this CTA, the same in all lanes; nothing when the wait has run out.
   auto read_item = [&](int n, uint32_t code, bool& ok) -> int4 {
@@ -484,7 +487,7 @@ RbStatus launch(const AttMaps& maps, const AttParams& p, int batch, int items, c
   void (*const kern)(const AttMaps, const AttParams, const int) =
       p.trans_k ? attention_prefill_kernel<BF16, KSTEPS, true> : attention_prefill_kernel<BF16, KSTEPS, false>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), PrefillSmem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
-  kern<<<(unsigned)items, kPrefillThreads, PrefillSmem::kTotal, stream>>>(maps, p, batch);
+  RB_CUDA_TRY(launch_after(kern, (unsigned)items, kPrefillThreads, PrefillSmem::kTotal, stream, 1, maps, p, batch));
   return RB_SUCCESS;
 }
 

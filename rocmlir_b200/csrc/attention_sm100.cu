@@ -29,6 +29,7 @@
 #include <string>
 
 #include "attention.cuh"
+#include "launch.cuh"
 
 namespace rb {
 namespace {
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   const uint32_t tmem_o = tmem_base + 256;   // S buffers at columns 0 and 128, O at 256
 
   const int d_atoms = p.D / 64, dv_chunks = p.Dv / 64;
@@ -571,11 +574,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
   if (warp == 1) {
     tmem_alloc<1>(tmem_holder, 64);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   const uint32_t tmem_o = tmem_base + 32;   // scores of two blocks at columns 0 and 16, O^T at 32
 
   const int d_atoms = p.D / 64, dv_chunks = p.Dv / 64;
@@ -900,6 +905,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -911,6 +917,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;   // S_A 0, S_B 128, O_A 256, O_B 384
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   const int d_atoms = p.D / 64, dv_chunks = p.Dv / 64;
   const uint32_t q_bytes = (uint32_t)kQT * p.D * 2, k_bytes = (uint32_t)kKT * p.D * 2, v_bytes = (uint32_t)kKT * p.Dv * 2;
@@ -1677,7 +1684,7 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   } else if (two_query_tiles(p)) {
     const long long ctas2 = (long long)p->g * ((kp.q_tiles + 1) / 2);
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attention_fwd2_kernel), Att2Smem::kTotal) != RB_SUCCESS) return RB_CUDA_ERROR;
-    attention_fwd2_kernel<<<(unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream>>>(maps, kp);
+    RB_CUDA_TRY(launch_after(attention_fwd2_kernel, (unsigned)ctas2, kAtt2Threads, Att2Smem::kTotal, stream, 1, maps, kp));
   } else {
     const bool few = few_queries(p);
     const bool mask_only = p->mask && !p->bias && !p->scale_tensor && !quantized && !p->causal;
@@ -1698,22 +1705,7 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
         : p->seq_q == 1 ? attention_decode_kernel<1> : attention_decode_kernel<kDecodeQ>;
     const int threads = few ? kDecodeThreads : kAttThreads, smem = few ? DecodeSmem::total((int)Dp, (int)Dvp) : AttSmem::kTotal;
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != RB_SUCCESS) return RB_CUDA_ERROR;
-    if (kp.splits == 1) {
-      kern<<<(unsigned)ctas, threads, smem, stream>>>(maps, kp);
-    } else {
-      cudaLaunchConfig_t lc;
-      memset(&lc, 0, sizeof(lc));
-      lc.gridDim = dim3((unsigned)(ctas * kp.splits), 1, 1);
-      lc.blockDim = dim3((unsigned)threads, 1, 1);
-      lc.dynamicSmemBytes = (size_t)smem;
-      lc.stream = stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)kp.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-      lc.attrs = attr;
-      lc.numAttrs = 1;
-      RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
-    }
+    RB_CUDA_TRY(launch_after(kern, (unsigned)(ctas * kp.splits), threads, smem, stream, (unsigned)kp.splits, maps, kp));
   }
   RB_CUDA_TRY(cudaGetLastError());
   count_launch();

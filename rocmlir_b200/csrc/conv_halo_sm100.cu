@@ -26,6 +26,7 @@
 #include <string>
 
 #include "epilogue.cuh"
+#include "launch.cuh"
 #include "lib_state.h"
 #include "ptx.cuh"
 
@@ -117,8 +118,10 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.in); prefetch_tmap(&maps.fil); }
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   if constexpr (EPI) {
     if (epi_col_bias(p.epi.flags))
       for (int j = threadIdx.x; j < p.Kout; j += kHaloThreads) {
@@ -550,9 +553,8 @@ RbStatus conv_halo_run_group(const HaloConv* cs, int count, const void* image, c
   if (st != RB_SUCCESS) return st;
   unsigned long long* trace = trace_buffer((size_t)grid * 16);
   for (int i = 0; i < count; ++i) g.prm[i].trace = trace;
-  if (with_epi) conv_halo_kernel<true><<<grid, kHaloThreads, smem, static_cast<cudaStream_t>(stream_v)>>>(g);
-  else conv_halo_kernel<false><<<grid, kHaloThreads, smem, static_cast<cudaStream_t>(stream_v)>>>(g);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(with_epi ? conv_halo_kernel<true> : conv_halo_kernel<false>, grid, kHaloThreads, smem,
+                           static_cast<cudaStream_t>(stream_v), 1, g));
   count_launch();
   return RB_SUCCESS;
 }

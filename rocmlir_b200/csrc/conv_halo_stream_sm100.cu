@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <string>
 
+#include "launch.cuh"
 #include "lib_state.h"
 #include "ptx.cuh"
 
@@ -84,6 +85,7 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) {
     for (int i = 0; i < PL; ++i) { prefetch_tmap(&maps.in[i]); prefetch_tmap(&maps.fil[i]); }
@@ -92,6 +94,7 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   const int taps = p.Y * p.X;
 
   if (warp == 0) {
@@ -381,9 +384,8 @@ RbStatus conv_halo_stream_run(const HaloConv& c, int elem_bytes, const void* ima
   if (st != RB_SUCCESS) return st;
   const int grid = std::min(p.num_tiles, dev->sm_count);
   p.trace = trace_buffer((size_t)grid * 16);
-  if (f32) conv_halo_stream_kernel<true><<<grid, kStThreads, smem, static_cast<cudaStream_t>(stream_v)>>>(maps, p);
-  else conv_halo_stream_kernel<false><<<grid, kStThreads, smem, static_cast<cudaStream_t>(stream_v)>>>(maps, p);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(f32 ? conv_halo_stream_kernel<true> : conv_halo_stream_kernel<false>, grid, kStThreads, smem,
+                           static_cast<cudaStream_t>(stream_v), 1, maps, p));
   count_launch();
   return RB_SUCCESS;
 }

@@ -33,6 +33,7 @@
 
 #include "conv_patch.cuh"
 #include "lib_state.h"
+#include "launch.cuh"
 
 namespace rb {
 namespace {
@@ -190,7 +191,9 @@ conv_patch_kernel(const PatchParams p) {
   if (warp == 0) {
     tmem_alloc<1>(tmem_holder, p.tmem_cols);
     tmem_relinquish<1>();
+    griddep_launch();
   }
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   load_window(p, PatchTile(p, tile), win);   // (the grid has no more CTAs per pass than there are tiles)
   // offsets of every k inside a window, and (in the operand area, which is not in use yet) inside a filter row
   int* foffs = reinterpret_cast<int*>(a_smem);
@@ -482,8 +485,7 @@ RbStatus conv_patch_run(const PatchConv& c, const void* image, const void* filte
   if (st != RB_SUCCESS) return st;
   const long long per_pass = std::max<long long>(1, (long long)dev->sm_count * s.ctas_per_sm / s.passes);
   const int grid = (int)std::min<long long>((long long)p.num_tiles, per_pass) * s.passes;
-  kern<<<grid, kPatchThreads, s.smem, static_cast<cudaStream_t>(stream_v)>>>(p);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(kern, grid, kPatchThreads, s.smem, static_cast<cudaStream_t>(stream_v), 1, p));
   count_launch();
   return RB_SUCCESS;
 }

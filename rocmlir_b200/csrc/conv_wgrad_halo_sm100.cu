@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <string>
 
+#include "launch.cuh"
 #include "lib_state.h"
 #include "ptx.cuh"
 
@@ -109,12 +110,14 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.x[0]); prefetch_tmap(&maps.dy); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
@@ -235,6 +238,8 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
 __global__ void __launch_bounds__(256)
 conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, void* __restrict__ out, int is_bf16) {
   __shared__ float4 part[8][32];
+  griddep_launch();
+  griddep_wait();
   const int lane4 = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int i4 = blockIdx.x * 32 + lane4;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -501,12 +506,10 @@ RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* o
   if (st != RB_SUCCESS) return st;
   const int grid = wgrad_grid(c, s, dev->sm_count);
   p.trace = trace_buffer((size_t)grid * 16);
-  conv_wgrad_halo_kernel<<<grid, kWgThreads, smem, stream>>>(maps, p);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(conv_wgrad_halo_kernel, grid, kWgThreads, smem, stream, 1, maps, p));
   count_launch();
   const int elems = c.Kout * p.yxc;
-  conv_wgrad_sum_kernel<<<(elems / 4 + 31) / 32, 256, 0, stream>>>(p.slabs, grid / s.groups, elems, filter_grad, c.is_bf16);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(conv_wgrad_sum_kernel, (elems / 4 + 31) / 32, 256, 0, stream, 1, p.slabs, grid / s.groups, elems, filter_grad, c.is_bf16));
   count_launch();
   return RB_SUCCESS;
 }

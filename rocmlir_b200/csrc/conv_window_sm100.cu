@@ -34,6 +34,7 @@
 
 #include "conv_patch.cuh"
 #include "lib_state.h"
+#include "launch.cuh"
 
 namespace rb {
 namespace {
@@ -275,11 +276,10 @@ __global__ void __launch_bounds__(kWindowThreads, 1) conv_window_kernel(const __
   if (warp == kWorkers / 32) {
     tmem_alloc<1>(tmem_holder, p.tmem_cols);
     tmem_relinquish<1>();
+    griddep_launch();
     for (int i = lane; i < kZeroBytes / 16; i += 32) *reinterpret_cast<uint4*>(smem_raw + base + p.zero_off + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
   }
   if (worker) {   // (the grid has no more CTAs per pass than there are items)
-    if constexpr (FETCH == kDirect) load_direct(p, Item(p, first), win);
-    else load_raw(p, Item(p, first), raw);
     if constexpr (FETCH == kElements) {
       for (int i = threadIdx.x; i < p.planes * 8; i += kWorkers) {
         const int j = i / 8, t = i & 7;
@@ -304,6 +304,9 @@ __global__ void __launch_bounds__(kWindowThreads, 1) conv_window_kernel(const __
         *reinterpret_cast<uint4*>(smem_raw + tasks + 16u * (uint32_t)k) = task;
       }
     }
+    griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
+    if constexpr (FETCH == kDirect) load_direct(p, Item(p, first), win);
+    else load_raw(p, Item(p, first), raw);
     if constexpr (EPI) {
       for (int j = threadIdx.x; j < p.nt; j += kWorkers) {
         const int n = min(n0 + j, p.Kout - 1);
@@ -675,8 +678,7 @@ RbStatus conv_window_run(const PatchConv& c, const void* image, const void* filt
   if (st != RB_SUCCESS) return st;
   const long long per_pass = std::max<long long>(1, dev->sm_count / s.passes);
   const int grid = (int)std::min<long long>((long long)p.num_items, per_pass) * s.passes;
-  kern<<<grid, kWindowThreads, s.smem, static_cast<cudaStream_t>(stream_v)>>>(p);
-  RB_CUDA_TRY(cudaGetLastError());
+  RB_CUDA_TRY(launch_after(kern, grid, kWindowThreads, s.smem, static_cast<cudaStream_t>(stream_v), 1, p));
   count_launch();
   return RB_SUCCESS;
 }

@@ -85,12 +85,12 @@ gemm_skinny_kernel(const __grid_constant__ SkinnyMaps maps, const SkinnyParams p
   if (warp == 1) {
     tmem_alloc<1>(tmem_holder, p.tmem_cols);
     tmem_relinquish<1>();
+    griddep_launch();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  griddep_launch();
   griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
 
   uint32_t* part_smem = reinterpret_cast<uint32_t*>(smem);   // [nt][128] accumulators of this part, after the main loop
@@ -223,7 +223,10 @@ bool gemm_skinny_applicable(const RbGemmProblem* p, uint32_t epi_flags) {
   const int sms = planning_sm_count(), kblocks = (int)((p->k * es + 127) / 128);
   const long long slots = 2LL * sms, tiles = (long long)p->g * ((p->n + kTileN - 1) / kTileN);
   const int rows = p->c_type == RB_I32 && epi_flags == 0 ? (p->m + 2) / 3 : p->m;
-  if ((p->n * (long long)dtype_bytes(p->c_type)) % 16) return rows <= 36 || kblocks > 8 || skinny_splits(p, tiles, kblocks, sms) > 1;
+  // Rows of C off 16 bytes are stored element by element here and copied out of a staging tile there, K in one part up to eight blocks. us
+  // of 131, 1030 and 10245 columns, K = 256, 16 rows: 6.3 / 6.6, 6.4 / 6.6, 6.8 / 9.0; 24: 7.3 / 6.7, 7.5 / 6.8, 7.7 / 9.1; 48: 10.3 / 6.7, 10.5 / 7.0, 10.8 / 9.3.
+  if ((p->n * (long long)dtype_bytes(p->c_type)) % 16)
+    return rows <= (kblocks > 4 ? 26 : 20) + (tiles > 64 ? 14 : 0) || kblocks > 8 || skinny_splits(p, tiles, kblocks, sms) > 1;
   if (tiles > slots) return (kblocks >= 8 && 2 * rows <= kblocks) || (tiles <= 2 * slots && rows <= 6);
   const int splits = skinny_splits(p, tiles, kblocks, sms);
   if (splits == 1) return rows <= (kblocks >= 4 ? std::max(16, kblocks / 2) : 12);

@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "gemm_skinny.h"
+#include "launch.cuh"
 #include "lib_state.h"
 
 namespace rb {
@@ -69,6 +70,7 @@ __device__ __forceinline__ uint4 load_row16(const uint8_t* row, unsigned at, uns
 // the 3 x 1024 x 1024 x 769 product took 28.7 us, now 16.4.
 __global__ void pad_rows_kernel(const PadJobs p) {
   griddep_launch();   // the product is set up meanwhile
+  griddep_wait();
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < p.first[2];
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const bool second = i >= p.first[1];
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p) {
   __shared__ float tile[64][65];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();   // the product is set up meanwhile
+  griddep_wait();
   for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
     const bool second = t >= p.first[1];
     const F32Job j = second ? p.job[1] : p.job[0];
@@ -186,7 +189,7 @@ void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaSt
   for (int i = 0; i < 2; ++i)
     jobs.first[i + 1] = jobs.first[i] + (i < count ? groups * (long long)jobs.job[i].tiles_x * jobs.job[i].tiles_y : 0);
   const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * 32);
-  f32_prepare_kernel<<<grid, 256, 0, stream>>>(jobs);
+  launch_after(f32_prepare_kernel, grid, 256, 0, stream, 1, jobs);   // (an error stays for the launch of the product)
   count_launch();
 }
 
@@ -397,6 +400,8 @@ template <int VEC>
 __global__ void splitk_reduce_kernel(const void* __restrict__ partial, int splits, long long plane, int G, int M, int N,
                                      void* __restrict__ c, int c_type, int trans_c, int acc_is_int, EpiParams epi) {
   const long long total = (long long)G * M * N / VEC;
+  griddep_launch();
+  griddep_wait();
   for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < total; i0 += (long long)gridDim.x * blockDim.x) {
     const long long i = i0 * VEC;
     const long long gm = (i >> 32) ? i / N : (long long)((unsigned)i / (unsigned)N);
@@ -818,7 +823,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     if (nj > 0) {
       if (nj == 1) pj.first[2] = pj.first[1];
       const int pb = (int)std::min<unsigned long long>((pj.first[2] + 255) / 256, (unsigned long long)dev->sm_count * 8);
-      pad_rows_kernel<<<pb, 256, 0, stream>>>(pj);
+      RB_CUDA_TRY(launch_after(pad_rows_kernel, pb, 256, 0, stream, 1, pj));
       count_launch();
     }
   }
@@ -1058,11 +1063,11 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     const long long threads = total / (vec ? 4 : 1);
     const int blocks = (int)std::min<long long>((threads + 127) / 128, (long long)dev->sm_count * 16);
     if (vec)
-      splitk_reduce_kernel<4><<<blocks, 128, 0, stream>>>(partial, splits, total, p->g, p->m, p->n, c, p->c_type,
-                                                          p->trans_c ? 1 : 0, is_int ? 1 : 0, ep);
+      RB_CUDA_TRY(launch_after(splitk_reduce_kernel<4>, blocks, 128, 0, stream, 1, partial, splits, total, p->g, p->m, p->n, c, p->c_type,
+                               p->trans_c ? 1 : 0, is_int ? 1 : 0, ep));
     else
-      splitk_reduce_kernel<1><<<blocks, 128, 0, stream>>>(partial, splits, total, p->g, p->m, p->n, c, p->c_type,
-                                                          p->trans_c ? 1 : 0, is_int ? 1 : 0, ep);
+      RB_CUDA_TRY(launch_after(splitk_reduce_kernel<1>, blocks, 128, 0, stream, 1, partial, splits, total, p->g, p->m, p->n, c, p->c_type,
+                               p->trans_c ? 1 : 0, is_int ? 1 : 0, ep));
     count_launch();
   }
   return RB_SUCCESS;

@@ -593,6 +593,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   if (warp == 2) {
     tmem_alloc<CTAS>(tmem_holder, kTmemCols);
     tmem_relinquish<CTAS>();
+    griddep_launch();   // what follows may be set up; it waits for the end of this kernel itself
   }
   if (warp == 0 && lane_id() == 0) {
     for (int s = 0; s < (two_planes ? 2 : 1); ++s) {
