@@ -1081,7 +1081,12 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
   void* C;
   const void* a_hi = input;
   const void* a_lo = nullptr;
-  if (p->direction == 0 && pl.a_implicit && pl.a_planes > 0) {
+  const bool planes_by_gemm = p->direction == 0 && pl.a_implicit && pl.a_planes == 2 && !f32_stream;
+  if (planes_by_gemm) {
+    if (off16(ws)) return fail(RB_UNSUPPORTED, "f32 planes: the workspace must be 16-byte aligned");
+    a_hi = ws + pl.a_off;
+    a_lo = ws + pl.a_off + pl.a_bytes / 2;
+  } else if (p->direction == 0 && pl.a_implicit && pl.a_planes > 0) {
     float* hi = reinterpret_cast<float*>(ws + pl.a_off);
     float* lo = pl.a_planes == 2 ? reinterpret_cast<float*>(ws + pl.a_off + pl.a_bytes / 2) : nullptr;
     const long long pix = (long long)p->n * p->h * p->w;
@@ -1161,6 +1166,13 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     if (p->direction == 0) {
       cv.tensor = a_hi;
       cv.tensor_lo = a_lo;
+      if (planes_by_gemm) {
+        cv.src = static_cast<const float*>(input);
+        cv.src_groups = pl.a_nchw ? p->n : 1;
+        cv.src_rows = pl.a_nchw ? p->c : (int)((long long)p->n * p->h * p->w);
+        cv.src_cols = pl.a_nchw ? p->h * p->w : p->c;
+        cv.src_transpose = pl.a_nchw;
+      }
       cv.N = p->n; cv.H = p->h; cv.W = p->w; cv.C = p->c;
       cv.P = (int)ho; cv.Q = (int)wo; cv.Y = p->y; cv.X = p->x;
       cv.stride_h = p->stride_h; cv.stride_w = p->stride_w; cv.dil_h = p->dil_h; cv.dil_w = p->dil_w;

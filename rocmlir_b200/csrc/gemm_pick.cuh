@@ -10,6 +10,7 @@ typedef void (*GemmKernel)(const GemmTensorMaps, const GemmParams);
 GemmKernel gemm_kernel_plain(int kind, bool a_mn, bool b_mn, int ctas);    // gemm_plain_sm100.cu
 GemmKernel gemm_kernel_fused(int kind, bool a_mn, bool b_mn, int ctas);    // gemm_fused_sm100.cu
 GemmKernel gemm_kernel_copied(int kind, bool a_mn, bool b_mn, int ctas);   // gemm_copied_sm100.cu
+GemmKernel gemm_kernel_halves(int ctas, int tail);                          // gemm_halves_sm100.cu
 
 template <int KIND, int CTAS, int TAIL>
 GemmKernel pick_major(bool a_mn, bool b_mn) {

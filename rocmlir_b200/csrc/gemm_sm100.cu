@@ -125,11 +125,12 @@ __device__ __forceinline__ void store_planes4(const F32Job& j, long long o, cons
     *reinterpret_cast<float4*>(j.hi + o) = make_float4(x[0], x[1], x[2], x[3]);
   }
 }
-__global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p) {
+__global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p, const unsigned int* gate) {
   __shared__ float tile[64][65];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();   // the product is set up meanwhile
   griddep_wait();
+  if (gate && *reinterpret_cast<const volatile unsigned int*>(gate) == 0u) return;   // f16 planes will do
   for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
     const bool second = t >= p.first[1];
     const F32Job j = second ? p.job[1] : p.job[0];
@@ -184,13 +185,181 @@ F32Job f32_job(const float* src, float* hi, float* lo, int R, int C, int pitch, 
   j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
   return j;
 }
-void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream) {
+void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream, const unsigned int* gate = nullptr) {
   jobs.first[0] = 0;
   for (int i = 0; i < 2; ++i)
     jobs.first[i + 1] = jobs.first[i] + (i < count ? groups * (long long)jobs.job[i].tiles_x * jobs.job[i].tiles_y : 0);
-  const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * 32);
-  launch_after(f32_prepare_kernel, grid, 256, 0, stream, 1, jobs);   // (an error stays for the launch of the product)
+  const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * (gate ? 8 : 32));   // (one wave of blocks that may have to end at once)
+  launch_after(f32_prepare_kernel, grid, 256, 0, stream, 1, jobs, gate);   // (an error stays for the launch of the product)
   count_launch();
+}
+
+// ---- f32 operands as f16 planes (see kMaxPlanes) -----------------------------------------------------------------------------
+// Scales of the two operands, from 512 runs of 32 elements of each: a power of two that brings the largest to 2^13, and the flag, which stands when
+// no such scales exist. One block, a warp per run, the loads in flight together: single elements, 16384 lines of each operand, took 20 us from L2 and 117
+// from memory.
+struct HalvesState {
+  float scale[2], out_scale;
+  unsigned int flag;        // not zero: an operand does not fit, TF32 planes it is
+};
+struct HalvesSample {
+  const float* src[2];
+  long long n[2];
+  HalvesState* state;
+};
+__global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p) {
+  __shared__ float top[2][32];
+  __shared__ int low_runs;
+  griddep_launch();
+  griddep_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[2][16];
+  if (threadIdx.x == 0) low_runs = 0;
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    const long long step = p.n[o] / 512;   // (products this large have more than 16384 elements an operand)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long at = (i * 32 + warp) * step + lane;
+      v[o][i] = at < p.n[o] ? fabsf(__ldg(p.src[o] + at)) : 0.0f;
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, v[o][i]);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if (lane == 0) top[o][warp] = m;
+  }
+  __syncthreads();
+  int e[2];
+  bool fits = true;
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    float m = top[o][lane];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    const int x = (int)(__float_as_uint(m) >> 23);   // the biased exponent: 0 for zeros and subnormal numbers, 255 for infinities
+    fits = fits && x < 255;
+    e[o] = x == 0 ? 0 : 140 - x;                     // 2^e * m lies in [2^13, 2^14)
+    fits = fits && e[o] <= 126 && e[o] >= -126;
+    // runs that will not fit, seen here already: more than a quarter below 2^-15 of the largest
+    bool low = false;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) low = low || __popc(__ballot_sync(0xffffffffu, v[o][i] != 0.0f && v[o][i] < m * 3.0517578125e-5f)) > 8;
+    if (low && lane == 0) low_runs = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int sum = -(e[0] + e[1]);
+    fits = fits && sum <= 126 && sum >= -126;
+    p.state->scale[0] = fits ? __uint_as_float((uint32_t)(127 + e[0]) << 23) : 1.0f;
+    p.state->scale[1] = fits ? __uint_as_float((uint32_t)(127 + e[1]) << 23) : 1.0f;
+    p.state->out_scale = fits ? __uint_as_float((uint32_t)(127 + sum) << 23) : 1.0f;
+    p.state->flag = fits && low_runs == 0 ? 0u : 1u;
+  }
+}
+// The planes: hi = f16(y), lo = f16(y - hi) of y = scale * x, K-major like the TF32 ones. |y| >= 2^16 does not fit; below 2^-2 lo (steps of
+// 2^-24 there) holds less than hi's 11 further bits, and a run of 64 along K with more than 16 such values that are not zero raises the flag. So
+// what is lost against TF32 planes lies below 2^-38 of the operand's largest values, in a quarter of them at most: less than the last of the
+// three products that both forms leave out (lo.lo, 2^-22 of a product each).
+// Bound by one read and one write of the operand. 4096^3, both operands: TF32 planes 62 us, these 46, with the sample 53.
+struct HalvesJob {
+  const float* src;
+  __half* hi;
+  __half* lo;
+  int R, C, pitch;          // as in F32Job; pitch in elements, a multiple of eight
+  int transpose;
+  int tiles_x, tiles_y;
+};
+struct HalvesJobs {
+  HalvesJob job[2];
+  long long first[3];
+  HalvesState* state;
+};
+__global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
+  __shared__ float tile[64][65];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
+  griddep_launch();
+  griddep_wait();
+  if (*reinterpret_cast<const volatile unsigned int*>(&p.state->flag)) return;
+  bool bad = false;
+  // four neighbours along K of one row; the 16 lanes of a row hold a run of 64
+  auto store4 = [&](const HalvesJob& j, long long o, const float* x, float scale, bool inside) {
+    __half h[4], l[4];
+    int low = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float y = x[e] * scale;
+      bad = bad || !(fabsf(y) < 65504.0f);
+      low += y != 0.0f && fabsf(y) < 0.25f ? 1 : 0;
+      h[e] = __float2half_rn(y);
+      l[e] = __float2half_rn(y - __half2float(h[e]));
+    }
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) low += __shfl_xor_sync(0xffffffffu, low, d);
+    bad = bad || low > 16;
+    if (inside) {
+      *reinterpret_cast<uint2*>(j.hi + o) = *reinterpret_cast<const uint2*>(h);
+      *reinterpret_cast<uint2*>(j.lo + o) = *reinterpret_cast<const uint2*>(l);
+    }
+  };
+  for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
+    const bool second = t >= p.first[1];
+    const HalvesJob j = second ? p.job[1] : p.job[0];
+    const float scale = p.state->scale[second ? 1 : 0];
+    const long long lt = t - (second ? p.first[1] : 0), per_g = (long long)j.tiles_x * j.tiles_y;
+    const long long g = lt / per_g;
+    const int rem = (int)(lt - g * per_g);
+    const int c0 = (rem % j.tiles_x) * 64, r0 = (rem / j.tiles_x) * 64;
+    const float* s = j.src + g * (long long)j.R * j.C;
+    const bool vec = j.C % 4 == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
+    float x[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // all four reads in flight
+      const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+      const float* q = s + (long long)r * j.C + c;
+      if (vec && r < j.R && c < j.C) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
+      }
+    }
+    if (!j.transpose) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+        store4(j, (g * j.R + r) * (long long)j.pitch + c, x[i], scale, r < j.R && c < j.pitch);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tile[ty + 16 * i][tx * 4 + e] = x[i][e];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int oc = c0 + ty + 16 * i, orr = r0 + tx * 4;   // output row = source column, output column = source row
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
+        store4(j, (g * j.C + oc) * (long long)j.pitch + orr, y, scale, oc < j.C && orr < j.pitch);
+      }
+      __syncthreads();
+    }
+  }
+  if (__syncthreads_or(bad ? 1 : 0) && threadIdx.x == 0) p.state->flag = 1u;
+}
+HalvesJob halves_job(const float* src, __half* hi, __half* lo, int R, int C, int pitch, bool transpose) {
+  HalvesJob j;
+  j.src = src; j.hi = hi; j.lo = lo; j.R = R; j.C = C; j.pitch = pitch; j.transpose = transpose ? 1 : 0;
+  j.tiles_x = ((transpose ? C : pitch) + 63) / 64;
+  j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
+  return j;
 }
 
 // Zeros for a C that both K ranges of an f32 product are added to; a kernel and not a memset, which does not start before its predecessor has
@@ -502,6 +671,16 @@ RbStatus check_problem(const RbGemmProblem* p) {
   return RB_SUCCESS;
 }
 
+// Products that gain from f16 planes: two more passes and the launches of a form that is not taken, 8 to 10 us, against half of the tensor core's
+// time - and of the im2col loads of a convolution, where filters of several taps gain from a quarter of the size on. us, f16 and TF32 planes:
+// 1536^3 46 and 43, 2048 x 2048 x 1024 44 and 46, 1800^3 61 and 74, 2500^3 124 and 173; 3x3, 128 -> 128, 28x28, 10 images 40 and 43, 24 images 47
+// and 58, 64 images 88 and 125; pointwise 128 -> 256, 28x28, 64 images 63 and 60. Explicit variants keep the TF32 form.
+bool halves_pay(const RbGemmProblem* p, bool conv) {
+  return p->ab_type == RB_F32 && p->f32_mode == 0 && 2.0 * p->g * p->m * (double)p->n * p->k >= (conv && p->k >= 512 ? 2e9 : 8e9);
+}
+size_t halves_state_at(size_t total) { return align_up(total, 256); }
+size_t halves_workspace(size_t total) { return halves_state_at(total) + 256; }
+
 struct Workspace {
   size_t a_off[2], b_off[2];  // [0] = copy / hi, [1] = lo
   size_t partial_off;         // K-split partial planes
@@ -556,8 +735,9 @@ size_t rb::gemm_workspace_bytes(const RbGemmProblem* p, int implicit_operand, bo
   OperandPlan ob = plan_operand(p->trans_b == 0, p->n, p->k, es, f32, split);
   if (implicit_operand == 0) oa.needs_copy = false;
   if (implicit_operand == 1) ob.needs_copy = false;
-  return plan_workspace(p, oa, ob, (least ? choose_one_kernel(p, t_variant, false, implicit_operand >= 0)
-                                          : choose_config(p, t_variant, false, implicit_operand >= 0))).total;
+  const size_t total = plan_workspace(p, oa, ob, (least ? choose_one_kernel(p, t_variant, false, implicit_operand >= 0)
+                                                        : choose_config(p, t_variant, false, implicit_operand >= 0))).total;
+  return !least && implicit_operand <= 0 && halves_pay(p, implicit_operand == 0) ? halves_workspace(total) : total;
 }
 
 extern "C" size_t rbGemmWorkspaceSize(const RbGemmProblem* p) { return rb::gemm_workspace_bytes(p, -1); }
@@ -787,7 +967,16 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   const bool add_ranges = cfg.splits == 2 && split && p->c_type == RB_F32 && ep.flags == 0 && !p->trans_c && !cfg.plain_stores && !chain &&
                           p->n % 4 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0;
 
+  // without room for their state, or as a part of something else, TF32 planes
+  const bool conv_src = conv_a && conva->src != nullptr;
+  const bool halves = halves_pay(p, conv_a) && t_variant == 0 && !capture && !chain && (!conva || (conv_src && conva->tensor_lo && conva->C % 64 == 0)) &&
+                      (oa.needs_copy || conv_src) && ob.needs_copy && workspace && workspace_bytes >= halves_workspace(ws.total);
+
   uint8_t* wsb = static_cast<uint8_t*>(workspace);
+  HalvesState* const state = halves ? reinterpret_cast<HalvesState*>(wsb + halves_state_at(ws.total)) : nullptr;
+  const int half_pitch = (int)align_up((size_t)p->k, 8);
+  const void* a_half[2] = {nullptr, nullptr};
+  const void* b_half[2] = {nullptr, nullptr};
   const void* a_src[2] = {a, nullptr};
   const void* b_src[2] = {b, nullptr};
   if (is_f32) {
@@ -803,7 +992,45 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     };
     if (oa.needs_copy) add(a, oa, ws.a_off, a_src);
     if (ob.needs_copy) add(b, ob, ws.b_off, b_src);
-    if (nj > 0) launch_f32_jobs(jobs, nj, p->g, dev->sm_count, stream);
+    if (halves) {
+      // the f16 planes lie where the TF32 ones would: whichever form is not taken is never read
+      HalvesSample sample;
+      sample.src[0] = conv_src ? conva->src : static_cast<const float*>(a); sample.src[1] = static_cast<const float*>(b);
+      sample.n[0] = conv_src ? (long long)conva->src_groups * conva->src_rows * conva->src_cols : (long long)p->g * p->m * p->k;
+      sample.n[1] = (long long)p->g * p->k * p->n;
+      sample.state = state;
+      HalvesJobs hj;
+      memset(&hj, 0, sizeof(hj));
+      hj.state = state;
+      auto add_half = [&](int i, const void* src, const OperandPlan& o, const size_t* off, const void** planes) {
+        __half* hi = reinterpret_cast<__half*>(wsb + off[0]);
+        __half* lo = hi + align_up((size_t)p->g * o.rows * half_pitch, 128);
+        hj.job[i] = halves_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, half_pitch, o.src_mn_major);
+        hj.first[i + 1] = hj.first[i] + p->g * (long long)hj.job[i].tiles_x * hj.job[i].tiles_y;
+        planes[0] = hi;
+        planes[1] = lo;
+      };
+      if (conv_src) {
+        hj.job[0] = halves_job(conva->src, reinterpret_cast<__half*>(const_cast<void*>(conva->tensor)),
+                               reinterpret_cast<__half*>(const_cast<void*>(conva->tensor_lo)), conva->src_rows, conva->src_cols, conva->C,
+                               conva->src_transpose);
+        hj.first[1] = conva->src_groups * (long long)hj.job[0].tiles_x * hj.job[0].tiles_y;
+      } else {
+        add_half(0, a, oa, ws.a_off, a_half);
+      }
+      add_half(1, b, ob, ws.b_off, b_half);
+      RB_CUDA_TRY(launch_after(halves_scale_kernel, 1, 1024, 0, stream, 1, sample));
+      RB_CUDA_TRY(launch_after(f32_halves_kernel, (unsigned)std::min<long long>(hj.first[2], (long long)dev->sm_count * 32), 256, 0, stream, 1, hj));
+      count_launch(2);
+    }
+    if (conv_src) {
+      F32Jobs image;
+      memset(&image, 0, sizeof(image));
+      image.job[0] = f32_job(conva->src, static_cast<float*>(const_cast<void*>(conva->tensor)), static_cast<float*>(const_cast<void*>(conva->tensor_lo)),
+                             conva->src_rows, conva->src_cols, conva->C, conva->src_transpose);
+      launch_f32_jobs(image, 1, conva->src_groups, dev->sm_count, stream, halves ? &state->flag : nullptr);
+    }
+    if (nj > 0) launch_f32_jobs(jobs, nj, p->g, dev->sm_count, stream, halves ? &state->flag : nullptr);
   } else {
     PadJobs pj;
     memset(&pj, 0, sizeof(pj));
@@ -834,10 +1061,17 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   // 2 = 128, 3 = 256); bits 16-23 K-split count. Zero fields mean "choose" (see choose_config).
   const int ctas = cfg.ctas, bn = cfg.bn, stages = cfg.stages, splits = cfg.splits;
 
-  const int bke = (int)(kRowBytes / es);
+  const size_t es_c = dtype_bytes(p->c_type);
+  void* partial = splits > 1 ? static_cast<void*>(wsb + ws.partial_off) : nullptr;
+
+  // f32 products that may run on f16 planes are launched in both forms; the operands' state says on the device which one works
+  for (int form = halves ? 0 : 1; form < 2; ++form) {
+  const bool half = form == 0;
+  const size_t es_op = half ? 2 : es;                    // of the planes that this form reads
+  const int bke = (int)(kRowBytes / es_op);
   GemmTensorMaps maps;
   memset(&maps, 0, sizeof(maps));
-  CUtensorMapDataType dt = abt == RB_F16   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+  CUtensorMapDataType dt = abt == RB_F16 || half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                            : abt == RB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : abt == RB_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                             : CU_TENSOR_MAP_DATA_TYPE_UINT8;
@@ -849,16 +1083,17 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
                             std::string* err) {
     const bool fused = (&o == &oa) ? a_fused : b_fused;
     const int ci = (&o == &oa) ? 0 : 1;
-    const uint64_t gstride = chain ? chain_stride[ci] : (uint64_t)o.rows * o.pitch * es;
+    const uint64_t pitch = (uint64_t)(half ? half_pitch : o.pitch) * es_op;
+    const uint64_t gstride = chain ? chain_stride[ci] : (uint64_t)o.rows * pitch;
     if (chain) base = (chain_flip >> ci) & 1 ? chain_ptr[ci][1] : chain_ptr[ci][0];
     if (fused) {
       const uint64_t dims[4] = {(uint64_t)bke, (uint64_t)o.rows, (uint64_t)(o.cols / bke), (uint64_t)p->g};
-      const uint64_t strides[3] = {(uint64_t)o.pitch * es, (uint64_t)kRowBytes, gstride};
+      const uint64_t strides[3] = {pitch, (uint64_t)kRowBytes, gstride};
       const uint32_t box[4] = {(uint32_t)bke, (uint32_t)bke, (uint32_t)(box_rows_kmajor / bke), 1u};
       return encode_tiled(m, dt, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
     }
     const uint64_t dims[3] = {(uint64_t)o.cols, (uint64_t)o.rows, (uint64_t)p->g};
-    const uint64_t strides[2] = {(uint64_t)o.pitch * es, gstride};
+    const uint64_t strides[2] = {pitch, gstride};
     // K-major: box = BKE k-elements x tile rows. MN-major: box = one 128-byte chunk of MN x BKE k-rows.
     const uint32_t box[3] = {(uint32_t)bke, (uint32_t)(o.mn_major ? bke : box_rows_kmajor), 1u};
     return encode_tiled(m, dt, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
@@ -867,13 +1102,13 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   const int planes = gemm_planes(p);   // [0] hi (or the operand itself), [1] lo
   if (conva) {
     const ConvAOperand& cv = *conva;
-    const int che = kRowBytes / (int)es;   // elements per 128-byte run of channels
+    const int che = bke;                   // elements per 128-byte run of channels
     if (cv.C % che != 0) return fail(RB_UNSUPPORTED, "implicit operand: channels must be a multiple of 128 bytes");
     const long long pixels = (long long)cv.N * cv.P * cv.Q, taps = (long long)cv.Y * cv.X * cv.C;
     if (conv_a ? (pixels != p->m || taps != p->k) : (pixels != p->k || taps != p->n))
       return fail(RB_INVALID_PARAM, "implicit operand does not match the GEMM extents");
     const uint64_t dims[4] = {(uint64_t)cv.C, (uint64_t)cv.W, (uint64_t)cv.H, (uint64_t)cv.N};
-    const uint64_t strides[3] = {(uint64_t)cv.C * es, (uint64_t)cv.W * cv.C * es, (uint64_t)cv.H * cv.W * cv.C * es};
+    const uint64_t strides[3] = {(uint64_t)cv.C * es_op, (uint64_t)cv.W * cv.C * es_op, (uint64_t)cv.H * cv.W * cv.C * es_op};
     // bounding box of the base pixel: from -pad to (extent - 1) + upper corner, so that stepping by the stride
     // visits exactly P x Q positions (CUTLASS states the same rule for its fprop maps)
     const int lower[2] = {-cv.pad_w, -cv.pad_h};
@@ -888,8 +1123,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     }
   }
   for (int s = 0; s < planes; ++s) {
-    if (!conv_a && !encode_operand(&maps.a[s], a_src[s], oa, kBM, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
-    if (!conv_b && !encode_operand(&maps.b[s], b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
+    if (!conv_a && !encode_operand(&maps.a[s], half ? a_half[s] : a_src[s], oa, kBM, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
+    if (!conv_b && !encode_operand(&maps.b[s], half ? b_half[s] : b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
   }
 
   GemmParams kp;
@@ -901,10 +1136,9 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.tiles_n = (p->n + bn - 1) / bn;
   kp.kblocks = (p->k + bke - 1) / bke;
   kp.planes = planes;
-  kp.idesc = make_idesc(cfmt, fmt, fmt_b == 0xffffffffu ? fmt : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
+  const uint32_t fmt_op = half ? 0u : fmt;
+  kp.idesc = make_idesc(cfmt, fmt_op, fmt_b == 0xffffffffu ? fmt_op : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
   kp.acc_is_int = is_int ? 1 : 0;
-  const size_t es_c = dtype_bytes(p->c_type);
-  void* partial = splits > 1 ? static_cast<void*>(wsb + ws.partial_off) : nullptr;
   if (splits > 1 && conva && conva->c_rows_per_img > 0)
     return fail(RB_UNSUPPORTED, "a channel-major result cannot be combined with a K split");
   if (splits > 1 && !add_ranges) {
@@ -960,7 +1194,12 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.kpr = cfg.kpr;
   kp.probe = kProbeBuild ? (t_variant >> 24) & 7 : 0;
   kp.wait_cycles = t_wait_cycles;
-  if (t_stall_launches > 0) { kp.stall = 1; --t_stall_launches; }
+  if (t_stall_launches > 0) { kp.stall = 1; t_stall_launches -= form; }
+  if (halves) {
+    kp.gate = &state->flag;
+    kp.gate_want = half ? 0u : 1u;
+    kp.halves_scale = &state->out_scale;
+  }
   if (conva) {
     kp.conva.enabled = conv_a ? 1 : 2; kp.conva.P = conva->P; kp.conva.Q = conva->Q; kp.conva.X = conva->X;
     kp.conva.cchunks = conva->C / bke;
@@ -994,7 +1233,8 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
 
   // fused elementwise code and copied rows only in launches that have such work (see GemmTail)
   const int tail = kp.c_tma == 2 ? kTailCopied : kp.epi.flags != 0 ? kTailFused : kTailNone;
-  const GemmKernel kern = tail == kTailCopied  ? gemm_kernel_copied(kind, a_mn, b_mn, ctas)
+  const GemmKernel kern = half                 ? gemm_kernel_halves(ctas, tail)
+                          : tail == kTailCopied  ? gemm_kernel_copied(kind, a_mn, b_mn, ctas)
                           : tail == kTailFused ? gemm_kernel_fused(kind, a_mn, b_mn, ctas)
                                                : gemm_kernel_plain(kind, a_mn, b_mn, ctas);
   const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
@@ -1043,7 +1283,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     return RB_SUCCESS;
   }
   kp.trace = trace_buffer((size_t)lc.gridDim.x * 16);
-  if (add_ranges) {
+  if (add_ranges && (half || !halves)) {
     const long long n4 = (long long)p->g * p->m * p->n / 4;
     cudaLaunchConfig_t zc;
     memset(&zc, 0, sizeof(zc));
@@ -1057,6 +1297,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   }
   RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
   count_launch();
+  }
   if (splits > 1 && !add_ranges) {
     const long long total = (long long)p->g * p->m * p->n;
     const bool vec = p->n % 4 == 0 && !p->trans_c && reinterpret_cast<uintptr_t>(c) % (4 * es_c) == 0;

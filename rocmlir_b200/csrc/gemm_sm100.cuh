@@ -47,6 +47,8 @@ struct KindTraits<kKindF16> { static constexpr int ES = 2, UMMA_K = 16; };
 template <>
 struct KindTraits<kKindTF32> { static constexpr int ES = 4, UMMA_K = 8; };
 template <>
+struct KindTraits<kKindHalves> { static constexpr int ES = 2, UMMA_K = 16; };
+template <>
 struct KindTraits<kKindI8> { static constexpr int ES = 1, UMMA_K = 32; };
 template <>
 struct KindTraits<kKindF8> { static constexpr int ES = 1, UMMA_K = 32; };
@@ -60,6 +62,11 @@ struct KindTraits<kKindF8> { static constexpr int ES = 1, UMMA_K = 32; };
 //   round-to-nearest: the tensor core truncates what it adds to the magnitude of the accumulator, and they are 2^-11 of it.
 //   Both fit beside each other in tensor memory: two buffers of 128 + 128 columns, or one of 256 + 256.
 // 4096^3: 841 -> 707 us in all, 492 of them in this kernel (838 TFLOP/s of TF32 products); error against 64 bits unchanged.
+//
+// Large products take f16 planes instead (kKindHalves): hi and lo of x * 2^s have the 11 bits each that TF32 ones have, and their products
+// run at twice the rate. What f16 lacks is range: a power of two per operand brings a sample's largest value to 2^13, which leaves 2^3 above it
+// and full accuracy down to 2^-15 of it. Operands that do not fit - a value of 2^16 or more, or a run of 64 along K of which more than a
+// quarter lies below - raise a flag, and the launches behind it do the TF32 form instead (f32_halves_kernel in gemm_sm100.cu).
 constexpr int kMaxPlanes = 2;
 
 struct GemmTensorMaps {
@@ -133,6 +140,10 @@ struct GemmParams {
   unsigned int* chain_flags;
   unsigned int chain_token;
   int chain_flip;
+  // A launch that may turn out not to be wanted: it ends at once unless *gate == gate_want. halves_scale: 2^-(s of A + s of B).
+  const unsigned int* gate;
+  unsigned int gate_want;
+  const float* halves_scale;
 };
 
 // Implicit B operand: base coordinates of output pixel `pix` (row-major n, p, q) and the tap / channel chunk of
@@ -367,7 +378,7 @@ __device__ __forceinline__ void emit_staged(const EpiCopyCtx& c, const uint8_t* 
 // Rows without fused work that are copied out: 16-bit C, or 32-bit words as they are (f32 with `small_cols` columns further on its small
 // accumulator, added with round-to-nearest; raw i32; the planes of a K split). Out of line, so that the loops of aligned rows stay short.
 static __device__ __noinline__ void epi_copy_tile(uint8_t* staging, uint32_t taddr, uint8_t* dst, long long pitch, int es, int col0, int col_end,
-                                                  int rows, int lane, int c_type, bool bits32, uint32_t small_cols) {
+                                                  int rows, int lane, int c_type, bool bits32, uint32_t small_cols, float small_scale) {
   const int width = bits32 ? 32 : 64;   // columns of a staged row
   uint8_t* rowp = staging + lane * kRowBytes;
 #pragma unroll 1
@@ -381,7 +392,7 @@ static __device__ __noinline__ void epi_copy_tile(uint8_t* staging, uint32_t tad
         tmem_ld32(taddr + small_cols, u);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])) * small_scale);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
@@ -541,6 +552,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   const uint32_t eflags = EPI ? p.epi.flags : 0u;   // compile-time zero without EPI
   const int c_tma = COPY ? 2 : p.c_tma;             // 0 or 1 otherwise
   const bool acc_is_int = EPI ? KIND == kKindI8 : p.acc_is_int != 0;   // (the plain instantiation keeps the code it was measured with)
+  constexpr bool kPlanes = KIND == kKindTF32 || KIND == kKindHalves;   // f32 operands
+  if constexpr (kPlanes) {
+    if (p.gate) {
+      griddep_wait();
+      if (*reinterpret_cast<const volatile unsigned int*>(p.gate) != p.gate_want) return;
+    }
+  }
   using KT = KindTraits<KIND>;
   using L = GemmSmemLayout<CTAS>;
   constexpr int ES = KT::ES;
@@ -549,7 +567,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   constexpr int KSTEPS = BKE / KT::UMMA_K;     // MMAs per stage (always 4)
   constexpr int CHUNK_BYTES = BKE * kRowBytes; // one MN-major chunk: BKE k-rows of 128 B
   const int bn_cta = p.bn / CTAS;              // columns of B this CTA loads
-  const bool two_planes = KIND == kKindTF32 && p.planes == 2;   // folds to false in every other kind
+  const bool two_planes = KIND == kKindHalves || (KIND == kKindTF32 && p.planes == 2);   // folds to false in every other kind
   const int stage_bytes = L::stage_bytes(p.bn, two_planes ? 2 : 1);
   // tensor memory: two buffers of 256 columns; with two planes a buffer is the main and the small accumulator, and a tile
   // of 256 columns takes both buffers
@@ -728,7 +746,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
                   tma_load_3d_bar(sb + c * CHUNK_BYTES, &maps.b[0], lead_full, n0 + c * CHE, k0, gb);
               }
             }
-            if constexpr (KIND == kKindTF32) {
+            if constexpr (kPlanes) {
               if (two_planes && !((probe & 1) || p.stall)) {   // the lo planes, behind the hi planes
                 uint8_t* sa_lo = sa + L::kABytes;
                 uint8_t* sb_lo = sb + bn_cta * kRowBytes;
@@ -813,7 +831,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
             const uint32_t a_lo = a_lo0 + s * kStageStep;
             const uint32_t b_lo = b_lo0 + s * kStageStep;
             bool done = false;
-            if constexpr (KIND == kKindTF32) {
+            if constexpr (kPlanes) {
               if (two_planes) {   // lo.hi and hi.lo into the small accumulator, hi.hi into the main one
                 const uint32_t a_l = a_lo + (L::kABytes >> 4), b_l = b_lo + ((uint32_t)(bn_cta * kRowBytes) >> 4);
                 const uint32_t tmem_s = tmem_d + small_cols;
@@ -932,7 +950,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       const long long row = row0 + lane;
       const bool row_ok = row < p.M;
       const int ngroups = p.bn / 32;
-      const int gz = (KIND == kKindTF32 && p.c_add ? 0 : w.split * p.G) + (g ^ ((p.chain_flip >> 2) & 1));   // group coordinate of the store map (K-split planes are stacked groups)
+      const int gz = (kPlanes && p.c_add ? 0 : w.split * p.G) + (g ^ ((p.chain_flip >> 2) & 1));   // group coordinate of the store map (K-split planes are stacked groups)
       // Per-column scales / biases of this tile, converted to f32, in this warp's private copy.
       float* vec_scale = epi_vecs + q * (2 * kMaxBN);
       float* vec_bias = vec_scale + kMaxBN;
@@ -985,12 +1003,16 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         if (!got) break;
       }
       // f32: 32 columns of the small accumulator, added with round-to-nearest to those of the main one in v
+      const float halves_scale = KIND == kKindHalves ? __ldg(p.halves_scale) : 1.0f;
       auto add_small = [&](uint32_t taddr_main, uint32_t* v) {
         uint32_t u[32];
         tmem_ld32(taddr_main + small_cols, u);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
+        for (int j = 0; j < 32; ++j) {
+          const float x = __fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j]));
+          v[j] = __float_as_uint(KIND == kKindHalves ? x * halves_scale : x);   // (a power of two)
+        }
       };
       // Fast path (whole tiles, float accumulators, no fused elementwise work, 16-bit C through TMA stores): a
       // compact loop - 64 columns = one 128-byte staging row per step. The general loop below handles every other
@@ -1013,7 +1035,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         fence_proxy_async();
         __syncwarp();
         if (lane == 0 && row0 < p.M) {
-          if (KIND == kKindTF32 && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
+          if (kPlanes && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
           else tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
           bulk_commit();
         }
@@ -1021,7 +1043,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       if constexpr (COPY) {
         if (fast16 || fast32)
           epi_copy_tile(my_staging, tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN, copy_base(), p.c_stride_m, es_c, nb * p.bn,
-                        min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u);
+                        min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u, halves_scale);
       } else if (fast16) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
         const int nsteps = p.bn / 64;

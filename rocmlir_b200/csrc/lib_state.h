@@ -48,6 +48,11 @@ struct ConvAOperand {
                              // convolution (GEMM K = N*P*Q, N = Y*X*C; B stored K x N, i.e. trans_b = 0)
   const void* tensor;        // NHWC (dense), element type = the GEMM's ab_type (f32: the hi TF32 plane)
   const void* tensor_lo = nullptr;  // f32 in accurate mode: the lo TF32 plane of the same tensor (see f32_planes)
+  // f32: the tensor that the planes are made of, [src_groups][src_rows][src_cols], turned within a group when src_transpose; gemm_run
+  // makes them (hi at `tensor`, lo at `tensor_lo`, or f16 planes there). Null: they are there.
+  const float* src = nullptr;
+  int src_groups = 0, src_rows = 0, src_cols = 0;
+  bool src_transpose = false;
   int N, H, W, C;            // tensor extents
   int P, Q;                  // output image (GEMM M = N * P * Q)
   int Y, X;                  // filter (GEMM K = Y * X * C)

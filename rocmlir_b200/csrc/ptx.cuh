@@ -347,7 +347,7 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t cta_smem_addr, uint32_t ct
 }
 
 // MMA kinds
-enum : int { kKindF16 = 0, kKindTF32 = 1, kKindI8 = 2, kKindF8 = 3 };
+enum : int { kKindF16 = 0, kKindTF32 = 1, kKindI8 = 2, kKindF8 = 3, kKindHalves = 4 };   // (halves: f32 as two f16 planes, see kMaxPlanes)
 
 template <int KIND, int CTAS>
 __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -359,12 +359,12 @@ __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t adesc, uint64_
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                 \
       : "memory")
   if constexpr (CTAS == 1) {
-    if constexpr (KIND == kKindF16) RB_UMMA("f16", "1");
+    if constexpr (KIND == kKindF16 || KIND == kKindHalves) RB_UMMA("f16", "1");
     if constexpr (KIND == kKindTF32) RB_UMMA("tf32", "1");
     if constexpr (KIND == kKindI8) RB_UMMA("i8", "1");
     if constexpr (KIND == kKindF8) RB_UMMA("f8f6f4", "1");
   } else {
-    if constexpr (KIND == kKindF16) RB_UMMA("f16", "2");
+    if constexpr (KIND == kKindF16 || KIND == kKindHalves) RB_UMMA("f16", "2");
     if constexpr (KIND == kKindTF32) RB_UMMA("tf32", "2");
     if constexpr (KIND == kKindI8) RB_UMMA("i8", "2");
     if constexpr (KIND == kKindF8) RB_UMMA("f8f6f4", "2");

@@ -1,0 +1,151 @@
+"""f32 operands as two f16 planes (large products): no further from the 64-bit result than the TF32 planes that a call without room for their state
+takes, and bit for bit those wherever an operand does not fit f16's range - seen in the sample or only by the pass itself."""
+import math
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+RULE = 1 << 27   # an explicit variant word: TF32 planes
+
+
+def both(a, b, out=None, **kw):
+    """The product with all of its workspace and with 256 bytes less."""
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200.gemm import gemm, problem, workspace_size
+    p = problem(a, b, kw.get("trans_a", False), kw.get("trans_b", False), False, torch.float32)
+    res = []
+    for room in (0, 256):
+        ws = torch.empty(workspace_size(p) - room, dtype=torch.uint8, device="cuda")
+        res.append(gemm(a, b, out_dtype=torch.float32, workspace=ws, **kw).clone())
+        torch.cuda.synchronize()
+    assert L.kernel_status() == 0
+    return res
+
+
+def normal(*shape, seed=0):
+    import torch
+    return torch.randn(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+
+
+def error(got, want):
+    return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("g,m,n,k,ta,tb", [(1, 2048, 2048, 1024, False, False), (1, 1999, 2001, 1003, False, True), (1, 1024, 1024, 4160, True, False),
+                                           (1, 2300, 900, 2049, True, True), (3, 1100, 1300, 1000, False, True), (1, 64, 8192, 8192, False, True),
+                                           (1, 8200, 4100, 130, False, False)])
+def test_error_is_no_larger(cuda_device, g, m, n, k, ta, tb):
+    import torch
+    for scale in (1.0, 1e-25, 1e15):
+        a, b = normal(*((g, k, m) if ta else (g, m, k)), seed=1) * scale, normal(*((g, n, k) if tb else (g, k, n)), seed=2)
+        half, tf32 = both(a, b, trans_a=ta, trans_b=tb)
+        want = (a.double().transpose(1, 2) if ta else a.double()) @ (b.double().transpose(1, 2) if tb else b.double())
+        assert not torch.equal(half, tf32)   # the f16 planes were taken
+        assert error(half, want) <= 1.001 * error(tf32, want)
+
+
+@pytest.mark.parametrize("kind", ["relu", "uniform", "rows", "sparse", "integers"])
+def test_other_distributions(cuda_device, kind):
+    import torch
+    a, b = normal(1, 2048, 2048, seed=3), normal(1, 2048, 2048, seed=4)
+    if kind == "relu":
+        a = a.relu()
+    if kind == "uniform":
+        a, b = torch.rand_like(a), torch.rand_like(b) * 2 - 1
+    if kind == "rows":      # three decades, row by row and column by column
+        a = a * torch.logspace(-1.5, 1.5, 2048, device="cuda")[None, :, None]
+        b = b * torch.logspace(-1.5, 1.5, 2048, device="cuda")[None, None, :]
+    if kind == "sparse":
+        a = a * (torch.rand_like(a) < 0.01)
+    if kind == "integers":  # exact in both
+        a, b = a.mul(3).round(), b.mul(3).round()
+    half, tf32 = both(a, b)
+    want = a.double() @ b.double()
+    assert error(half, want) <= 1.001 * error(tf32, want)
+    if kind == "integers":
+        assert torch.equal(half.double(), want)
+
+
+@pytest.mark.parametrize("kind", ["huge", "huge_unsampled", "rows", "row_unsampled", "k", "inf", "nan", "subnormal", "largest", "alternate"])
+@pytest.mark.parametrize("which", [0, 1])
+def test_operands_that_do_not_fit_take_tf32_planes(cuda_device, kind, which):
+    import torch
+    x, y = normal(1, 2048, 2048, seed=5), normal(1, 2048, 2048, seed=6)
+    if which:   # the other operand, whose K runs down the rows
+        x = x.transpose(1, 2).contiguous()
+    rows, cols = ((2, 1) if which else (1, 2))
+    if kind == "huge":
+        x.select(rows, 17).mul_(1e9)
+    if kind == "huge_unsampled":
+        x[0, 1031, 77] = 1e7
+    if kind == "rows":
+        x = x * torch.logspace(-9, 9, 2048, device="cuda").view((1, 2048, 1) if rows == 1 else (1, 1, 2048))
+    if kind == "row_unsampled":
+        x.select(rows, 1033).mul_(1e-9)
+    if kind == "k":
+        x = x * torch.logspace(-6, 6, 2048, device="cuda").view((1, 1, 2048) if cols == 2 else (1, 2048, 1))
+    if kind == "inf":
+        x[0, 3, 1999] = math.inf
+    if kind == "nan":
+        x[0, 1500, 2] = math.nan
+    if kind == "subnormal":
+        x = x * 1e-41
+    if kind == "largest":
+        x[0, 5, 6] = 3.4e38
+    if kind == "alternate":
+        mask = (torch.arange(2048, device="cuda") % 2 == 0).view((1, 1, 2048) if cols == 2 else (1, 2048, 1))
+        x = torch.where(mask, x * 1e-7, x)
+    half, tf32 = both(y, x) if which else both(x, y)
+    assert torch.equal(half.view(torch.int32), tf32.view(torch.int32))
+
+
+def test_zeros_epilogue_and_result_over_an_operand(cuda_device):
+    import torch
+    from rocmlir_b200.gemm import Epilogue, gemm, problem, workspace_size
+    a, b, bias = normal(1, 2048, 2048, seed=7), normal(1, 2048, 2048, seed=8), normal(2048, seed=9)
+    for x in both(torch.zeros_like(a), b):
+        assert not x.any()
+    plain, fused = both(a, b)[0], both(a, b, epilogue=Epilogue(bias=bias, relu=True))[0]
+    assert torch.equal(fused, (plain + bias).relu())
+    ws = torch.empty(workspace_size(problem(a, b, False, False, False, torch.float32)), dtype=torch.uint8, device="cuda")
+    over = a.clone()
+    gemm(over, b, out=over, workspace=ws)
+    assert torch.equal(over, plain)
+
+
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+@pytest.mark.parametrize("n,c,k,hw,fil,stride,fits", [(24, 128, 128, 28, 3, 1, True), (20, 256, 64, 28, 3, 1, True), (20, 192, 130, 33, 3, 2, True),
+                                                      (24, 128, 128, 28, 3, 1, False)])
+def test_convolution(cuda_device, layout, n, c, k, hw, fil, stride, fits):
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200 import conv as rb_conv
+    last = layout == "nhwc"
+    lay = ("gkyxc", "nhwgc", "nhwgk") if last else ("gkcyx", "ngchw", "ngkhw")
+    cfg = rb_conv.ConvConfig(n, c, k, hw, hw, fil, fil, stride_h=stride, stride_w=stride, pad_h=1, pad_w=1, fil_layout=lay[0], in_layout=lay[1],
+                             out_layout=lay[2])
+    x, w = normal(n, c, hw, hw, seed=10), normal(k, c, fil, fil, seed=11)
+    if not fits:
+        x[n // 2] *= 1e8
+    order = (0, 2, 3, 1) if last else (0, 1, 2, 3)
+    xs, wsrc = x.permute(order).contiguous(), w.permute(order).contiguous()
+    got = []
+    for variant in (0, RULE):
+        out = torch.empty(cfg.numel("out"), device="cuda")
+        L.lib().rbSetGemmVariant(variant)
+        try:
+            ws = torch.empty(max(16, rb_conv.workspace_size(cfg, torch.float32, rb_conv.OPERATIONS["conv"])), dtype=torch.uint8, device="cuda")
+            rb_conv.conv(cfg, rb_conv.OPERATIONS["conv"], wsrc.view(-1), xs.view(-1), out, workspace=ws)
+        finally:
+            L.lib().rbSetGemmVariant(0)
+        torch.cuda.synchronize()
+        o = out.view(n, cfg.ho, cfg.wo, k).permute(0, 3, 1, 2) if last else out.view(n, k, cfg.ho, cfg.wo)
+        got.append(o.contiguous())
+    assert L.kernel_status() == 0
+    if not fits:
+        assert torch.equal(got[0], got[1])
+        return
+    with torch.backends.cudnn.flags(enabled=False):
+        want = torch.nn.functional.conv2d(x.double(), w.double(), stride=stride, padding=1)
+    assert not torch.equal(got[0], got[1]) and error(got[0], want) <= 1.001 * error(got[1], want)
