@@ -391,6 +391,14 @@ struct GemmConfig {
 // TF32 planes per operand (see kMaxPlanes)
 int gemm_planes(const RbGemmProblem* p) { return p->ab_type == RB_F32 && p->f32_mode == 0 ? 2 : 1; }
 
+// Products that gain from f16 planes: two more passes and the launches of a form that is not taken, 8 to 10 us, against half of the tensor core's
+// time - and of the im2col loads of a convolution, where filters of several taps gain from a quarter of the size on. us, f16 and TF32 planes:
+// 1536^3 46 and 43, 2048 x 2048 x 1024 44 and 46, 1800^3 61 and 74, 2500^3 124 and 173; 3x3, 128 -> 128, 28x28, 10 images 40 and 43, 24 images 47
+// and 58, 64 images 88 and 125; pointwise 128 -> 256, 28x28, 64 images 63 and 60. Explicit variants keep the TF32 form.
+bool halves_pay(const RbGemmProblem* p, bool conv) {
+  return p->ab_type == RB_F32 && p->f32_mode == 0 && 2.0 * p->g * p->m * (double)p->n * p->k >= (conv && p->k >= 512 ? 2e9 : 8e9);
+}
+
 // Tile and K split of a plain product by an estimate of its time, where nobody has asked for one. A launch costs `fixed`; a CTA (or
 // pair) then walks its tiles, K block by K block: at least `block` (operand fetch and issue of its MMAs), and no faster than all
 // CTAs together draw operands through the L2 -> SM fabric; a tile shorter than the store of the tile before it waits for that; the
@@ -469,6 +477,7 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
 
 GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = false, bool implicit = false, bool whole = false) {
   GemmConfig c;
+  const int asked = variant;
   if (variant == 0) variant = (int)tuned_variant_gemm(p);   // the measured table, when it knows the problem
   const int es = (int)dtype_bytes(p->ab_type);
   const bool b_mn = p->ab_type != RB_F32 && p->trans_b == 0;
@@ -533,7 +542,10 @@ GemmConfig choose_config(const RbGemmProblem* p, int variant, bool epi_vec = fal
   }
   if (c.splits > kblocks) c.splits = (int)kblocks;
   // every range must be non-empty with ceil-division ranges
-  while (c.splits > 1 && (long long)(c.splits - 1) * ((kblocks + c.splits - 1) / c.splits) >= kblocks) --c.splits;
+  // (also of the blocks of 64 that f16 planes have: 29 ranges of K = 50176 are 28 of them, and the sum read a plane that nobody had written)
+  const bool both = halves_pay(p, implicit) && (asked == 0 || ((variant >> 16) & 0xFF) == 0);
+  auto empty = [&](long long blocks) { return (c.splits - 1) * ((blocks + c.splits - 1) / c.splits) >= blocks; };
+  while (c.splits > 1 && (empty(kblocks) || (both && empty((p->k + 63LL) / 64)))) --c.splits;
   // Stream-K tail (variant bit 9 switches it ON): when the last wave of whole tiles would leave more than 5 % of the
   // GPU idle, the tiles of the last full wave plus the remainder are dealt out by K blocks instead. Measured on
   // B200 it does not pay for the shapes tried (4096^3 f16: 1090 vs 1120 TFLOP/s sustained; 2048x11008x4096 i8:
@@ -671,13 +683,6 @@ RbStatus check_problem(const RbGemmProblem* p) {
   return RB_SUCCESS;
 }
 
-// Products that gain from f16 planes: two more passes and the launches of a form that is not taken, 8 to 10 us, against half of the tensor core's
-// time - and of the im2col loads of a convolution, where filters of several taps gain from a quarter of the size on. us, f16 and TF32 planes:
-// 1536^3 46 and 43, 2048 x 2048 x 1024 44 and 46, 1800^3 61 and 74, 2500^3 124 and 173; 3x3, 128 -> 128, 28x28, 10 images 40 and 43, 24 images 47
-// and 58, 64 images 88 and 125; pointwise 128 -> 256, 28x28, 64 images 63 and 60. Explicit variants keep the TF32 form.
-bool halves_pay(const RbGemmProblem* p, bool conv) {
-  return p->ab_type == RB_F32 && p->f32_mode == 0 && 2.0 * p->g * p->m * (double)p->n * p->k >= (conv && p->k >= 512 ? 2e9 : 8e9);
-}
 size_t halves_state_at(size_t total) { return align_up(total, 256); }
 size_t halves_workspace(size_t total) { return halves_state_at(total) + 256; }
 

@@ -149,3 +149,17 @@ def test_convolution(cuda_device, layout, n, c, k, hw, fil, stride, fits):
     with torch.backends.cudnn.flags(enabled=False):
         want = torch.nn.functional.conv2d(x.double(), w.double(), stride=stride, padding=1)
     assert not torch.equal(got[0], got[1]) and error(got[0], want) <= 1.001 * error(got[1], want)
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 1152, 50176), (128, 1100, 49920), (100, 2048, 20544), (300, 384, 40000)])
+def test_every_range_of_k_has_blocks(cuda_device, m, n, k):
+    """Ranges counted in blocks of 32, of which a range of blocks of 64 may have none left: every plane that is summed has been written. The
+    workspace starts as NaN; sums of small whole numbers are exact."""
+    import torch
+    from rocmlir_b200.gemm import gemm, problem, workspace_size
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = (torch.randint(-2, 3, (1, r, k), generator=g, device="cuda").float() for r in (m, n))
+    ws = torch.full((workspace_size(problem(a, b, False, True, False, torch.float32)) // 4 + 64,), float("nan"), device="cuda").view(torch.uint8)
+    c = torch.empty(1, m, n, device="cuda")
+    gemm(a, b, trans_b=True, out=c, workspace=ws)
+    assert torch.equal(c.double(), torch.bmm(a.double(), b.double().transpose(1, 2)))
