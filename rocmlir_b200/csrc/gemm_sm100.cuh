@@ -365,9 +365,9 @@ static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t
 __device__ __forceinline__ void emit_staged(const EpiStoreCtx& c, const uint8_t* stg, int n0) {
   fence_proxy_async();
   __syncwarp();
-  if (c.lane == 0 && c.row0 < c.M) {
-    tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
-    bulk_commit();
+  if (c.lane == 0) {
+    if (c.row0 < c.M) tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
+    bulk_commit();   // without a store too: the waits count groups, and what they wait for may be a tile back
   }
 }
 __device__ __forceinline__ void emit_staged(const EpiCopyCtx& c, const uint8_t* stg, int n0) {
@@ -1034,10 +1034,12 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       auto store_map = [&](const uint8_t* stg, int n0) {
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0 && row0 < p.M) {
-          if (kPlanes && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
-          else tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
-          bulk_commit();
+        if (lane == 0) {
+          if (row0 < p.M) {
+            if (kPlanes && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
+            else tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
+          }
+          bulk_commit();   // without a store too: the waits count groups, and what they wait for may be a tile back
         }
       };
       if constexpr (COPY) {
