@@ -126,7 +126,6 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) attention_prefill_kernel(c
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -224,6 +223,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) attention_prefill_kernel(c
         j = sj;
         if (++s == NS) { s = 0; par ^= 1u; }
       }
+      griddep_launch();   // the last load is under way
     } else if (warp == 1 || warp == 3) {
       // ------------------------------ MMA issuer of one tile ------------------------------
       const int t = warp >> 1;

@@ -142,7 +142,6 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -182,6 +181,7 @@ __global__ void __launch_bounds__(kAttThreads, 1) attention_fwd_kernel(const __g
         for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, (j0 + j) * kKT, g);
         if (++s == NS) { s = 0; par ^= 1u; }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -574,7 +574,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
   if (warp == 1) {
     tmem_alloc<1>(tmem_holder, 64);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   tc_fence_before();
   __syncthreads();
@@ -609,6 +608,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
         for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, key0, g);
         if (++s == NS) { s = 0; par ^= 1u; }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -905,7 +905,6 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.q);
@@ -946,6 +945,7 @@ __global__ void __launch_bounds__(kAtt2Threads, 1) attention_fwd2_kernel(const _
         for (int c = 0; c < dv_chunks; ++c) tma_load_3d(vs + c * (kKT * 128), &maps.v, &v_full[s], c * 64, j * kKT, g);
         if (++s == NS) { s = 0; par ^= 1u; }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------

@@ -118,7 +118,6 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.in); prefetch_tmap(&maps.fil); }
   griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
@@ -164,6 +163,7 @@ conv_halo_kernel(const __grid_constant__ HaloGroup g) {
           if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
         }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------

@@ -85,7 +85,6 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) {
     for (int i = 0; i < PL; ++i) { prefetch_tmap(&maps.in[i]); prefetch_tmap(&maps.fil[i]); }
@@ -123,6 +122,7 @@ conv_halo_stream_kernel(const __grid_constant__ StreamMaps maps, const __grid_co
           }
         }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------

@@ -191,7 +191,6 @@ conv_patch_kernel(const PatchParams p) {
   if (warp == 0) {
     tmem_alloc<1>(tmem_holder, p.tmem_cols);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   griddep_wait();   // nothing above touches what an earlier kernel of the stream reads or writes
   load_window(p, PatchTile(p, tile), win);   // (the grid has no more CTAs per pass than there are tiles)
@@ -301,6 +300,7 @@ conv_patch_kernel(const PatchParams p) {
     prev = cur;
     cur = next;
   }
+  griddep_launch();   // the last load is under way
   cp_async_wait_all();
   if (ok && t > 0) {
     ok = mbar_wait(bar, (groups - 1) & 1u, p.status, kStatusTimeoutEpilogue, p.wait_cycles);

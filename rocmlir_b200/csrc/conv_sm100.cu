@@ -27,9 +27,7 @@
 #include <algorithm>
 #include <string>
 
-#include "launch.cuh"
 #include "lib_state.h"
-#include "ptx.cuh"
 
 namespace rb {
 namespace {
@@ -43,8 +41,6 @@ struct Dims5 {
 // to_dense: dst[dense] = src[strided]; else dst[strided] = src[dense]. ES = element bytes.
 template <int ES>
 __global__ void permute5_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, Dims5 d, int to_dense) {
-  griddep_launch();
-  griddep_wait();
   const long long total = d.size[0] * d.size[1] * d.size[2] * d.size[3] * d.size[4];
   if (total <= 0xffffffffLL) {
     // the usual case: 32-bit index arithmetic (64-bit divisions cost an order of magnitude more)
@@ -96,8 +92,6 @@ struct Transpose2 {
 
 template <typename T>
 __global__ void transpose_tiles_kernel(const T* __restrict__ src, T* __restrict__ dst, Transpose2 t, int to_dense) {
-  griddep_launch();
-  griddep_wait();
   __shared__ T tile[32][33];
   const long long tiles_r = (t.R + 31) / 32, tiles_c = (t.C + 31) / 32;
   const long long total = t.B0 * t.B1 * tiles_r * tiles_c;
@@ -146,8 +140,6 @@ struct GatherParams {
 
 template <int ES>
 __global__ void conv_gather_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, GatherParams g) {
-  griddep_launch();
-  griddep_wait();
   // Rows, columns and every per-tensor extent fit 32 bits (checked by the plan); only the flat index is 64-bit, so
   // all but the first division are 32-bit.
   const unsigned cols = (unsigned)(g.Y * g.X * g.CH), pitch = (unsigned)g.pitch;
@@ -191,8 +183,6 @@ __global__ void conv_gather_kernel(const uint8_t* __restrict__ src, uint8_t* __r
 // row pitch to be multiples of 16 bytes and 16-byte aligned buffers.
 template <int ES>
 __global__ void conv_gather_vec_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, GatherParams g) {
-  griddep_launch();
-  griddep_wait();
   constexpr int VE = 16 / ES;                      // elements per vector
   const unsigned pitch_v = (unsigned)(g.pitch / VE), chv = (unsigned)(g.CH / VE);
   const unsigned rows = (unsigned)(g.N * g.P * g.Q);
@@ -233,8 +223,6 @@ __global__ void conv_gather_vec_kernel(const uint8_t* __restrict__ src, uint8_t*
 // zeros elsewhere (out is N x ((P-1)*sh+1) x ((Q-1)*sw+1) x CH). One 16-byte vector of channels per thread and step.
 __global__ void upsample_nhwc_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int N, int P, int Q, int UP,
                                      int UQ, int chv, int sh, int sw) {
-  griddep_launch();
-  griddep_wait();
   const long long total = (long long)N * UP * UQ * chv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -267,8 +255,6 @@ struct ClassTable {
 
 template <int ES>
 __global__ void interleave_classes_kernel(const uint8_t* __restrict__ cls, uint8_t* __restrict__ dst, ClassTable t) {
-  griddep_launch();
-  griddep_wait();
   // One thread per 16-byte vector of channels when the destination is channel-contiguous, else per element. One
   // block row of threads walks one image row (n, h): the class row, and with it every division by a run-time
   // extent, is computed once per row; along w the class alternates with w mod stride_w.
@@ -341,8 +327,6 @@ struct ClassFilters {
 
 template <int ES>
 __global__ void class_filters_kernel(const uint8_t* __restrict__ fil, uint8_t* __restrict__ ws, ClassFilters f) {
-  griddep_launch();
-  griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < f.first[f.n]; i += (long long)gridDim.x * blockDim.x) {
     int c = 0;
     while (i >= f.first[c + 1]) ++c;
@@ -712,7 +696,9 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, b
 
 template <typename K, typename... Args>
 void launch_es(size_t es, int blocks, cudaStream_t st, K k1, K k2, K k4, Args... args) {
-  launch_after(es == 1 ? k1 : es == 2 ? k2 : k4, blocks, 256, 0, st, 1, args...);
+  if (es == 1) k1<<<blocks, 256, 0, st>>>(args...);
+  else if (es == 2) k2<<<blocks, 256, 0, st>>>(args...);
+  else k4<<<blocks, 256, 0, st>>>(args...);
 }
 
 }  // namespace
@@ -937,11 +923,11 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
       const int tb = (int)std::min<long long>(tiles, (long long)dev->sm_count * 16);
       const int td = to_dense ? 1 : 0;
       if (esz == 1)
-        launch_after(transpose_tiles_kernel<uint8_t>, tb, 256, 0, stream, 1, static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), t, td);
+        transpose_tiles_kernel<uint8_t><<<tb, 256, 0, stream>>>(static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), t, td);
       else if (esz == 2)
-        launch_after(transpose_tiles_kernel<uint16_t>, tb, 256, 0, stream, 1, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), t, td);
+        transpose_tiles_kernel<uint16_t><<<tb, 256, 0, stream>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), t, td);
       else
-        launch_after(transpose_tiles_kernel<uint32_t>, tb, 256, 0, stream, 1, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), t, td);
+        transpose_tiles_kernel<uint32_t><<<tb, 256, 0, stream>>>(static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), t, td);
       count_launch();
       return;
     }
@@ -986,8 +972,8 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
         ft.first[j + 1] = ft.first[j] + (long long)p->c * c.q.y * c.q.x * p->k;
       }
       const int fb = (int)std::max<long long>(1, std::min<long long>(blocks, (ft.first[ft.n] + 1023) / 1024));
-      if (es == 2) launch_after(class_filters_kernel<2>, fb, 256, 0, stream, 1, static_cast<const uint8_t*>(filter), ws, ft);
-      else launch_after(class_filters_kernel<4>, fb, 256, 0, stream, 1, static_cast<const uint8_t*>(filter), ws, ft);
+      if (es == 2) class_filters_kernel<2><<<fb, 256, 0, stream>>>(static_cast<const uint8_t*>(filter), ws, ft);
+      else class_filters_kernel<4><<<fb, 256, 0, stream>>>(static_cast<const uint8_t*>(filter), ws, ft);
       count_launch();
     }
     if (cls_on_halo) {
@@ -1059,9 +1045,9 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     const int ithreads = row_items <= 1024 ? (int)((row_items + 31) / 32 * 32) : 256;
     const int ib = (int)std::min<long long>((long long)p->n * p->h, (long long)dev->sm_count * (2048 / ithreads) * 2);
     if (es == 2)
-      launch_after(interleave_classes_kernel<2>, ib, ithreads, 0, stream, 1, ws, static_cast<uint8_t*>(input), tb);
+      interleave_classes_kernel<2><<<ib, ithreads, 0, stream>>>(ws, static_cast<uint8_t*>(input), tb);
     else
-      launch_after(interleave_classes_kernel<4>, ib, ithreads, 0, stream, 1, ws, static_cast<uint8_t*>(input), tb);
+      interleave_classes_kernel<4><<<ib, ithreads, 0, stream>>>(ws, static_cast<uint8_t*>(input), tb);
     count_launch();
     RB_CUDA_TRY(cudaGetLastError());
     return RB_SUCCESS;
@@ -1184,7 +1170,7 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
       cv.tensor = output;
       if (pl.a_up) {
         const int chv = (int)((size_t)p->k * es / 16);
-        launch_after(upsample_nhwc_kernel, blocks, 256, 0, stream, 1, static_cast<const uint4*>(output), reinterpret_cast<uint4*>(ws + pl.a_off),
+        upsample_nhwc_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint4*>(output), reinterpret_cast<uint4*>(ws + pl.a_off),
                                                           p->n, (int)ho, (int)wo, uh, uw, chv, p->stride_h, p->stride_w);
         count_launch();
         cv.tensor = ws + pl.a_off;

@@ -110,7 +110,6 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
   if (warp == 2) {
     tmem_alloc<1>(tmem_holder, 512);
     tmem_relinquish<1>();
-    griddep_launch();
   }
   if (warp == 0 && lane_id() == 0) { prefetch_tmap(&maps.x[0]); prefetch_tmap(&maps.dy); }
   tc_fence_before();
@@ -140,6 +139,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
           tma_load_4d(dy + (size_t)kc * p.dy_plane_bytes, &maps.dy, &full_bar[s], kc * 64, 0, p0, n);
         if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
       }
+      griddep_launch();   // the last load is under way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------

@@ -276,7 +276,6 @@ __global__ void __launch_bounds__(kWindowThreads, 1) conv_window_kernel(const __
   if (warp == kWorkers / 32) {
     tmem_alloc<1>(tmem_holder, p.tmem_cols);
     tmem_relinquish<1>();
-    griddep_launch();
     for (int i = lane; i < kZeroBytes / 16; i += 32) *reinterpret_cast<uint4*>(smem_raw + base + p.zero_off + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
   }
   if (worker) {   // (the grid has no more CTAs per pass than there are items)
@@ -403,6 +402,7 @@ __global__ void __launch_bounds__(kWindowThreads, 1) conv_window_kernel(const __
       prev = cur;
       cur = next;
     }
+    griddep_launch();   // the last load is under way
     cp_async_wait_all();
     if (t > 0 && ok && mbar_wait_warp(&done[(t - 1u) & 1u], ((t - 1u) >> 1) & 1u, p.status, kStatusTimeoutEpilogue, p.wait_cycles)) {
       tc_fence_after();

@@ -277,11 +277,10 @@ struct EpiCopyCtx : EpiStoreCtx {
 // anywhere: row r goes to dst + r * pitch, of which `cols` elements and the first `rows` rows exist. Stored straight from the
 // registers, as the general loop does, every store instruction touches 32 rows.
 //
-// 2- and 4-byte elements: eight lanes to a row, each an aligned 16 bytes of C put together from the two staged pieces it lies across;
-// what is left of a 128-byte run at its ends, 16 bytes in all, element by element. Bound by the load/store unit's instructions: 16 stores
+// 2-byte elements: eight lanes to a row, each an aligned 16 bytes of C put together from the two staged pieces it lies across; what is
+// left of a 128-byte run at its ends, 16 bytes in all, element by element. Bound by the load/store unit's instructions: 16 stores
 // for 32 rows of 64 columns where one per 32 neighbouring elements makes 64. 1344x997x144 f16 13.2 -> 12.5 us, 1675x918x1960 bf16
 // 24.1 -> 22.8 (18.0 with 920 columns). All rows' loads ahead of the stores: 13.2 and 23.2 (twice the code, and a tile runs it once).
-template <int ES>
 __device__ __forceinline__ void copy_rows_wide(const uint8_t* stg, uint8_t* dst, long long pitch_bytes, int rows, int bytes, int lane) {
   const int j = lane & 7;
 #pragma unroll 2
@@ -301,21 +300,20 @@ __device__ __forceinline__ void copy_rows_wide(const uint8_t* stg, uint8_t* dst,
 #pragma unroll
     for (int i = 0; i < 5; ++i) v[i] = (a & 4) ? u[i] : u[i + 1];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = ES == 4 ? v[i + 1] : __funnelshift_rc(v[i], v[i + 1], (4 - (a & 3)) * 8);
+    for (int i = 0; i < 4; ++i) o[i] = __funnelshift_rc(v[i], v[i + 1], (4 - (a & 3)) * 8);
     const int at = 16 * j - a;
     const bool there = row < rows;
     if (there && at >= 0 && at + 16 <= bytes) *reinterpret_cast<uint4*>(g + at) = make_uint4(o[0], o[1], o[2], o[3]);
     const int head = a ? min(16 - a, bytes) : 0, tail = head + ((bytes - head) & ~15);
     const int rest = there ? head + bytes - tail : 0;
-    for (int e = j * ES; e < rest; e += 8 * ES) {
+    for (int e = 2 * j; e < rest; e += 16) {
       const int off = e < head ? e : tail + e - head;
       const uint8_t* from = srow + ((off & ~15) ^ x) + (off & 15);
-      if (ES == 4) *reinterpret_cast<uint32_t*>(g + off) = *reinterpret_cast<const uint32_t*>(from);
-      else *reinterpret_cast<uint16_t*>(g + off) = *reinterpret_cast<const uint16_t*>(from);
+      *reinterpret_cast<uint16_t*>(g + off) = *reinterpret_cast<const uint16_t*>(from);
     }
   }
 }
-// Single bytes: a store per 32 neighbouring elements.
+// Single bytes and words of four: a store per 32 neighbouring elements (words: a whole run; 296 x 314 x 1472 f32 32.9 us, by 16 bytes to a lane 36.6).
 template <typename T>
 __device__ __forceinline__ void copy_rows(const uint8_t* stg, T* dst, long long pitch, int rows, int cols, int lane) {
   constexpr int kPer = kRowBytes / 32 / (int)sizeof(T);   // elements of a row per lane: columns lane, lane + 32, ...
@@ -355,8 +353,8 @@ static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t
       const int r = i / pieces, j = i - r * pieces;
       *reinterpret_cast<uint4*>(dst + r * pitch * es + j * 16) = *reinterpret_cast<const uint4*>(stg + r * kRowBytes + ((j ^ (r & 7)) << 4));
     }
-  } else if (es == 2) copy_rows_wide<2>(stg, dst, pitch * 2, rows, bytes, lane);
-  else if (es == 4) copy_rows_wide<4>(stg, dst, pitch * 4, rows, bytes, lane);
+  } else if (es == 2) copy_rows_wide(stg, dst, pitch * 2, rows, bytes, lane);
+  else if (es == 4) copy_rows(stg, reinterpret_cast<uint32_t*>(dst), pitch, rows, cols, lane);
   else copy_rows(stg, dst, pitch, rows, cols, lane);
   __syncwarp();
 }
@@ -611,7 +609,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
   if (warp == 2) {
     tmem_alloc<CTAS>(tmem_holder, kTmemCols);
     tmem_relinquish<CTAS>();
-    griddep_launch();   // what follows may be set up; it waits for the end of this kernel itself
   }
   if (warp == 0 && lane_id() == 0) {
     for (int s = 0; s < (two_planes ? 2 : 1); ++s) {
@@ -779,6 +776,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           if (++s == (uint32_t)rounds) { s = 0; ph ^= 1u; }
         }
       }
+      griddep_launch();   // the last load is under way
       if (p.trace) p.trace[blockIdx.x * 16 + 1] = (unsigned long long)w_empty;
     }
   } else if (warp == 1) {
