@@ -377,6 +377,7 @@ struct ConvPlan {
   bool a_up;         // backward data with a stride: the output gradient is zero-upsampled into the workspace first
   int a_planes;      // f32 forward implicit GEMM: TF32 planes of the input kept in the workspace (0, 1 or 2)
   bool a_nchw;       //   the input is NCHW: the plane pass transposes it to NHWC
+  int c_pad;         //   channels of the planes and of the filter matrix: the problem's, or padded with zeros to whole 128-byte runs
   size_t a_bytes, b_bytes, c_bytes, gemm_ws;
   size_t a_off, b_off, c_off, gemm_off, total;
   // backward data by stride classes (see interleave_classes_kernel): sub-problems and their places in the workspace
@@ -454,6 +455,7 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, b
   pl->a_up = false;
   pl->a_planes = 0;
   pl->a_nchw = false;
+  pl->c_pad = p->c;
   gp.g = (int)G;
   gp.ab_type = t;
   gp.f32_mode = p->f32_mode;
@@ -477,11 +479,22 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, b
     const int act_nchw[5] = {0, 1, 2, 3, 4};
     const bool in_is_nchw = is_dense_in_order(pl->is, isz, act_nchw, 5);
     const bool in_ok = (t != RB_F32) ? in_is_mat : (in_is_mat || in_is_nchw);
-    pl->a_implicit = !pl->a_direct && in_ok && G == 1 && (p->c * es) % 128 == 0 &&
+    // f32 with 16, 24, 40, ... channels: planes padded to a multiple of 32. The im2col matrix that such layers took otherwise is taps times the
+    // input, written, split in two and read again; small ones of it cost less than the padded filter (us, padded and matrix: 10 x 16 -> 128, 47x47,
+    // 3x3 40 and 61; 60 x 16 -> 256, 40x40 123 and 277; pointwise 7 x 16 -> 128, 53x53 23 and 28; 1 x 16 -> 64, 20x20, 3x3 24 and 19). Whole
+    // steps of eight channels: others would have more steps, and truncated sums, than the matrix. Variant bit 26 keeps the matrix.
+    if (t == RB_F32 && p->f32_mode == 0 && p->c >= 16 && p->c % 8 == 0 && pix_o * yxc * (long long)es >= (1 << 20) && !((rbGetGemmVariant() >> 26) & 1))
+      pl->c_pad = (p->c + 31) / 32 * 32;
+    pl->a_implicit = !pl->a_direct && in_ok && G == 1 && (pl->c_pad * es) % 128 == 0 &&
                      p->pad_h < 64 && p->pad_w < 64 && (p->y - 1) * p->dil_h < 256 && (p->x - 1) * p->dil_w < 256 &&
                      p->stride_h <= 8 && p->stride_w <= 8 && pix_i < 0x7fffffffLL;
     pl->a_planes = 0;
     pl->a_nchw = false;
+    if (!pl->a_implicit) pl->c_pad = p->c;
+    if (pl->c_pad != p->c) {
+      gp.k = p->y * p->x * pl->c_pad;
+      pl->b_direct = false;
+    }
     if (pl->a_implicit && t == RB_F32) {
       pl->a_nchw = !in_is_mat;
       pl->a_planes = p->f32_mode == 0 ? 2 : (in_is_mat ? 0 : 1);
@@ -511,9 +524,10 @@ RbStatus make_plan(const RbConvProblem* p, ConvPlan* pl, int result_type = -1, b
       }
     }
     if (pl->a_implicit) pl->a_direct = true;   // nothing to gather
-    pl->a_bytes = pl->a_implicit ? (size_t)pl->a_planes * up256((size_t)pix_i * p->c * es)
+    pl->a_bytes = pl->a_implicit ? (size_t)pl->a_planes * up256((size_t)pix_i * pl->c_pad * es)
                                  : (pl->a_direct ? 0 : (size_t)G * pix_o * yxc * es);
-    pl->b_bytes = pl->b_direct ? 0 : (size_t)G * p->k * yxc * es;
+    // (a padded filter matrix, and before it the dense one)
+    pl->b_bytes = pl->b_direct ? 0 : pl->c_pad != p->c ? up256((size_t)p->k * gp.k * es) + (size_t)p->k * yxc * es : (size_t)G * p->k * yxc * es;
     pl->c_bytes = pl->c_direct ? 0 : (size_t)G * pix_o * p->k * es_o;
   } else if (p->direction == 2) {
     gp.m = p->k; gp.n = (int)yxc; gp.k = (int)pix_o;
@@ -735,7 +749,7 @@ static bool f32_streamed(const RbConvProblem* p, const ConvPlan& pl, HaloConv* s
   const size_t fil_plane = up256((size_t)p->k * p->y * p->x * p->c * 4);
   if (!(pl.a_implicit && !pl.a_up && p->direction == 0 && p->stride_h == 1 && p->stride_w == 1 && p->g == 1 &&
         !((rbGetGemmVariant() >> 26) & 1) && p->data_type == RB_F32 && pl.a_planes == 2 && pl.gemm.c_type == RB_F32 &&
-        pl.gemm_ws >= 2 * fil_plane))
+        pl.gemm_ws >= 2 * fil_plane) || pl.c_pad != p->c)
     return false;
   halo_geometry(p, sc);
   *o_k = 1;
@@ -1088,6 +1102,18 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
     if (pl.a_direct) A = input; else { gather(input, ws + pl.a_off, false, false, ho, wo, p->c); A = ws + pl.a_off; }
     if (pl.b_direct) B = filter;
     else if (f32_stream && fil_kcyx) B = nullptr;   // transposed and split in one pass below
+    else if (pl.c_pad != p->c) {   // rows of channels, each padded
+      const void* dense = filter;
+      if (!is_dense_in_order(pl.fs, fsz, fil_kyxc, 5)) {
+        uint8_t* at = ws + pl.b_off + up256((size_t)p->k * pl.gemm.k * es);
+        permute(filter, at, fsz, pl.fs, fil_kyxc, true, es);
+        dense = at;
+      }
+      st = f32_planes(static_cast<const float*>(dense), reinterpret_cast<float*>(ws + pl.b_off), nullptr, 1, p->k * p->y * p->x, p->c, pl.c_pad, false,
+                      false, stream_v);
+      if (st != RB_SUCCESS) return st;
+      B = ws + pl.b_off;
+    }
     else { permute(filter, ws + pl.b_off, fsz, pl.fs, fil_kyxc, true, es); B = ws + pl.b_off; }
     C = (pl.c_direct || pl.c_remap) ? output : static_cast<void*>(ws + pl.c_off);
   } else if (p->direction == 2) {
@@ -1159,7 +1185,7 @@ RbStatus rb::conv_run(const RbConvProblem* p, int result_type, void* filter, voi
         cv.src_cols = pl.a_nchw ? p->h * p->w : p->c;
         cv.src_transpose = pl.a_nchw;
       }
-      cv.N = p->n; cv.H = p->h; cv.W = p->w; cv.C = p->c;
+      cv.N = p->n; cv.H = p->h; cv.W = p->w; cv.C = pl.c_pad;
       cv.P = (int)ho; cv.Q = (int)wo; cv.Y = p->y; cv.X = p->x;
       cv.stride_h = p->stride_h; cv.stride_w = p->stride_w; cv.dil_h = p->dil_h; cv.dil_w = p->dil_w;
       cv.pad_h = p->pad_h; cv.pad_w = p->pad_w; cv.pad_h_hi = p->pad_h_r; cv.pad_w_hi = p->pad_w_r;
