@@ -1124,8 +1124,12 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
         return fail(RB_UNSUPPORTED, "implicit operand (im2col): " + err);
     }
   }
+  // An A of fewer rows than a tile: no others are asked for (what the stage then holds there goes into rows of the sum that nothing reads).
+  // Rows beyond the tensor cost a TMA load more than rows of it do - us a call, fp8, K = 1344: 42 x 6560 9.8 -> 8.8, 42 x 8192 10.7 -> 8.8, 128 rows
+  // 8.8 and 8.9 - where every CTA's tile has them; in the last row of tiles alone they are not seen.
+  const int a_box = ctas == 1 && !conv_a && !chain && !oa.mn_major && p->m < kBM ? (int)(p->m + 7) / 8 * 8 : kBM;
   for (int s = 0; s < planes; ++s) {
-    if (!conv_a && !encode_operand(&maps.a[s], half ? a_half[s] : a_src[s], oa, kBM, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
+    if (!conv_a && !encode_operand(&maps.a[s], half ? a_half[s] : a_src[s], oa, a_box, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
     if (!conv_b && !encode_operand(&maps.b[s], half ? b_half[s] : b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
   }
 
@@ -1138,6 +1142,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.tiles_n = (p->n + bn - 1) / bn;
   kp.kblocks = (p->k + bke - 1) / bke;
   kp.planes = planes;
+  kp.a_short = planes * (kBM - a_box) * (int)kRowBytes;
   const uint32_t fmt_op = half ? 0u : fmt;
   kp.idesc = make_idesc(cfmt, fmt_op, fmt_b == 0xffffffffu ? fmt_op : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
   kp.acc_is_int = is_int ? 1 : 0;

@@ -119,6 +119,7 @@ struct GemmParams {
   unsigned int* sk_flags;      // [units][8]: one word per (CTA of the pair, epilogue warp), set to sk_token when written
   unsigned int sk_token;       // unique per launch, so stale words of earlier launches never match
   ConvAParams conva;
+  int a_short;                // bytes of a stage that are not loaded: rows that no row of a short A needs (one row tile, not a pair's)
   int a_fused, b_fused;       // MN-major operand loaded with one 4-D box per stage (extent a multiple of the chunk)
   int probe;                  // instrumentation, only in builds with -DRB_ENABLE_PROBE (results become meaningless):
                               // bit0 = no loads, bit1 = no epilogue work, bit2 = epilogue without its global stores
@@ -666,7 +667,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           } else if (probe & 1) {
             if (CTAS == 1 || rank == 0) mbar_arrive(&full_bar[s]);
           } else if constexpr (CTAS == 1) {
-            mbar_expect_tx(&full_bar[s], nblk * stage_bytes);
+            mbar_expect_tx(&full_bar[s], nblk * (stage_bytes - p.a_short));
           } else {
             if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * nblk * stage_bytes);
           }
