@@ -423,55 +423,67 @@ struct StoreCost {
 };
 constexpr TileCost kTileCosts[] = {{1, 64, 4.75, 0.239, 24}, {1, 128, 4.35, 0.311, 32}, {2, 128, 5.68, 0.233, 24}, {1, 256, 3.50, 0.446, 48}, {2, 256, 4.91, 0.324, 32}};
 constexpr StoreCost kStoreCost = {0.0087, 0.84, 0.0084, 2.58, 0.97};
-// f32 with two planes; only where the rule does not cut K, so that no accumulation chain gets longer
-constexpr TileCost kTileCostsF32[] = {{1, 64, 6.9, 0.57, 48}, {1, 128, 5.3, 0.67, 64}, {2, 128, 6.4, 0.56, 48}, {1, 256, 5.5, 0.95, 96}, {2, 256, 4.4, 0.87, 64}};
-constexpr StoreCost kStoreCostF32 = {0.025, 0.0, 0.025, 2.0, 0.85};
+// f32 with two TF32 planes: fitted to 131000 tiles and K ranges of 18000 products of 12 to 4096 rows and columns, K of 64 to 8192, alone and in groups
+// of three, 5 % off on average (the pass over the operands, the same for all of them, left out here). Of 959
+// products new to the fit one is more than 5 % slower than by the estimate before (fitted to six products, no K ranges) and 23 more than 2 %, the mean is 0.95:
+// 64 x 246 x 2019 29.8 -> 17.2 us, 128 x 1739 x 620 35.4 -> 21.1, 3 x 64 x 650 x 595 33.3 -> 19.4; 27 x 192 x 64 7.9 -> 8.1.
+constexpr TileCost kTileCostsF32[] = {{1, 64, 7.47, 0.518, 48}, {1, 128, 7.37, 0.608, 64}, {2, 128, 8.24, 0.526, 48}, {1, 256, 7.60, 1.069, 96}, {2, 256, 8.65, 0.818, 64}};
+constexpr StoreCost kStoreCostF32 = {0.0031, 0.58, 0.037, 11.9, 0.97};
 
 // *ctas and *bn come in as the rule gives them and stay unless another tile, or fewer K ranges, is estimated faster by the margin. K is not cut where
 // the rule does not cut it: such a product needs no planes in its workspace and can be handed out as one kernel. An f32 result keeps
 // accumulation chains no longer than the rule's: the tensor core truncates what it adds, and of two chains in place of one the error of f16 and
 // fp8 products against 64 bits is half (1.2e-6 -> 0.6e-6 at K = 1024; values of one sign 6.1e-6 -> 2.8e-6). In a 16-bit result its rounding hides that
 // (2.067e-4 both ways). whole: only all of K at once, whatever the result, where that is no slower than the rule (see choose_one_kernel).
+// f32 operands: where the rule cuts K (for speed, or to keep chains to 2048 elements), as many ranges as any tile gains by, down to eight blocks each;
+// with whole, and for what f16 planes may take over, the rule.
 void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks, int sms, bool whole, int* ctas, int* bn, int* splits) {
   const bool f32 = p->ab_type == RB_F32;
+  const int need = f32 ? (int)((p->k + 2047LL) / 2048) : 1;   // (see choose_config)
   const TileCost* const costs = f32 ? kTileCostsF32 : kTileCosts;
   const StoreCost& sc = f32 ? kStoreCostF32 : kStoreCost;
   const int es_c = (int)dtype_bytes(p->c_type);
   // an 8-bit result is requantised, 4-byte ones (and planes) are two staged rows for one; rows off 16 bytes are copied out by the warps
   const double words = f32 ? 1.0 : 1.45;
   const double width = (p->c_type == RB_I8 ? 2.76 : es_c == 4 ? words : 1.0) * ((long long)p->n * es_c % 16 ? sc.ragged : 1.0);
-  auto estimate = [&](const TileCost& t, bool split, long long* s, long long* waves) {
+  // *s comes in as the ranges wanted, 0 for the rule's
+  auto estimate = [&](const TileCost& t, long long* s, long long* waves) {
     const long long tiles = (long long)p->g * ((p->m + kBM * t.ctas - 1) / (kBM * t.ctas)) * ((p->n + t.bn - 1) / t.bn);
     const long long units = sms / t.ctas;
-    *s = split && tiles * 2 <= units && kblocks >= 16 ? std::max<long long>(1, std::min<long long>(std::min(units / tiles, kblocks / 8), 128)) : 1;
+    if (*s == 0) *s = tiles * 2 <= units && kblocks >= 16 ? std::max<long long>(1, std::min<long long>(std::min(units / tiles, kblocks / 8), 128)) : 1;
+    *s = std::min<long long>(std::max<long long>(*s, need), kblocks);
     const long long items = tiles * *s, kb = (kblocks + *s - 1) / *s;
     *waves = (items + units - 1) / units;
     const double busy = (double)std::min(items, units) * t.ctas;
     const double block = std::max(t.block, busy * t.kb_per_block / 12500.0);
     // (a byte per element in 64 columns: half of a staged row, copied out by the warps)
-    const double columns = t.bn * (*s > 1 ? words : t.bn == 64 && es_c == 1 ? 1.52 * width : width);
+    const double columns = (f32 ? std::min(t.bn, (int)p->n) : t.bn) * (*s > 1 ? words : t.bn == 64 && es_c == 1 ? 1.52 * width : width);
     double us = t.fixed + std::max(kb * block, sc.tile + sc.column * columns) * (double)(*waves - 1) + kb * block + sc.last * columns;
-    if (*s > 1) us += 2.13 + (double)*s * p->g * p->m * p->n * 4 / 1e6 * 0.265;
+    const double plane_mb = (double)p->g * p->m * p->n * 4 / 1e6;
+    if (f32 && *s > 1) us += *s == 2 && p->n % 4 == 0 ? 0.88 + plane_mb * 0.368 : 1.51 + (double)*s * plane_mb * 0.298;   // (two: see add_ranges)
+    if (!f32 && *s > 1) us += 2.13 + (double)*s * plane_mb * 0.265;
     return us;
   };
   const int rule_ctas = *ctas, rule_bn = *bn;
   double best = 0;
-  long long s = 1, waves = 1;
+  long long s = 0, waves = 1;
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
-    if (t.ctas == rule_ctas && t.bn == rule_bn) best = (whole ? 1.0 : sc.margin) * estimate(t, true, &s, &waves);
+    if (t.ctas == rule_ctas && t.bn == rule_bn) best = (whole ? 1.0 : sc.margin) * estimate(t, &s, &waves);
   }
-  if (best == 0 || waves > 3 || (f32 && (s > 1 || p->k > 2048))) return;   // (s and waves are those of the rule's tile)
+  if (best == 0 || waves > 3 || (f32 && s > 1 && (whole || halves_pay(p, false)))) return;   // (s and waves are those of the rule's tile)
   const long long rule_splits = whole ? 1 : s;
   const long long chain = p->c_type == RB_F32 && p->ab_type != RB_I8 && !whole ? (kblocks + s - 1) / s : kblocks;   // longest accumulation chain allowed
   for (int i = 0; i < 5; ++i) {
     const TileCost& t = costs[i];
-    if (f32 && t.ctas == 1 && t.bn == 256) continue;
-    if (b_mn && (t.bn / t.ctas) % che != 0) continue;
+    if ((b_mn && (t.bn / t.ctas) % che != 0) || (f32 && t.bn > 64 && t.bn >= 2 * p->n)) continue;
     if (t.ctas == 2 && (p->m <= kBM || kblocks <= 2)) continue;   // (see choose_config)
-    for (int split = 0; split < (rule_splits > 1 ? 2 : 1); ++split) {
-      double us = estimate(t, split != 0, &s, &waves);
-      if (s > 1) us *= 1.08;   // (K ranges other than the rule's are the less certain ones)
+    const long long tiles = (long long)p->g * ((p->m + kBM * t.ctas - 1) / (kBM * t.ctas)) * ((p->n + t.bn - 1) / t.bn);
+    const long long most = f32 && rule_splits > 1 ? std::max<long long>(rule_splits, std::min<long long>(std::min(sms / t.ctas / tiles, kblocks / 8), 128)) : 1;
+    for (long long want = f32 ? rule_splits : 1; want <= (f32 || rule_splits == 1 ? most : 2); ++want) {   // (f32: fewer than the rule's have longer chains)
+      s = f32 || want == 1 ? want : 0;
+      double us = estimate(t, &s, &waves);
+      if (s > 1 && !f32) us *= 1.08;   // (K ranges other than the rule's are the less certain ones)
       if (us < best && (kblocks + s - 1) / s <= chain) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
     }
   }
@@ -572,7 +584,7 @@ GemmConfig choose_one_kernel(const RbGemmProblem* p, int variant, bool epi_vec =
   const GemmConfig c = choose_config(p, variant, epi_vec, implicit);
   if (c.splits == 1) return c;
   const GemmConfig whole = choose_config(p, variant, epi_vec, implicit, true);
-  return whole.splits == 1 ? whole : c;
+  return whole.splits == 1 || p->ab_type == RB_F32 ? whole : c;
 }
 
 // Sums the partial planes of a K split in a fixed order (range 0, 1, 2, ...), applies the epilogue and
