@@ -59,7 +59,7 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// Two query tiles per CTA, without side tensors (attention_prefill_sm100.cu).
+// Two query tiles per CTA, without side tensors, scale above zero (attention_prefill_sm100.cu).
 constexpr int kPrefillThreads = 384;
 RbStatus attention_prefill_launch(const AttMaps& maps, const AttParams& p, cudaStream_t stream);
 

@@ -1,4 +1,4 @@
-// rock.attention over more than one query tile, no side tensors: two 128-row query tiles per CTA, each with a softmax group and an
+// rock.attention over more than one query tile, no side tensors, a scale above zero: two 128-row query tiles per CTA, each with a softmax group and an
 // issuing warp of its own, so that one tile's products run while the other tile's scores become probabilities.
 //
 // 384 threads: warp 0 producer (TMA loads, work items), warps 1 and 3 MMA issuers of tile A and B, warp 2 TMEM allocator, warps 4-7
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) attention_prefill_kernel(c
         float alpha = 1.0f;
         bool sure = false;
         if (j == 0) {
-          const float mb = row_max<0, kKT>(v, -INFINITY) * p.scale_log2;   // the scale is not negative
+          const float mb = row_max<0, kKT>(v, -INFINITY) * p.scale_log2;   // the scale is positive
           m_ref = mb > -INFINITY ? mb : -INFINITY;
           sure = true;
         }

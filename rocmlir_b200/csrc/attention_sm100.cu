@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) attention_decode_kernel(con
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Two query tiles per CTA, scores with side tensors (scale, bias, mask, quantised) or without a softmax; without side tensors
+// Two query tiles per CTA, scores with side tensors (scale, bias, mask, quantised), with a scale of zero or without a softmax; all others
 // attention_prefill_sm100.cu. One softmax group alone leaves the tensor pipe idle while it works: P_j.V_j has to wait
 // for softmax(j). With two 128-row query tiles (A, B) that share every K/V tile, the products of one tile run while
 // the other tile's softmax group computes:   ... PV_A(j)  S_A(j+1)  PV_B(j)  S_B(j+1) ...
@@ -1678,7 +1678,8 @@ static RbStatus rb::attention_run(const RbAttentionProblem* p, const void* q, co
   if (ctas > 0x7fffffffLL) return fail(RB_UNSUPPORTED, "too many query tiles");
   kp.o = o;
   kp.o_cols = p->head_v;
-  if (two_query_tiles(p) && !p->bias && !p->scale_tensor && !p->mask && !quantized && !kp.linear) {
+  // (the prefill kernel masks scores before it scales them: -inf times a scale of zero would be NaN)
+  if (two_query_tiles(p) && kp.scale_log2 > 0.0f && !p->bias && !p->scale_tensor && !p->mask && !quantized && !kp.linear) {
     const RbStatus st = attention_prefill_launch(maps, kp, stream);
     if (st != RB_SUCCESS) return st;
   } else if (two_query_tiles(p)) {

@@ -96,3 +96,16 @@ def test_scores_that_are_not_finite(cuda_device, bad):
     assert torch.equal(got.isnan(), seen.expand_as(got))
     ok = ~seen.expand_as(got)
     assert (got.double() - want)[ok].abs().max().item() <= 2.1 * 2.0 ** -11 * v.max().item()
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("scale", [0.0, -0.0, 2.0 ** -149, 2.0 ** -126])
+@pytest.mark.parametrize("g,s,sk,d,causal", [(2, 129, 128, 64, True), (2, 256, 256, 128, True), (3, 300, 300, 64, True), (1, 129, 1, 64, False),
+                                             (2, 257, 130, 128, False), (2, 900, 897, 64, False), (2, 256, 256, 64, False)])
+def test_scale_of_zero(cuda_device, dtype, scale, g, s, sk, d, causal):
+    """Every visible key weighs the same; keys past the end and above the diagonal weigh nothing."""
+    import torch
+    from rocmlir_b200.attention import attention
+    gen = torch.Generator(device="cuda").manual_seed(s + sk)
+    q, k, v = (torch.randn(shape, device="cuda", generator=gen).to(getattr(torch, dtype)) for shape in ((g, s, d), (g, sk, d), (g, sk, d)))
+    check(attention(q, k, v, trans_k=True, scale=scale, causal=causal), q, k, v, scale, causal)
