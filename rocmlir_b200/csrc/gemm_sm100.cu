@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();
   griddep_wait();
-  if (*reinterpret_cast<const volatile unsigned int*>(&p.state->flag)) return;
+  // other blocks may raise the flag at any time: one thread reads it for the block
+  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<const volatile unsigned int*>(&p.state->flag) != 0u)) return;
   bool bad = false;
   // four neighbours along K of one row; the 16 lanes of a row hold a run of 64
   auto store4 = [&](const HalvesJob& j, long long o, const float* x, float scale, bool inside) {
