@@ -129,7 +129,9 @@ typedef struct RbGemmProblem {
   int32_t trans_a, trans_b, trans_c;
   int32_t ab_type; /* RbDType of A and B */
   int32_t c_type;  /* RbDType of C */
-  int32_t f32_mode; /* for ab_type RB_F32: 0 = 3xTF32 split (fp32-class accuracy), 1 = single TF32 pass */
+  int32_t f32_mode; /* for ab_type RB_F32: 0 = every operand as the sum of two parts of 11 bits, three products of them (fp32-class accuracy):
+                       TF32 parts, or f16 parts in large products whose operands are seen on the device to hold as many bits in them;
+                       1 = single TF32 pass */
   int32_t store_method; /* 0 = set: C = A.B; 1 = add: C = C + A.B on a C the caller has filled (rock.gemm's
                            store_method = atomic_add, rocmlir-gen --store-method, rocmlir-gen.cpp:325-331). The product is
                            rounded to C's type and added in it; f32 / f16 / bf16 results. Deterministic: no atomics. */

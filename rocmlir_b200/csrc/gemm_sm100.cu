@@ -197,9 +197,11 @@ void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaSt
 }
 
 // ---- f32 operands as f16 planes (see kMaxPlanes) -----------------------------------------------------------------------------
-// Scales of the two operands, from 512 runs of 32 elements of each: a power of two that brings the largest to 2^13, and the flag, which stands when
-// no such scales exist. One block, a warp per run, the loads in flight together: single elements, 16384 lines of each operand, took 20 us from L2 and 117
-// from memory.
+// Scales of the two operands, from 512 runs of 32 elements of each: a power of two that brings the largest to 2^13 (1 where all are zero), and the flag,
+// which stands when no such scales exist. One block, a warp per run, the loads in flight together: single elements, 16384 lines of each operand, took 20
+// us from L2 and 117 from memory.
+// Values of |y| < kHalfFull, y = scale * x, have fewer bits in f16 planes (steps of 2^-36) than in TF32 ones: kHalfLeast has 18 of 22.
+constexpr float kHalfFull = 1.0f / 16384, kHalfLeast = kHalfFull / 16;
 struct HalvesState {
   float scale[2], out_scale;
   unsigned int flag;        // not zero: an operand does not fit, TF32 planes it is
@@ -219,7 +221,8 @@ __global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p
   if (threadIdx.x == 0) low_runs = 0;
 #pragma unroll
   for (int o = 0; o < 2; ++o) {
-    const long long step = p.n[o] / 512;   // (products this large have more than 16384 elements an operand)
+    // an odd number of runs apart, so that rows of any length are met in all their columns (small operands: the runs overlap)
+    const long long runs = p.n[o] / 512 / 32, step = runs > 1 ? ((runs - 1) | 1) * 32 : p.n[o] / 512;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const long long at = (i * 32 + warp) * step + lane;
@@ -247,10 +250,15 @@ __global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p
     fits = fits && x < 255;
     e[o] = x == 0 ? 0 : 140 - x;                     // 2^e * m lies in [2^13, 2^14)
     fits = fits && e[o] <= 126 && e[o] >= -126;
-    // runs that will not fit, seen here already: more than a quarter below 2^-15 of the largest
+    // values that will not fit, seen here already
+    const float scale = e[o] <= 126 && e[o] >= -126 ? __uint_as_float((uint32_t)(127 + e[o]) << 23) : 1.0f;
     bool low = false;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) low = low || __popc(__ballot_sync(0xffffffffu, v[o][i] != 0.0f && v[o][i] < m * 3.0517578125e-5f)) > 8;
+    for (int i = 0; i < 16; ++i) {
+      const float y = v[o][i] * scale;
+      const int below = __popc(__ballot_sync(0xffffffffu, v[o][i] != 0.0f && y < kHalfFull));
+      low = low || below > 1 || __any_sync(0xffffffffu, v[o][i] != 0.0f && y < kHalfLeast);
+    }
     if (low && lane == 0) low_runs = 1;
   }
   __syncthreads();
@@ -263,10 +271,11 @@ __global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p
     p.state->flag = fits && low_runs == 0 ? 0u : 1u;
   }
 }
-// The planes: hi = f16(y), lo = f16(y - hi) of y = scale * x, K-major like the TF32 ones. |y| >= 2^16 does not fit; below 2^-2 lo (steps of
-// 2^-24 there) holds less than hi's 11 further bits, and a run of 64 along K with more than 16 such values that are not zero raises the flag. So
-// what is lost against TF32 planes lies below 2^-38 of the operand's largest values, in a quarter of them at most: less than the last of the
-// three products that both forms leave out (lo.lo, 2^-22 of a product each).
+// The planes: hi = f16(y), lo = f16((y - hi) * kLoFactor) of y = scale * x, K-major like the TF32 ones. |y| >= 65504 does not fit. From kHalfFull up
+// they are off by 2^-23 of y at most, as TF32 planes are (2^-22 where the residual is half a step of the largest numbers). Nothing is lost to a value below, wherever it stands, because it raises the flag: what
+// selects it in the other operand - a diagonal, a few rows that are not zero - is not known here. The one exception keeps ordinary data on this form, where
+// one value in 3e7 is that small (normal ones; 4096 x 4096 of them have such a value in 4 cases of 10): one value of kHalfLeast or more in all
+// tiles of a block, among three others at least that are not zero in its 64 of a row and in its 64 of a column. Zeros are exact and count for nothing.
 // Bound by one read and one write of the operand. 4096^3, both operands: TF32 planes 62 us, these 46, with the sample 53.
 struct HalvesJob {
   const float* src;
@@ -281,33 +290,39 @@ struct HalvesJobs {
   long long first[3];
   HalvesState* state;
 };
+// Whether the value at (r, c) of a source of R x C, below kHalfFull, may stay in f16 planes (see above).
+__device__ __noinline__ bool low_value_fits(const float* s, int R, int C, int r, int c, float scale) {
+  if (fabsf(s[(long long)r * C + c] * scale) < kHalfLeast) return false;
+  int in_row = 0, in_col = 0;
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i) {
+    const int rr = (r & ~63) + i, cc = (c & ~63) + i;
+    in_row += cc < C && s[(long long)r * C + cc] != 0.0f ? 1 : 0;
+    in_col += rr < R && s[(long long)rr * C + c] != 0.0f ? 1 : 0;
+  }
+  return in_row >= 4 && in_col >= 4;
+}
 __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
   __shared__ float tile[64][65];
+  __shared__ int lows;      // values below kHalfFull
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();
   griddep_wait();
+  if (threadIdx.x == 0) lows = 0;
   // other blocks may raise the flag at any time: one thread reads it for the block
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<const volatile unsigned int*>(&p.state->flag) != 0u)) return;
   bool bad = false;
-  // four neighbours along K of one row; the 16 lanes of a row hold a run of 64
-  auto store4 = [&](const HalvesJob& j, long long o, const float* x, float scale, bool inside) {
+  auto store4 = [&](const HalvesJob& j, long long o, const float* x, float scale) {   // four neighbours along K of one row
     __half h[4], l[4];
-    int low = 0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float y = x[e] * scale;
-      bad = bad || !(fabsf(y) < 65504.0f);
-      low += y != 0.0f && fabsf(y) < 0.25f ? 1 : 0;
       h[e] = __float2half_rn(y);
-      l[e] = __float2half_rn(y - __half2float(h[e]));
+      // (a residual of 16, half a step of the largest numbers, would round up to infinity)
+      l[e] = __float2half_rn(fminf(fmaxf((y - __half2float(h[e])) * kLoFactor, -65504.0f), 65504.0f));
     }
-#pragma unroll
-    for (int d = 8; d > 0; d >>= 1) low += __shfl_xor_sync(0xffffffffu, low, d);
-    bad = bad || low > 16;
-    if (inside) {
-      *reinterpret_cast<uint2*>(j.hi + o) = *reinterpret_cast<const uint2*>(h);
-      *reinterpret_cast<uint2*>(j.lo + o) = *reinterpret_cast<const uint2*>(l);
-    }
+    *reinterpret_cast<uint2*>(j.hi + o) = *reinterpret_cast<const uint2*>(h);
+    *reinterpret_cast<uint2*>(j.lo + o) = *reinterpret_cast<const uint2*>(l);
   };
   for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
     const bool second = t >= p.first[1];
@@ -332,11 +347,22 @@ __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
         for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
       }
     }
+    uint32_t low = 0;   // (a lane's sixteen values)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float v = x[i >> 2][i & 3], y = fabsf(v * scale);
+      bad = bad || !(y < 65504.0f);
+      if (y < kHalfFull && v != 0.0f) low |= 1u << i;
+    }
+    if (low && !bad) {
+      const int i = __ffs(low) - 1;
+      bad = (low & (low - 1)) != 0 || atomicAdd(&lows, 1) != 0 || !low_value_fits(s, j.R, j.C, r0 + ty + 16 * (i >> 2), c0 + tx * 4 + (i & 3), scale);
+    }
     if (!j.transpose) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
-        store4(j, (g * j.R + r) * (long long)j.pitch + c, x[i], scale, r < j.R && c < j.pitch);
+        if (r < j.R && c < j.pitch) store4(j, (g * j.R + r) * (long long)j.pitch + c, x[i], scale);
       }
     } else {
 #pragma unroll
@@ -350,7 +376,7 @@ __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
         float y[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
-        store4(j, (g * j.C + oc) * (long long)j.pitch + orr, y, scale, oc < j.C && orr < j.pitch);
+        if (oc < j.C && orr < j.pitch) store4(j, (g * j.C + oc) * (long long)j.pitch + orr, y, scale);
       }
       __syncthreads();
     }

@@ -63,10 +63,12 @@ struct KindTraits<kKindF8> { static constexpr int ES = 1, UMMA_K = 32; };
 //   Both fit beside each other in tensor memory: two buffers of 128 + 128 columns, or one of 256 + 256.
 // 4096^3: 841 -> 707 us in all, 492 of them in this kernel (838 TFLOP/s of TF32 products); error against 64 bits unchanged.
 //
-// Large products take f16 planes instead (kKindHalves): hi and lo of x * 2^s have the 11 bits each that TF32 ones have, and their products
-// run at twice the rate. What f16 lacks is range: a power of two per operand brings a sample's largest value to 2^13, which leaves 2^3 above it
-// and full accuracy down to 2^-15 of it. Operands that do not fit - a value of 2^16 or more, or a run of 64 along K of which more than a
-// quarter lies below - raise a flag, and the launches behind it do the TF32 form instead (f32_halves_kernel in gemm_sm100.cu).
+// Large products take f16 planes instead (kKindHalves): hi = f16(y) and lo = f16((y - hi) * 2^12) of y = x * 2^s have the 11 bits each that TF32
+// ones have, and their products run at twice the rate. What f16 lacks is range. A power of two per operand brings a sample's largest value to 2^13,
+// which leaves 2^3 above it; lo, with a factor of its own that the epilogue takes out of the small accumulator, keeps all its bits down to |y| = 2^-14,
+// 2^-27 of that value (without the factor 2^-15 of it). Operands with values beyond either end raise a flag, and the launches behind it do
+// the TF32 form instead (f32_halves_kernel in gemm_sm100.cu).
+constexpr float kLoFactor = 4096.0f;
 constexpr int kMaxPlanes = 2;
 
 struct GemmTensorMaps {
@@ -377,7 +379,7 @@ __device__ __forceinline__ void emit_staged(const EpiCopyCtx& c, const uint8_t* 
 // Rows without fused work that are copied out: 16-bit C, or 32-bit words as they are (f32 with `small_cols` columns further on its small
 // accumulator, added with round-to-nearest; raw i32; the planes of a K split). Out of line, so that the loops of aligned rows stay short.
 static __device__ __noinline__ void epi_copy_tile(uint8_t* staging, uint32_t taddr, uint8_t* dst, long long pitch, int es, int col0, int col_end,
-                                                  int rows, int lane, int c_type, bool bits32, uint32_t small_cols, float small_scale) {
+                                                  int rows, int lane, int c_type, bool bits32, uint32_t small_cols, float small_by, float scale) {
   const int width = bits32 ? 32 : 64;   // columns of a staged row
   uint8_t* rowp = staging + lane * kRowBytes;
 #pragma unroll 1
@@ -391,7 +393,7 @@ static __device__ __noinline__ void epi_copy_tile(uint8_t* staging, uint32_t tad
         tmem_ld32(taddr + small_cols, u);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])) * small_scale);
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fmaf_rn(__uint_as_float(u[j]), small_by, __uint_as_float(v[j])) * scale);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
@@ -1009,8 +1011,9 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const float x = __fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j]));
-          v[j] = __float_as_uint(KIND == kKindHalves ? x * halves_scale : x);   // (a power of two)
+          // (both factors are powers of two)
+          v[j] = __float_as_uint(KIND == kKindHalves ? __fmaf_rn(__uint_as_float(u[j]), 1.0f / kLoFactor, __uint_as_float(v[j])) * halves_scale
+                                                     : __fadd_rn(__uint_as_float(v[j]), __uint_as_float(u[j])));
         }
       };
       // Fast path (whole tiles, float accumulators, no fused elementwise work, 16-bit C through TMA stores): a
@@ -1044,7 +1047,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       if constexpr (COPY) {
         if (fast16 || fast32)
           epi_copy_tile(my_staging, tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN, copy_base(), p.c_stride_m, es_c, nb * p.bn,
-                        min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u, halves_scale);
+                        min(p.N, (nb + 1) * p.bn), min(32, p.M - (int)row0), lane, p.c_type, fast32, two_planes ? small_cols : 0u,
+                        KIND == kKindHalves ? 1.0f / kLoFactor : 1.0f, halves_scale);
       } else if (fast16) {
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * kMaxBN;
         const int nsteps = p.bn / 64;

@@ -163,3 +163,126 @@ def test_every_range_of_k_has_blocks(cuda_device, m, n, k):
     c = torch.empty(1, m, n, device="cuda")
     gemm(a, b, trans_b=True, out=c, workspace=ws)
     assert torch.equal(c.double(), torch.bmm(a.double(), b.double().transpose(1, 2)))
+
+
+def worst(got, want, size, dim):
+    """Largest error along `dim` in units of the sum of the magnitudes that were added (|A||B|)."""
+    return ((got.double() - want).abs() / size.clamp(min=1e-300)).amax(dim)
+
+
+def no_worse(half, tf32, a, b):
+    """Row by row and column by column, no further from the 64-bit result than the TF32 form, apart from what both may leave of each single
+    product: lo.lo, 2^-22 of it, and 2^-23 of it for the rounding of each lo, 2^-21 together."""
+    want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    for dim in (1, 2):
+        assert (worst(half, want, size, dim) <= 2 * worst(tf32, want, size, dim) + 2.0 ** -21).all()
+
+
+def uneven(kind, shape, seed):
+    """Operands most of which are zero, or some of whose values are far below the others, rows first."""
+    import torch
+    x = normal(*shape, seed=seed)
+    rows, cols = shape[1], shape[2]
+    r, c = torch.arange(rows, device="cuda")[:, None], torch.arange(cols, device="cuda")[None, :]
+    gen = torch.Generator(device="cuda").manual_seed(seed + 1)
+    some = torch.rand(shape, device="cuda", generator=gen)
+    fall = lambda lo, n: torch.logspace(0, lo, n, device="cuda", dtype=torch.float64).float()
+    if kind.startswith("superdiagonal"):
+        x = torch.where(c == r + 64, 1 + some, 0) * float(kind[13:])
+    if kind == "diagonal":
+        x = torch.where(c == r, 1 + some, 0) * fall(-9, rows)[None, :, None]
+    if kind == "few":
+        x = x * (some < 0.05) * 1e-4 * (c >= 32)
+    if kind == "few_by_rows":
+        x = x * (some < 0.05) * fall(-8, rows)[None, :, None]
+    if kind == "sparse_row":
+        x = torch.where(r == 1033, x * (some < 0.2) * 1e-9, x)
+    if kind == "relu_row":
+        x = torch.where(r == 1033, x.relu() * (c % 4 == 0) * 1e-12, x)
+    if kind == "dense_row_underflows":
+        x = torch.where(r == 1033, x * 1e-25, x * 1e30)
+    if kind == "low_columns":
+        x = torch.where(c % 64 < 12, x * 1e-9, x)
+    if kind == "one_low_column":
+        x = torch.where(c == 77, x * 1e-8, x)
+    if kind == "scattered":
+        x = torch.where(some < 1e-3, x * 1e-10, x)
+    if kind == "one_value":
+        x[0, 1033, 77] = 1e-9
+    return x.contiguous()
+
+
+UNEVEN = ["superdiagonal1.1e-3", "superdiagonal1e-4", "superdiagonal1e-9", "diagonal", "few", "few_by_rows", "sparse_row", "relu_row",
+          "dense_row_underflows", "low_columns", "one_low_column", "scattered", "one_value"]
+
+
+@pytest.mark.parametrize("kind", UNEVEN)
+@pytest.mark.parametrize("other", ["normal", "identity"])
+@pytest.mark.parametrize("which", [0, 1])
+def test_small_values_keep_their_digits(cuda_device, kind, other, which):
+    import torch
+    x = uneven(kind, (1, 2048, 2048), 21)
+    y = torch.eye(2048, device="cuda")[None].contiguous() if other == "identity" else normal(1, 2048, 2048, seed=23)
+    if which:
+        x = x.transpose(1, 2).contiguous()
+    a, b = (y, x) if which else (x, y)
+    no_worse(*both(a, b), a, b)
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_short_sums_keep_the_digits_of_small_rows(cuda_device, which):
+    import torch
+    x, y = normal(1, 16384, 16, seed=31), normal(1, 16384, 16, seed=32)
+    x[:, 1::2] *= 1e-9
+    a, b = (y, x) if which else (x, y)
+    half, tf32 = both(a, b, trans_b=True)
+    no_worse(half, tf32, a, b.transpose(1, 2))
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_ordinary_operands_take_f16_planes(cuda_device, seed):
+    """4096 x 4096 normal values: now and then a single one lies below what f16 planes hold in full (none of these four below 2^-18)."""
+    import torch
+    a, b = normal(1, 4096, 4096, seed=100 + seed), normal(1, 4096, 4096, seed=200 + seed)
+    half, tf32 = both(a, b)
+    assert not torch.equal(half, tf32)
+    no_worse(half, tf32, a, b)
+
+
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+@pytest.mark.parametrize("c", [40, 128])
+@pytest.mark.parametrize("kind", ["dim_image", "few", "dim_filter"])
+def test_convolution_keeps_the_digits_of_small_values(cuda_device, layout, c, kind):
+    import torch
+    from rocmlir_b200 import _lib as L
+    from rocmlir_b200 import conv as rb_conv
+    n, k, hw, last = 48, 128, 28, layout == "nhwc"
+    lay = ("gkyxc", "nhwgc", "nhwgk") if last else ("gkcyx", "ngchw", "ngkhw")
+    cfg = rb_conv.ConvConfig(n, c, k, hw, hw, 3, 3, pad_h=1, pad_w=1, fil_layout=lay[0], in_layout=lay[1], out_layout=lay[2])
+    x, w = normal(n, c, hw, hw, seed=41), normal(k, c, 3, 3, seed=42)
+    if kind == "dim_image":
+        x[n // 2] *= (normal(c, hw, hw, seed=43) > 1.0) * 1e-9
+    if kind == "few":
+        x = x * (normal(n, c, hw, hw, seed=43) > 2.0) * 1e-4
+        x[:, :32] = 0
+        x[0, 0, 0, 0] = 1.0
+    if kind == "dim_filter":
+        w[17] *= (normal(c, 3, 3, seed=43) > 1.0) * 1e-9
+    order = (0, 2, 3, 1) if last else (0, 1, 2, 3)
+    xs, wsrc = x.permute(order).contiguous(), w.permute(order).contiguous()
+    got = []
+    for variant in (0, RULE):
+        out = torch.empty(cfg.numel("out"), device="cuda")
+        L.lib().rbSetGemmVariant(variant)
+        try:
+            ws = torch.empty(max(16, rb_conv.workspace_size(cfg, torch.float32, rb_conv.OPERATIONS["conv"])), dtype=torch.uint8, device="cuda")
+            rb_conv.conv(cfg, rb_conv.OPERATIONS["conv"], wsrc.view(-1), xs.view(-1), out, workspace=ws)
+        finally:
+            L.lib().rbSetGemmVariant(0)
+        torch.cuda.synchronize()
+        got.append((out.view(n, cfg.ho, cfg.wo, k).permute(0, 3, 1, 2) if last else out.view(n, k, cfg.ho, cfg.wo)).reshape(n * k, -1))
+    assert L.kernel_status() == 0
+    with torch.backends.cudnn.flags(enabled=False):
+        want, size = (torch.nn.functional.conv2d(p.double(), q.double(), padding=1).reshape(n * k, -1) for p, q in ((x, w), (x.abs(), w.abs())))
+    for dim in (0, 1):   # (per image and filter, per filter and pixel over the images)
+        assert (worst(got[0], want, size, dim) <= 2 * worst(got[1], want, size, dim) + 2.0 ** -21).all()
