@@ -22,8 +22,9 @@
 // into one buffer were measured several times slower than the MMAs of a small problem). Filters whose accumulators
 // exceed the 512 TMEM columns are divided among groups of CTAs (each group walks all pixels for its share of the taps).
 //
-// Non-finite inputs: a zero of the padded raster multiplies whatever pixel the shifted window holds there, so an Inf
-// or NaN in the input can reach taps that the reference's gather would not pair it with.
+// Non-finite inputs: a zero of the padded raster multiplies whatever pixel the shifted window holds there, so an Inf or NaN in the input makes a NaN of
+// taps that do not meet it. With a stride, where the im2col form of this library would run otherwise, the second kernel computes whatever it finds to be NaN
+// once more, pixel by pixel; at unit stride such taps are NaN.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -52,7 +53,7 @@ struct WgradMaps {
 };
 
 struct WgradParams {
-  int Kout, cchunks, kchunks, yxc;
+  int Kout, kchunks, yxc;
   int Wp, R, ksteps;                 // padded raster width, output rows per tile, 16-pixel reduction steps per tile
   int tiles_per_img, num_tiles;
   int x_plane_bytes, dy_plane_bytes, x_box_bytes, dy_box_bytes, stage_bytes, stages, dy_off;
@@ -233,10 +234,84 @@ conv_wgrad_halo_kernel(const __grid_constant__ WgradMaps maps, const __grid_cons
   }
 }
 
+// What elements of the filter gradient are computed from by themselves.
+struct WgradDirect {
+  const uint16_t* x;     // [N][H][W][C]; null: they are left as they are
+  const uint16_t* dy;    // [N][P][Q][Kout]
+  int H, W, C, P, Q, Kout, X, yxc;
+  int stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
+  int pixels;            // N * P * Q
+};
+__device__ __forceinline__ float elem16(uint32_t bits, int is_bf16) {
+  return is_bf16 ? __bfloat162float(__ushort_as_bfloat16((unsigned short)bits)) : __half2float(__ushort_as_half((unsigned short)bits));
+}
+__device__ __forceinline__ void store4_16(void* out, int i4, float4 a, int is_bf16) {
+  uint2 w;
+  if (is_bf16) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+    w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
+  } else {
+    __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(a.z, a.w);
+    w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
+  }
+  reinterpret_cast<uint2*>(out)[i4] = w;
+}
+// The block's quads of elements (neighbouring channels of one tap) whose sums, in part[0 .. 31], hold a NaN: such elements once more, pixel by pixel, the
+// output pixels shared out among all threads. A padding pixel is a zero that is multiplied like any other, as in the im2col form. A sum that
+// is NaN stays one: a quad is done when one of its threads has that of all that are asked for.
+__device__ __noinline__ void wgrad_direct(const WgradDirect& d, float4* part, int first, int elems, void* out, int is_bf16) {
+  __shared__ int done[32];
+  const int lane = threadIdx.x & 31;
+  const float4 mine = part[lane];
+  const uint32_t quads = __ballot_sync(0xffffffffu, first + 4 * lane < elems && (isnan(mine.x) || isnan(mine.y) || isnan(mine.z) || isnan(mine.w)));
+  int bits = 0;
+  while ((1 << bits) < __popc(quads)) ++bits;
+  const int quad = threadIdx.x & ((1 << bits) - 1), groups = 256 >> bits, group = threadIdx.x >> bits;
+  const bool active = quad < __popc(quads);
+  const int at = active ? (int)__fns(quads, 0, quad + 1) : 0, i = first + 4 * at;
+  const float4 sum = part[at];
+  const int k = i / d.yxc, tap = i % d.yxc / d.C, c = i % d.C, y = tap / d.X, x = tap % d.X;
+  if (threadIdx.x < 32) done[threadIdx.x] = 0;
+  __syncthreads();   // and part may be written again
+  float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int pix0 = group; active && pix0 < d.pixels; pix0 += 8 * groups) {
+    if (reinterpret_cast<volatile int*>(done)[quad]) break;
+    float g[8];
+    uint2 t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int pix = pix0 + u * groups;
+      const int row = pix / d.Q, q = pix - row * d.Q, n = row / d.P;
+      const int h = (row - n * d.P) * d.stride_h - d.pad_h + y * d.dil_h, v = q * d.stride_w - d.pad_w + x * d.dil_w;
+      const bool there = pix < d.pixels;
+      g[u] = there ? elem16(__ldg(d.dy + (size_t)pix * d.Kout + k), is_bf16) : 0.0f;
+      t[u] = make_uint2(0u, 0u);
+      if (there && h >= 0 && h < d.H && v >= 0 && v < d.W) t[u] = __ldg(reinterpret_cast<const uint2*>(d.x + (((size_t)n * d.H + h) * d.W + v) * d.C + c));
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      a[0] = fmaf(g[u], elem16(t[u].x & 0xffffu, is_bf16), a[0]);
+      a[1] = fmaf(g[u], elem16(t[u].x >> 16, is_bf16), a[1]);
+      a[2] = fmaf(g[u], elem16(t[u].y & 0xffffu, is_bf16), a[2]);
+      a[3] = fmaf(g[u], elem16(t[u].y >> 16, is_bf16), a[3]);
+    }
+    if ((!isnan(sum.x) || isnan(a[0])) && (!isnan(sum.y) || isnan(a[1])) && (!isnan(sum.z) || isnan(a[2])) && (!isnan(sum.w) || isnan(a[3])))
+      done[quad] = 1;
+  }
+  part[threadIdx.x] = make_float4(a[0], a[1], a[2], a[3]);
+  __syncthreads();
+  if (active && group == 0) {
+    float4 r = part[quad];
+    for (int s = 1; s < groups; ++s) { const float4 v = part[(s << bits) + quad]; r.x += v.x; r.y += v.y; r.z += v.z; r.w += v.w; }
+    store4_16(out, i / 4, make_float4(isnan(sum.x) ? r.x : sum.x, isnan(sum.y) ? r.y : sum.y, isnan(sum.z) ? r.z : sum.z, isnan(sum.w) ? r.w : sum.w), is_bf16);
+  }
+}
+
 // Adds the slabs and converts: a block covers 32 float4 columns x 8 slices of the slabs (eight independent 16-byte
-// loads in flight per thread); the slices meet in shared memory.
+// loads in flight per thread); the slices meet in shared memory. Sums that are NaN go to wgrad_direct, all warps of the block together.
 __global__ void __launch_bounds__(256)
-conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, void* __restrict__ out, int is_bf16) {
+conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, void* __restrict__ out, int is_bf16, const __grid_constant__ WgradDirect direct) {
   __shared__ float4 part[8][32];
   griddep_launch();
   griddep_wait();
@@ -261,18 +336,17 @@ conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, vo
   }
   part[slice][lane4] = a;
   __syncthreads();
+  bool nan = false;
   if (slice == 0 && i4 * 4 < elems) {
 #pragma unroll
     for (int s = 1; s < 8; ++s) { const float4 v = part[s][lane4]; a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; }
-    uint2 w;
-    if (is_bf16) {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
-      w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
-    } else {
-      __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(a.z, a.w);
-      w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
-    }
-    reinterpret_cast<uint2*>(out)[i4] = w;
+    store4_16(out, i4, a, is_bf16);
+    nan = isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(a.w);
+  }
+  if (direct.x && __syncthreads_or(nan)) {
+    if (slice == 0) part[0][lane4] = a;
+    __syncthreads();
+    wgrad_direct(direct, &part[0][0], blockIdx.x * 128, elems, out, is_bf16);
   }
 }
 
@@ -280,7 +354,6 @@ conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, vo
 struct WgradPhase {
   int a_h, a_w;              // first pixel of the phase
   int lo_h, hi_h, lo_w, hi_w;  // smallest and largest o of its taps
-  int taps;
 };
 
 struct WgradShape {
@@ -354,12 +427,11 @@ bool wgrad_shape(const HaloConv& c, WgradShape* s) {
     while (f < s->nphases && (s->phase[f].a_h != ah || s->phase[f].a_w != aw)) ++f;
     if (f == s->nphases) {
       if (f == kWgMaxPhases) return false;
-      s->phase[s->nphases++] = {ah, aw, oh, oh, ow, ow, 0};
+      s->phase[s->nphases++] = {ah, aw, oh, oh, ow, ow};
     }
     WgradPhase& q = s->phase[f];
     q.lo_h = std::min(q.lo_h, oh); q.hi_h = std::max(q.hi_h, oh);
     q.lo_w = std::min(q.lo_w, ow); q.hi_w = std::max(q.hi_w, ow);
-    ++q.taps;
   }
   int n = 0, more_w = 0, more_h = 0;
   for (int f = 0; f < s->nphases; ++f) {
@@ -455,7 +527,7 @@ RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* o
 
   WgradParams p;
   memset(&p, 0, sizeof(p));
-  p.Kout = c.Kout; p.cchunks = s.cchunks; p.kchunks = s.kchunks; p.yxc = c.Y * c.X * c.C;
+  p.Kout = c.Kout; p.kchunks = s.kchunks; p.yxc = c.Y * c.X * c.C;
   p.Wp = s.Wp; p.R = s.R; p.ksteps = s.ksteps;
   p.tiles_per_img = (c.P + s.R - 1) / s.R;
   p.num_tiles = c.N * p.tiles_per_img;
@@ -509,7 +581,13 @@ RbStatus conv_wgrad_halo_run(const HaloConv& c, const void* image, const void* o
   RB_CUDA_TRY(launch_after(conv_wgrad_halo_kernel, grid, kWgThreads, smem, stream, 1, maps, p));
   count_launch();
   const int elems = c.Kout * p.yxc;
-  RB_CUDA_TRY(launch_after(conv_wgrad_sum_kernel, (elems / 4 + 31) / 32, 256, 0, stream, 1, p.slabs, grid / s.groups, elems, filter_grad, c.is_bf16));
+  WgradDirect d;
+  d.x = c.stride_h > 1 || c.stride_w > 1 ? static_cast<const uint16_t*>(image) : nullptr;
+  d.dy = static_cast<const uint16_t*>(out_grad);
+  d.H = c.H; d.W = c.W; d.C = c.C; d.P = c.P; d.Q = c.Q; d.Kout = c.Kout; d.X = c.X; d.yxc = p.yxc;
+  d.stride_h = c.stride_h; d.stride_w = c.stride_w; d.dil_h = c.dil_h; d.dil_w = c.dil_w; d.pad_h = c.pad_h; d.pad_w = c.pad_w;
+  d.pixels = c.N * c.P * c.Q;
+  RB_CUDA_TRY(launch_after(conv_wgrad_sum_kernel, (elems / 4 + 31) / 32, 256, 0, stream, 1, p.slabs, grid / s.groups, elems, filter_grad, c.is_bf16, d));
   count_launch();
   return RB_SUCCESS;
 }
