@@ -250,14 +250,16 @@ __global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p
     fits = fits && x < 255;
     e[o] = x == 0 ? 0 : 140 - x;                     // 2^e * m lies in [2^13, 2^14)
     fits = fits && e[o] <= 126 && e[o] >= -126;
-    // values that will not fit, seen here already
+    // values that will not fit, seen here already: two in a run, or one below the least
     const float scale = e[o] <= 126 && e[o] >= -126 ? __uint_as_float((uint32_t)(127 + e[o]) << 23) : 1.0f;
-    bool low = false;
+    float least = kHalfFull;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float y = v[o][i] * scale;
-      const int below = __popc(__ballot_sync(0xffffffffu, v[o][i] != 0.0f && y < kHalfFull));
-      low = low || below > 1 || __any_sync(0xffffffffu, v[o][i] != 0.0f && y < kHalfLeast);
+    for (int i = 0; i < 16; ++i) least = fminf(least, v[o][i] != 0.0f ? v[o][i] * scale : kHalfFull);
+    bool low = false;
+    if (__any_sync(0xffffffffu, least < kHalfFull)) {
+      low = __any_sync(0xffffffffu, least < kHalfLeast);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) low = low || __popc(__ballot_sync(0xffffffffu, v[o][i] != 0.0f && v[o][i] * scale < kHalfFull)) > 1;
     }
     if (low && lane == 0) low_runs = 1;
   }
@@ -290,19 +292,30 @@ struct HalvesJobs {
   long long first[3];
   HalvesState* state;
 };
-// Whether the value at (r, c) of a source of R x C, below kHalfFull, may stay in f16 planes (see above).
-__device__ __noinline__ bool low_value_fits(const float* s, int R, int C, int r, int c, float scale) {
-  if (fabsf(s[(long long)r * C + c] * scale) < kHalfLeast) return false;
-  int in_row = 0, in_col = 0;
+// Whether the values below kHalfFull among a thread's sixteen (rows r, r + 16, ..., columns c ... c + 3 of a source of R x C) may stay in f16
+// planes (see above); lows counts those of the block.
+__device__ __noinline__ bool low_values_fit(const float* s, int R, int C, int r, int c, float scale, int* lows) {
+  bool fit = true;
 #pragma unroll 1
-  for (int i = 0; i < 64; ++i) {
-    const int rr = (r & ~63) + i, cc = (c & ~63) + i;
-    in_row += cc < C && s[(long long)r * C + cc] != 0.0f ? 1 : 0;
-    in_col += rr < R && s[(long long)rr * C + c] != 0.0f ? 1 : 0;
+  for (int e = 0; e < 16 && fit; ++e) {
+    const int rr = r + 16 * (e >> 2), cc = c + (e & 3);
+    if (rr >= R || cc >= C) continue;
+    const float v = s[(long long)rr * C + cc], y = fabsf(v * scale);
+    if (v == 0.0f || y >= kHalfFull) continue;
+    fit = y >= kHalfLeast && atomicAdd(lows, 1) == 0;
+    if (!fit) break;
+    int in_row = 0, in_col = 0;
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i) {
+      const int ri = (rr & ~63) + i, ci = (cc & ~63) + i;
+      in_row += ci < C && s[(long long)rr * C + ci] != 0.0f ? 1 : 0;
+      in_col += ri < R && s[(long long)ri * C + cc] != 0.0f ? 1 : 0;
+    }
+    fit = in_row >= 4 && in_col >= 4;
   }
-  return in_row >= 4 && in_col >= 4;
+  return fit;
 }
-__global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
+__global__ void __launch_bounds__(256, 5) f32_halves_kernel(const HalvesJobs p) {
   __shared__ float tile[64][65];
   __shared__ int lows;      // values below kHalfFull
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
@@ -347,16 +360,12 @@ __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
         for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
       }
     }
-    uint32_t low = 0;   // (a lane's sixteen values)
+    bool low = false;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const float v = x[i >> 2][i & 3], y = fabsf(v * scale);
       bad = bad || !(y < 65504.0f);
-      if (y < kHalfFull && v != 0.0f) low |= 1u << i;
-    }
-    if (low && !bad) {
-      const int i = __ffs(low) - 1;
-      bad = (low & (low - 1)) != 0 || atomicAdd(&lows, 1) != 0 || !low_value_fits(s, j.R, j.C, r0 + ty + 16 * (i >> 2), c0 + tx * 4 + (i & 3), scale);
+      low = low || (y < kHalfFull && v != 0.0f);
     }
     if (!j.transpose) {
 #pragma unroll
@@ -380,6 +389,7 @@ __global__ void __launch_bounds__(256) f32_halves_kernel(const HalvesJobs p) {
       }
       __syncthreads();
     }
+    if (low && !bad) bad = !low_values_fit(s, j.R, j.C, r0 + ty, c0 + tx * 4, scale, &lows);
   }
   if (__syncthreads_or(bad ? 1 : 0) && threadIdx.x == 0) p.state->flag = 1u;
 }
