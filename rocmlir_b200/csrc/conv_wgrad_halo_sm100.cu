@@ -275,12 +275,12 @@ __device__ __noinline__ void wgrad_direct(const WgradDirect& d, float4* part, in
   __syncthreads();   // and part may be written again
   float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int pix0 = group; active && pix0 < d.pixels; pix0 += 8 * groups) {
+  for (int pix0 = group; active && pix0 < d.pixels; pix0 += 4 * groups) {
     if (reinterpret_cast<volatile int*>(done)[quad]) break;
-    float g[8];
-    uint2 t[8];
+    float g[4];
+    uint2 t[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < 4; ++u) {
       const int pix = pix0 + u * groups;
       const int row = pix / d.Q, q = pix - row * d.Q, n = row / d.P;
       const int h = (row - n * d.P) * d.stride_h - d.pad_h + y * d.dil_h, v = q * d.stride_w - d.pad_w + x * d.dil_w;
@@ -290,7 +290,7 @@ __device__ __noinline__ void wgrad_direct(const WgradDirect& d, float4* part, in
       if (there && h >= 0 && h < d.H && v >= 0 && v < d.W) t[u] = __ldg(reinterpret_cast<const uint2*>(d.x + (((size_t)n * d.H + h) * d.W + v) * d.C + c));
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < 4; ++u) {
       a[0] = fmaf(g[u], elem16(t[u].x & 0xffffu, is_bf16), a[0]);
       a[1] = fmaf(g[u], elem16(t[u].x >> 16, is_bf16), a[1]);
       a[2] = fmaf(g[u], elem16(t[u].y & 0xffffu, is_bf16), a[2]);
@@ -309,8 +309,9 @@ __device__ __noinline__ void wgrad_direct(const WgradDirect& d, float4* part, in
 }
 
 // Adds the slabs and converts: a block covers 32 float4 columns x 8 slices of the slabs (eight independent 16-byte
-// loads in flight per thread); the slices meet in shared memory. Sums that are NaN go to wgrad_direct, all warps of the block together.
-__global__ void __launch_bounds__(256)
+// loads in flight per thread); the slices meet in shared memory. Sums that are NaN go to wgrad_direct, all warps of the block together;
+// its registers may not cost the others a block of six (N = 32, 128 -> 128, 28x28, unit stride 20.9 -> 22.0 us a call with three).
+__global__ void __launch_bounds__(256, 6)
 conv_wgrad_sum_kernel(const float* __restrict__ slabs, int nslabs, int elems, void* __restrict__ out, int is_bf16, const __grid_constant__ WgradDirect direct) {
   __shared__ float4 part[8][32];
   griddep_launch();
