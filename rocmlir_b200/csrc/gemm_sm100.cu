@@ -185,15 +185,14 @@ F32Job f32_job(const float* src, float* hi, float* lo, int R, int C, int pitch, 
   j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
   return j;
 }
-void launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream, const unsigned int* gate = nullptr) {
+RbStatus launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream, const unsigned int* gate = nullptr) {
   jobs.first[0] = 0;
   for (int i = 0; i < 2; ++i)
     jobs.first[i + 1] = jobs.first[i] + (i < count ? groups * (long long)jobs.job[i].tiles_x * jobs.job[i].tiles_y : 0);
   const unsigned grid = (unsigned)std::min<long long>(jobs.first[2], (long long)sms * (gate ? 8 : 32));   // (one wave of blocks that may have to end at once)
-  // a pass that will most likely have nothing to do is set up early (64 images 128 -> 128, 28x28, 3x3 f32 96 us a call -> 89); see launch.cuh for the others
-  if (gate) launch_after(f32_prepare_kernel, grid, 256, 0, stream, 1, jobs, gate);   // (an error stays for the launch of the product)
-  else f32_prepare_kernel<<<grid, 256, 0, stream>>>(jobs, gate);
+  RB_CUDA_TRY(launch_after(f32_prepare_kernel, grid, 256, 0, stream, 1, jobs, gate));
   count_launch();
+  return RB_SUCCESS;
 }
 
 // ---- f32 operands as f16 planes (see kMaxPlanes) -----------------------------------------------------------------------------
@@ -808,9 +807,7 @@ RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int 
   F32Jobs jobs;
   memset(&jobs, 0, sizeof(jobs));
   jobs.job[0] = f32_job(src, hi, split ? lo : nullptr, R, C, pitch, transpose);
-  launch_f32_jobs(jobs, 1, groups, dev->sm_count, stream);
-  RB_CUDA_TRY(cudaGetLastError());
-  return RB_SUCCESS;
+  return launch_f32_jobs(jobs, 1, groups, dev->sm_count, stream);
 }
 
 extern "C" RbStatus rbGemmGetConfig(const RbGemmProblem* p, RbGemmConfigInfo* out) { return rb::gemm_config(p, -1, out); }
@@ -1083,9 +1080,11 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
       memset(&image, 0, sizeof(image));
       image.job[0] = f32_job(conva->src, static_cast<float*>(const_cast<void*>(conva->tensor)), static_cast<float*>(const_cast<void*>(conva->tensor_lo)),
                              conva->src_rows, conva->src_cols, conva->C, conva->src_transpose);
-      launch_f32_jobs(image, 1, conva->src_groups, dev->sm_count, stream, halves ? &state->flag : nullptr);
+      st = launch_f32_jobs(image, 1, conva->src_groups, dev->sm_count, stream, halves ? &state->flag : nullptr);
+      if (st != RB_SUCCESS) return st;
     }
-    if (nj > 0) launch_f32_jobs(jobs, nj, p->g, dev->sm_count, stream, halves ? &state->flag : nullptr);
+    if (nj > 0) st = launch_f32_jobs(jobs, nj, p->g, dev->sm_count, stream, halves ? &state->flag : nullptr);
+    if (st != RB_SUCCESS) return st;
   } else {
     PadJobs pj;
     memset(&pj, 0, sizeof(pj));
@@ -1195,7 +1194,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.tiles_n = (p->n + bn - 1) / bn;
   kp.kblocks = (p->k + bke - 1) / bke;
   kp.planes = planes;
-  kp.a_short = planes * (kBM - a_box) * (int)kRowBytes;
+  kp.stage_tx = (ctas == 2 ? GemmSmemLayout<2>::stage_bytes(bn, planes) : GemmSmemLayout<1>::stage_bytes(bn, planes)) - planes * (kBM - a_box) * (int)kRowBytes;
   const uint32_t fmt_op = half ? 0u : fmt;
   kp.idesc = make_idesc(cfmt, fmt_op, fmt_b == 0xffffffffu ? fmt_op : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
   kp.acc_is_int = is_int ? 1 : 0;
@@ -1255,6 +1254,19 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
   kp.probe = kProbeBuild ? (t_variant >> 24) & 7 : 0;
   kp.wait_cycles = t_wait_cycles;
   if (t_stall_launches > 0) { kp.stall = 1; t_stall_launches -= form; }
+  // Set up early, a successor overlaps its launch with this kernel's tail; between launches of a stream the early start itself costs 0.4 to 0.8 us, which
+  // is not always won back. us a call in a stream, early and not: 1791 x 1024 x 2944 i8 13.6 / 13.8, 2048^3 f16 19.2 / 19.7, 13 images 512 -> 128, 35x35,
+  // pointwise, stride 2, 8.4 / 9.0. Not where
+  // * the call has other launches, small blocks that wait beside the CTAs at work (300 x 700 x 4096, K in ranges, 15.5 / 15.2, 64 x 246 x 2019 f32
+  //   19.6 / 18.6, 543 x 768 x 365 x 3, rows copied, 12.9 / 11.8, 3 x 1024 x 1024 x 769 14.7 / 14.3) - but the launch of the form that is not taken;
+  // * few rows draw a large B, which is what bounds them (45 x 6080 x 3392 fp8 12.4 / 11.9, 256 x 4096 x 4096 i8 13.9 / 13.4, 66 x 4336 x 1920 fp8 still
+  //   8.9 / 9.3);
+  // * single CTAs work on several short tiles each, the next tile's loads under way behind a tile's stores (171 images 64 -> 256, 44x44, input gradient,
+  //   47.1 / 45.7, 148 images 64 -> 128, 45x45, input gradient, 32.6 / 31.9, 21 images 512 -> 64, 39x39 10.7 / 10.2; ten K blocks gain, 755 x 6416 x 1280 i8
+  //   17.2 / 17.5, and so do pairs, 10 images 256 -> 512, 55x55, 19.4 / 20.0).
+  const bool streams_b = p->m <= 3 * kBM && (double)p->n * p->k * es >= 12e6;
+  const bool several = ctas == 1 && kp.kblocks <= 8 && (long long)p->g * kp.tiles_m * kp.tiles_n > dev->sm_count;
+  kp.early = halves || !(splits > 1 || oa.needs_copy || ob.needs_copy || streams_b || several) ? 1 : 0;
   if (halves) {
     kp.gate = &state->flag;
     kp.gate_want = half ? 0u : 1u;

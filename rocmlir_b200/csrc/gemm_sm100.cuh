@@ -121,7 +121,7 @@ struct GemmParams {
   unsigned int* sk_flags;      // [units][8]: one word per (CTA of the pair, epilogue warp), set to sk_token when written
   unsigned int sk_token;       // unique per launch, so stale words of earlier launches never match
   ConvAParams conva;
-  int a_short;                // bytes of a stage that are not loaded: rows that no row of a short A needs (one row tile, not a pair's)
+  int stage_tx;               // bytes of a stage that are loaded by one CTA: less than all of it where A is shorter than a tile
   int a_fused, b_fused;       // MN-major operand loaded with one 4-D box per stage (extent a multiple of the chunk)
   int probe;                  // instrumentation, only in builds with -DRB_ENABLE_PROBE (results become meaningless):
                               // bit0 = no loads, bit1 = no epilogue work, bit2 = epilogue without its global stores
@@ -143,6 +143,7 @@ struct GemmParams {
   unsigned int* chain_flags;
   unsigned int chain_token;
   int chain_flip;
+  int early;                  // the next kernel of the stream may be set up when a CTA has issued its last load, not only when it ends
   // A launch that may turn out not to be wanted: it ends at once unless *gate == gate_want. halves_scale: 2^-(s of A + s of B).
   const unsigned int* gate;
   unsigned int gate_want;
@@ -366,9 +367,9 @@ static __device__ __noinline__ void copy_staged_rows(const uint8_t* stg, uint8_t
 __device__ __forceinline__ void emit_staged(const EpiStoreCtx& c, const uint8_t* stg, int n0) {
   fence_proxy_async();
   __syncwarp();
-  if (c.lane == 0) {
-    if (c.row0 < c.M) tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
-    bulk_commit();   // without a store too: the waits count groups, and what they wait for may be a tile back
+  if (c.lane == 0) {   // (see store_map)
+    tma_store_3d(c.cmap, stg, n0, c.row0, c.gz);
+    bulk_commit();
   }
 }
 __device__ __forceinline__ void emit_staged(const EpiCopyCtx& c, const uint8_t* stg, int n0) {
@@ -669,7 +670,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           } else if (probe & 1) {
             if (CTAS == 1 || rank == 0) mbar_arrive(&full_bar[s]);
           } else if constexpr (CTAS == 1) {
-            mbar_expect_tx(&full_bar[s], nblk * (stage_bytes - p.a_short));
+            mbar_expect_tx(&full_bar[s], nblk * p.stage_tx);
           } else {
             if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * nblk * stage_bytes);
           }
@@ -779,7 +780,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
           if (++s == (uint32_t)rounds) { s = 0; ph ^= 1u; }
         }
       }
-      griddep_launch();   // the last load is under way
+      if (p.early) griddep_launch();   // the last load is under way
       if (p.trace) p.trace[blockIdx.x * 16 + 1] = (unsigned long long)w_empty;
     }
   } else if (warp == 1) {
@@ -1036,12 +1037,14 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmTensorMaps maps, const GemmParam
       auto store_map = [&](const uint8_t* stg, int n0) {
         fence_proxy_async();
         __syncwarp();
+        // Rows beyond the last are clipped, all 32 of them too: a group must be committed for every staged row, because the waits count groups.
         if (lane == 0) {
-          if (row0 < p.M) {
-            if (kPlanes && p.c_add) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
-            else tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
+          if (kPlanes && p.c_add) {
+            if (row0 < p.M) tma_add_3d(&maps.c, stg, n0, (int)row0, gz);
+          } else {
+            tma_store_3d(&maps.c, stg, n0, (int)row0, gz);
           }
-          bulk_commit();   // without a store too: the waits count groups, and what they wait for may be a tile back
+          bulk_commit();
         }
       };
       if constexpr (COPY) {
