@@ -1120,255 +1120,255 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
 
   // f32 products that may run on f16 planes are launched in both forms; the operands' state says on the device which one works
   for (int form = halves ? 0 : 1; form < 2; ++form) {
-  const bool half = form == 0;
-  const size_t es_op = half ? 2 : es;                    // of the planes that this form reads
-  const int bke = (int)(kRowBytes / es_op);
-  GemmTensorMaps maps;
-  memset(&maps, 0, sizeof(maps));
-  CUtensorMapDataType dt = abt == RB_F16 || half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                           : abt == RB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                           : abt == RB_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                            : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  // An MN-major tile is 128-byte chunks of M/N x K rows; when the extent is a whole number of chunks the chunk
-  // index becomes a tensor dimension of its own and one 4-D box fetches the whole tile of a stage.
-  const bool a_fused = oa.mn_major && oa.cols % bke == 0 && oa.pitch == oa.cols;
-  const bool b_fused = ob.mn_major && ob.cols % bke == 0 && ob.pitch == ob.cols;
-  auto encode_operand = [&](CUtensorMap* m, const void* base, const OperandPlan& o, int box_rows_kmajor,
-                            std::string* err) {
-    const bool fused = (&o == &oa) ? a_fused : b_fused;
-    const int ci = (&o == &oa) ? 0 : 1;
-    const uint64_t pitch = (uint64_t)(half ? half_pitch : o.pitch) * es_op;
-    const uint64_t gstride = chain ? chain_stride[ci] : (uint64_t)o.rows * pitch;
-    if (chain) base = (chain_flip >> ci) & 1 ? chain_ptr[ci][1] : chain_ptr[ci][0];
-    if (fused) {
-      const uint64_t dims[4] = {(uint64_t)bke, (uint64_t)o.rows, (uint64_t)(o.cols / bke), (uint64_t)p->g};
-      const uint64_t strides[3] = {pitch, (uint64_t)kRowBytes, gstride};
-      const uint32_t box[4] = {(uint32_t)bke, (uint32_t)bke, (uint32_t)(box_rows_kmajor / bke), 1u};
-      return encode_tiled(m, dt, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
+    const bool half = form == 0;
+    const size_t es_op = half ? 2 : es;                    // of the planes that this form reads
+    const int bke = (int)(kRowBytes / es_op);
+    GemmTensorMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    CUtensorMapDataType dt = abt == RB_F16 || half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                             : abt == RB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                             : abt == RB_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                              : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    // An MN-major tile is 128-byte chunks of M/N x K rows; when the extent is a whole number of chunks the chunk
+    // index becomes a tensor dimension of its own and one 4-D box fetches the whole tile of a stage.
+    const bool a_fused = oa.mn_major && oa.cols % bke == 0 && oa.pitch == oa.cols;
+    const bool b_fused = ob.mn_major && ob.cols % bke == 0 && ob.pitch == ob.cols;
+    auto encode_operand = [&](CUtensorMap* m, const void* base, const OperandPlan& o, int box_rows_kmajor,
+                              std::string* err) {
+      const bool fused = (&o == &oa) ? a_fused : b_fused;
+      const int ci = (&o == &oa) ? 0 : 1;
+      const uint64_t pitch = (uint64_t)(half ? half_pitch : o.pitch) * es_op;
+      const uint64_t gstride = chain ? chain_stride[ci] : (uint64_t)o.rows * pitch;
+      if (chain) base = (chain_flip >> ci) & 1 ? chain_ptr[ci][1] : chain_ptr[ci][0];
+      if (fused) {
+        const uint64_t dims[4] = {(uint64_t)bke, (uint64_t)o.rows, (uint64_t)(o.cols / bke), (uint64_t)p->g};
+        const uint64_t strides[3] = {pitch, (uint64_t)kRowBytes, gstride};
+        const uint32_t box[4] = {(uint32_t)bke, (uint32_t)bke, (uint32_t)(box_rows_kmajor / bke), 1u};
+        return encode_tiled(m, dt, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
+      }
+      const uint64_t dims[3] = {(uint64_t)o.cols, (uint64_t)o.rows, (uint64_t)p->g};
+      const uint64_t strides[2] = {pitch, gstride};
+      // K-major: box = BKE k-elements x tile rows. MN-major: box = one 128-byte chunk of MN x BKE k-rows.
+      const uint32_t box[3] = {(uint32_t)bke, (uint32_t)(o.mn_major ? bke : box_rows_kmajor), 1u};
+      return encode_tiled(m, dt, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
+    };
+    std::string err;
+    const int planes = gemm_planes(p);   // [0] hi (or the operand itself), [1] lo
+    if (conva) {
+      const ConvAOperand& cv = *conva;
+      const int che = bke;                   // elements per 128-byte run of channels
+      if (cv.C % che != 0) return fail(RB_UNSUPPORTED, "implicit operand: channels must be a multiple of 128 bytes");
+      const long long pixels = (long long)cv.N * cv.P * cv.Q, taps = (long long)cv.Y * cv.X * cv.C;
+      if (conv_a ? (pixels != p->m || taps != p->k) : (pixels != p->k || taps != p->n))
+        return fail(RB_INVALID_PARAM, "implicit operand does not match the GEMM extents");
+      const uint64_t dims[4] = {(uint64_t)cv.C, (uint64_t)cv.W, (uint64_t)cv.H, (uint64_t)cv.N};
+      const uint64_t strides[3] = {(uint64_t)cv.C * es_op, (uint64_t)cv.W * cv.C * es_op, (uint64_t)cv.H * cv.W * cv.C * es_op};
+      // bounding box of the base pixel: from -pad to (extent - 1) + upper corner, so that stepping by the stride
+      // visits exactly P x Q positions (CUTLASS states the same rule for its fprop maps)
+      const int lower[2] = {-cv.pad_w, -cv.pad_h};
+      const int upper[2] = {cv.pad_w_hi - (cv.X - 1) * cv.dil_w, cv.pad_h_hi - (cv.Y - 1) * cv.dil_h};
+      const uint32_t trav[2] = {(uint32_t)cv.stride_w, (uint32_t)cv.stride_h};
+      // A: a tile is 128 pixels (rows) x one K block of channels. B: a chunk is one K block of pixels x 64 channels.
+      for (int sg = 0; sg < (conv_a ? planes : 1); ++sg) {
+        const void* plane = sg == 1 ? cv.tensor_lo : cv.tensor;
+        if (!encode_im2col_nhwc(conv_a ? &maps.a[sg] : &maps.b[0], dt, plane, dims, strides, lower, upper, (uint32_t)che,
+                                (uint32_t)(conv_a ? kBM : bke), trav, &err))
+          return fail(RB_UNSUPPORTED, "implicit operand (im2col): " + err);
+      }
     }
-    const uint64_t dims[3] = {(uint64_t)o.cols, (uint64_t)o.rows, (uint64_t)p->g};
-    const uint64_t strides[2] = {pitch, gstride};
-    // K-major: box = BKE k-elements x tile rows. MN-major: box = one 128-byte chunk of MN x BKE k-rows.
-    const uint32_t box[3] = {(uint32_t)bke, (uint32_t)(o.mn_major ? bke : box_rows_kmajor), 1u};
-    return encode_tiled(m, dt, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, err);
-  };
-  std::string err;
-  const int planes = gemm_planes(p);   // [0] hi (or the operand itself), [1] lo
-  if (conva) {
-    const ConvAOperand& cv = *conva;
-    const int che = bke;                   // elements per 128-byte run of channels
-    if (cv.C % che != 0) return fail(RB_UNSUPPORTED, "implicit operand: channels must be a multiple of 128 bytes");
-    const long long pixels = (long long)cv.N * cv.P * cv.Q, taps = (long long)cv.Y * cv.X * cv.C;
-    if (conv_a ? (pixels != p->m || taps != p->k) : (pixels != p->k || taps != p->n))
-      return fail(RB_INVALID_PARAM, "implicit operand does not match the GEMM extents");
-    const uint64_t dims[4] = {(uint64_t)cv.C, (uint64_t)cv.W, (uint64_t)cv.H, (uint64_t)cv.N};
-    const uint64_t strides[3] = {(uint64_t)cv.C * es_op, (uint64_t)cv.W * cv.C * es_op, (uint64_t)cv.H * cv.W * cv.C * es_op};
-    // bounding box of the base pixel: from -pad to (extent - 1) + upper corner, so that stepping by the stride
-    // visits exactly P x Q positions (CUTLASS states the same rule for its fprop maps)
-    const int lower[2] = {-cv.pad_w, -cv.pad_h};
-    const int upper[2] = {cv.pad_w_hi - (cv.X - 1) * cv.dil_w, cv.pad_h_hi - (cv.Y - 1) * cv.dil_h};
-    const uint32_t trav[2] = {(uint32_t)cv.stride_w, (uint32_t)cv.stride_h};
-    // A: a tile is 128 pixels (rows) x one K block of channels. B: a chunk is one K block of pixels x 64 channels.
-    for (int sg = 0; sg < (conv_a ? planes : 1); ++sg) {
-      const void* plane = sg == 1 ? cv.tensor_lo : cv.tensor;
-      if (!encode_im2col_nhwc(conv_a ? &maps.a[sg] : &maps.b[0], dt, plane, dims, strides, lower, upper, (uint32_t)che,
-                              (uint32_t)(conv_a ? kBM : bke), trav, &err))
-        return fail(RB_UNSUPPORTED, "implicit operand (im2col): " + err);
+    // An A of fewer rows than a tile: no others are asked for (what the stage then holds there goes into rows of the sum that nothing reads).
+    // Rows beyond the tensor cost a TMA load more than rows of it do - us a call, fp8, K = 1344: 42 x 6560 9.8 -> 8.8, 42 x 8192 10.7 -> 8.8, 128 rows
+    // 8.8 and 8.9 - where every CTA's tile has them; in the last row of tiles alone they are not seen.
+    const int a_box = ctas == 1 && !conv_a && !chain && !oa.mn_major && p->m < kBM ? (int)(p->m + 7) / 8 * 8 : kBM;
+    for (int s = 0; s < planes; ++s) {
+      if (!conv_a && !encode_operand(&maps.a[s], half ? a_half[s] : a_src[s], oa, a_box, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
+      if (!conv_b && !encode_operand(&maps.b[s], half ? b_half[s] : b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
     }
-  }
-  // An A of fewer rows than a tile: no others are asked for (what the stage then holds there goes into rows of the sum that nothing reads).
-  // Rows beyond the tensor cost a TMA load more than rows of it do - us a call, fp8, K = 1344: 42 x 6560 9.8 -> 8.8, 42 x 8192 10.7 -> 8.8, 128 rows
-  // 8.8 and 8.9 - where every CTA's tile has them; in the last row of tiles alone they are not seen.
-  const int a_box = ctas == 1 && !conv_a && !chain && !oa.mn_major && p->m < kBM ? (int)(p->m + 7) / 8 * 8 : kBM;
-  for (int s = 0; s < planes; ++s) {
-    if (!conv_a && !encode_operand(&maps.a[s], half ? a_half[s] : a_src[s], oa, a_box, &err)) return fail(RB_UNSUPPORTED, "A: " + err);
-    if (!conv_b && !encode_operand(&maps.b[s], half ? b_half[s] : b_src[s], ob, bn / ctas, &err)) return fail(RB_UNSUPPORTED, "B: " + err);
-  }
 
-  GemmParams kp;
-  memset(&kp, 0, sizeof(kp));
-  kp.G = p->g; kp.M = p->m; kp.N = p->n; kp.K = p->k;
-  kp.bn = bn;
-  kp.splits = splits;
-  kp.tiles_m = (p->m + kBM * ctas - 1) / (kBM * ctas);
-  kp.tiles_n = (p->n + bn - 1) / bn;
-  kp.kblocks = (p->k + bke - 1) / bke;
-  kp.planes = planes;
-  kp.stage_tx = (ctas == 2 ? GemmSmemLayout<2>::stage_bytes(bn, planes) : GemmSmemLayout<1>::stage_bytes(bn, planes)) - planes * (kBM - a_box) * (int)kRowBytes;
-  const uint32_t fmt_op = half ? 0u : fmt;
-  kp.idesc = make_idesc(cfmt, fmt_op, fmt_b == 0xffffffffu ? fmt_op : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
-  kp.acc_is_int = is_int ? 1 : 0;
-  if (splits > 1 && conva && conva->c_rows_per_img > 0)
-    return fail(RB_UNSUPPORTED, "a channel-major result cannot be combined with a K split");
-  if (splits > 1 && !add_ranges) {
-    // every K range writes raw accumulators into its own plane; the reduction applies the epilogue
-    kp.c = partial;
-    kp.c_type = is_int ? RB_I32 : RB_F32;
-    kp.c_stride_m = p->n; kp.c_stride_n = 1;
-    kp.c_stride_g = (long long)p->m * p->n;
-    kp.split_stride = (long long)p->g * p->m * p->n;
-    kp.vec_ok = (p->n % 4 == 0) ? 1 : 0;
-    kp.c_tma = cfg.plain_stores ? 0 : kp.vec_ok ? 1 : 2;   // planes are stored like a C of splits * g groups
-  } else {
-    kp.c = c;
-    kp.c_type = p->c_type;
-    if (p->trans_c) { kp.c_stride_m = 1; kp.c_stride_n = p->m; } else { kp.c_stride_m = p->n; kp.c_stride_n = 1; }
-    kp.c_stride_g = (long long)p->m * p->n;
-    if (chain)   // signed distance from group 0's result to group 1's, in elements
-      kp.c_stride_g = (reinterpret_cast<intptr_t>(chain->c2) - reinterpret_cast<intptr_t>(c)) / (intptr_t)es_c;
-    kp.vec_ok = (!p->trans_c && ((size_t)p->n * es_c) % 16 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0) ? 1 : 0;
-    // rows off 16-byte boundaries: staged like the others, copied out by the warps (us, element stores from the registers before): 3 x 640 x
-    // 2279, K = 768, bf16 with bias and ReLU 179 -> 30; 2000 x 3001 x 640 95 -> 29; 4096 x 4095 x 4096 f16 243 -> 149; f32 768 x 1043 x 3648
-    // 98 -> 64
-    // (and so is an 8-bit result in tiles of 64 columns: the box of the store map is a staged row, 128 of them)
-    kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok && bn * es_c >= (size_t)kRowBytes ? 1 : 2;
-    if (conva && conva->c_rows_per_img > 0) {   // NKHW result: strided element stores, coalesced along the pixels
-      kp.c_rows_per_img = conva->c_rows_per_img;
-      kp.c_img_stride = conva->c_img_stride;
-      kp.c_stride_m = 1;
-      kp.c_stride_n = conva->c_col_stride;
-      kp.vec_ok = 0;
-      kp.c_tma = 0;
+    GemmParams kp;
+    memset(&kp, 0, sizeof(kp));
+    kp.G = p->g; kp.M = p->m; kp.N = p->n; kp.K = p->k;
+    kp.bn = bn;
+    kp.splits = splits;
+    kp.tiles_m = (p->m + kBM * ctas - 1) / (kBM * ctas);
+    kp.tiles_n = (p->n + bn - 1) / bn;
+    kp.kblocks = (p->k + bke - 1) / bke;
+    kp.planes = planes;
+    kp.stage_tx = (ctas == 2 ? GemmSmemLayout<2>::stage_bytes(bn, planes) : GemmSmemLayout<1>::stage_bytes(bn, planes)) - planes * (kBM - a_box) * (int)kRowBytes;
+    const uint32_t fmt_op = half ? 0u : fmt;
+    kp.idesc = make_idesc(cfmt, fmt_op, fmt_b == 0xffffffffu ? fmt_op : fmt_b, a_mn ? 1u : 0u, b_mn ? 1u : 0u, (uint32_t)(kBM * ctas), (uint32_t)bn);
+    kp.acc_is_int = is_int ? 1 : 0;
+    if (splits > 1 && conva && conva->c_rows_per_img > 0)
+      return fail(RB_UNSUPPORTED, "a channel-major result cannot be combined with a K split");
+    if (splits > 1 && !add_ranges) {
+      // every K range writes raw accumulators into its own plane; the reduction applies the epilogue
+      kp.c = partial;
+      kp.c_type = is_int ? RB_I32 : RB_F32;
+      kp.c_stride_m = p->n; kp.c_stride_n = 1;
+      kp.c_stride_g = (long long)p->m * p->n;
+      kp.split_stride = (long long)p->g * p->m * p->n;
+      kp.vec_ok = (p->n % 4 == 0) ? 1 : 0;
+      kp.c_tma = cfg.plain_stores ? 0 : kp.vec_ok ? 1 : 2;   // planes are stored like a C of splits * g groups
+    } else {
+      kp.c = c;
+      kp.c_type = p->c_type;
+      if (p->trans_c) { kp.c_stride_m = 1; kp.c_stride_n = p->m; } else { kp.c_stride_m = p->n; kp.c_stride_n = 1; }
+      kp.c_stride_g = (long long)p->m * p->n;
+      if (chain)   // signed distance from group 0's result to group 1's, in elements
+        kp.c_stride_g = (reinterpret_cast<intptr_t>(chain->c2) - reinterpret_cast<intptr_t>(c)) / (intptr_t)es_c;
+      kp.vec_ok = (!p->trans_c && ((size_t)p->n * es_c) % 16 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0) ? 1 : 0;
+      // rows off 16-byte boundaries: staged like the others, copied out by the warps (us, element stores from the registers before): 3 x 640 x
+      // 2279, K = 768, bf16 with bias and ReLU 179 -> 30; 2000 x 3001 x 640 95 -> 29; 4096 x 4095 x 4096 f16 243 -> 149; f32 768 x 1043 x 3648
+      // 98 -> 64
+      // (and so is an 8-bit result in tiles of 64 columns: the box of the store map is a staged row, 128 of them)
+      kp.c_tma = cfg.plain_stores || p->trans_c ? 0 : kp.vec_ok && bn * es_c >= (size_t)kRowBytes ? 1 : 2;
+      if (conva && conva->c_rows_per_img > 0) {   // NKHW result: strided element stores, coalesced along the pixels
+        kp.c_rows_per_img = conva->c_rows_per_img;
+        kp.c_img_stride = conva->c_img_stride;
+        kp.c_stride_m = 1;
+        kp.c_stride_n = conva->c_col_stride;
+        kp.vec_ok = 0;
+        kp.c_tma = 0;
+      }
+      kp.epi = ep;
     }
-    kp.epi = ep;
-  }
-  if (kp.c_tma == 1) {
-    const int st_type = kp.c_type;                      // what the kernel stores: C's type, or raw planes
-    const size_t es_st = dtype_bytes(st_type);
-    const CUtensorMapDataType cdt = st_type == RB_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                    : st_type == RB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                                    : st_type == RB_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                    : st_type == RB_I32  ? CU_TENSOR_MAP_DATA_TYPE_INT32
-                                                         : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    const uint64_t cdims[3] = {(uint64_t)p->n, (uint64_t)p->m, (uint64_t)p->g * (add_ranges ? 1 : splits)};
-    const uint64_t cstrides[2] = {(uint64_t)p->n * es_st, chain ? chain_stride[2] : (uint64_t)p->m * p->n * es_st};
-    const uint32_t cbox[3] = {(uint32_t)(kRowBytes / es_st), 32u, 1u};
-    void* cbase = (chain && (chain_flip & 4)) ? chain->c2 : kp.c;
-    if (!encode_tiled(&maps.c, cdt, 3, cbase, cdims, cstrides, cbox, CU_TENSOR_MAP_SWIZZLE_128B, &err))
-      return fail(RB_UNSUPPORTED, "C: " + err);
-  }
-  kp.c_add = add_ranges ? 1 : 0;
-  kp.status = dev->status_word;
-  kp.stages = stages;
-  kp.kpr = cfg.kpr;
-  kp.probe = kProbeBuild ? (t_variant >> 24) & 7 : 0;
-  kp.wait_cycles = t_wait_cycles;
-  if (t_stall_launches > 0) { kp.stall = 1; t_stall_launches -= form; }
-  // Set up early, a successor overlaps its launch with this kernel's tail; between launches of a stream the early start itself costs 0.4 to 0.8 us, which
-  // is not always won back. us a call in a stream, early and not: 1791 x 1024 x 2944 i8 13.6 / 13.8, 2048^3 f16 19.2 / 19.7, 13 images 512 -> 128, 35x35,
-  // pointwise, stride 2, 8.4 / 9.0. Not where
-  // * the call has other launches, small blocks that wait beside the CTAs at work (300 x 700 x 4096, K in ranges, 15.5 / 15.2, 64 x 246 x 2019 f32
-  //   19.6 / 18.6, 543 x 768 x 365 x 3, rows copied, 12.9 / 11.8, 3 x 1024 x 1024 x 769 14.7 / 14.3) - but the launch of the form that is not taken;
-  // * few rows draw a large B, which is what bounds them (45 x 6080 x 3392 fp8 12.4 / 11.9, 256 x 4096 x 4096 i8 13.9 / 13.4, 66 x 4336 x 1920 fp8 still
-  //   8.9 / 9.3);
-  // * single CTAs work on several short tiles each, the next tile's loads under way behind a tile's stores (171 images 64 -> 256, 44x44, input gradient,
-  //   47.1 / 45.7, 148 images 64 -> 128, 45x45, input gradient, 32.6 / 31.9, 21 images 512 -> 64, 39x39 10.7 / 10.2; ten K blocks gain, 755 x 6416 x 1280 i8
-  //   17.2 / 17.5, and so do pairs, 10 images 256 -> 512, 55x55, 19.4 / 20.0).
-  const bool streams_b = p->m <= 3 * kBM && (double)p->n * p->k * es >= 12e6;
-  const bool several = ctas == 1 && kp.kblocks <= 8 && (long long)p->g * kp.tiles_m * kp.tiles_n > dev->sm_count;
-  kp.early = halves || !(splits > 1 || oa.needs_copy || ob.needs_copy || streams_b || several) ? 1 : 0;
-  if (halves) {
-    kp.gate = &state->flag;
-    kp.gate_want = half ? 0u : 1u;
-    kp.halves_scale = &state->out_scale;
-  }
-  if (conva) {
-    kp.conva.enabled = conv_a ? 1 : 2; kp.conva.P = conva->P; kp.conva.Q = conva->Q; kp.conva.X = conva->X;
-    kp.conva.cchunks = conva->C / bke;
-    kp.conva.stride_h = conva->stride_h; kp.conva.stride_w = conva->stride_w;
-    kp.conva.dil_h = conva->dil_h; kp.conva.dil_w = conva->dil_w; kp.conva.pad_h = conva->pad_h; kp.conva.pad_w = conva->pad_w;
-  }
-  kp.a_fused = a_fused ? 1 : 0;
-  kp.b_fused = b_fused ? 1 : 0;
+    if (kp.c_tma == 1) {
+      const int st_type = kp.c_type;                      // what the kernel stores: C's type, or raw planes
+      const size_t es_st = dtype_bytes(st_type);
+      const CUtensorMapDataType cdt = st_type == RB_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                      : st_type == RB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                      : st_type == RB_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                      : st_type == RB_I32  ? CU_TENSOR_MAP_DATA_TYPE_INT32
+                                                           : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+      const uint64_t cdims[3] = {(uint64_t)p->n, (uint64_t)p->m, (uint64_t)p->g * (add_ranges ? 1 : splits)};
+      const uint64_t cstrides[2] = {(uint64_t)p->n * es_st, chain ? chain_stride[2] : (uint64_t)p->m * p->n * es_st};
+      const uint32_t cbox[3] = {(uint32_t)(kRowBytes / es_st), 32u, 1u};
+      void* cbase = (chain && (chain_flip & 4)) ? chain->c2 : kp.c;
+      if (!encode_tiled(&maps.c, cdt, 3, cbase, cdims, cstrides, cbox, CU_TENSOR_MAP_SWIZZLE_128B, &err))
+        return fail(RB_UNSUPPORTED, "C: " + err);
+    }
+    kp.c_add = add_ranges ? 1 : 0;
+    kp.status = dev->status_word;
+    kp.stages = stages;
+    kp.kpr = cfg.kpr;
+    kp.probe = kProbeBuild ? (t_variant >> 24) & 7 : 0;
+    kp.wait_cycles = t_wait_cycles;
+    if (t_stall_launches > 0) { kp.stall = 1; t_stall_launches -= form; }
+    // Set up early, a successor overlaps its launch with this kernel's tail; between launches of a stream the early start itself costs 0.4 to 0.8 us, which
+    // is not always won back. us a call in a stream, early and not: 1791 x 1024 x 2944 i8 13.6 / 13.8, 2048^3 f16 19.2 / 19.7, 13 images 512 -> 128, 35x35,
+    // pointwise, stride 2, 8.4 / 9.0. Not where
+    // * the call has other launches, small blocks that wait beside the CTAs at work (300 x 700 x 4096, K in ranges, 15.5 / 15.2, 64 x 246 x 2019 f32
+    //   19.6 / 18.6, 543 x 768 x 365 x 3, rows copied, 12.9 / 11.8, 3 x 1024 x 1024 x 769 14.7 / 14.3) - but the launch of the form that is not taken;
+    // * few rows draw a large B, which is what bounds them (45 x 6080 x 3392 fp8 12.4 / 11.9, 256 x 4096 x 4096 i8 13.9 / 13.4, 66 x 4336 x 1920 fp8 still
+    //   8.9 / 9.3);
+    // * single CTAs work on several short tiles each, the next tile's loads under way behind a tile's stores (171 images 64 -> 256, 44x44, input gradient,
+    //   47.1 / 45.7, 148 images 64 -> 128, 45x45, input gradient, 32.6 / 31.9, 21 images 512 -> 64, 39x39 10.7 / 10.2; ten K blocks gain, 755 x 6416 x 1280 i8
+    //   17.2 / 17.5, and so do pairs, 10 images 256 -> 512, 55x55, 19.4 / 20.0).
+    const bool streams_b = p->m <= 3 * kBM && (double)p->n * p->k * es >= 12e6;
+    const bool several = ctas == 1 && kp.kblocks <= 8 && (long long)p->g * kp.tiles_m * kp.tiles_n > dev->sm_count;
+    kp.early = halves || !(splits > 1 || oa.needs_copy || ob.needs_copy || streams_b || several) ? 1 : 0;
+    if (halves) {
+      kp.gate = &state->flag;
+      kp.gate_want = half ? 0u : 1u;
+      kp.halves_scale = &state->out_scale;
+    }
+    if (conva) {
+      kp.conva.enabled = conv_a ? 1 : 2; kp.conva.P = conva->P; kp.conva.Q = conva->Q; kp.conva.X = conva->X;
+      kp.conva.cchunks = conva->C / bke;
+      kp.conva.stride_h = conva->stride_h; kp.conva.stride_w = conva->stride_w;
+      kp.conva.dil_h = conva->dil_h; kp.conva.dil_w = conva->dil_w; kp.conva.pad_h = conva->pad_h; kp.conva.pad_w = conva->pad_w;
+    }
+    kp.a_fused = a_fused ? 1 : 0;
+    kp.b_fused = b_fused ? 1 : 0;
 
-  if (chain) {
-    if ((size_t)kp.tiles_m * kp.tiles_n * ctas * 4 * sizeof(unsigned int) > chain->flags_bytes)
-      return fail(RB_UNSUPPORTED, "chained launch: too many tiles for the flag words");
-    static std::atomic<unsigned int> next_chain_token{0xc4a10001u};
-    kp.chain_flags = chain->flags;
-    kp.chain_token = next_chain_token.fetch_add(1, std::memory_order_relaxed);
-    kp.chain_flip = chain_flip;
-  }
-  const long long num_tiles = (long long)kp.G * kp.tiles_m * kp.tiles_n;
-  const long long num_items = num_tiles * splits;
-  if (num_items > 0x7fffffffLL) return fail(RB_UNSUPPORTED, "too many tiles");
-  // the stream-K split was planned for a B200's SM count; on anything else every tile is computed whole
-  const bool use_sk = cfg.sk_tiles > 0 && dev->sm_count == planned_sms();
-  kp.dp_tiles = use_sk ? cfg.dp_tiles : (int)num_tiles;
-  kp.sk_tiles = use_sk ? cfg.sk_tiles : 0;
-  if (use_sk) {
-    kp.sk_partial = wsb + ws.sk_off;
-    kp.sk_flags = reinterpret_cast<unsigned int*>(wsb + ws.sk_flags_off);
-    static std::atomic<unsigned int> next_token{0x5eed0001u};
-    kp.sk_token = next_token.fetch_add(1, std::memory_order_relaxed);
-  }
+    if (chain) {
+      if ((size_t)kp.tiles_m * kp.tiles_n * ctas * 4 * sizeof(unsigned int) > chain->flags_bytes)
+        return fail(RB_UNSUPPORTED, "chained launch: too many tiles for the flag words");
+      static std::atomic<unsigned int> next_chain_token{0xc4a10001u};
+      kp.chain_flags = chain->flags;
+      kp.chain_token = next_chain_token.fetch_add(1, std::memory_order_relaxed);
+      kp.chain_flip = chain_flip;
+    }
+    const long long num_tiles = (long long)kp.G * kp.tiles_m * kp.tiles_n;
+    const long long num_items = num_tiles * splits;
+    if (num_items > 0x7fffffffLL) return fail(RB_UNSUPPORTED, "too many tiles");
+    // the stream-K split was planned for a B200's SM count; on anything else every tile is computed whole
+    const bool use_sk = cfg.sk_tiles > 0 && dev->sm_count == planned_sms();
+    kp.dp_tiles = use_sk ? cfg.dp_tiles : (int)num_tiles;
+    kp.sk_tiles = use_sk ? cfg.sk_tiles : 0;
+    if (use_sk) {
+      kp.sk_partial = wsb + ws.sk_off;
+      kp.sk_flags = reinterpret_cast<unsigned int*>(wsb + ws.sk_flags_off);
+      static std::atomic<unsigned int> next_token{0x5eed0001u};
+      kp.sk_token = next_token.fetch_add(1, std::memory_order_relaxed);
+    }
 
-  // fused elementwise code and copied rows only in launches that have such work (see GemmTail)
-  const int tail = kp.c_tma == 2 ? kTailCopied : kp.epi.flags != 0 ? kTailFused : kTailNone;
-  const GemmKernel kern = half                 ? gemm_kernel_halves(ctas, tail)
-                          : tail == kTailCopied  ? gemm_kernel_copied(kind, a_mn, b_mn, ctas)
-                          : tail == kTailFused ? gemm_kernel_fused(kind, a_mn, b_mn, ctas)
-                                               : gemm_kernel_plain(kind, a_mn, b_mn, ctas);
-  const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
-  const int smem = ctas == 2 ? GemmSmemLayout<2>::total(stages, bn, kernel_epi_vec, planes) : GemmSmemLayout<1>::total(stages, bn, kernel_epi_vec, planes);
-  {
-    const RbStatus sst = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    if (sst != RB_SUCCESS) return sst;
-  }
+    // fused elementwise code and copied rows only in launches that have such work (see GemmTail)
+    const int tail = kp.c_tma == 2 ? kTailCopied : kp.epi.flags != 0 ? kTailFused : kTailNone;
+    const GemmKernel kern = half                 ? gemm_kernel_halves(ctas, tail)
+                            : tail == kTailCopied  ? gemm_kernel_copied(kind, a_mn, b_mn, ctas)
+                            : tail == kTailFused ? gemm_kernel_fused(kind, a_mn, b_mn, ctas)
+                                                 : gemm_kernel_plain(kind, a_mn, b_mn, ctas);
+    const bool kernel_epi_vec = splits == 1 && epi_vec;  // with a K split the reduction kernel applies the epilogue
+    const int smem = ctas == 2 ? GemmSmemLayout<2>::total(stages, bn, kernel_epi_vec, planes) : GemmSmemLayout<1>::total(stages, bn, kernel_epi_vec, planes);
+    {
+      const RbStatus sst = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+      if (sst != RB_SUCCESS) return sst;
+    }
 
-  cudaLaunchConfig_t lc;
-  memset(&lc, 0, sizeof(lc));
-  lc.blockDim = dim3(kGemmThreads, 1, 1);
-  lc.dynamicSmemBytes = (size_t)smem;
-  lc.stream = stream;
-  cudaLaunchAttribute attr[2];
-  lc.attrs = attr;
-  attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
-  ++lc.numAttrs;
-  if (ctas == 2) {
-    attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[lc.numAttrs].val.clusterDim.x = 2; attr[lc.numAttrs].val.clusterDim.y = 1; attr[lc.numAttrs].val.clusterDim.z = 1;
+    cudaLaunchConfig_t lc;
+    memset(&lc, 0, sizeof(lc));
+    lc.blockDim = dim3(kGemmThreads, 1, 1);
+    lc.dynamicSmemBytes = (size_t)smem;
+    lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    lc.attrs = attr;
+    attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++lc.numAttrs;
-    const int pairs = dev->sm_count / 2;
-    lc.gridDim = dim3((unsigned)(2 * (int)std::min<long long>(num_items, pairs)), 1, 1);
-  } else {
-    lc.gridDim = dim3((unsigned)std::min<long long>(num_items, dev->sm_count), 1, 1);
-  }
-  if (capture) {
-    static_assert(sizeof(GemmTensorMaps) + sizeof(GemmParams) + 64 <= sizeof(capture->params), "parameter block too small");
-    memset(capture, 0, sizeof(*capture));
-    const std::string sym = kernel_symbol(kind, kind == kKindTF32 ? false : a_mn, kind == kKindTF32 ? false : b_mn, ctas, tail);
-    snprintf(capture->symbol, sizeof(capture->symbol), "%s", sym.c_str());
-    capture->grid = lc.gridDim.x;
-    capture->block = kGemmThreads;
-    capture->cluster = (uint32_t)ctas;
-    capture->dynamic_smem = (uint32_t)smem;
-    capture->param_count = 2;
-    capture->param_offset[0] = 0;
-    capture->param_size[0] = (uint32_t)sizeof(GemmTensorMaps);
-    capture->param_offset[1] = (uint32_t)((sizeof(GemmTensorMaps) + 63) / 64 * 64);
-    capture->param_size[1] = (uint32_t)sizeof(GemmParams);
-    kp.trace = nullptr;
-    memcpy(capture->params + capture->param_offset[0], &maps, sizeof(maps));
-    memcpy(capture->params + capture->param_offset[1], &kp, sizeof(kp));
-    return RB_SUCCESS;
-  }
-  kp.trace = trace_buffer((size_t)lc.gridDim.x * 16);
-  if (add_ranges && (half || !halves)) {
-    const long long n4 = (long long)p->g * p->m * p->n / 4;
-    cudaLaunchConfig_t zc;
-    memset(&zc, 0, sizeof(zc));
-    zc.gridDim = dim3((unsigned)std::min<long long>((n4 + 1023) / 1024, (long long)dev->sm_count * 4), 1, 1);
-    zc.blockDim = dim3(256, 1, 1);
-    zc.stream = stream;
-    zc.attrs = attr;   // (the first is the programmatic launch)
-    zc.numAttrs = 1;
-    RB_CUDA_TRY(cudaLaunchKernelEx(&zc, zero_kernel, static_cast<float4*>(c), n4));
+    if (ctas == 2) {
+      attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      attr[lc.numAttrs].val.clusterDim.x = 2; attr[lc.numAttrs].val.clusterDim.y = 1; attr[lc.numAttrs].val.clusterDim.z = 1;
+      ++lc.numAttrs;
+      const int pairs = dev->sm_count / 2;
+      lc.gridDim = dim3((unsigned)(2 * (int)std::min<long long>(num_items, pairs)), 1, 1);
+    } else {
+      lc.gridDim = dim3((unsigned)std::min<long long>(num_items, dev->sm_count), 1, 1);
+    }
+    if (capture) {
+      static_assert(sizeof(GemmTensorMaps) + sizeof(GemmParams) + 64 <= sizeof(capture->params), "parameter block too small");
+      memset(capture, 0, sizeof(*capture));
+      const std::string sym = kernel_symbol(kind, kind == kKindTF32 ? false : a_mn, kind == kKindTF32 ? false : b_mn, ctas, tail);
+      snprintf(capture->symbol, sizeof(capture->symbol), "%s", sym.c_str());
+      capture->grid = lc.gridDim.x;
+      capture->block = kGemmThreads;
+      capture->cluster = (uint32_t)ctas;
+      capture->dynamic_smem = (uint32_t)smem;
+      capture->param_count = 2;
+      capture->param_offset[0] = 0;
+      capture->param_size[0] = (uint32_t)sizeof(GemmTensorMaps);
+      capture->param_offset[1] = (uint32_t)((sizeof(GemmTensorMaps) + 63) / 64 * 64);
+      capture->param_size[1] = (uint32_t)sizeof(GemmParams);
+      kp.trace = nullptr;
+      memcpy(capture->params + capture->param_offset[0], &maps, sizeof(maps));
+      memcpy(capture->params + capture->param_offset[1], &kp, sizeof(kp));
+      return RB_SUCCESS;
+    }
+    kp.trace = trace_buffer((size_t)lc.gridDim.x * 16);
+    if (add_ranges && (half || !halves)) {
+      const long long n4 = (long long)p->g * p->m * p->n / 4;
+      cudaLaunchConfig_t zc;
+      memset(&zc, 0, sizeof(zc));
+      zc.gridDim = dim3((unsigned)std::min<long long>((n4 + 1023) / 1024, (long long)dev->sm_count * 4), 1, 1);
+      zc.blockDim = dim3(256, 1, 1);
+      zc.stream = stream;
+      zc.attrs = attr;   // (the first is the programmatic launch)
+      zc.numAttrs = 1;
+      RB_CUDA_TRY(cudaLaunchKernelEx(&zc, zero_kernel, static_cast<float4*>(c), n4));
+      count_launch();
+    }
+    RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
     count_launch();
-  }
-  RB_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, maps, kp));
-  count_launch();
   }
   if (splits > 1 && !add_ranges) {
     const long long total = (long long)p->g * p->m * p->n;
