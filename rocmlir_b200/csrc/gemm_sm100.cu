@@ -99,14 +99,79 @@ __device__ __forceinline__ float tf32_round(float x) {
 // Up to two operands per launch, dealt out in 64 x 64 tiles. Bound by one read and `planes` writes of the operand, so both
 // sides move 16 bytes per thread (the read element by element where the rows of the source do not allow it). Two operands of
 // 4096 x 4096: 61 us, 6.6 TB/s.
-struct F32Job {
+template <typename T>
+struct PlaneJob {
   const float* src;
-  float* hi;
-  float* lo;              // nullptr: one plane, the value itself
+  T* hi;
+  T* lo;                  // nullptr (f32 planes only): one plane, the value itself
   int R, C, pitch;        // src [G][R][C]; out [G][R][pitch], or with transpose [G][C][pitch]
   int transpose;
   int tiles_x, tiles_y;   // tiles of the output-padded extent along C and R
 };
+// The tiles of both jobs, a block per tile: seen() gets a thread's sixteen values as they lie, store() four neighbours along K of one row of the
+// planes at offset o, after() the tile's place when it is done.
+template <typename T, typename Seen, typename Store, typename After>
+__device__ __forceinline__ void plane_tiles(const PlaneJob<T>* jobs, const long long* first, Seen&& seen, Store&& store, After&& after) {
+  __shared__ float tile[64][65];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
+  for (long long t = blockIdx.x; t < first[2]; t += gridDim.x) {
+    const bool second = t >= first[1];
+    const PlaneJob<T> j = second ? jobs[1] : jobs[0];
+    const long long lt = t - (second ? first[1] : 0), per_g = (long long)j.tiles_x * j.tiles_y;
+    const long long g = lt / per_g;
+    const int rem = (int)(lt - g * per_g);
+    const int c0 = (rem % j.tiles_x) * 64, r0 = (rem / j.tiles_x) * 64;
+    const float* s = j.src + g * (long long)j.R * j.C;
+    const bool vec = j.C % 4 == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
+    float x[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // all four reads in flight
+      const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+      const float* q = s + (long long)r * j.C + c;
+      if (vec && r < j.R && c < j.C) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
+      }
+    }
+    seen(second, x);
+    if (!j.transpose) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
+        if (r < j.R && c < j.pitch) store(j, (g * j.R + r) * (long long)j.pitch + c, x[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tile[ty + 16 * i][tx * 4 + e] = x[i][e];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int oc = c0 + ty + 16 * i, orr = r0 + tx * 4;   // output row = source column, output column = source row
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
+        if (oc < j.C && orr < j.pitch) store(j, (g * j.C + oc) * (long long)j.pitch + orr, y);
+      }
+      __syncthreads();
+    }
+    after(j, s, r0 + ty, c0 + tx * 4);
+  }
+}
+// The grid covers the padded extent of whichever dimension becomes the output row (zeros past the source's extent).
+template <typename T>
+PlaneJob<T> plane_job(const float* src, T* hi, T* lo, int R, int C, int pitch, bool transpose) {
+  PlaneJob<T> j;
+  j.src = src; j.hi = hi; j.lo = lo; j.R = R; j.C = C; j.pitch = pitch; j.transpose = transpose ? 1 : 0;
+  j.tiles_x = ((transpose ? C : pitch) + 63) / 64;
+  j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
+  return j;
+}
+typedef PlaneJob<float> F32Job;
 struct F32Jobs {
   F32Job job[2];
   long long first[3];     // tiles before each job
@@ -126,64 +191,11 @@ __device__ __forceinline__ void store_planes4(const F32Job& j, long long o, cons
   }
 }
 __global__ void __launch_bounds__(256) f32_prepare_kernel(const F32Jobs p, const unsigned int* gate) {
-  __shared__ float tile[64][65];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();   // the product is set up meanwhile
   griddep_wait();
   if (gate && *reinterpret_cast<const volatile unsigned int*>(gate) == 0u) return;   // f16 planes will do
-  for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
-    const bool second = t >= p.first[1];
-    const F32Job j = second ? p.job[1] : p.job[0];
-    const long long lt = t - (second ? p.first[1] : 0), per_g = (long long)j.tiles_x * j.tiles_y;
-    const long long g = lt / per_g;
-    const int rem = (int)(lt - g * per_g);
-    const int c0 = (rem % j.tiles_x) * 64, r0 = (rem / j.tiles_x) * 64;
-    const float* s = j.src + g * (long long)j.R * j.C;
-    const bool vec = j.C % 4 == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
-    float x[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {   // all four reads in flight
-      const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
-      const float* q = s + (long long)r * j.C + c;
-      if (vec && r < j.R && c < j.C) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(q));
-        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
-      }
-    }
-    if (!j.transpose) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
-        if (r < j.R && c < j.pitch) store_planes4(j, (g * j.R + r) * (long long)j.pitch + c, x[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) tile[ty + 16 * i][tx * 4 + e] = x[i][e];
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int oc = c0 + ty + 16 * i, orr = r0 + tx * 4;   // output row = source column, output column = source row
-        float y[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
-        if (oc < j.C && orr < j.pitch) store_planes4(j, (g * j.C + oc) * (long long)j.pitch + orr, y);
-      }
-      __syncthreads();
-    }
-  }
-}
-// The grid covers the padded extent of whichever dimension becomes the output row (zeros past the source's extent).
-F32Job f32_job(const float* src, float* hi, float* lo, int R, int C, int pitch, bool transpose) {
-  F32Job j;
-  j.src = src; j.hi = hi; j.lo = lo; j.R = R; j.C = C; j.pitch = pitch; j.transpose = transpose ? 1 : 0;
-  j.tiles_x = ((transpose ? C : pitch) + 63) / 64;
-  j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
-  return j;
+  plane_tiles(p.job, p.first, [](bool, const float (*)[4]) {}, [](const F32Job& j, long long o, const float* x) { store_planes4(j, o, x); },
+              [](const F32Job&, const float*, int, int) {});
 }
 RbStatus launch_f32_jobs(F32Jobs& jobs, int count, long long groups, int sms, cudaStream_t stream, const unsigned int* gate = nullptr) {
   jobs.first[0] = 0;
@@ -278,14 +290,7 @@ __global__ void __launch_bounds__(1024) halves_scale_kernel(const HalvesSample p
 // one value in 3e7 is that small (normal ones; 4096 x 4096 of them have such a value in 4 cases of 10): one value of kHalfLeast or more in all
 // tiles of a block, among three others at least that are not zero in its 64 of a row and in its 64 of a column. Zeros are exact and count for nothing.
 // Bound by one read and one write of the operand. 4096^3, both operands: TF32 planes 62 us, these 46, with the sample 53.
-struct HalvesJob {
-  const float* src;
-  __half* hi;
-  __half* lo;
-  int R, C, pitch;          // as in F32Job; pitch in elements, a multiple of eight
-  int transpose;
-  int tiles_x, tiles_y;
-};
+typedef PlaneJob<__half> HalvesJob;   // pitch: a multiple of eight
 struct HalvesJobs {
   HalvesJob job[2];
   long long first[3];
@@ -315,89 +320,42 @@ __device__ __noinline__ bool low_values_fit(const float* s, int R, int C, int r,
   return fit;
 }
 __global__ void __launch_bounds__(256, 5) f32_halves_kernel(const HalvesJobs p) {
-  __shared__ float tile[64][65];
   __shared__ int lows;      // values below kHalfFull
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 vectors of four x 16 rows
   griddep_launch();
   griddep_wait();
   if (threadIdx.x == 0) lows = 0;
   // other blocks may raise the flag at any time: one thread reads it for the block
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<const volatile unsigned int*>(&p.state->flag) != 0u)) return;
-  bool bad = false;
-  auto store4 = [&](const HalvesJob& j, long long o, const float* x, float scale) {   // four neighbours along K of one row
-    __half h[4], l[4];
+  bool bad = false, low = false;
+  float scale = 1.0f;
+  plane_tiles(
+      p.job, p.first,
+      [&](bool second, const float (*x)[4]) {
+        scale = p.state->scale[second ? 1 : 0];
+        low = false;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float y = x[e] * scale;
-      h[e] = __float2half_rn(y);
-      // (a residual of 16, half a step of the largest numbers, would round up to infinity)
-      l[e] = __float2half_rn(fminf(fmaxf((y - __half2float(h[e])) * kLoFactor, -65504.0f), 65504.0f));
-    }
-    *reinterpret_cast<uint2*>(j.hi + o) = *reinterpret_cast<const uint2*>(h);
-    *reinterpret_cast<uint2*>(j.lo + o) = *reinterpret_cast<const uint2*>(l);
-  };
-  for (long long t = blockIdx.x; t < p.first[2]; t += gridDim.x) {
-    const bool second = t >= p.first[1];
-    const HalvesJob j = second ? p.job[1] : p.job[0];
-    const float scale = p.state->scale[second ? 1 : 0];
-    const long long lt = t - (second ? p.first[1] : 0), per_g = (long long)j.tiles_x * j.tiles_y;
-    const long long g = lt / per_g;
-    const int rem = (int)(lt - g * per_g);
-    const int c0 = (rem % j.tiles_x) * 64, r0 = (rem / j.tiles_x) * 64;
-    const float* s = j.src + g * (long long)j.R * j.C;
-    const bool vec = j.C % 4 == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
-    float x[4][4];
+        for (int i = 0; i < 16; ++i) {
+          const float v = x[i >> 2][i & 3], y = fabsf(v * scale);
+          bad = bad || !(y < 65504.0f);
+          low = low || (y < kHalfFull && v != 0.0f);
+        }
+      },
+      [&](const HalvesJob& j, long long o, const float* x) {
+        __half h[4], l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {   // all four reads in flight
-      const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
-      const float* q = s + (long long)r * j.C + c;
-      if (vec && r < j.R && c < j.C) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(q));
-        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[i][e] = (r < j.R && c + e < j.C) ? __ldg(q + e) : 0.0f;
-      }
-    }
-    bool low = false;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float v = x[i >> 2][i & 3], y = fabsf(v * scale);
-      bad = bad || !(y < 65504.0f);
-      low = low || (y < kHalfFull && v != 0.0f);
-    }
-    if (!j.transpose) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + ty + 16 * i, c = c0 + tx * 4;
-        if (r < j.R && c < j.pitch) store4(j, (g * j.R + r) * (long long)j.pitch + c, x[i], scale);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) tile[ty + 16 * i][tx * 4 + e] = x[i][e];
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int oc = c0 + ty + 16 * i, orr = r0 + tx * 4;   // output row = source column, output column = source row
-        float y[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = tile[tx * 4 + e][ty + 16 * i];
-        if (oc < j.C && orr < j.pitch) store4(j, (g * j.C + oc) * (long long)j.pitch + orr, y, scale);
-      }
-      __syncthreads();
-    }
-    if (low && !bad) bad = !low_values_fit(s, j.R, j.C, r0 + ty, c0 + tx * 4, scale, &lows);
-  }
+        for (int e = 0; e < 4; ++e) {
+          const float y = x[e] * scale;
+          h[e] = __float2half_rn(y);
+          // (a residual of 16, half a step of the largest numbers, would round up to infinity)
+          l[e] = __float2half_rn(fminf(fmaxf((y - __half2float(h[e])) * kLoFactor, -65504.0f), 65504.0f));
+        }
+        *reinterpret_cast<uint2*>(j.hi + o) = *reinterpret_cast<const uint2*>(h);
+        *reinterpret_cast<uint2*>(j.lo + o) = *reinterpret_cast<const uint2*>(l);
+      },
+      [&](const HalvesJob& j, const float* s, int r, int c) {
+        if (low && !bad) bad = !low_values_fit(s, j.R, j.C, r, c, scale, &lows);
+      });
   if (__syncthreads_or(bad ? 1 : 0) && threadIdx.x == 0) p.state->flag = 1u;
-}
-HalvesJob halves_job(const float* src, __half* hi, __half* lo, int R, int C, int pitch, bool transpose) {
-  HalvesJob j;
-  j.src = src; j.hi = hi; j.lo = lo; j.R = R; j.C = C; j.pitch = pitch; j.transpose = transpose ? 1 : 0;
-  j.tiles_x = ((transpose ? C : pitch) + 63) / 64;
-  j.tiles_y = ((transpose ? pitch : R) + 63) / 64;
-  return j;
 }
 
 // Zeros for a C that both K ranges of an f32 product are added to; a kernel and not a memset, which does not start before its predecessor has
@@ -806,7 +764,7 @@ RbStatus rb::f32_planes(const float* src, float* hi, float* lo, int groups, int 
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   F32Jobs jobs;
   memset(&jobs, 0, sizeof(jobs));
-  jobs.job[0] = f32_job(src, hi, split ? lo : nullptr, R, C, pitch, transpose);
+  jobs.job[0] = plane_job(src, hi, split ? lo : nullptr, R, C, pitch, transpose);
   return launch_f32_jobs(jobs, 1, groups, dev->sm_count, stream);
 }
 
@@ -1038,7 +996,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     auto add = [&](const void* src, const OperandPlan& o, const size_t* off, const void** planes) {
       float* hi = reinterpret_cast<float*>(wsb + off[0]);
       float* lo = split ? reinterpret_cast<float*>(wsb + off[1]) : nullptr;
-      jobs.job[nj++] = f32_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, o.pitch, o.src_mn_major);
+      jobs.job[nj++] = plane_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, o.pitch, o.src_mn_major);
       planes[0] = hi;
       planes[1] = lo;
     };
@@ -1057,13 +1015,13 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
       auto add_half = [&](int i, const void* src, const OperandPlan& o, const size_t* off, const void** planes) {
         __half* hi = reinterpret_cast<__half*>(wsb + off[0]);
         __half* lo = hi + align_up((size_t)p->g * o.rows * half_pitch, 128);
-        hj.job[i] = halves_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, half_pitch, o.src_mn_major);
+        hj.job[i] = plane_job(static_cast<const float*>(src), hi, lo, o.src_rows, o.src_cols, half_pitch, o.src_mn_major);
         hj.first[i + 1] = hj.first[i] + p->g * (long long)hj.job[i].tiles_x * hj.job[i].tiles_y;
         planes[0] = hi;
         planes[1] = lo;
       };
       if (conv_src) {
-        hj.job[0] = halves_job(conva->src, reinterpret_cast<__half*>(const_cast<void*>(conva->tensor)),
+        hj.job[0] = plane_job(conva->src, reinterpret_cast<__half*>(const_cast<void*>(conva->tensor)),
                                reinterpret_cast<__half*>(const_cast<void*>(conva->tensor_lo)), conva->src_rows, conva->src_cols, conva->C,
                                conva->src_transpose);
         hj.first[1] = conva->src_groups * (long long)hj.job[0].tiles_x * hj.job[0].tiles_y;
@@ -1078,7 +1036,7 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     if (conv_src) {
       F32Jobs image;
       memset(&image, 0, sizeof(image));
-      image.job[0] = f32_job(conva->src, static_cast<float*>(const_cast<void*>(conva->tensor)), static_cast<float*>(const_cast<void*>(conva->tensor_lo)),
+      image.job[0] = plane_job(conva->src, static_cast<float*>(const_cast<void*>(conva->tensor)), static_cast<float*>(const_cast<void*>(conva->tensor_lo)),
                              conva->src_rows, conva->src_cols, conva->C, conva->src_transpose);
       st = launch_f32_jobs(image, 1, conva->src_groups, dev->sm_count, stream, halves ? &state->flag : nullptr);
       if (st != RB_SUCCESS) return st;
