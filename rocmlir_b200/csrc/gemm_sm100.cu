@@ -414,15 +414,19 @@ struct TileCost {
 };
 struct StoreCost {
   double last, tile, column, ragged, margin;   // a column of the exposed store; a tile and a column of the others; rows off 16 bytes; what an estimate must beat
+  double ragged_tile;                          // rows off 16 bytes in the others
 };
 constexpr TileCost kTileCosts[] = {{1, 64, 4.75, 0.239, 24}, {1, 128, 4.35, 0.311, 32}, {2, 128, 5.68, 0.233, 24}, {1, 256, 3.50, 0.446, 48}, {2, 256, 4.91, 0.324, 32}};
-constexpr StoreCost kStoreCost = {0.0087, 0.84, 0.0084, 2.58, 0.97};
+constexpr StoreCost kStoreCost = {0.0087, 0.84, 0.0084, 2.58, 0.97, 2.58};
 // f32 with two TF32 planes: fitted to 131000 tiles and K ranges of 18000 products of 12 to 4096 rows and columns, K of 64 to 8192, alone and in groups
 // of three, 5 % off on average (the pass over the operands, the same for all of them, left out here). Of 959
 // products new to the fit one is more than 5 % slower than by the estimate before (fitted to six products, no K ranges) and 23 more than 2 %, the mean is 0.95:
 // 64 x 246 x 2019 29.8 -> 17.2 us, 128 x 1739 x 620 35.4 -> 21.1, 3 x 64 x 650 x 595 33.3 -> 19.4; 27 x 192 x 64 7.9 -> 8.1.
+// Fitted apart, from 35 products of several waves: rows off 16 bytes cost a tile that is not the last twice an aligned one's store, where the common
+// factor of 11.9, that of the exposed store, chose 256 columns for 704 x 3098 x 128 (17.0 -> 21.6 us) and 64 for 2304 x 2157 x 384 (37.7 -> 48.6); and beyond three
+// waves tiles of 64 columns are 4 to 13 % slower than estimated.
 constexpr TileCost kTileCostsF32[] = {{1, 64, 7.47, 0.518, 48}, {1, 128, 7.37, 0.608, 64}, {2, 128, 8.24, 0.526, 48}, {1, 256, 7.60, 1.069, 96}, {2, 256, 8.65, 0.818, 64}};
-constexpr StoreCost kStoreCostF32 = {0.0031, 0.58, 0.037, 11.9, 0.97};
+constexpr StoreCost kStoreCostF32 = {0.0031, 0.58, 0.037, 11.9, 0.97, 2.0};
 
 // *ctas and *bn come in as the rule gives them and stay unless another tile, or fewer K ranges, is estimated faster by the margin. K is not cut where
 // the rule does not cut it: such a product needs no planes in its workspace and can be handed out as one kernel. An f32 result keeps
@@ -439,7 +443,8 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
   const int es_c = (int)dtype_bytes(p->c_type);
   // an 8-bit result is requantised, 4-byte ones (and planes) are two staged rows for one; rows off 16 bytes are copied out by the warps
   const double words = f32 ? 1.0 : 1.45;
-  const double width = (p->c_type == RB_I8 ? 2.76 : es_c == 4 ? words : 1.0) * ((long long)p->n * es_c % 16 ? sc.ragged : 1.0);
+  const bool off16 = (long long)p->n * es_c % 16 != 0;
+  const double width = (p->c_type == RB_I8 ? 2.76 : es_c == 4 ? words : 1.0) * (off16 ? sc.ragged : 1.0);
   // *s comes in as the ranges wanted, 0 for the rule's
   auto estimate = [&](const TileCost& t, long long* s, long long* waves) {
     const long long tiles = (long long)p->g * ((p->m + kBM * t.ctas - 1) / (kBM * t.ctas)) * ((p->n + t.bn - 1) / t.bn);
@@ -452,7 +457,8 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
     const double block = std::max(t.block, busy * t.kb_per_block / 12500.0);
     // (a byte per element in 64 columns: half of a staged row, copied out by the warps)
     const double columns = (f32 ? std::min(t.bn, (int)p->n) : t.bn) * (*s > 1 ? words : t.bn == 64 && es_c == 1 ? 1.52 * width : width);
-    double us = t.fixed + std::max(kb * block, sc.tile + sc.column * columns) * (double)(*waves - 1) + kb * block + sc.last * columns;
+    const double others = off16 && *s == 1 ? columns / sc.ragged * sc.ragged_tile : columns;
+    double us = t.fixed + std::max(kb * block, sc.tile + sc.column * others) * (double)(*waves - 1) + kb * block + sc.last * columns;
     const double plane_mb = (double)p->g * p->m * p->n * 4 / 1e6;
     if (f32 && *s > 1) us += *s == 2 && p->n % 4 == 0 ? 0.88 + plane_mb * 0.368 : 1.51 + (double)*s * plane_mb * 0.298;   // (two: see add_ranges)
     if (!f32 && *s > 1) us += 2.13 + (double)*s * plane_mb * 0.265;
@@ -478,6 +484,7 @@ void estimate_tile(const RbGemmProblem* p, bool b_mn, int che, long long kblocks
       s = f32 || want == 1 ? want : 0;
       double us = estimate(t, &s, &waves);
       if (s > 1 && !f32) us *= 1.08;   // (K ranges other than the rule's are the less certain ones)
+      if (f32 && t.bn == 64 && waves > 3) continue;   // (see kStoreCostF32)
       if (us < best && (kblocks + s - 1) / s <= chain) { best = us; *ctas = t.ctas; *bn = t.bn; *splits = (int)s; }
     }
   }
@@ -1217,13 +1224,14 @@ RbStatus rb::gemm_run(const RbGemmProblem* p, const RbEpilogue* epi, const void*
     // pointwise, stride 2, 8.4 / 9.0. Not where
     // * the call has other launches, small blocks that wait beside the CTAs at work (300 x 700 x 4096, K in ranges, 15.5 / 15.2, 64 x 246 x 2019 f32
     //   19.6 / 18.6, 543 x 768 x 365 x 3, rows copied, 12.9 / 11.8, 3 x 1024 x 1024 x 769 14.7 / 14.3) - but the launch of the form that is not taken;
-    // * few rows draw a large B, which is what bounds them (45 x 6080 x 3392 fp8 12.4 / 11.9, 256 x 4096 x 4096 i8 13.9 / 13.4, 66 x 4336 x 1920 fp8 still
-    //   8.9 / 9.3);
+    // * few rows draw a large B, which is what bounds them, on more than half of the SMs, so that a successor's CTAs have to wait for one (45 x 6080 x 3392
+    //   fp8 12.4 / 11.9, 256 x 4096 x 4096 i8 13.9 / 13.4, 164 x 2848 x 2688 fp8 10.9 / 10.4; 66 x 4336 x 1920 fp8, 68 CTAs, 8.9 / 9.3);
     // * single CTAs work on several short tiles each, the next tile's loads under way behind a tile's stores (171 images 64 -> 256, 44x44, input gradient,
     //   47.1 / 45.7, 148 images 64 -> 128, 45x45, input gradient, 32.6 / 31.9, 21 images 512 -> 64, 39x39 10.7 / 10.2; ten K blocks gain, 755 x 6416 x 1280 i8
     //   17.2 / 17.5, and so do pairs, 10 images 256 -> 512, 55x55, 19.4 / 20.0).
-    const bool streams_b = p->m <= 3 * kBM && (double)p->n * p->k * es >= 12e6;
-    const bool several = ctas == 1 && kp.kblocks <= 8 && (long long)p->g * kp.tiles_m * kp.tiles_n > dev->sm_count;
+    const long long own = (long long)p->g * kp.tiles_m * kp.tiles_n * ctas;   // CTAs, were there one for every tile
+    const bool streams_b = p->m <= 3 * kBM && (double)p->n * p->k * es >= 7e6 && 2 * own > dev->sm_count;
+    const bool several = ctas == 1 && kp.kblocks <= 8 && own > dev->sm_count;
     kp.early = halves || !(splits > 1 || oa.needs_copy || ob.needs_copy || streams_b || several) ? 1 : 0;
     if (halves) {
       kp.gate = &state->flag;
