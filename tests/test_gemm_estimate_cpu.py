@@ -4,6 +4,8 @@ import ctypes as C
 import math
 import random
 
+import pytest
+
 from rocmlir_b200 import _lib as L
 
 RULE = 1 << 27
@@ -69,10 +71,5 @@ def test_dimensions_of_a_handle_are_those_of_the_one_kernel():
     (3405, 1344, 192, 1, 0, (256, 128)), (3246, 1541, 263, 0, 0, (256, 128)), (2368, 1920, 640, 0, 1, (128, 128))])
 def test_f32_products_of_several_waves(m, n, k, trans_a, trans_b, tile):
     """The tile that was the fastest of those measured, rows of C on and off 16 bytes (others took 1.1 to 1.4 times as long)."""
-    import ctypes
-
-    from rocmlir_b200 import _lib as L
-    p = L.RbGemmProblem(1, m, n, k, trans_a, trans_b, 0, L.F32, L.F32, 0, 0)
-    info = L.RbGemmConfigInfo()
-    assert L.lib().rbGemmGetConfig(ctypes.byref(p), ctypes.byref(info)) == 0
+    info, _ = query(L.RbGemmProblem(1, m, n, k, trans_a, trans_b, 0, L.F32, L.F32, 0, 0), 0)
     assert (info.tile_m, info.tile_n, info.splits) == (*tile, 1)
