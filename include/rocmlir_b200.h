@@ -373,7 +373,7 @@ RB_EXPORT int rbGetGemmVariant(void);
  * without one). `variant` is the explicit variant word that
  * reproduces the configuration. */
 typedef struct RbGemmConfigInfo {
-  int32_t tile_m, tile_n, tile_k; /* output tile of one CTA group; K elements per pipeline stage */
+  int32_t tile_m, tile_n, tile_k; /* output tile of one CTA group; K elements per pipeline stage (f32: of the TF32 form) */
   int32_t ctas;                   /* CTAs per cluster (1, or 2 = cta_group::2 pair) */
   int32_t stages;                 /* depth of the shared-memory ring */
   int32_t splits;                 /* K ranges (1 = no split) */
